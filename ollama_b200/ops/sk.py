@@ -53,6 +53,20 @@ class Quant256Args(C.Structure):
                 ("xd", C.c_void_p), ("xbs", C.c_void_p), ("perm", C.c_int)]
 
 
+class SgSeg(C.Structure):
+    _fields_ = [("w", C.c_void_p), ("bias", C.c_void_p), ("type", C.c_int), ("n", C.c_int), ("out_off", C.c_int), ("tile0", C.c_int)]
+
+
+class SgArgs(C.Structure):
+    _fields_ = [("seg", SgSeg * 4), ("nseg", C.c_int), ("k", C.c_int), ("nb", C.c_int), ("x", C.c_void_p), ("mode", C.c_int), ("out", C.c_void_p), ("ldo", C.c_int),
+                ("act", C.c_int), ("alpha", C.c_float), ("limit", C.c_float), ("ws", C.c_void_p), ("flags", C.c_void_p), ("status", C.c_void_p), ("tiles", C.c_int),
+                ("ring", C.c_int), ("slot_bytes", C.c_int), ("x_slots", C.c_int)]
+
+
+class Rows16Args(C.Structure):
+    _fields_ = [("x", C.c_void_p), ("ldx", C.c_int), ("bf16", C.c_int), ("norm_w", C.c_void_p), ("eps", C.c_float), ("k", C.c_int), ("out", C.c_void_p)]
+
+
 MODE_STORE, MODE_ACCUM, MODE_GLU = 0, 1, 2
 
 
@@ -266,6 +280,47 @@ def gemv(weights: list[SkWeight], x: torch.Tensor | tuple[torch.Tensor, torch.Te
     a.mode, a.out, a.ldo = mode, out.data_ptr(), out.stride(0)
     a.act, a.alpha, a.limit = K._ACT[act], alpha, limit
     K._check(K.lib().b2_gemv_sk(C.byref(a), max_ctas, split, ring, int(pdl), K.stream()), "gemv_sk")
+    return out
+
+
+ROWS16_CHUNK = 4384              # bytes of the activation chunk of one 256-block and eight rows (kernels/gemm_sk.cu)
+ROWS16_MAX_NORM = 16384          # longest row that is normalised on the way
+
+
+def rows16_bytes(nb: int, k: int) -> int:
+    return (k // 256) * ((nb + 7) // 8) * ROWS16_CHUNK
+
+
+def rows16(x: torch.Tensor, norm_w: torch.Tensor | None = None, eps: float = 0.0, out: torch.Tensor | None = None, pdl: bool = False) -> torch.Tensor:
+    """fp32 or bf16 rows [nb, k] (optionally RMS-normalised first) as the f16 activation chunks that :func:`gemm16` reads."""
+    nb, k = x.shape
+    if x.dtype not in (torch.float32, torch.bfloat16) or x.stride(1) != 1:
+        raise ValueError("rows16 takes fp32 or bf16 rows")
+    n = rows16_bytes(nb, k)
+    if out is None:
+        out = torch.empty(n, device=x.device, dtype=torch.uint8)
+    elif out.numel() < n:
+        raise ValueError(f"rows16: {out.numel()} bytes for chunks of {n}")
+    a = Rows16Args(K.ptr(x), x.stride(0), int(x.dtype == torch.bfloat16), K.ptr(norm_w), eps, k, K.ptr(out))
+    K._check(K.lib().b2_rows16(C.byref(a), nb, int(pdl), K.stream()), "rows16")
+    return out
+
+
+def gemm16(weights: list[SkWeight], x: torch.Tensor, nb: int, *, out: torch.Tensor | None = None, mode: int = MODE_STORE, act: str = "silu", alpha: float = 1.702,
+           limit: float = 7.0, max_ctas: int = 0, pdl: bool = False) -> torch.Tensor:
+    """y[b] = concat_i(W_i x[b] + bias_i) of 1..32 rows in the chunks of :func:`rows16`; modes and results as in :func:`gemv`, activations in 16 bits."""
+    dev, total = weights[0].units.device, sum(w.n for w in weights)
+    if out is None:
+        out = torch.empty(nb, total // 2 if mode == MODE_GLU else total, device=dev, dtype=torch.float32)
+    a, ws, off = SgArgs(), workspace(dev), 0
+    for i, w in enumerate(weights):
+        s = a.seg[i]
+        s.w, s.bias, s.type, s.n, s.out_off = w.units.data_ptr(), K.ptr(w.bias), w.wtype, w.n, off
+        off += w.n
+    a.nseg, a.k, a.nb, a.x = len(weights), weights[0].k, nb, K.ptr(x)
+    a.mode, a.out, a.ldo, a.act, a.alpha, a.limit = mode, out.data_ptr(), out.stride(0), K._ACT[act], alpha, limit
+    a.ws, a.flags, a.status = ws.ws.data_ptr(), ws.flags.data_ptr(), ws.status.data_ptr()
+    K._check(K.lib().b2_gemm_sk(C.byref(a), max_ctas, int(pdl), K.stream()), "gemm_sk")
     return out
 
 

@@ -186,3 +186,46 @@ def test_engine_decodes_up_to_32_sequences_in_one_step(tmp_path):
         assert eng.decode_argmax(list(range(nb)), toks[:nb], pos[:nb]) == got.argmax(-1).tolist()
     from ollama_b200.ops import sk
     sk.workspace("cuda").check()
+
+
+@pytest.mark.parametrize("segs,k", [([(16, GGMLType.Q4_K)], 256), ([(272, GGMLType.Q6_K), (16, GGMLType.Q4_K), (32, GGMLType.Q6_K)], 512), ([(4096, GGMLType.Q4_K)], 2816)])
+@pytest.mark.parametrize("nb", [1, 8, 9, 24, 32])
+def test_gemm16_matches_reference(segs, k, nb):
+    """Rows in 16-bit activations (kernels/gemm_sk.cu): groups of one tile, groups that matrices of both encodings share, groups split between CTAs; stored, added, normalised, in
+    bf16 rows.  Bound: activations keep 2^-12 of a 256-block's largest value (about 3.5 of their deviations), Q6_K codes times scales 2^-12, so 2^-9 of a result's deviation at worst."""
+    _, sk = _mods()
+    gen = torch.Generator().manual_seed(nb + k)
+    ws = [sk.repack(QWeight.from_float("w", torch.randn(n, k, generator=gen) * 0.05, t), "cuda", bias=torch.randn(n, generator=gen)) for n, t in segs]
+    W = torch.cat([sk.unit_weights(w) for w in ws]).double()
+    bias = torch.cat([w.bias for w in ws]).double()
+    W, bias = W.cuda(), bias.cuda()
+    x, nw = torch.randn(nb, k, generator=gen).cuda() * 3, torch.rand(k, generator=gen).cuda() + 0.5
+    x[0] *= 1e4                                        # rows have scales of their own
+    x[-1, :256] = 0
+
+    def check(got, rows):
+        ref = rows.double() @ W.t()
+        tol = 2 ** -9 * ref.std(1, keepdim=True) + 1e-6
+        assert ((got.double() - ref - bias).abs() <= tol + 1e-6 * ref.abs()).all(), ((got.double() - ref - bias).abs() / tol).max()
+
+    check(sk.gemm16(ws, sk.rows16(x), nb), x)
+    out = torch.randn(nb, W.shape[0], generator=gen).cuda()
+    was = out.clone()
+    sk.gemm16(ws, sk.rows16(x), nb, out=out, mode=sk.MODE_ACCUM)
+    assert torch.allclose(out - was, sk.gemm16(ws, sk.rows16(x), nb), rtol=1e-4, atol=1e-4 * float(out.abs().max()))
+    normed = (x.double() * torch.rsqrt((x.double() ** 2).mean(1, keepdim=True) + 1e-5) * nw.double())
+    check(sk.gemm16(ws, sk.rows16(x, nw, 1e-5), nb), normed)
+    b16 = x.to(torch.bfloat16)
+    check(sk.gemm16(ws, sk.rows16(b16), nb), b16)
+    sk.workspace("cuda").check()
+
+
+def test_gemm16_glu_matches_reference():
+    _, sk = _mods()
+    gen = torch.Generator().manual_seed(3)
+    w = sk.repack(QWeight.from_float("w", torch.randn(1376, 512, generator=gen) * 0.05, GGMLType.Q4_K), "cuda")
+    x = torch.randn(19, 512, generator=gen).cuda()
+    y = x.double() @ sk.unit_weights(w).double().t()
+    ref = torch.nn.functional.silu(y[:, 0::2]) * y[:, 1::2]
+    got = sk.gemm16([w], sk.rows16(x), 19, mode=sk.MODE_GLU)
+    assert (got.double() - ref).norm() < 2 ** -9 * ref.norm()
