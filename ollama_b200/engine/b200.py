@@ -632,7 +632,7 @@ class B200Backend(StepEngine):
         if c.head_dim in K.ATTN_PREFILL_HEAD_DIMS and not spans:
             self.kernel_launches += 1
             return K.attn_prefill(q, self.k_cache[i], self.v_cache[i], slot, pos0, p_end, self.attn_scale, c.causal, window,
-                                  c.attn_softcap, L.sinks, k_scale=self.k_scale[i], v_scale=self.v_scale[i])
+                                  c.attn_softcap, L.sinks, k_scale=self.k_scale[i], v_scale=self.v_scale[i], pdl=self.pdl)
         # head sizes without a flash-attention instantiation (32, 256): plain torch attention over the same cache rows
         kk = self.k_cache[i][slot, :, :p_end].transpose(0, 1).float()        # [S, Hkv, hd]
         vv = self.v_cache[i][slot, :, :p_end].transpose(0, 1).float()
@@ -669,7 +669,7 @@ class B200Backend(StepEngine):
             if embeds is not None and len(embeds[0]):      # image rows: projected features, not scaled like token embeddings
                 x[torch.as_tensor(list(embeds[0]), device=dev)] = embeds[1].to(dev, x.dtype)
         for i, L in enumerate(self.layers):
-            h = K.rmsnorm_bf16(x, L.attn_norm, c.norm_eps)
+            h = K.rmsnorm_bf16(x, L.attn_norm, c.norm_eps, pdl=self.pdl)
             qkv = torch.empty(T, (c.n_heads + 2 * c.n_kv_heads) * c.head_dim, device=dev, dtype=torch.float32)
             if getattr(L, "wqkv16", None) is not None:      # resident 16-bit copies: one GEMM for Q, K and V
                 K.gemm_bf16(h, L.wqkv16, L.bqkv, out=qkv)
@@ -682,7 +682,7 @@ class B200Backend(StepEngine):
             q = K.rope_kv(qkv, pos, slots, self.inv_freq_local if local else self.inv_freq, n_heads=c.n_heads, n_kv_heads=c.n_kv_heads,
                           hd=c.head_dim, n_rot=c.rope_dim, neox=c.rope_style == "neox", mscale=1.0 if local else self.mscale,
                           k_cache=self.k_cache[i], v_cache=self.v_cache[i], q_norm=L.q_norm, k_norm=L.k_norm, eps=c.norm_eps,
-                          k_scale=self.k_scale[i], v_scale=self.v_scale[i])
+                          k_scale=self.k_scale[i], v_scale=self.v_scale[i], pdl=self.pdl)
             if len(bounds) == 1:
                 o = self._attn_prefill(q, i, L, bounds[0][2], bounds[0][3], bounds[0][3] + T, spans)
             else:
@@ -691,7 +691,7 @@ class B200Backend(StepEngine):
                 x = x + R.rmsnorm(self._mm(o, L.wo), L.post_attn_norm, c.norm_eps)
             else:
                 self._mm(o, L.wo, x, 0, accumulate=True)                  # residual add in the GEMM epilogue
-            h = K.rmsnorm_bf16(x, L.ffn_norm, c.norm_eps)
+            h = K.rmsnorm_bf16(x, L.ffn_norm, c.norm_eps, pdl=self.pdl)
             if L.moe:
                 x = x + self._moe_prefill(h, L)
                 continue

@@ -16,22 +16,7 @@
 #include <mma.h>
 
 #include "common.cuh"
-
-struct AttnPrefillArgs {
-    const float* q;          // [T][H][D] fp32, rotary embedding already applied
-    const __half* k_cache;   // [slots][Hkv][n_ctx][D]
-    const __half* v_cache;
-    __nv_bfloat16* out;      // [T][H * D]
-    const float* sinks;      // [H] or null
-    int T, H, Hkv, n_ctx;
-    int slot, pos0;
-    int kv_len;              // keys visible to the chunk: positions [0, kv_len)
-    int causal;
-    int window;              // 0 = none; key k is visible to query p when p - k < window
-    float scale, softcap;
-    const __half* k_scale;   // q8_0 cache (k_cache / v_cache hold int8): [slots][Hkv][n_ctx][D/32] scales, or null for f16
-    const __half* v_scale;
-};
+#include "pass_args.cuh"
 
 namespace {
 

@@ -20,22 +20,7 @@
 // and head sizes other than 64 / 128.  In the reference stack this is ggml-cuda's fattn family (mma / tile / vec).
 #include "tc_common.cuh"
 #include "rows.cuh"
-
-struct AttnPrefillArgs {      // the same block as in attn_prefill.cu
-    const float* q;          // [T][H][D] fp32, rotary embedding already applied
-    const __half* k_cache;   // [slots][Hkv][n_ctx][D]
-    const __half* v_cache;
-    __nv_bfloat16* out;      // [T][H * D]
-    const float* sinks;      // [H] or null
-    int T, H, Hkv, n_ctx;
-    int slot, pos0;
-    int kv_len;              // keys visible to the chunk: positions [0, kv_len)
-    int causal;
-    int window;              // 0 = none; key k is visible to query p when p - k < window
-    float scale, softcap;
-    const __half* k_scale;   // int8 cache: not taken by this kernel
-    const __half* v_scale;
-};
+#include "pass_args.cuh"
 
 // Paged form of the pipelined kernel: the query tiles of a step (portions of several sequences) come as a list, K / V tiles are
 // read through a page table (two 64-position pages per tile; caches [page][Hkv][64][D], pad columns zero), the mask may be chunked or a window
@@ -536,6 +521,7 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS2) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    pdl_wait();      // launches of flat caches may overlap the end of the kernel before them
     if (warp < SOFTMAX_WARPS) {
         const int r = 32 * (warp & 3) + lane, c = warp >> 2, qi = DIFF ? r & 63 : r;
         const bool live = qi < rows;
@@ -567,6 +553,7 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_launch();      // not before the tensor memory is there: CTAs of the next kernel that came first would keep it until this one ends
     const int row0 = FORM == PARTS ? tile.z + k_begin : PAGED ? 0 : (a.slot * a.Hkv + hkv) * a.n_ctx + k_begin;
     const int* table = FORM == PAGED_CACHE ? pg.page_table + (size_t)tile.z * pg.max_pages : nullptr;
 
@@ -871,15 +858,18 @@ int launch(const AttnPrefillArgs& a, int n_slots, cudaStream_t st) {
 }
 
 template <int D>
-int launch2(const AttnPrefillArgs& a, int n_slots, cudaStream_t st) {
+int launch2(const AttnPrefillArgs& a, int n_slots, int pdl, cudaStream_t st) {
     CUtensorMap mk, mv;
     const size_t rows = (size_t)n_slots * a.Hkv * a.n_ctx;
     if (!cached_kv_map(&mk, a.k_cache, rows, D) || !cached_kv_map(&mv, a.v_cache, rows, D)) return (int)cudaErrorNotSupported;
     static PerDeviceOnce once;
     if (once.first()) cudaFuncSetAttribute(attn_prefill_tc2_kernel<D, D, FLAT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay2<D, D>::TOTAL);
     dim3 grid((a.T + BQ - 1) / BQ, a.H);
-    attn_prefill_tc2_kernel<D, D, FLAT><<<grid, THREADS2, Lay2<D, D>::TOTAL, st>>>(mk, mv, a, AttnPagedArgs{}, AttnPartsArgs{});
-    return (int)cudaGetLastError();
+    AttnPrefillArgs copy = a;
+    AttnPagedArgs pg = {};
+    AttnPartsArgs pt = {};
+    void* args[] = {&mk, &mv, &copy, &pg, &pt};
+    return launch_rows((const void*)attn_prefill_tc2_kernel<D, D, FLAT>, grid, dim3(THREADS2), Lay2<D, D>::TOTAL, args, st, pdl);
 }
 
 template <int D, bool DIFF>
@@ -954,15 +944,15 @@ B2_API int b2_attn_prefill_paged(const AttnPrefillArgs* a, const AttnPagedArgs* 
 
 // Prefill attention on tcgen05: f16 caches, head size 64 or 128 (anything else: cudaErrorNotSupported, nothing launched; the
 // caller then runs b2_attn_prefill).  `n_slots`: slots of the cache tensors (the extent of the TMA maps).  Returns a cudaError_t value.
-B2_API int b2_attn_prefill_tc(const AttnPrefillArgs* a, int head_dim, int n_slots, cudaStream_t st) {
+B2_API int b2_attn_prefill_tc(const AttnPrefillArgs* a, int head_dim, int n_slots, int pdl, cudaStream_t st) {
     if (!a || a->T < 1 || a->H < 1 || a->Hkv < 1 || a->H % a->Hkv || a->kv_len < 1 || a->kv_len > a->n_ctx || n_slots < 1 || a->slot < 0 ||
         a->slot >= n_slots)
         return (int)cudaErrorInvalidValue;
     if (a->k_scale || a->v_scale) return (int)cudaErrorNotSupported;
     if (((uintptr_t)a->k_cache & 15) || ((uintptr_t)a->v_cache & 15) || ((uintptr_t)a->q & 15) || ((uintptr_t)a->out & 15)) return (int)cudaErrorNotSupported;
     if ((size_t)n_slots * a->Hkv * a->n_ctx >= ((size_t)1 << 31)) return (int)cudaErrorNotSupported;
-    if (g_variant == 2 && head_dim == 128) return launch2<128>(*a, n_slots, st);
-    if (g_variant == 2 && head_dim == 64) return launch2<64>(*a, n_slots, st);
+    if (g_variant == 2 && head_dim == 128) return launch2<128>(*a, n_slots, pdl, st);
+    if (g_variant == 2 && head_dim == 64) return launch2<64>(*a, n_slots, pdl, st);
     if (head_dim == 128) return g_variant ? launch<128, true>(*a, n_slots, st) : launch<128, false>(*a, n_slots, st);
     if (head_dim == 64) return g_variant ? launch<64, true>(*a, n_slots, st) : launch<64, false>(*a, n_slots, st);
     return (int)cudaErrorNotSupported;

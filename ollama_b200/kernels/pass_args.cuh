@@ -1,6 +1,30 @@
-// Arguments of the products of unit-ordered matrices in 16-bit rows.
+// Arguments of kernels that more than one source file launches.
 #pragma once
 #include "common.cuh"
+
+struct RopeKvArgs {
+    const float* qkv;        // [nt][(H + 2 Hkv) * hd]  (q | k | v)
+    const int* positions;    // [nt]
+    const int* slots;        // [nt]
+    const float* inv_freq;   // [n_rot/2]
+    const float* q_norm;     // [hd] or null
+    const float* k_norm;     // [hd] or null
+    float eps, mscale;
+    int n_heads, n_kv_heads, hd, n_rot, neox, n_ctx;
+    float* q_out;            // [nt][H][hd]
+    __half* k_cache;         // [slots][Hkv][n_ctx][hd]  (int8 when the scale arrays are given)
+    __half* v_cache;
+    __half* k_scale;         // q8_0 cache: [slots][Hkv][n_ctx][hd/32] one f16 scale per 32 dims, or null for an f16 cache
+    __half* v_scale;
+};
+
+struct NormCastArgs {
+    const float* x;
+    const float* w;
+    float eps;
+    int k, do_norm;
+    __nv_bfloat16* out;
+};
 
 // Products of unit-ordered matrices (gemm_sk.cu).
 struct SgSeg {
@@ -34,4 +58,20 @@ struct Rows16Args {
     float eps;
     int k;
     uint8_t* out;         // [k / 256][ceil(nb / 8)][SG_CHUNK] regrouped: per 256-block all values, then all sums, then all scales
+};
+
+struct AttnPrefillArgs {
+    const float* q;          // [T][H][D] fp32, rotary embedding already applied
+    const __half* k_cache;   // [slots][Hkv][n_ctx][D]
+    const __half* v_cache;
+    __nv_bfloat16* out;      // [T][H * D]
+    const float* sinks;      // [H] or null
+    int T, H, Hkv, n_ctx;
+    int slot, pos0;
+    int kv_len;              // keys visible to the chunk: positions [0, kv_len)
+    int causal;
+    int window;              // 0 = none; key k is visible to query p when p - k < window
+    float scale, softcap;
+    const __half* k_scale;   // q8_0 cache (k_cache / v_cache hold int8): [slots][Hkv][n_ctx][D/32] scales, or null for f16
+    const __half* v_scale;
 };

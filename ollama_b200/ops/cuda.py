@@ -572,12 +572,12 @@ def glu_rows(gu: torch.Tensor, act: str, alpha: float = 1.702, limit: float = 7.
     return out
 
 
-def rmsnorm_bf16(x: torch.Tensor, w: torch.Tensor | None, eps: float, do_norm: bool = True) -> torch.Tensor:
+def rmsnorm_bf16(x: torch.Tensor, w: torch.Tensor | None, eps: float, do_norm: bool = True, pdl: bool = False) -> torch.Tensor:
     """Row-wise RMSNorm of fp32 [rows, k] with a bf16 result (the A operand of the prefill GEMMs)."""
     rows, k = x.shape
     out = torch.empty(rows, k, device=x.device, dtype=torch.bfloat16)
     a = NormCastArgs(ptr(x), ptr(w), eps, k, int(do_norm), ptr(out))
-    _check(lib().b2_rmsnorm_bf16(C.byref(a), rows, stream()), "rmsnorm_bf16")
+    _check(lib().b2_rmsnorm_bf16(C.byref(a), rows, int(pdl), stream()), "rmsnorm_bf16")
     return out
 
 
@@ -594,7 +594,7 @@ ATTN_PREFILL_DEFAULT = "auto"       # the kernel prefill attention runs on unles
 
 def attn_prefill(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, slot: int, pos0: int, kv_len: int, scale: float,
                  causal: bool = True, window: int = 0, softcap: float = 0.0, sinks: torch.Tensor | None = None,
-                 k_scale: torch.Tensor | None = None, v_scale: torch.Tensor | None = None, mode: str | None = None) -> torch.Tensor:
+                 k_scale: torch.Tensor | None = None, v_scale: torch.Tensor | None = None, mode: str | None = None, pdl: bool = False) -> torch.Tensor:
     """Flash attention of a prefill chunk: q [T, H, D] fp32 -> bf16 [T, H * D].  ``mode``: "tc" = the tcgen05 kernel
     (kernels/attn_prefill_tc.cu: f16 caches, head size 64 / 128), "mma" = the mma.sync kernel (kernels/attn_prefill.cu), "auto" =
     tcgen05 where it applies.  Default: B200_ATTN_PREFILL, else ATTN_PREFILL_DEFAULT."""
@@ -605,7 +605,7 @@ def attn_prefill(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
                         int(causal), window, scale, softcap, ptr(k_scale), ptr(v_scale))
     mode = mode or os.environ.get("B200_ATTN_PREFILL", ATTN_PREFILL_DEFAULT)
     if mode in ("auto", "tc") and D in (64, 128) and k_scale is None and q.dtype == torch.float32:
-        rc = lib().b2_attn_prefill_tc(C.byref(a), D, n_slots, stream())
+        rc = lib().b2_attn_prefill_tc(C.byref(a), D, n_slots, int(pdl), stream())
         if rc == 0:
             return out
         if rc != 801 or mode == "tc":              # 801 = cudaErrorNotSupported: nothing was launched

@@ -152,6 +152,18 @@ def test_rope_kv(neox, qk_norm, hd, n_rot):
         assert torch.allclose(vc[slots[t], :, pos[t]].float().cpu(), vr[t], atol=5e-3, rtol=2e-3)
 
 
+@pytest.mark.parametrize("k", [4, 30, 1028, 8192, 8196])
+def test_rmsnorm_bf16(k):
+    """Rows kept in registers (multiples of four up to 8192), other lengths and rows that start off 16 bytes in two passes; one rounding to bf16 after about k 2^-24 in fp32."""
+    K = _K()
+    gen = torch.Generator().manual_seed(k)
+    flat, w = torch.randn(5 * k + 1, generator=gen).cuda(), (torch.rand(k, generator=gen) + 0.5).cuda()
+    for x in (flat[:5 * k].view(5, k), flat[1:].view(5, k)):
+        ref = R.rmsnorm(x.double(), w.double(), 1e-5)
+        assert ((K.rmsnorm_bf16(x, w, 1e-5).double() - ref).abs() <= 2 ** -8 * ref.abs()).all()
+        assert torch.equal(K.rmsnorm_bf16(x, None, 1e-5, do_norm=False), x.to(torch.bfloat16))
+
+
 @pytest.mark.parametrize("neox,qk_norm,hd,n_rot,H,Hkv,q8", [(False, False, 128, 128, 12, 2, False), (True, True, 64, 64, 9, 3, False),
                                                           (True, False, 64, 32, 4, 2, True), (True, True, 256, 256, 3, 1, False)])
 def test_rope_kv_of_a_prefill_chunk(neox, qk_norm, hd, n_rot, H, Hkv, q8):
