@@ -349,7 +349,7 @@ class B200Backend(StepEngine):
         a16 = xf.view(-1)[:nb * k].view(nb, k).to(torch.bfloat16)      # activation rows are packed at the matrix's row length
         off = 0
         for w, b16 in zip(ws, b16s):
-            K.gemm_bf16(a16, b16, w.bias if bias is None else bias, out=out[:nb, off:off + b16.shape[0]], accumulate=accumulate)
+            K.gemm_bf16(a16, b16, w.bias if bias is None else bias, out=out[:nb, off:off + b16.shape[0]], accumulate=accumulate, pdl=2 * self.pdl)
             off += b16.shape[0]
         self._n += 1 + len(ws)
 
@@ -596,16 +596,16 @@ class B200Backend(StepEngine):
             self.kernel_launches += 1
             y = K.gemm_q(x_bf16, w, out=out, accumulate=accumulate, out_off=out_off)
             return y.to(torch.bfloat16) if out16 else y
-        wb = getattr(w, "bf16", None)
+        wb, pdl = getattr(w, "bf16", None), 2 * self.pdl
         if wb is None:
-            wb = K.dequant_to_bf16(w)        # scratch: freed (back to the caching allocator) when this call returns
+            wb, pdl = K.dequant_to_bf16(w), 0        # scratch: freed (back to the caching allocator) when this call returns
             self.kernel_launches += 1
         self.kernel_launches += 1
         if out16:
-            return K.gemm_bf16_out16(x_bf16, wb, w.bias)
+            return K.gemm_bf16_out16(x_bf16, wb, w.bias, pdl=pdl)
         if out is not None:
-            return K.gemm_bf16(x_bf16, wb, w.bias, out=out[:, out_off:out_off + w.n], accumulate=accumulate)
-        return K.gemm_bf16(x_bf16, wb, w.bias)
+            return K.gemm_bf16(x_bf16, wb, w.bias, out=out[:, out_off:out_off + w.n], accumulate=accumulate, pdl=pdl)
+        return K.gemm_bf16(x_bf16, wb, w.bias, pdl=pdl)
 
     def _mm_glu(self, x_bf16: torch.Tensor, w: K.DevWeight) -> torch.Tensor:
         """act(gate) * up of the interleaved gate/up matrix for a prefill chunk, bf16 [T, d_ff]."""
@@ -614,12 +614,12 @@ class B200Backend(StepEngine):
             self.kernel_launches += 2
             gu = K.gemm_q(x_bf16, w).to(torch.bfloat16)                  # columns interleaved: even = gate, odd = up
             return K.glu_rows(gu, c.act, c.swiglu_alpha, c.swiglu_limit)
-        wb = getattr(w, "bf16", None)
+        wb, pdl = getattr(w, "bf16", None), 2 * self.pdl
         if wb is None:
-            wb = K.dequant_to_bf16(w)
+            wb, pdl = K.dequant_to_bf16(w), 0
             self.kernel_launches += 1
         self.kernel_launches += 1
-        return K.gemm_bf16_glu(x_bf16, wb, c.act, w.bias, c.swiglu_alpha, c.swiglu_limit)
+        return K.gemm_bf16_glu(x_bf16, wb, c.act, w.bias, c.swiglu_alpha, c.swiglu_limit, pdl=pdl)
 
     def _attn_prefill(self, q: torch.Tensor, i: int, L, slot: int, pos0: int, p_end: int, spans=()) -> torch.Tensor:
         """Attention of a prefill chunk over cache positions [0, p_end): q [T, H, hd] fp32 -> bf16 [T, H * hd].  ``spans``
@@ -672,7 +672,7 @@ class B200Backend(StepEngine):
             h = K.rmsnorm_bf16(x, L.attn_norm, c.norm_eps, pdl=self.pdl)
             qkv = torch.empty(T, (c.n_heads + 2 * c.n_kv_heads) * c.head_dim, device=dev, dtype=torch.float32)
             if getattr(L, "wqkv16", None) is not None:      # resident 16-bit copies: one GEMM for Q, K and V
-                K.gemm_bf16(h, L.wqkv16, L.bqkv, out=qkv)
+                K.gemm_bf16(h, L.wqkv16, L.bqkv, out=qkv, pdl=2 * self.pdl)
                 self.kernel_launches += 1
             else:
                 self._mm(h, L.wq, qkv, 0)

@@ -2,7 +2,7 @@
 //
 // Blackwell path: operand tiles are fetched by TMA (cp.async.bulk.tensor, 128-byte swizzle) into a
 // multi-stage shared-memory ring, one elected thread issues tcgen05.mma (cta_group::1, M = 128, N up to
-// 256, K = 16 per instruction) with the accumulator in tensor memory, and four epilogue warps read the
+// 256, K = 16 per instruction; larger products cta_group::2, M = 256 on two SMs) with the accumulator in tensor memory, and four epilogue warps read the
 // accumulator back with tcgen05.ld, add the bias and store / accumulate into the output.  Roles are
 // warp-specialised: warp 0 = TMA producer, warp 1 = MMA issuer (+ TMEM allocation), warps 2..5 = epilogue.
 //
@@ -63,13 +63,17 @@ struct GemmParams {
     long long part_stride;
     int part_ld;
     float act_p, act_q;     // numbers of the activation
+    int pdl;                // 1: may start while the kernel before it ends (programmatic dependent launch), 2: and b does not depend on that kernel
 };
 
-template <int BN>
+// PAIR: two CTAs of a cluster share a tile of 256 rows (cta_group::2).  Each holds its 128 rows of a and half of b's rows, so a k block brings 32 KB to an SM for the
+// products of 48.
+template <int BN, bool PAIR>
 struct Cfg {
-    static constexpr int STAGES = BN == 256 ? 4 : (BN == 192 ? 5 : 6);
+    static constexpr int STAGES = PAIR ? (BN == 256 ? 6 : 7) : BN == 256 ? 4 : (BN == 192 ? 5 : 6);
+    static constexpr int B_ROWS = PAIR ? BN / 2 : BN;
     static constexpr int A_BYTES = BM * BK * 2;
-    static constexpr int B_BYTES = BN * BK * 2;
+    static constexpr int B_BYTES = B_ROWS * BK * 2;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
     static constexpr int EPI_LD = 36;                                   // padded row of the epilogue's 32 x 32 transpose tile (floats)
     static constexpr int EPI_BYTES = 4 * 32 * EPI_LD * 4;              // one tile per epilogue warp
@@ -77,6 +81,40 @@ struct Cfg {
     static constexpr int ACC_STRIDE = BN == 192 ? 256 : BN;            // column distance of the two accumulators
     static constexpr int TMEM_COLS = 2 * ACC_STRIDE < 32 ? 32 : 2 * ACC_STRIDE;      // a power of two
 };
+
+// ---- cta_group::2 -----------------------------------------------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// Address of the first CTA's copy of a shared-memory object.
+__device__ __forceinline__ uint32_t leader_addr(const void* p) {
+    uint32_t d;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(d) : "r"(smem_u32(p)));
+    return d;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// A tile into this CTA's shared memory whose bytes count at a barrier of the pair's first CTA.
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4}], [%2];"
+                 ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+// Arrives on the barrier at this offset in both CTAs.
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void arrive_leader(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(leader_addr(bar)) : "memory");
+}
 
 __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int& mt, int& nt) {
     const int per_group = GROUP_M * tiles_n;
@@ -142,11 +180,14 @@ __device__ __forceinline__ void store4(const GemmParams& p, float4 r, int row, i
 }
 
 // TAIL: some columns are p.tail's.  A form of its own, since a test per stored element made all products 8 % longer.
-template <int BN, bool SPLIT, bool TAIL, bool XIELU>
+// PAIR: a launch of CTA pairs.  One CTA per tile is bound by what the L2 delivers to an SM, 47 to 55 bytes a cycle whatever the tile (880 cycles for the 48 KB of a 128 x 256 x 64 block
+// whose products take 512); the pair asks for 32 KB.
+template <int BN, bool SPLIT, bool TAIL, bool XIELU, bool PAIR>
 __global__ void __launch_bounds__(192, 1) gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                                                               const __grid_constant__ GemmParams p) {
     extern __shared__ uint8_t smem_raw[];
-    using L = Cfg<BN>;
+    using L = Cfg<BN, PAIR>;
+    constexpr int TM = PAIR ? 2 * BM : BM;
     constexpr int STAGES = L::STAGES;
     uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);     // 128-byte swizzle wants 1024-byte alignment
     float* epi = reinterpret_cast<float*>(tiles + STAGES * L::STAGE_BYTES);
@@ -158,7 +199,8 @@ __global__ void __launch_bounds__(192, 1) gemm_bf16_tc_kernel(const __grid_const
     __shared__ int s_failed;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tiles_m = (p.m + BM - 1) / BM, tiles_n = (p.n + BN - 1) / BN, n_tiles = tiles_m * tiles_n;
+    const int rank = PAIR ? (int)cluster_rank() : 0, first = PAIR ? blockIdx.x >> 1 : blockIdx.x, step = PAIR ? gridDim.x >> 1 : gridDim.x;
+    const int tiles_m = (p.m + TM - 1) / TM, tiles_n = (p.n + BN - 1) / BN, n_tiles = tiles_m * tiles_n;
     const int splits = SPLIT ? p.splits : 1, total = n_tiles * splits;
     const int k_all = (p.k + BK - 1) / BK;
     auto k_first = [&](int t) { return (int)((long long)k_all * (t / n_tiles) / splits); };      // k blocks of work item t: [k_first(t), k_first(t + n_tiles))
@@ -171,24 +213,43 @@ __global__ void __launch_bounds__(192, 1) gemm_bf16_tc_kernel(const __grid_const
         }
         for (int b = 0; b < 2; b++) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 4);       // one arrival per epilogue warp
+            mbar_init(&acc_empty[b], PAIR ? 8 : 4);       // one arrival per epilogue warp
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {     // one warp allocates the accumulator columns (power of two >= 32)
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(L::TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(L::TMEM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(L::TMEM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     tc_fence_before();
     __syncthreads();
+    if (PAIR) cluster_sync();            // both CTAs' barriers exist before either's copies or products arrive on them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_launch();      // not before the tensor memory is there: CTAs of the next kernel that came first would keep it until this one ends
 
     if (warp == 0) {
         if (lane == 0) {
-            int it = 0;
+            int it = 0, early = 0;
             bool ok = true;
-            for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+            auto load_b = [&](int s, int kb, int row) {      // and what the stage's barrier waits for: both CTAs' tiles
+                if (!PAIR || rank == 0) mbar_expect_tx(&full[s], (PAIR ? 2 : 1) * L::STAGE_BYTES);
+                uint8_t* dst = tiles + s * L::STAGE_BYTES + L::A_BYTES;
+                if (PAIR) tma_load_2d_pair(dst, &map_b, kb * BK, row + rank * L::B_ROWS, leader_addr(&full[s]));
+                else tma_load_2d(dst, &map_b, kb * BK, row, &full[s]);
+            };
+            if (p.pdl == 2 && !SPLIT && first < total) {                   // the matrix's blocks of the first stages are under way before the kernel ahead has ended
+                int mt, nt;
+                tile_coords(first, tiles_m, tiles_n, mt, nt);
+                for (; early < STAGES && early < k_all; early++) load_b(early, early, nt * BN);
+            }
+            pdl_wait();
+            for (int t = first; t < total && ok; t += step) {
                 int mt, nt;
                 tile_coords(SPLIT ? t % n_tiles : t, tiles_m, tiles_n, mt, nt);
                 const int e = p.tile_expert ? p.tile_expert[mt] : 0;
@@ -198,19 +259,19 @@ __global__ void __launch_bounds__(192, 1) gemm_bf16_tc_kernel(const __grid_const
                     const int s = it % STAGES;
                     if (it >= STAGES && !mbar_wait(&empty[s], ((it / STAGES) - 1) & 1)) { ok = false; break; }
                     uint8_t* a_dst = tiles + s * L::STAGE_BYTES;
-                    mbar_expect_tx(&full[s], L::STAGE_BYTES);
-                    tma_load_2d(a_dst, &map_a, kb * BK, mt * BM, &full[s]);
-                    tma_load_2d(a_dst + L::A_BYTES, &map_b, kb * BK, e * p.n + nt * BN, &full[s]);
+                    if (it >= early) load_b(s, kb, e * p.n + nt * BN);
+                    if (PAIR) tma_load_2d_pair(a_dst, &map_a, kb * BK, mt * TM + rank * BM, leader_addr(&full[s]));
+                    else tma_load_2d(a_dst, &map_a, kb * BK, mt * BM, &full[s]);
                 }
             }
             if (!ok) atomicExch(&s_failed, 1);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc(BM, BN);
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc = umma_idesc(TM, BN);
             int it = 0, i = 0;
             bool ok = true;
-            for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+            for (int t = first; t < total && ok; t += step) {
                 if (p.tile_expert) {
                     int mt, nt;
                     tile_coords(SPLIT ? t % n_tiles : t, tiles_m, tiles_n, mt, nt);
@@ -231,11 +292,14 @@ __global__ void __launch_bounds__(192, 1) gemm_bf16_tc_kernel(const __grid_const
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; k++) {
                         // advancing 16 elements along K inside the swizzle span = 32 bytes = 2 descriptor units
-                        umma_bf16(acc, adesc + 2 * k, bdesc + 2 * k, idesc, kb != kb0 || k != 0);
+                        if (PAIR) umma_bf16_pair(acc, adesc + 2 * k, bdesc + 2 * k, idesc, kb != kb0 || k != 0);
+                        else umma_bf16(acc, adesc + 2 * k, bdesc + 2 * k, idesc, kb != kb0 || k != 0);
                     }
-                    umma_commit(&empty[s]);        // frees the stage once these MMAs have read it
+                    if (PAIR) umma_commit_pair(&empty[s]);
+                    else umma_commit(&empty[s]);   // frees the stage once these MMAs have read it
                 }
-                if (ok) umma_commit(&acc_full[buf]);
+                if (ok && PAIR) umma_commit_pair(&acc_full[buf]);
+                else if (ok) umma_commit(&acc_full[buf]);
             }
             if (!ok) atomicExch(&s_failed, 1);
         }
@@ -244,15 +308,16 @@ __global__ void __launch_bounds__(192, 1) gemm_bf16_tc_kernel(const __grid_const
         const int q = warp & 3;
         int i = 0;
         bool ok = true;
-        for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+        pdl_wait();
+        for (int t = first; t < total && ok; t += step) {
             int mt, nt;
             tile_coords(SPLIT ? t % n_tiles : t, tiles_m, tiles_n, mt, nt);
             const int e = p.tile_expert ? p.tile_expert[mt] : 0;
             if (e < 0) continue;
-            const int buf = i & 1, use = i >> 1;
+            const int buf = i & 1, use = i >> 1, row_base = mt * TM + rank * BM;
             i++;
-            if (!SPLIT && p.mul && mt * BM + q * 32 + lane < p.m) {      // the table's rows are anywhere in memory: asked for while the products run
-                const __nv_bfloat16* r = p.mul + (size_t)p.mul_row[mt * BM + q * 32 + lane] * p.ldm;
+            if (!SPLIT && p.mul && row_base + q * 32 + lane < p.m) {      // the table's rows are anywhere in memory: asked for while the products run
+                const __nv_bfloat16* r = p.mul + (size_t)p.mul_row[row_base + q * 32 + lane] * p.ldm;
                 for (int c = nt * BN; c < min(nt * BN + BN, p.n); c += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(r + c));
             }
             if (!mbar_wait(&acc_full[buf], use & 1)) { ok = false; break; }
@@ -271,7 +336,7 @@ __global__ void __launch_bounds__(192, 1) gemm_bf16_tc_kernel(const __grid_const
                 if (!SPLIT && !XIELU && (p.accumulate || p.mul)) {
 #pragma unroll
                     for (int rr = 0; rr < 8; rr++) {
-                        const int row = mt * BM + q * 32 + rr * 4 + sub;
+                        const int row = row_base + q * 32 + rr * 4 + sub;
                         if (row < p.m && col < p.n) with[rr] = fetch4(p, row, col);
                     }
                 }
@@ -286,7 +351,7 @@ __global__ void __launch_bounds__(192, 1) gemm_bf16_tc_kernel(const __grid_const
                 if (TAIL && n0 + c0 + 32 > p.tail_col) {      // warp-uniform
 #pragma unroll 1
                     for (int rr = 0; rr < 8; rr++) {
-                        const int lr = rr * 4 + sub, row = mt * BM + q * 32 + lr;
+                        const int lr = rr * 4 + sub, row = row_base + q * 32 + lr;
                         if (row >= p.m || col >= p.n) continue;
                         float4 r = *(const float4*)(st + lr * L::EPI_LD + cq);
                         r.x += bias.x; r.y += bias.y; r.z += bias.z; r.w += bias.w;
@@ -299,7 +364,7 @@ __global__ void __launch_bounds__(192, 1) gemm_bf16_tc_kernel(const __grid_const
 #pragma unroll
                 for (int rr = 0; rr < 8; rr++) {
                     const int lr = rr * 4 + sub;
-                    const int row = mt * BM + q * 32 + lr;
+                    const int row = row_base + q * 32 + lr;
                     if (row >= p.m || col >= p.n) continue;
                     float4 r = *(const float4*)(st + lr * L::EPI_LD + cq);
                     if (SPLIT) {
@@ -313,15 +378,18 @@ __global__ void __launch_bounds__(192, 1) gemm_bf16_tc_kernel(const __grid_const
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[buf])) : "memory");
+            if (lane == 0 && PAIR) arrive_leader(&acc_empty[buf]);
+            else if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[buf])) : "memory");
         }
         if (!ok) atomicExch(&s_failed, 1);
     }
     tc_fence_before();
     __syncthreads();
+    if (PAIR) cluster_sync();            // neither CTA's memory goes while the other's copies, products or arrivals may still use it
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(L::TMEM_COLS) : "memory");
+        if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(L::TMEM_COLS) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(L::TMEM_COLS) : "memory");
     }
     if (threadIdx.x == 0 && s_failed) atomicExch(&g_gemm_status, KS_TIMEOUT);
     if (p.cm.n_dst > 0) comm_publish(p.cm, gridDim.x, comm_next_epoch(p.cm));
@@ -338,20 +406,62 @@ int sm_count() {
     return n;
 }
 
-template <int BN, bool SPLIT = false, bool TAIL = false, bool XIELU = false>
+template <int BN, bool SPLIT = false, bool TAIL = false, bool XIELU = false, bool PAIR = false>
 int launch(const void* a, const void* b, const GemmParams& p, cudaStream_t st, int b_rows = 0) {
+    using L = Cfg<BN, PAIR>;
+    constexpr int TM = PAIR ? 2 * BM : BM;
     CUtensorMap ma, mb;
-    if (!make_map(&ma, a, p.m, p.k, BM, p.lda) || !make_map(&mb, b, b_rows ? b_rows : p.n, p.k, BN)) return (int)cudaErrorNotSupported;
+    if (!make_map(&ma, a, p.m, p.k, BM, p.lda) || !make_map(&mb, b, b_rows ? b_rows : p.n, p.k, L::B_ROWS)) return (int)cudaErrorNotSupported;
+    const void* fn = (const void*)gemm_bf16_tc_kernel<BN, SPLIT, TAIL, XIELU, PAIR>;
     static PerDeviceOnce once;
-    if (once.first()) cudaFuncSetAttribute(gemm_bf16_tc_kernel<BN, SPLIT, TAIL, XIELU>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::TOTAL);
-    const int total = ((p.m + BM - 1) / BM) * ((p.n + BN - 1) / BN) * (SPLIT ? p.splits : 1);
-    const int grid = total < sm_count() ? total : sm_count();
-    gemm_bf16_tc_kernel<BN, SPLIT, TAIL, XIELU><<<grid, 192, Cfg<BN>::TOTAL, st>>>(ma, mb, p);
-    return (int)cudaGetLastError();
+    if (once.first()) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
+    const int total = ((p.m + TM - 1) / TM) * ((p.n + BN - 1) / BN) * (SPLIT ? p.splits : 1), units = PAIR ? sm_count() / 2 : sm_count();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((total < units ? total : units) * (PAIR ? 2 : 1));
+    cfg.blockDim = dim3(192);
+    cfg.dynamicSmemBytes = L::TOTAL;
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = p.pdl ? 1 : 0;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = 2;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = PAIR ? 2 : 1;
+    GemmParams copy = p;
+    void* args[] = {&ma, &mb, &copy};
+    return (int)cudaLaunchKernelExC(&cfg, fn, args);
+}
+
+// Cycles that a product takes, as measured: rounds of tiles, times the k blocks of 64, times what a block takes by the bytes that an SM gets for it (128 x 128: 613, 128 x 256: 885,
+// pairs of 256 x 128: 632, of 256 x 256: 736); a launch of pairs takes about two microseconds more to begin and end.
+double tile_cycles(const GemmParams& p, int bn, bool pair) {
+    const long tm = pair ? 2 * BM : BM, tiles = ((p.m + tm - 1) / tm) * ((p.n + bn - 1) / bn), units = pair ? sm_count() / 2 : sm_count();
+    const int bytes = 128 * (BM + (pair ? bn / 2 : bn));
+    return (double)((tiles + units - 1) / units) * ((p.k + BK - 1) / BK) * (pair ? 320 + bytes / 79 : 80 + bytes / 61) + (pair ? 4500 : 0);
 }
 
 template <bool TAIL = false, bool XIELU = false>
 int dispatch(const void* a, const void* b, const GemmParams& p, cudaStream_t st, int b_rows = 0) {
+    if (!TAIL && !XIELU && p.m > BM && p.n >= 64 && p.splits <= 1 && !p.tile_expert && p.cm.n_dst == 0 && !b_rows) {
+        // the form and width with the fewest cycles, at equal ones the wider tile
+        double best = 0;
+        int width = 0;
+        bool pair = false;
+        for (int form = 0; form < 2; form++)
+            for (int bn : {256, 192, 128, 64}) {
+                if (p.n < bn || (form && bn < 192)) continue;      // narrower pairs are never the fastest
+                const double c = tile_cycles(p, bn, form);
+                if (!width || c < best) {
+                    best = c;
+                    width = bn;
+                    pair = form;
+                }
+            }
+        if (pair) return width == 256 ? launch<256, false, false, false, true>(a, b, p, st) : launch<192, false, false, false, true>(a, b, p, st);
+        return width == 256 ? launch<256>(a, b, p, st) : width == 192 ? launch<192>(a, b, p, st) : width == 128 ? launch<128>(a, b, p, st) : launch<64>(a, b, p, st);
+    }
     // wide tiles once they fill the machine; narrower ones keep more SMs busy on small problems
     const long tiles_m = (p.m + BM - 1) / BM;
     // a handful of rows (a decode step of several sequences): the product streams b once, so the narrowest tile that spreads
@@ -409,17 +519,19 @@ bool bad_operands(const void* a, const void* b, int m, int n, int k, int ldo) {
 
 // out[m][n] (+)= a[m][k] . b[n][k]^T + bias[n];  a, b bf16 row-major with k % 8 == 0 and 16-byte aligned bases,
 // out fp32 with ldo % 4 == 0, n % 4 == 0.  Returns a cudaError_t value.
-B2_API int b2_gemm_bf16(const void* a, const void* b, int m, int n, int k, float* out, int ldo, const float* bias, int accumulate,
+B2_API int b2_gemm_bf16(const void* a, const void* b, int m, int n, int k, float* out, int ldo, const float* bias, int accumulate, int pdl,
                         cudaStream_t st) {
     if (bad_operands(a, b, m, n, k, ldo) || ((uintptr_t)out & 15)) return (int)cudaErrorInvalidValue;
     GemmParams p{m, n, k, out, ldo, bias, accumulate, 0, {}, 0, nullptr, 0, 0.f, 0.f};
+    p.pdl = pdl;
     return dispatch(a, b, p, st);
 }
 
 // Same product with a bf16 result (n % 8 == 0, ldo % 8 == 0); no accumulation.
-B2_API int b2_gemm_bf16_out16(const void* a, const void* b, int m, int n, int k, void* out, int ldo, const float* bias, cudaStream_t st) {
+B2_API int b2_gemm_bf16_out16(const void* a, const void* b, int m, int n, int k, void* out, int ldo, const float* bias, int pdl, cudaStream_t st) {
     if (bad_operands(a, b, m, n, k, ldo) || (n & 7) || (ldo & 7) || ((uintptr_t)out & 15)) return (int)cudaErrorInvalidValue;
     GemmParams p{m, n, k, out, ldo, bias, 0, 1, {}, 0, nullptr, 0, 0.f, 0.f};
+    p.pdl = pdl;
     return dispatch(a, b, p, st);
 }
 
@@ -441,6 +553,7 @@ B2_API int b2_gemm_rows(const GemmRowsArgs* g, cudaStream_t st) {
                  (const __nv_bfloat16*)g->mul, g->mul_row, g->ldm, (__nv_bfloat16*)g->copy, g->lda, g->tail, g->tail_col, g->ld_tail};
     p.act_p = g->act_p;
     p.act_q = g->act_q;
+    p.pdl = g->tile_expert ? 0 : g->pdl;
     const bool xielu = p.act == ACT_XIELU;
     if (xielu && (g->tile_expert || g->tail || g->mul || g->accumulate || g->copy || g->out_type > 1 || g->alpha != 1.f)) return (int)cudaErrorNotSupported;
     if (g->tile_expert) return dispatch(g->a, g->b, p, st, g->experts * n);
@@ -480,9 +593,10 @@ B2_API int b2_gemm_bf16_scatter(const void* a, const void* b, int m, int n, int 
 // Gate/up product with the gated activation in the epilogue: out[m][n / 2] (bf16) = act(gate, up) of the interleaved columns of
 // a . b^T + bias.  act: 0 silu, 1 gelu_tanh, 2 clamped swiglu (alpha, limit).
 B2_API int b2_gemm_bf16_glu(const void* a, const void* b, int m, int n, int k, void* out, int ldo, const float* bias, int act, float alpha,
-                            float limit, cudaStream_t st) {
+                            float limit, int pdl, cudaStream_t st) {
     if (bad_operands(a, b, m, n, k, ldo) || (n & 7) || (ldo & 1) || ((uintptr_t)out & 3) || act < 0 || act > 2) return (int)cudaErrorInvalidValue;
     GemmParams p{m, n, k, out, ldo, bias, 0, 1, {}, 0, nullptr, 1 + act, alpha, limit};
+    p.pdl = pdl;
     return dispatch(a, b, p, st);
 }
 

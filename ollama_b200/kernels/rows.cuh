@@ -90,4 +90,5 @@ struct GemmRowsArgs {
     float* tail;              // [m][ld_tail]
     int tail_col, ld_tail;
     float act_p, act_q;       // numbers of the activation, where it has some
+    int pdl;                  // bf16 products: 1 programmatic dependent launch, 2: and b does not depend on the kernel before
 };

@@ -463,8 +463,8 @@ def attn_decode_rope(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
 
 
 def gemm_bf16(a: torch.Tensor, b: torch.Tensor, bias: torch.Tensor | None = None, out: torch.Tensor | None = None,
-              accumulate: bool = False) -> torch.Tensor:
-    """out[m, n] (+)= a[m, k] @ b[n, k]^T + bias on the tcgen05 tensor-core kernel (bf16 operands, fp32 result)."""
+              accumulate: bool = False, pdl: int = 0) -> torch.Tensor:
+    """out[m, n] (+)= a[m, k] @ b[n, k]^T + bias on the tcgen05 tensor-core kernel (bf16 operands, fp32 result).  ``pdl``: 1 the launch may begin while the kernel before it ends, 2 and ``b`` does not depend on that kernel."""
     m, k = a.shape
     n = b.shape[0]
     if a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16 or b.shape[1] != k:
@@ -473,12 +473,13 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, bias: torch.Tensor | None = None
     if out is None:
         out = torch.empty(m, n, device=a.device, dtype=torch.float32)
     f = lib().b2_gemm_bf16
-    f.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_void_p]
-    _check(f(ptr(a), ptr(b), m, n, k, ptr(out), out.stride(0), ptr(bias), int(accumulate), stream()), "gemm_bf16")
+    f.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_int, C.c_void_p]
+    _check(f(ptr(a), ptr(b), m, n, k, ptr(out), out.stride(0), ptr(bias), int(accumulate), pdl, stream()), "gemm_bf16")
     return out
 
 
-def gemm_bf16_out16(a: torch.Tensor, b: torch.Tensor, bias: torch.Tensor | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
+def gemm_bf16_out16(a: torch.Tensor, b: torch.Tensor, bias: torch.Tensor | None = None, out: torch.Tensor | None = None,
+                    pdl: int = 0) -> torch.Tensor:
     """Same product as :func:`gemm_bf16` with a bf16 result (n % 8 == 0)."""
     m, k = a.shape
     n = b.shape[0]
@@ -486,8 +487,8 @@ def gemm_bf16_out16(a: torch.Tensor, b: torch.Tensor, bias: torch.Tensor | None 
     if out is None:
         out = torch.empty(m, n, device=a.device, dtype=torch.bfloat16)
     f = lib().b2_gemm_bf16_out16
-    f.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]
-    _check(f(ptr(a), ptr(b), m, n, k, ptr(out), out.stride(0), ptr(bias), stream()), "gemm_bf16_out16")
+    f.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_void_p]
+    _check(f(ptr(a), ptr(b), m, n, k, ptr(out), out.stride(0), ptr(bias), pdl, stream()), "gemm_bf16_out16")
     return out
 
 
@@ -755,13 +756,14 @@ def gemm_q_grouped(a: torch.Tensor, w: DevWeight, tile_expert: torch.Tensor, glu
     return out
 
 
-def gemm_bf16_glu(a: torch.Tensor, b: torch.Tensor, act: str, bias: torch.Tensor | None = None, alpha: float = 1.702, limit: float = 7.0) -> torch.Tensor:
+def gemm_bf16_glu(a: torch.Tensor, b: torch.Tensor, act: str, bias: torch.Tensor | None = None, alpha: float = 1.702, limit: float = 7.0,
+                  pdl: int = 0) -> torch.Tensor:
     """Gate/up product of a dense FFN with the gated activation in the GEMM epilogue: bf16 [m, n / 2]."""
     m, k = a.shape
     n = b.shape[0]
     a, b = a.contiguous(), b.contiguous()
     out = torch.empty(m, n // 2, device=a.device, dtype=torch.bfloat16)
     f = lib().b2_gemm_bf16_glu
-    f.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_float, C.c_float, C.c_void_p]
-    _check(f(ptr(a), ptr(b), m, n, k, ptr(out), out.stride(0), ptr(bias), _ACT[act], alpha, limit, stream()), "gemm_bf16_glu")
+    f.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_float, C.c_float, C.c_int, C.c_void_p]
+    _check(f(ptr(a), ptr(b), m, n, k, ptr(out), out.stride(0), ptr(bias), _ACT[act], alpha, limit, pdl, stream()), "gemm_bf16_glu")
     return out

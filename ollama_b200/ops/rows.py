@@ -31,7 +31,7 @@ RowSeg = _st("RowSeg", [("w", P), ("g", P), ("rs", P), ("rc", P), ("out", P), ("
 GemmRowsArgs = _st("GemmRowsArgs", [("a", P), ("b", P), ("out", P), ("bias", P), ("mul", P), ("mul_row", P), ("tile_expert", P), ("copy", P), ("ws", P),
                                     ("ws_floats", C.c_longlong), ("m", I), ("n", I), ("k", I), ("lda", I), ("ldb", I), ("ldo", I), ("out_type", I), ("act", I),
                                     ("accumulate", I), ("experts", I), ("ldm", I), ("alpha", F), ("limit", F), ("tail", P), ("tail_col", I), ("ld_tail", I),
-                                    ("act_p", F), ("act_q", F)])
+                                    ("act_p", F), ("act_q", F), ("pdl", I)])
 GemvRowsArgs = _st("GemvRowsArgs", [("seg", RowSeg * 4), ("nseg", I), ("nb", I), ("k", I), ("src", I), ("f32", I), ("x", P), ("ldx", I), ("x2", P),
                                     ("ldx2", I), ("k1", I), ("eps", F), ("kn", I), ("conv_seg", I), ("conv_n", I), ("taps", I), ("conv_w", P),
                                     ("conv_b", P), ("conv_state", P), ("conv_silu", I), ("conv_shift", I), ("conv_out", P), ("ldu", I), ("slots", P), ("positions", P),
@@ -144,7 +144,7 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: str = "", acc
     ws = torch.empty(size, device=a.device) if size else None
     g = GemmRowsArgs(ptr(a), ptr(w), ptr(out), ptr(bias), ptr(mul), ptr(mul_row), ptr(tile_expert), ptr(copy), ptr(ws), size, m, n, k, a.stride(0), w.stride(0), out.stride(0),
                      OUT_TYPE[out.dtype], ACT[act], int(accumulate), experts, mul.stride(0) if mul is not None else 0, alpha, limit, ptr(tail), n - nt,
-                     tail.stride(0) if nt else 0, *nums)
+                     tail.stride(0) if nt else 0, *nums, 1)      # 1: w may come from the kernel just before
     _call("b2_gemm_rows_f32" if f32 else "b2_gemm_rows", g)
 
 

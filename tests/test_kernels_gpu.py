@@ -695,6 +695,29 @@ def test_engine_moe_prefill_on_mxfp4_experts(tmp_path, monkeypatch, stream_q):
     eng.close()
 
 
+@pytest.mark.parametrize("m,n,k", [(129, 64, 64), (257, 304, 520), (300, 192, 72), (1153, 5584, 1032), (769, 5408, 2056)])
+@pytest.mark.parametrize("pdl", [0, 2])
+def test_gemm_bf16_shapes(m, n, k, pdl):
+    """Products of more than 128 rows in the form and width that the estimate picks (the last two: CTA pairs, 256 and 192 columns), ragged in every direction, all outputs.
+    Exact products of bf16 values, fp32 sums: k 2^-24 of the sum of magnitudes; 16-bit results one rounding more."""
+    K = _K()
+    gen = torch.Generator().manual_seed(m + n)
+    a, b = (torch.randn(r, k, generator=gen).to(torch.bfloat16).cuda() for r in (m, n))
+    bias, x = torch.randn(n, generator=gen).cuda(), torch.randn(m, n, generator=gen).cuda()
+    ref = a.double() @ b.double().t() + bias.double()
+    tol = (k + 2) * 2 ** -24 * (a.double().abs() @ b.double().abs().t() + bias.double().abs() + x.double().abs())
+    assert ((K.gemm_bf16(a, b, bias, pdl=pdl).double() - ref).abs() <= tol).all()
+    out = x.clone()
+    K.gemm_bf16(a, b, bias, out=out, accumulate=True, pdl=pdl)
+    assert ((out.double() - x.double() - ref).abs() <= tol).all()
+    assert ((K.gemm_bf16_out16(a, b, bias, pdl=pdl).double() - ref).abs() <= tol + 2 ** -8 * ref.abs()).all()
+    g, u = ref[:, 0::2], ref[:, 1::2]
+    h = g * torch.sigmoid(g) * u
+    got = K.gemm_bf16_glu(a, b, "silu", bias, pdl=pdl).double()
+    assert ((got - h).abs() <= 2 ** -8 * h.abs() + 1.1 * tol[:, 0::2] * u.abs() + g.abs() * tol[:, 1::2]).all()      # the slope of silu is at most 1.1
+    assert K_status_ok()
+
+
 def K_status_ok() -> bool:
     return _K().gemm_status() == 0
 
