@@ -484,14 +484,14 @@ class B200Backend(StepEngine):
         inv_freq, mscale = (self.inv_freq_local, 1.0) if local else (self.inv_freq, self.mscale)
         ca = K.AttnCombineArgs(K.ptr(b.part_acc), K.ptr(b.part_ml), K.ptr(L.sinks), c.n_heads, self.n_splits, c.head_dim,
                                K.ptr(b.ao), None, None)
-        fused = self.fuse_rope and L.q_norm is None and L.k_norm is None and self.k_scale[i] is None
+        fused = self.fuse_rope and (L.q_norm is None) == (L.k_norm is None) and self.k_scale[i] is None
         aa = K.AttnDecodeArgs(None if fused else K.ptr(b.q), K.ptr(self.k_cache[i]), K.ptr(self.v_cache[i]), K.ptr(b.positions), K.ptr(b.slots),
                               c.n_heads, c.n_kv_heads, self.n_ctx, self.n_splits, self.attn_scale, c.attn_softcap,
                               c.sliding_window if L.swa else 0, K.ptr(b.part_acc), K.ptr(b.part_ml), K.ptr(self.k_scale[i]),
                               K.ptr(self.v_scale[i]))
         if fused:
             # rotary embedding of the queries, rotation + cache append of the new key / value and the attention in one launch
-            rr = K.AttnRopeArgs(K.ptr(b.qkv), K.ptr(inv_freq), mscale, c.rope_dim, int(c.rope_style == "neox"))
+            rr = K.AttnRopeArgs(K.ptr(b.qkv), K.ptr(inv_freq), mscale, c.rope_dim, int(c.rope_style == "neox"), K.ptr(L.q_norm), K.ptr(L.k_norm), c.norm_eps)
             lib.b2_attn_decode_rope.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p]
             rc = lib.b2_attn_decode_rope(C.byref(aa), C.byref(rr), C.byref(ca), nb, c.head_dim, int(self.pdl), st())
             if rc == 801:               # cudaErrorNotSupported: nothing was launched; this model keeps the separate kernel

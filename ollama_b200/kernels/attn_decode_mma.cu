@@ -38,13 +38,26 @@ __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-template <int D, int NS, bool PAGED>
+// Four int8 values times a block's scale, as two f16 pairs, each rounded once (1024 + 128 + value under the exponent of 1024, less 1152, is exact).
+__device__ __forceinline__ uint2 expand_q8x4(uint32_t w, __half2 d) {
+    w ^= 0x80808080u;
+    uint32_t lo = __byte_perm(w, 0x64646464u, 0x4140), hi = __byte_perm(w, 0x64646464u, 0x4342);
+    const __half2 base = __half2half2(__ushort_as_half(0x6480));
+    const __half2 a = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&lo), base), d), b = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&hi), base), d);
+    return make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+
+// Q8: int8 caches.  Tiles arrive as they are in a ring of NS stages and are expanded into one f16 tile when they are used, so that as many requests are under way as of f16
+// caches; loads that were expanded on the way into the stage kept none (8 sequences of 3000 positions took 55 us a layer, their bytes 8).
+template <int D, int NS, bool PAGED, bool Q8>
 __global__ void __launch_bounds__(128) attn_decode_mma_kernel(const __grid_constant__ AttnDecodeArgs a, const __grid_constant__ AttnRopeArgs r) {
-    constexpr int LD = D + PAD;
+    constexpr int LD = D + PAD, TS = Q8 ? 1 : NS;
+    constexpr int RAW_ROW = D + D / 16, RAW = 2 * BN * RAW_ROW;  // bytes of a stage: [BN][D] keys, [BN][D / 32] their scales, the values likewise
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __half* sQ = reinterpret_cast<__half*>(smem_raw);            // [ROWS][LD]
-    __half* sK = sQ + ROWS * LD;                                 // [NS][BN][LD]
-    __half* sV = sK + NS * BN * LD;                              // [NS][BN][LD]
+    __half* sK = sQ + ROWS * LD;                                 // [TS][BN][LD]
+    __half* sV = sK + TS * BN * LD;                              // [TS][BN][LD]
+    unsigned char* sR = reinterpret_cast<unsigned char*>(sV + TS * BN * LD);      // Q8: [NS][RAW]
     __shared__ float s_m[4][ROWS], s_l[4][ROWS];
     __shared__ float s_cs[128], s_sn[128];                        // cos / sin of the query position per rotated pair (fused form)
     __shared__ __half s_newk[D], s_newv[D];                       // the query token's own key and value rows (fused form, owning split)
@@ -82,30 +95,24 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(const __grid_const
             asm volatile("cp.async.commit_group;" ::: "memory");
             return;
         }
-        if (a.k_scale) {      // q8_0 cache: plain loads, expanded to f16 on the way into shared memory
-            const int8_t* kq = reinterpret_cast<const int8_t*>(a.k_cache) + row0 * D;
-            const int8_t* vq = reinterpret_cast<const int8_t*>(a.v_cache) + row0 * D;
-            const __half* ks = a.k_scale + row0 * (D / 32);
-            const __half* vs = a.v_scale + row0 * (D / 32);
-            for (int c = tid; c < BN * (D / 16); c += 128) {
-                const int r = c / (D / 16), col = (c % (D / 16)) * 16;
-                const int pos = min(n0 + r, a.n_ctx - 1);
-                const uint4 k4 = *(const uint4*)(kq + (size_t)pos * D + col), v4 = *(const uint4*)(vq + (size_t)pos * D + col);
-                const float dkf = __half2float(ks[(size_t)pos * (D / 32) + (col >> 5)]), dvf = __half2float(vs[(size_t)pos * (D / 32) + (col >> 5)]);
-                const uint32_t kw[4] = {k4.x, k4.y, k4.z, k4.w}, vw[4] = {v4.x, v4.y, v4.z, v4.w};
-                uint32_t ko[8], vo[8];
+        if (Q8) {
+            const unsigned char* src[2] = {reinterpret_cast<const unsigned char*>(a.k_cache) + row0 * D, reinterpret_cast<const unsigned char*>(a.v_cache) + row0 * D};
+            const __half* sc[2] = {a.k_scale + row0 * (D / 32), a.v_scale + row0 * (D / 32)};
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const uint32_t kb = kw[i >> 1] >> (16 * (i & 1)), vb = vw[i >> 1] >> (16 * (i & 1));
-                    ko[i] = pack_half2(dkf * (float)(int8_t)(kb & 0xff), dkf * (float)(int8_t)((kb >> 8) & 0xff));
-                    vo[i] = pack_half2(dvf * (float)(int8_t)(vb & 0xff), dvf * (float)(int8_t)((vb >> 8) & 0xff));
+            for (int kv = 0; kv < 2; kv++) {
+                unsigned char* dst = sR + stage * RAW + kv * BN * RAW_ROW;
+                for (int c = tid; c < BN * (D / 16); c += 128) {
+                    const int rr = c / (D / 16), col = (c % (D / 16)) * 16;
+                    cp_async16(dst + rr * D + col, src[kv] + (size_t)min(n0 + rr, a.n_ctx - 1) * D + col);
                 }
-                *(uint4*)(dk + r * LD + col) = make_uint4(ko[0], ko[1], ko[2], ko[3]);
-                *(uint4*)(dk + r * LD + col + 8) = make_uint4(ko[4], ko[5], ko[6], ko[7]);
-                *(uint4*)(dv + r * LD + col) = make_uint4(vo[0], vo[1], vo[2], vo[3]);
-                *(uint4*)(dv + r * LD + col + 8) = make_uint4(vo[4], vo[5], vo[6], vo[7]);
+                for (int c = tid; c < BN; c += 128) {      // the row's scales: D / 16 bytes
+                    const __half* from = sc[kv] + (size_t)min(n0 + c, a.n_ctx - 1) * (D / 32);
+                    unsigned char* to = dst + BN * D + c * (D / 16);
+                    if (D == 128) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(to)), "l"(from) : "memory");
+                    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(to)), "l"(from) : "memory");
+                }
             }
-            asm volatile("cp.async.commit_group;" ::: "memory");      // keeps the group counting of the f16 path
+            asm volatile("cp.async.commit_group;" ::: "memory");
             return;
         }
         const __half* kbase = a.k_cache + row0 * D;
@@ -125,7 +132,7 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(const __grid_const
         if (t < n_tiles) load_kv(t, t);
         else asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    const bool fresh = r.qkv != nullptr;
+    const bool fresh = !Q8 && r.qkv != nullptr;
     const bool owner = fresh && !(PAGED && r.no_append) && n_tiles > 0 && qpos - shift >= p0 && qpos - shift < p1;      // this split holds the query token's own position
     // element i of a raw head row after the rotary embedding (pairs (2p, 2p+1), or (p, p + n_rot/2) in the neox order)
     // the second map's columns of a row of two (differential attention) turn like the first's
@@ -146,7 +153,7 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(const __grid_const
     if (fresh) {
         // the raw rows (query heads of this group, the key and the value) are staged in the last K stage, which stays unused
         // until the tile loop requests tile NS - 1; cos / sin of the position are computed once per CTA meanwhile
-        float* raw = reinterpret_cast<float*>(sK + (NS - 1) * BN * LD);       // [group + 2][D]
+        float* raw = reinterpret_cast<float*>(sK + (TS - 1) * BN * LD);       // [group + 2][D]
         const int nrows = group + (owner ? 2 : 0);
         if (PAGED) {
             const float* tok = r.qkv + (size_t)b * r.ldq;
@@ -232,6 +239,21 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(const __grid_const
             s_sn[p] = sn * r.mscale;
             s_cs[p] = cs * r.mscale;
         }
+        if (r.q_norm) {          // RMS norm of each head, a warp per head
+            __syncthreads();
+            for (int rr = warp; rr < group + (owner ? 1 : 0); rr += 4) {
+                const float* w = rr < group ? r.q_norm : r.k_norm;
+                float x[D / 32], s = 0.f;
+#pragma unroll
+                for (int i = 0; i < D / 32; i++) {
+                    x[i] = raw[rr * D + lane + 32 * i];
+                    s += x[i] * x[i];
+                }
+                const float inv = rsqrtf(warp_sum(s) / (float)D + r.eps);
+#pragma unroll
+                for (int i = 0; i < D / 32; i++) raw[rr * D + lane + 32 * i] = x[i] * inv * w[lane + 32 * i];
+            }
+        }
         }
         __syncthreads();
         if (owner) {      // append the new key / value rows to the cache and keep them for the last tile
@@ -279,11 +301,29 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(const __grid_const
     const float inv_cap = a.softcap > 0.f ? 1.f / a.softcap : 0.f;
 
     for (int tile = 0; tile < n_tiles; tile++) {
-        const int stage = tile % NS;
+        const int stage = Q8 ? 0 : tile % NS;
         if (tile + NS - 1 < n_tiles) load_kv(tile + NS - 1, (tile + NS - 1) % NS);      // into the stage that tile - 1 has just left
         else asm volatile("cp.async.commit_group;" ::: "memory");
         asm volatile("cp.async.wait_group %0;" ::"n"(NS - 1) : "memory");               // tile's own group is complete
         __syncthreads();
+        if (Q8) {
+#pragma unroll
+            for (int kv = 0; kv < 2; kv++) {
+                const unsigned char* src = sR + (tile % NS) * RAW + kv * BN * RAW_ROW;
+                const __half* sc = reinterpret_cast<const __half*>(src + BN * D);
+                __half* dst = kv ? sV : sK;
+#pragma unroll
+                for (int c = tid; c < BN * (D / 16); c += 128) {
+                    const int rr = c / (D / 16), col = (c % (D / 16)) * 16;
+                    const uint4 w = *reinterpret_cast<const uint4*>(src + rr * D + col);
+                    const __half2 d = __half2half2(sc[rr * (D / 32) + (col >> 5)]);
+                    const uint2 e0 = expand_q8x4(w.x, d), e1 = expand_q8x4(w.y, d), e2 = expand_q8x4(w.z, d), e3 = expand_q8x4(w.w, d);
+                    *reinterpret_cast<uint4*>(dst + rr * LD + col) = make_uint4(e0.x, e0.y, e1.x, e1.y);
+                    *reinterpret_cast<uint4*>(dst + rr * LD + col + 8) = make_uint4(e2.x, e2.y, e3.x, e3.y);
+                }
+            }
+            __syncthreads();
+        }
         if (owner && tile == n_tiles - 1) {      // the query's own row did not come from the cache: put it into the tile
             const int rr = qpos - shift - (p0 + tile * BN);
             for (int i = tid; i < D; i += 128) {
@@ -401,11 +441,12 @@ __global__ void __launch_bounds__(128) attn_decode_mma_kernel(const __grid_const
     }
 }
 
-template <int D, int NS, bool PAGED>
+template <int D, int NS, bool PAGED, bool Q8 = false>
 int launch(const AttnDecodeArgs& a, const AttnRopeArgs& r, int nb, int pdl, cudaStream_t st) {
-    constexpr int SMEM = (ROWS + 2 * NS * BN) * (D + PAD) * 2;
+    constexpr int SMEM = (ROWS + 2 * (Q8 ? 1 : NS) * BN) * (D + PAD) * 2 + (Q8 ? NS * 2 * BN * (D + D / 16) : 0);
+    const void* fn = (const void*)attn_decode_mma_kernel<D, NS, PAGED, Q8>;
     static PerDeviceOnce once;
-    if (once.first()) cudaFuncSetAttribute(attn_decode_mma_kernel<D, NS, PAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    if (once.first()) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(a.n_splits, a.n_kv_heads, nb);
     cfg.blockDim = dim3(128);
@@ -419,7 +460,7 @@ int launch(const AttnDecodeArgs& a, const AttnRopeArgs& r, int nb, int pdl, cuda
     AttnDecodeArgs copy = a;
     AttnRopeArgs rcopy = r;
     void* args[] = {&copy, &rcopy};
-    return (int)cudaLaunchKernelExC(&cfg, (const void*)attn_decode_mma_kernel<D, NS, PAGED>, args);
+    return (int)cudaLaunchKernelExC(&cfg, fn, args);
 }
 
 int g_stages = 0;      // 0: by the size of the launch; 2, 3 or 4: forced (tests)
@@ -444,6 +485,8 @@ int stages_for(const AttnDecodeArgs& a, int nb) {
 template <int D>
 int launch_d(const AttnDecodeArgs& a, const AttnRopeArgs& r, int nb, int pdl, cudaStream_t st) {
     const int ns = stages_for(a, nb);
+    // int8 stages are small: four of them and the f16 tile take 108 KB at 128 columns, two CTAs per SM, as many as three stages of f16
+    if (a.k_scale) return ns == 2 && a.n_ctx / a.n_splits < 2 * BN ? launch<D, 2, false, true>(a, r, nb, pdl, st) : launch<D, 4, false, true>(a, r, nb, pdl, st);
     if (a.page_table) return ns == 4 ? launch<D, 4, true>(a, r, nb, pdl, st) : ns == 3 ? launch<D, 3, true>(a, r, nb, pdl, st) : launch<D, 2, true>(a, r, nb, pdl, st);
     return ns == 4 ? launch<D, 4, false>(a, r, nb, pdl, st) : ns == 3 ? launch<D, 3, false>(a, r, nb, pdl, st) : launch<D, 2, false>(a, r, nb, pdl, st);
 }

@@ -266,6 +266,29 @@ def test_attn_decode_with_rotary_embedding_and_cache_append_inside(hd, H, Hkv, n
                               pos[:1], slots[:1] * 0, inv, n_heads=1, n_rot=64, neox=neox, mscale=1.0, scale=1.0, n_splits=1) is None
 
 
+@pytest.mark.parametrize("hd,H,Hkv", [(128, 8, 2), (64, 3, 3)])
+@pytest.mark.parametrize("n_splits", [1, 3, 16])
+def test_attn_decode_head_norm(hd, H, Hkv, n_splits, attn_mode):
+    """The norm of each query and key head inside the attention launch, parts without a position among them, against norm and rotation in a launch of their own and the scalar
+    kernel.  Bound as in the tests beside this one: f16 queries and probabilities."""
+    K = _K()
+    n_slots, n_ctx, nb = 3, 1100, 3
+    gen = torch.Generator().manual_seed(hd + n_splits)
+    kc, vc = ((torch.randn(n_slots, Hkv, n_ctx, hd, generator=gen) * 0.5).to(torch.float16).cuda() for _ in range(2))
+    qkv = torch.randn(nb, (H + 2 * Hkv) * hd, generator=gen).cuda()
+    pos, slots = torch.tensor([5, 700, 1099], dtype=torch.int32).cuda(), torch.tensor([2, 0, 1], dtype=torch.int32).cuda()
+    qn, kn = (torch.rand(hd, generator=gen).cuda() + 0.5 for _ in range(2))
+    inv = (1.0 / (10000.0 ** (torch.arange(0, hd, 2).float() / hd))).cuda()
+    kc2, vc2 = kc.clone(), vc.clone()
+    q = K.rope_kv(qkv, pos, slots, inv, n_heads=H, n_kv_heads=Hkv, hd=hd, n_rot=hd, neox=True, mscale=1.0, k_cache=kc, v_cache=vc, q_norm=qn, k_norm=kn, eps=1e-5)
+    attn_mode(0)
+    ref, _ = K.attn_decode(q, kc, vc, pos, slots, scale=hd ** -0.5, n_splits=n_splits)
+    attn_mode(1)
+    got = K.attn_decode_rope(qkv, kc2, vc2, pos, slots, inv, n_heads=H, n_rot=hd, neox=True, mscale=1.0, scale=hd ** -0.5, n_splits=n_splits, q_norm=qn, k_norm=kn, eps=1e-5)
+    assert torch.allclose(kc2, kc, atol=2e-3, rtol=2e-3) and torch.equal(vc2, vc)
+    assert torch.allclose(got, ref, atol=3e-3, rtol=2e-2)
+
+
 @pytest.mark.parametrize("hd,H,Hkv", [(128, 32, 8), (64, 16, 2), (128, 16, 1)])
 @pytest.mark.parametrize("q8", [False, True])
 def test_attn_decode_tensor_core_long_context(hd, H, Hkv, q8, attn_mode):
