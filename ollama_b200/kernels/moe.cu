@@ -132,6 +132,79 @@ B2_API int b2_moe_route(const MoeRouteArgs* a, int tokens, int pdl, cudaStream_t
     return (int)cudaLaunchKernelExC(&cfg, (const void*)moe_route_kernel, args);
 }
 
+// Router logits of a decode step in 32 bits: out[b][e] = w[e] . x[b] + bias[e].  A CTA multiplies four rows of each; its 256 threads share the row length, and fetch their weights
+// before the grid-dependency wait.  (The matrix-vector kernel gave 128 experts 32 CTAs and eight tokens a launch: 14 us twice a layer at 16 tokens.)
+struct RouterArgs {
+    const float* x;        // [nb][ldx]
+    const float* w;        // [n][k]
+    const float* bias;     // [n] or null
+    float* out;            // [nb][ldo]
+    int ldx, n, k, nb, ldo;
+};
+
+constexpr int ROUTER_AHEAD = 3;      // 16-byte pieces per thread and row fetched ahead: rows of up to 3072 values
+
+__global__ void __launch_bounds__(256) router_kernel(const __grid_constant__ RouterArgs a) {
+    __shared__ float part[8][16];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, e0 = blockIdx.x * 4, b0 = blockIdx.y * 4, k4 = a.k >> 2;
+    const float4* w[4];
+    const float4* x[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        w[i] = reinterpret_cast<const float4*>(a.w + (size_t)min(e0 + i, a.n - 1) * a.k);
+        x[i] = reinterpret_cast<const float4*>(a.x + (size_t)min(b0 + i, a.nb - 1) * a.ldx);
+    }
+    pdl_launch();
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 wv[ROUTER_AHEAD][4];
+#pragma unroll
+    for (int j = 0; j < ROUTER_AHEAD; j++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) wv[j][i] = tid + 256 * j < k4 ? w[i][tid + 256 * j] : zero;
+    pdl_wait();
+    float acc[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) acc[i] = 0.f;
+    auto add = [&](const float4 (&u)[4], int c) {
+        float4 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) v[i] = c < k4 ? x[i][c] : zero;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc[4 * i + j] += u[i].x * v[j].x + u[i].y * v[j].y + u[i].z * v[j].z + u[i].w * v[j].w;
+    };
+#pragma unroll
+    for (int j = 0; j < ROUTER_AHEAD; j++) add(wv[j], tid + 256 * j);
+    for (int c = tid + 256 * ROUTER_AHEAD; c < k4; c += 256) {
+        float4 u[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) u[i] = w[i][c];
+        add(u, c);
+    }
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+        const float v = warp_sum(acc[i]);
+        if (lane == 0) part[warp][i] = v;
+    }
+    __syncthreads();
+    if (tid < 16) {
+        const int e = e0 + (tid >> 2), b = b0 + (tid & 3);
+        float v = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; i++) v += part[i][tid];
+        if (e < a.n && b < a.nb) a.out[(size_t)b * a.ldo + e] = v + (a.bias ? a.bias[e] : 0.f);
+    }
+}
+
+// k and ldx multiples of 4, x and w 16-byte aligned.
+B2_API int b2_router(const RouterArgs* in, int pdl, cudaStream_t st) {
+    RouterArgs a = *in;
+    if (a.nb < 1 || a.n < 1 || a.k < 4 || (a.k & 3) || (a.ldx & 3) || (((uintptr_t)a.x | (uintptr_t)a.w) & 15)) return (int)cudaErrorInvalidValue;
+    void* args[] = {&a};
+    return launch_rows((const void*)router_kernel, dim3((a.n + 3) / 4, (a.nb + 3) / 4), dim3(256), 0, args, st, pdl);
+}
+
 // ---------------------------------------------------------------------------------------------
 // x[t] += sum_s wts[t][s] * y[t * k + s]      (y rows of experts that live elsewhere are zero)
 // With a CommSend (low-latency protocol) the weighted sum is not added locally: it is this GPU's partial

@@ -757,6 +757,18 @@ def gemm_q_grouped(a: torch.Tensor, w: DevWeight, tile_expert: torch.Tensor, glu
     return out
 
 
+class RouterArgs(C.Structure):
+    _fields_ = [("x", C.c_void_p), ("w", C.c_void_p), ("bias", C.c_void_p), ("out", C.c_void_p), ("ldx", C.c_int), ("n", C.c_int), ("k", C.c_int), ("nb", C.c_int),
+                ("ldo", C.c_int)]
+
+
+def router(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, out: torch.Tensor, pdl: bool = False) -> None:
+    """out[b, e] = w[e] . x[b] + bias[e], all fp32; row length a multiple of 4."""
+    a = RouterArgs(ptr(x), ptr(w), ptr(bias), ptr(out), x.stride(0), w.shape[0], w.shape[1], x.shape[0], out.stride(0))
+    _check(lib().b2_router(C.byref(a), int(pdl), stream()), "router")
+
+
+
 def gemm_bf16_glu(a: torch.Tensor, b: torch.Tensor, act: str, bias: torch.Tensor | None = None, alpha: float = 1.702, limit: float = 7.0,
                   pdl: int = 0) -> torch.Tensor:
     """Gate/up product of a dense FFN with the gated activation in the GEMM epilogue: bf16 [m, n / 2]."""

@@ -718,6 +718,18 @@ def test_engine_moe_prefill_on_mxfp4_experts(tmp_path, monkeypatch, stream_q):
     eng.close()
 
 
+@pytest.mark.parametrize("nb,n,k", [(1, 3, 4), (5, 128, 2880), (16, 33, 4100)])
+def test_router(nb, n, k):
+    """Router logits in 32 bits: sums of k products of about unit size, k 2^-24 at worst."""
+    K = _K()
+    gen = torch.Generator().manual_seed(k)
+    x, w, bias = torch.randn(nb, k, generator=gen).cuda(), (torch.randn(n, k, generator=gen) * k ** -0.5).cuda(), torch.randn(n, generator=gen).cuda()
+    out = torch.zeros(nb, n + 4, device="cuda")
+    K.router(x, w, bias, out)
+    assert (out[:, :n].double() - x.double() @ w.double().t() - bias.double()).abs().max() < 2 ** -24 * k ** 0.5 * 64
+    assert out[:, n:].abs().max() == 0
+
+
 @pytest.mark.parametrize("m,n,k", [(129, 64, 64), (257, 304, 520), (300, 192, 72), (1153, 5584, 1032), (769, 5408, 2056)])
 @pytest.mark.parametrize("pdl", [0, 2])
 def test_gemm_bf16_shapes(m, n, k, pdl):
