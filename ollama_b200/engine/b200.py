@@ -38,6 +38,12 @@ MAX_STREAM_BATCH = 32            # sequences per step when every matrix runs on 
 # Steps of more sequences than this multiply f16 activations (kernels/gemm_sk.cu) instead of int8 ones: a layer of Llama-8B takes 64 us of products against 70 at eight
 # sequences and 108 against 78 at thirteen.
 INT8_ROWS = 8
+# Steps of at least so many (token, expert) pairs, and of one for every eighth expert, read MXFP4 experts once for all rows that chose them (kernels/moe_fp4.cu), smaller ones
+# once per pair: a layer of 128 experts of 13 MB, four a token, takes 72 us against 75 at four tokens and 194 against 280 at sixteen, but 45 against 29 at one.
+FP4_MIN_PAIRS = 16
+# Prompts of up to so many rows an expert do too; beyond them the 128-row tiles of gemm_q_grouped.cu are full: 769 us against 1341 at 32 rows, 1227 against 1349 at 64, 1825
+# against 1358 at 96.
+FP4_MAX_ROWS = 64
 
 
 def supports(cfg: ModelConfig) -> bool:
@@ -304,6 +310,9 @@ class B200Backend(StepEngine):
             b.moe_lids = torch.zeros(hr, device=dev, dtype=i32)
             b.moe_w = torch.zeros(hr, device=dev, dtype=f32)
             b.ey = torch.zeros(hr, c.d_model, device=dev, dtype=f32)
+            b.fp4 = None
+            if type(self) is B200Backend and all(K.moe_fp4_supported(w) for L in self.layers if L.moe for w in (L.gu, L.down)):
+                b.fp4 = K.MoeFp4(hr, self.e_cnt, c.d_model, c.d_ff_expert, dev, 8)
         b.logits = torch.zeros(MB, c.vocab_size, device=dev, dtype=f32)
         b.part_acc = torch.zeros(MB * c.n_heads * self.n_splits * c.head_dim, device=dev, dtype=f32)
         b.part_ml = torch.zeros(MB * c.n_heads * self.n_splits * 2, device=dev, dtype=f32)
@@ -399,6 +408,17 @@ class B200Backend(StepEngine):
         else:
             self._gemv([L.router], nb, b.xq, b.xds, b.xf, b.rlogits, b.rlogits.stride(0), tc=False)
         self._route(b.rlogits, nb, b.moe_ids, b.moe_lids, b.moe_w, self.pdl)
+        if b.fp4 is not None and cm is None and pairs >= max(FP4_MIN_PAIRS, self.e_cnt // 8):
+            # each chosen expert is read once for all of its rows, in bf16 activations
+            m = b.fp4
+            m.sort(b.moe_lids, pairs, self.pdl)
+            m.take(b.xf.view(-1)[:nb * c.d_model].view(nb, c.d_model), k, pairs, self.pdl)
+            m.product(L.gu, pairs, c.act, c.swiglu_alpha, c.swiglu_limit, pdl=self.pdl)
+            m.product(L.down, pairs, out=b.ey, by_pair=True, pdl=self.pdl)
+            ca = K.MoeCombineArgs(K.ptr(b.ey), K.ptr(b.moe_w), k, c.d_model, K.ptr(b.x))
+            K._check(lib.b2_moe_combine(C.byref(ca), nb, int(self.pdl), st()), "moe_combine")
+            self._n += 6
+            return
         ga = K.GluArgs()
         ga.gu = L.gu.desc()
         ga.nb, ga.xq, ga.xds, ga.xf = 1, K.ptr(b.xq), K.ptr(b.xds), K.ptr(b.xf)
@@ -418,12 +438,12 @@ class B200Backend(StepEngine):
         K._check(lib.b2_moe_combine(C.byref(ca), nb, int(self.pdl), st()), "moe_combine")
         self._n += 4
 
-    def _moe_prefill(self, h: torch.Tensor, L) -> torch.Tensor:
+    def _moe_prefill(self, h: torch.Tensor, L, x: torch.Tensor | None = None) -> torch.Tensor:
         """Expert FFN of a prefill chunk without leaving the device: the (token, expert-slot) pairs are sorted by expert into
         128-row tiles, one grouped tensor-core GEMM runs gate/up with the gated activation in its epilogue, a second one the
         down projection, and the weighted rows are added back per token.
 
-        ``h``: [T, d_model] bf16.  Returns this GPU's (partial, under expert parallelism) FFN output [T, d_model] fp32.
+        ``h``: [T, d_model] bf16.  Returns this GPU's (partial, under expert parallelism) FFN output [T, d_model] fp32, added to ``x`` where that is given.
         """
         c = self.cfg
         T, k = h.shape[0], c.n_experts_used
@@ -438,6 +458,19 @@ class B200Backend(StepEngine):
         ids = torch.empty(T * k, device=self.device, dtype=torch.int32)
         lids, wts = torch.empty_like(ids), torch.empty(T * k, device=self.device, dtype=torch.float32)
         self._route(logits.contiguous(), T, ids, lids, wts, False)
+        per = T * k / c.n_experts
+        if (self.moe_stream_q and getattr(L.gu, "bf16", None) is None and K.moe_fp4_supported(L.gu) and K.moe_fp4_supported(L.down)
+                and (per <= FP4_MAX_ROWS or not (K.gemm_q_grouped_supported(L.gu) and K.gemm_q_grouped_supported(L.down)))):
+            # experts without a resident 16-bit copy: their 4-bit blocks are multiplied as they are, once for up to 64 rows.  Chunks of about twice
+            # the mean, so that few experts need a second one: at 32 rows 769 us a layer in chunks of 64, 830 of 32; at 8 rows 512 of 16, 541 of 32
+            m = K.MoeFp4(T * k, self.e_cnt, c.d_model, c.d_ff_expert, self.device, 8 if per <= 4 else 16 if per <= 8 else 32 if per <= 20 else 64)
+            m.sort(lids, T * k)
+            m.take(h, k, T * k)
+            m.product(L.gu, T * k, c.act, c.swiglu_alpha, c.swiglu_limit)
+            ys = torch.empty(m.rows, c.d_model, device=self.device, dtype=torch.float32)
+            m.product(L.down, T * k, out=ys)
+            self.kernel_launches += 6
+            return K.moe_scatter_combine(ys, m.row_of_pair, wts, T, k, out=x, accumulate=x is not None)
         row, tile_expert, rows = K.moe_plan(lids, self.e_cnt)
         xs = K.moe_gather(h, row, k, rows)
         if self.moe_stream_q and getattr(L.gu, "bf16", None) is None and K.gemm_q_grouped_supported(L.gu) and K.gemm_q_grouped_supported(L.down):
@@ -446,7 +479,7 @@ class B200Backend(StepEngine):
             ys = K.gemm_q_grouped(f, L.down, tile_expert) if f is not None else None
             if ys is not None:
                 self.kernel_launches += 6
-                return K.moe_scatter_combine(ys, row, wts, T, k)
+                return K.moe_scatter_combine(ys, row, wts, T, k, out=x, accumulate=x is not None)
         gu16 = getattr(L.gu, "bf16", None)
         if gu16 is None:
             gu16 = K.dequant_to_bf16(L.gu)                        # all resident experts at once: scratch until the call returns
@@ -460,7 +493,7 @@ class B200Backend(StepEngine):
         ys = K.gemm_bf16_grouped(f, dn16, self.e_cnt, tile_expert, L.down.bias)
         del dn16
         self.kernel_launches += 6
-        return K.moe_scatter_combine(ys, row, wts, T, k)
+        return K.moe_scatter_combine(ys, row, wts, T, k, out=x, accumulate=x is not None)
 
     def _sk(self, ws, x: torch.Tensor, out: torch.Tensor, nb: int, norm_w=None, mode: int = SK.MODE_STORE) -> None:
         """One streaming GEMV of the decode step: fp32 rows in (normalised with ``norm_w``), ``out`` stored / added to / gated."""
@@ -706,7 +739,7 @@ class B200Backend(StepEngine):
                 self._mm(o, L.wo, x, 0, accumulate=True)                  # residual add in the GEMM epilogue
             h = K.rmsnorm_bf16(x, L.ffn_norm, c.norm_eps, pdl=self.pdl)
             if L.moe:
-                x = x + self._moe_prefill(h, L)
+                x = self._moe_prefill(h, L, x)
                 continue
             f = self._mm_glu(h, L.gu)                                     # gate/up with the gated activation in the GEMM epilogue
             if c.sandwich_norm:

@@ -635,7 +635,7 @@ def attn_prefill_tc_status(clear: bool = False) -> int:
 
 def gemm_status() -> int:
     """0 = ok; 1 = a bounded wait inside a tensor-core kernel (the GEMMs, the tcgen05 attention) expired."""
-    return int(lib().b2_gemm_status()) | int(lib().b2_gemm_q_status()) | int(lib().b2_attn_prefill_tc_status()) | int(lib().b2_gemm_q_grouped_status())
+    return int(lib().b2_moe_fp4_status()) | int(lib().b2_gemm_status()) | int(lib().b2_gemm_q_status()) | int(lib().b2_attn_prefill_tc_status()) | int(lib().b2_gemm_q_grouped_status())
 
 
 GEMM_Q_TYPES = {WT_Q4_K, WT_Q6_K, WT_Q8_0, WT_BF16, WT_F16}
@@ -767,6 +767,67 @@ def router(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, out: tor
     a = RouterArgs(ptr(x), ptr(w), ptr(bias), ptr(out), x.stride(0), w.shape[0], w.shape[1], x.shape[0], out.stride(0))
     _check(lib().b2_router(C.byref(a), int(pdl), stream()), "router")
 
+
+class MoeSortArgs(C.Structure):
+    _fields_ = [("lids", C.c_void_p), ("pairs", C.c_int), ("n_experts", C.c_int), ("rows", C.c_int), ("max_chunks", C.c_int), ("chunks", C.c_void_p),
+                ("row_of_pair", C.c_void_p), ("pair_of_row", C.c_void_p)]
+
+
+class MoeFp4Args(C.Structure):
+    _fields_ = [("q", C.c_void_p), ("s", C.c_void_p), ("bias", C.c_void_p), ("n", C.c_int), ("k", C.c_int), ("x", C.c_void_p), ("chunks", C.c_void_p),
+                ("pair_of_row", C.c_void_p), ("out", C.c_void_p), ("glu", C.c_int), ("alpha", C.c_float), ("limit", C.c_float)]
+
+
+def moe_fp4_supported(w: DevWeight) -> bool:
+    """True when the stacked experts ``w`` can be read by :class:`MoeFp4` (MXFP4, rows a multiple of 16, row length of 32 up to 16384)."""
+    return w.wtype == WT_MXFP4 and w.n % 16 == 0 and w.k % 32 == 0 and w.k <= 16384
+
+
+class MoeFp4:
+    """The (token, expert) pairs of a step or a prompt times MXFP4 experts, each expert read once for all rows that chose it (kernels/moe_fp4.cu).
+
+    Holds the sorted places of the pairs and the row buffers, so that a decode step can keep one for its CUDA graph; sizes that depend on the choice of
+    experts never visit the host.  ``chunk``: rows of an expert that a block multiplies at once, 8 / 16 / 32 / 64."""
+
+    def __init__(self, pairs: int, n_experts: int, d: int, ff: int, device, chunk: int):
+        self.n_experts, self.d, self.ff, self.chunk = n_experts, d, ff, chunk
+        self.max_chunks = min(pairs, n_experts + pairs // chunk)      # full chunks, and one that is not for each expert
+        self.rows = self.max_chunks * chunk
+
+        def ints(n):
+            return torch.empty(n, device=device, dtype=torch.int32)
+
+        self.chunks, self.row_of_pair, self.pair_of_row = ints(1 + 2 * self.max_chunks), ints(pairs), ints(self.rows)
+        size = lib().b2_moe_rows_bytes
+        size.restype = C.c_longlong
+        self.x = torch.empty(size(self.max_chunks, chunk, max(d, ff)), device=device, dtype=torch.uint8)      # the given rows, then the hidden ones
+        self.h = torch.empty(self.rows, ff, device=device, dtype=torch.bfloat16)
+
+    def sort(self, lids: torch.Tensor, pairs: int, pdl: bool = False) -> None:
+        a = MoeSortArgs(ptr(lids), pairs, self.n_experts, self.chunk, self.max_chunks, ptr(self.chunks), ptr(self.row_of_pair), ptr(self.pair_of_row))
+        _check(lib().b2_moe_sort(C.byref(a), int(pdl), stream()), "moe_sort")
+
+    def take(self, x: torch.Tensor, per_token: int, pairs: int, pdl: bool = False) -> None:
+        """Rows of ``x`` (fp32 or bf16, [tokens, d]) to the places of their pairs."""
+        self._rows(x, per_token, self.row_of_pair, pairs, pdl)
+
+    def _rows(self, x, per_token, row_of_pair, n, pdl):
+        f = lib().b2_moe_rows
+        f.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_int, C.c_void_p]
+        _check(f(ptr(x), int(x.dtype == torch.bfloat16), x.stride(0), x.shape[1], per_token, ptr(row_of_pair), ptr(self.chunks), self.chunk, n, ptr(self.x), int(pdl), stream()),
+               "moe_rows")
+
+    def product(self, w: DevWeight, pairs: int, glu: str | None = None, alpha: float = 1.702, limit: float = 7.0, out: torch.Tensor | None = None,
+                by_pair: bool = False, pdl: bool = False) -> None:
+        """``glu``: the gate/up product, its activated rows stay here; else the down product of those into fp32 ``out``, by pair or by place."""
+        n = min(self.max_chunks, pairs)
+        a = MoeFp4Args(w.planes[0].data_ptr(), w.planes[1].data_ptr(), ptr(w.bias), w.n, w.k, ptr(self.x), ptr(self.chunks),
+                       ptr(self.pair_of_row) if by_pair else None, ptr(self.h if glu else out), 1 + _ACT[glu] if glu else 0, alpha, limit)
+        f = lib().b2_moe_fp4
+        f.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p]
+        _check(f(C.addressof(a), self.chunk, n, int(pdl), stream()), "moe_fp4")
+        if glu:
+            self._rows(self.h, 1, None, n * self.chunk, pdl)
 
 
 def gemm_bf16_glu(a: torch.Tensor, b: torch.Tensor, act: str, bias: torch.Tensor | None = None, alpha: float = 1.702, limit: float = 7.0,

@@ -730,6 +730,50 @@ def test_router(nb, n, k):
     assert out[:, n:].abs().max() == 0
 
 
+@pytest.mark.parametrize("E,d,ff,T,k,chunk", [(8, 256, 256, 1, 2, 8), (8, 96, 160, 37, 3, 16), (6, 288, 224, 100, 2, 64), (3, 2880, 2880, 70, 2, 32), (40, 64, 32, 9, 4, 8)])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_moe_fp4_products(E, d, ff, T, k, chunk, bf16):
+    """Pairs sorted by expert times MXFP4 experts (kernels/moe_fp4.cu): gate/up with activation, down, by pair and by place; rows of experts that live elsewhere, row lengths that fill a
+    128-column step partly, scales above 2 and of zero.  Bound: hidden rows
+    are rounded to bf16 (2^-9 of each term of a sum) and read to 2^-18 of a block's largest value, as the given ones are; weights are exact; as much again for fp32 sums and
+    the activation."""
+    from ollama_b200.models.weights import QWeight
+    K = _K()
+    gen = torch.Generator().manual_seed(d + T)
+
+    def blocks(n, kk):
+        e = torch.randint(117, 122, (E * n * kk // 32, 1), generator=gen)
+        e[0], e[-1] = 131, 0
+        return torch.cat([e.to(torch.uint8), torch.randint(0, 256, (E * n * kk // 32, 16), generator=gen).to(torch.uint8)], 1).view(-1)
+
+    qg, qd = QWeight("g", GGMLType.MXFP4, (E, 2 * ff, d), blocks(2 * ff, d)), QWeight("d", GGMLType.MXFP4, (E, d, ff), blocks(d, ff))
+    bg, bd = torch.randn(E * 2 * ff, generator=gen) * 0.1, torch.randn(E * d, generator=gen) * 0.1
+    gu, dn = K.repack(qg, "cuda", bias=bg), K.repack(qd, "cuda", bias=bd)
+    x = torch.randn(T, d, generator=gen)
+    x16 = x.to(torch.bfloat16)
+    lids = torch.stack([torch.randperm(E, generator=gen)[:k] for _ in range(T)]).to(torch.int32).view(-1)
+    lids[3::7] = -1
+    m = K.MoeFp4(T * k, E, d, ff, "cuda", chunk)
+    m.sort(lids.cuda(), T * k)
+    m.take((x16 if bf16 else x).cuda(), k, T * k)
+    m.product(gu, T * k, "swiglu_oai", 1.702, 7.0)
+    by_pair, by_place = torch.zeros(T * k, d, device="cuda"), torch.zeros(m.rows, d, device="cuda")
+    m.product(dn, T * k, out=by_pair, by_pair=True)
+    m.product(dn, T * k, out=by_place)
+    rows = m.row_of_pair.cpu()
+    assert torch.equal(rows < 0, lids < 0) and rows[rows >= 0].unique().numel() == int((lids >= 0).sum())
+    Wg, Wd = qg.dequant().double().view(E, 2 * ff, d), qd.dequant().double().view(E, d, ff)
+    for p in (lids >= 0).nonzero()[:, 0].tolist():
+        e = int(lids[p])
+        y = Wg[e] @ x16[p // k].double() + bg.view(E, -1)[e].double()
+        g, u = y[0::2].clamp(max=7.0), y[1::2].clamp(-7.0, 7.0)
+        h = g * torch.sigmoid(1.702 * g) * (u + 1.0)
+        ref = Wd[e] @ h + bd.view(E, -1)[e].double()
+        assert ((by_pair[p].cpu().double() - ref).abs() <= 2 ** -8 * (Wd[e].abs() @ (h.abs() + 0.05)) + 1e-5).all()      # 0.05: fp32 sums of up to 500 where up is near -1
+        assert torch.equal(by_place[rows[p]], by_pair[p])
+    assert torch.equal(by_pair[(lids < 0).cuda()], torch.zeros_like(by_pair[(lids < 0).cuda()]))
+
+
 @pytest.mark.parametrize("m,n,k", [(129, 64, 64), (257, 304, 520), (300, 192, 72), (1153, 5584, 1032), (769, 5408, 2056)])
 @pytest.mark.parametrize("pdl", [0, 2])
 def test_gemm_bf16_shapes(m, n, k, pdl):
