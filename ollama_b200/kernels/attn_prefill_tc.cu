@@ -628,7 +628,7 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
         const int qp = q_lo + (DIFF ? r & 63 : r);
         const int row_lo = first_key(qp, chunk, window), last_lo = first_key(q_hi, chunk, window);      // this row's first key (but for kept ones); the last row's
         const float LOG2E = 1.4426950408889634f;
-        const float sl2 = a.scale * LOG2E;
+        const float mult = a.softcap > 0.f ? 1.f : a.scale * LOG2E;      // scores times this are exponents of two; the running maximum is one of plain scores
         const uint32_t lane_base = (uint32_t)(32 * q) << 16;
         float o[OH];
 #pragma unroll
@@ -644,7 +644,11 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
                 uint32_t ov[32];
                 tmem_ld32(tmem + lane_base + (uint32_t)(256 + 128 * b + OH * c + j0), ov);
 #pragma unroll
-                for (int j = 0; j < 32; j++) o[j0 + j] = o[j0 + j] * corr + __uint_as_float(ov[j]);
+                for (int j = 0; j < 32; j += 2) {
+                    const float2 y = fma2(make_float2(o[j0 + j], o[j0 + j + 1]), make_float2(corr, corr), make_float2(__uint_as_float(ov[j]), __uint_as_float(ov[j + 1])));
+                    o[j0 + j] = y.x;
+                    o[j0 + j + 1] = y.y;
+                }
             }
             tc_fence_before();
         };
@@ -664,11 +668,6 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
                 for (int i = 0; i < 2; i++)
 #pragma unroll
                     for (int j = 0; j < 32; j++) v[i][j] = __float_as_uint(cap2 * tanh_exp(__uint_as_float(v[i][j]) * inv_cap));
-            } else {
-#pragma unroll
-                for (int i = 0; i < 2; i++)
-#pragma unroll
-                    for (int j = 0; j < 32; j++) v[i][j] = __float_as_uint(__uint_as_float(v[i][j]) * sl2);
             }
             if (masked) {
                 const int kp0 = n0 + 64 * c;
@@ -691,21 +690,23 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
             if (!mbar_wait(&pair[q], t & 1)) { ok = false; break; }
             mx = fmaxf(mx, x_max[(c ^ 1) * 128 + r]);
             const float m_new = fmaxf(m_run, mx);
-            const float corr = m_new == -INFINITY ? 1.f : ex2(m_run - m_new);
-            const float mref = m_new == -INFINITY ? 0.f : m_new;
+            const float corr = m_new == -INFINITY ? 1.f : ex2((m_run - m_new) * mult);
+            const float mref = m_new == -INFINITY ? 0.f : m_new * mult;
             m_run = m_new;
-            float ls = 0.f;
+            const float2 mult2 = make_float2(mult, mult), less = make_float2(-mref, -mref);
+            float2 ls2 = make_float2(0.f, 0.f);
             uint32_t pw[32];
 #pragma unroll
             for (int i = 0; i < 2; i++)
 #pragma unroll
                 for (int j = 0; j < 32; j += 2) {
-                    const float p0 = ex2(__uint_as_float(v[i][j]) - mref), p1 = ex2(__uint_as_float(v[i][j + 1]) - mref);
-                    ls += p0 + p1;
-                    pw[16 * i + (j >> 1)] = pack_h2(p0, p1);
+                    const float2 e = fma2(make_float2(__uint_as_float(v[i][j]), __uint_as_float(v[i][j + 1])), mult2, less);
+                    const float2 pr = make_float2(ex2(e.x), ex2(e.y));
+                    ls2 = add2(ls2, pr);
+                    pw[16 * i + (j >> 1)] = pack_h2(pr.x, pr.y);
                 }
             tmem_st32(tmem + lane_base + (uint32_t)(128 * b + 32 * c), pw);      // both warps of the quarter have read all of S(t) by now
-            l_run = l_run * corr + ls;
+            l_run = l_run * corr + (ls2.x + ls2.y);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&p_ready[b]);
@@ -770,8 +771,8 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
             float oc = 1.f;
             if (a.sinks) {
                 const float sk = a.sinks[h] * LOG2E;
-                const float m_new = fmaxf(m_run, sk);
-                oc = m_run == -INFINITY ? 0.f : ex2(m_run - m_new);
+                const float m = m_run * mult, m_new = fmaxf(m, sk);
+                oc = m_run == -INFINITY ? 0.f : ex2(m - m_new);
                 l = l * oc + ex2(sk - m_new);
             }
             const float inv = l > 0.f ? oc / l : 0.f;
