@@ -479,6 +479,8 @@ int dispatch(const void* a, const void* b, const GemmParams& p, cudaStream_t st,
 // Parts of a split product, added in order; bias, activation, factors, accumulation and output type of the whole.
 __global__ void __launch_bounds__(256) gemm_parts_kernel(const __grid_constant__ GemmParams p) {
     const int row = blockIdx.y, col = 4 * (blockIdx.x * 256 + threadIdx.x);
+    pdl_launch();
+    pdl_wait();
     if (col >= p.n) return;
     float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int s = 0; s < p.splits; s++) {
@@ -511,6 +513,39 @@ int split_count(int m, int n, int k) {
     return (int)(s > 16 ? 16 : s);
 }
 
+// Parts of the row length, and their tile width, for a product of more than 128 rows that one round of whole tiles leaves long: where the rounds of parts, their sums through
+// memory (about 3400 bytes a cycle) and the launch that adds them take a tenth less than the product in one piece.
+// 331 x 2048 x 5504: 31.6 -> 18.4 us; 512 x 4096 x 14336: 75 -> 61.5 us.
+int long_splits(int m, int n, int k, int& width) {
+    if (m <= BM || n < 128) return 1;
+    GemmParams p = {};
+    p.m = m;
+    p.n = n;
+    p.k = k;
+    double best = 0;
+    for (int bn : {256, 192, 128, 64})
+        for (int pair = 0; pair < 2; pair++) {
+            if (n < bn || (pair && bn < 192)) continue;
+            const double c = tile_cycles(p, bn, pair);
+            if (best == 0 || c < best) best = c;
+        }
+    best *= 0.9;
+    int splits = 1;
+    const long blocks = (k + BK - 1) / BK, tiles_m = (m + BM - 1) / BM;
+    for (int bn : {256, 128}) {
+        const long tiles = tiles_m * ((n + bn - 1) / bn);
+        for (int s = 2; n >= bn && s <= 8 && s * 8 <= blocks; s++) {
+            const double c = (double)((tiles * s + sm_count() - 1) / sm_count()) * ((blocks + s - 1) / s) * (80 + 128 * (BM + bn) / 61) + 8.0 * s * m * n / 3400 + 5000;
+            if (c < best) {
+                best = c;
+                splits = s;
+                width = bn;
+            }
+        }
+    }
+    return splits;
+}
+
 bool bad_operands(const void* a, const void* b, int m, int n, int k, int ldo) {
     return m < 1 || n < 1 || k < 8 || (k & 7) || (n & 3) || (ldo & 3) || ((uintptr_t)a & 15) || ((uintptr_t)b & 15);
 }
@@ -518,13 +553,32 @@ bool bad_operands(const void* a, const void* b, int m, int n, int k, int ldo) {
 }  // namespace
 
 // out[m][n] (+)= a[m][k] . b[n][k]^T + bias[n];  a, b bf16 row-major with k % 8 == 0 and 16-byte aligned bases,
-// out fp32 with ldo % 4 == 0, n % 4 == 0.  Returns a cudaError_t value.
-B2_API int b2_gemm_bf16(const void* a, const void* b, int m, int n, int k, float* out, int ldo, const float* bias, int accumulate, int pdl,
-                        cudaStream_t st) {
+// out fp32 with ldo % 4 == 0, n % 4 == 0.  With scratch (b2_gemm_bf16_scratch floats, 16-byte aligned) long products of few tiles are split along k.  Returns a cudaError_t value.
+B2_API int b2_gemm_bf16(const void* a, const void* b, int m, int n, int k, float* out, int ldo, const float* bias, int accumulate, int pdl, float* ws,
+                        long long ws_floats, cudaStream_t st) {
     if (bad_operands(a, b, m, n, k, ldo) || ((uintptr_t)out & 15)) return (int)cudaErrorInvalidValue;
     GemmParams p{m, n, k, out, ldo, bias, accumulate, 0, {}, 0, nullptr, 0, 0.f, 0.f};
     p.pdl = pdl;
+    int width = 0;
+    const int splits = ws && !((uintptr_t)ws & 15) && !((uintptr_t)bias & 15) ? long_splits(m, n, k, width) : 1;
+    if (splits > 1 && (long long)splits * m * n <= ws_floats && m <= 65535) {
+        p.splits = splits;
+        p.part = ws;
+        p.part_ld = n;
+        p.part_stride = (long long)m * n;
+        const int rc = width == 256 ? launch<256, true>(a, b, p, st) : launch<128, true>(a, b, p, st);
+        if (rc) return rc;
+        void* args[] = {&p};
+        return launch_rows((const void*)gemm_parts_kernel, dim3((n + 1023) / 1024, m), dim3(256), 0, args, st, pdl ? 1 : 0);
+    }
     return dispatch(a, b, p, st);
+}
+
+// Floats of scratch with which b2_gemm_bf16 would split a product of this size (0: it would not).
+B2_API long long b2_gemm_bf16_scratch(int m, int n, int k) {
+    int width = 0;
+    const int s = long_splits(m, n, k, width);
+    return s > 1 ? (long long)s * m * n : 0;
 }
 
 // Same product with a bf16 result (n % 8 == 0, ldo % 8 == 0); no accumulation.

@@ -7,6 +7,7 @@ library cannot be loaded this module raises: there is no silent fallback on a GP
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import os
 from dataclasses import dataclass, field
 
@@ -463,6 +464,14 @@ def attn_decode_rope(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
     return out
 
 
+@functools.lru_cache(maxsize=4096)
+def gemm_bf16_scratch(m: int, n: int, k: int) -> int:
+    """Floats of scratch with which the tcgen05 product of this size is split along k (0: it is not)."""
+    f = lib().b2_gemm_bf16_scratch
+    f.restype, f.argtypes = C.c_longlong, [C.c_int, C.c_int, C.c_int]
+    return int(f(m, n, k))
+
+
 def gemm_bf16(a: torch.Tensor, b: torch.Tensor, bias: torch.Tensor | None = None, out: torch.Tensor | None = None,
               accumulate: bool = False, pdl: int = 0) -> torch.Tensor:
     """out[m, n] (+)= a[m, k] @ b[n, k]^T + bias on the tcgen05 tensor-core kernel (bf16 operands, fp32 result).  ``pdl``: 1 the launch may begin while the kernel before it ends, 2 and ``b`` does not depend on that kernel."""
@@ -473,9 +482,11 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, bias: torch.Tensor | None = None
     a, b = a.contiguous(), b.contiguous()
     if out is None:
         out = torch.empty(m, n, device=a.device, dtype=torch.float32)
+    size = gemm_bf16_scratch(m, n, k)
+    ws = torch.empty(size, device=a.device, dtype=torch.float32) if size else None
     f = lib().b2_gemm_bf16
-    f.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_int, C.c_void_p]
-    _check(f(ptr(a), ptr(b), m, n, k, ptr(out), out.stride(0), ptr(bias), int(accumulate), pdl, stream()), "gemm_bf16")
+    f.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_longlong, C.c_void_p]
+    _check(f(ptr(a), ptr(b), m, n, k, ptr(out), out.stride(0), ptr(bias), int(accumulate), pdl, ptr(ws), size, stream()), "gemm_bf16")
     return out
 
 
