@@ -31,6 +31,7 @@ from ..models.weights import QWeight, load_tensor
 from ..ops import cuda as K
 from ..ops import reference as R
 from ..ops import sk as SK
+from ..ops.prompt import PromptPass
 from .steps import StepEngine
 
 MAX_DECODE_BATCH = 8             # sequences per launch of the dp4a kernels (kernels/gemv.cu)
@@ -38,6 +39,9 @@ MAX_STREAM_BATCH = 32            # sequences per step when every matrix runs on 
 # Steps of more sequences than this multiply f16 activations (kernels/gemm_sk.cu) instead of int8 ones: a layer of Llama-8B takes 64 us of products against 70 at eight
 # sequences and 108 against 78 at thirteen.
 INT8_ROWS = 8
+# Prompt passes of at most this many rows read the units too, 32 rows a launch, instead of the 16-bit copies: a layer of Llama-8B is 124 MB against 436 (70 us of products
+# against 200 up to eight rows, 105 for every 32).
+UNIT_ROWS = 64
 # Steps of at least so many (token, expert) pairs, and of one for every eighth expert, read MXFP4 experts once for all rows that chose them (kernels/moe_fp4.cu), smaller ones
 # once per pair: a layer of 128 experts of 13 MB, four a token, takes 72 us against 75 at four tokens and 194 against 280 at sixteen, but 45 against 29 at one.
 FP4_MIN_PAIRS = 16
@@ -328,13 +332,16 @@ class B200Backend(StepEngine):
         b.host_in = torch.zeros(3, MB, dtype=i32).pin_memory()
         b.host_out = torch.zeros(MB, dtype=i32).pin_memory()
         b.host_np, b.host_out_np = b.host_in.numpy(), b.host_out.numpy()
+        # dense layers of a prompt are launched from native code (kernels/prefill_pass.cu)
+        plain = type(self) is B200Backend and self.prefill_gemm == "bf16" and not c.sandwich_norm and c.head_dim in K.ATTN_PREFILL_HEAD_DIMS
+        self._pass = PromptPass(self) if plain and not any(L.moe for L in self.layers) else None
         self._graphs.clear()
         self._warm.clear()
 
     def close(self) -> None:
         self._graphs.clear()
         self.k_cache = self.v_cache = self.k_scale = self.v_scale = []
-        self.buf = None
+        self.buf = self._pass = None
 
     # -- decode ---------------------------------------------------------------------------------------
     def _norm_quant(self, x, w, nb, k, *, do_norm=True, residual=None, src=None):
@@ -513,13 +520,13 @@ class B200Backend(StepEngine):
         SK.gemv(ws, xin, norm_w=norm_w, eps=c.norm_eps, out=out, mode=mode, act=c.act, alpha=c.swiglu_alpha, limit=c.swiglu_limit, pdl=self.pdl)
         self._n += 1
 
-    def _rows_sk(self, ws, x: torch.Tensor, out: torch.Tensor, norm_w=None, mode: int = SK.MODE_STORE, buf: torch.Tensor | None = None) -> None:
+    def _rows_sk(self, ws, x: torch.Tensor, out: torch.Tensor, norm_w=None, mode: int = SK.MODE_STORE, buf: torch.Tensor | None = None, wsp=None) -> None:
         """Rows times unit-ordered matrices in f16 activations, 32 rows a launch: ``out`` stored / added to / gated."""
         c = self.cfg
         for r in range(0, x.shape[0], SK.MAX_TOKENS):
             xs = x[r:r + SK.MAX_TOKENS]
             x16 = SK.rows16(xs, norm_w, c.norm_eps, out=buf, pdl=self.pdl)
-            SK.gemm16(ws, x16, xs.shape[0], out=out[r:], mode=mode, act=c.act, alpha=c.swiglu_alpha, limit=c.swiglu_limit, pdl=self.pdl)
+            SK.gemm16(ws, x16, xs.shape[0], out=out[r:], mode=mode, act=c.act, alpha=c.swiglu_alpha, limit=c.swiglu_limit, pdl=self.pdl, ws=wsp)
 
     def _decode_layer_sk(self, i: int, L, nb: int) -> None:
         """A layer on the streaming GEMV: both RMSNorms, both residual adds, the gated activation and every activation
@@ -714,6 +721,11 @@ class B200Backend(StepEngine):
             x = K.embed(self.embd, ids, c.embed_scale)
             if embeds is not None and len(embeds[0]):      # image rows: projected features, not scaled like token embeddings
                 x[torch.as_tensor(list(embeds[0]), device=dev)] = embeds[1].to(dev, x.dtype)
+        units = self._unit_rows(T) and self._pass is not None and self._pass.units
+        mode = os.environ.get("B200_ATTN_PREFILL", K.ATTN_PREFILL_DEFAULT)
+        if self._pass is not None and (self._pass.units if units else self._pass.wide) and not spans and mode in ("auto", "mma") and x.is_contiguous() and x.dtype == torch.float32:
+            self.kernel_launches += self._pass.run(self, x, pos, slots, [(r0, r1 - r0, sl, p0) for r0, r1, sl, p0 in bounds], units, mode == "auto")
+            return x
         for i, L in enumerate(self.layers):
             h = K.rmsnorm_bf16(x, L.attn_norm, c.norm_eps, pdl=self.pdl)
             qkv = torch.empty(T, (c.n_heads + 2 * c.n_kv_heads) * c.head_dim, device=dev, dtype=torch.float32)
@@ -752,7 +764,16 @@ class B200Backend(StepEngine):
     def _final_norm(self, x: torch.Tensor) -> torch.Tensor:
         return R.rmsnorm(x, self.out_norm, self.cfg.norm_eps)
 
+    def _unit_rows(self, rows: int) -> bool:
+        """True when a prompt pass of so many rows multiplies with the unit-ordered matrices (the widest rows have to fit the normalising pass)."""
+        return 0 < rows <= UNIT_ROWS and self.prefill_gemm == "bf16" and self.cfg.d_model <= SK.ROWS16_MAX_NORM
+
     def _logits(self, x: torch.Tensor) -> torch.Tensor:
+        if self._unit_rows(x.shape[0]) and getattr(self, "sk_head", None) is not None:
+            out = torch.empty(x.shape[0], self.cfg.vocab_size, device=self.device, dtype=torch.float32)
+            self._rows_sk([self.sk_head], x.contiguous(), out, self.out_norm, wsp=self._pass.ws if self._pass is not None else None)
+            self.kernel_launches += 2 * ((x.shape[0] + SK.MAX_TOKENS - 1) // SK.MAX_TOKENS)
+            return R.softcap(out, self.cfg.final_softcap)
         return R.softcap(self._mm(self._final_norm(x).to(torch.bfloat16), self.head), self.cfg.final_softcap)
 
     @torch.no_grad()

@@ -187,16 +187,14 @@ class PipelineBackend:
             return None
         last = self.stages[-1]
         with torch.cuda.device(last.device):
-            h = R.rmsnorm(x[-1:], last.out_norm, self.cfg.norm_eps).to(torch.bfloat16)
-            return R.softcap(last._mm(h, last.head)[0], self.cfg.final_softcap)
+            return last._logits(x[-1:])[0]
 
     @torch.no_grad()
     def verify(self, slot: int, tokens: Sequence[int], pos0: int) -> torch.Tensor:
         x = self._chunk(slot, tokens, pos0)
         last = self.stages[-1]
         with torch.cuda.device(last.device):
-            h = R.rmsnorm(x, last.out_norm, self.cfg.norm_eps).to(torch.bfloat16)
-            return R.softcap(last._mm(h, last.head), self.cfg.final_softcap)
+            return last._logits(x)
 
     @torch.no_grad()
     def hidden(self, slot: int, tokens: Sequence[int]) -> torch.Tensor:

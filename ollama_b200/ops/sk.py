@@ -195,7 +195,7 @@ def unit_weights(w: SkWeight) -> torch.Tensor:
 
 
 class Workspace:
-    """Hand-over buffers of split tiles and the status word, one set per device (launches of one stream share it)."""
+    """Hand-over buffers of split tiles and the status word, one set per device (launches of one stream share it; prompt passes have their own)."""
 
     def __init__(self, device):
         rows = int(K.lib().b2_gemv_sk_max_groups())
@@ -307,12 +307,12 @@ def rows16(x: torch.Tensor, norm_w: torch.Tensor | None = None, eps: float = 0.0
 
 
 def gemm16(weights: list[SkWeight], x: torch.Tensor, nb: int, *, out: torch.Tensor | None = None, mode: int = MODE_STORE, act: str = "silu", alpha: float = 1.702,
-           limit: float = 7.0, max_ctas: int = 0, pdl: bool = False) -> torch.Tensor:
+           limit: float = 7.0, max_ctas: int = 0, pdl: bool = False, ws: Workspace | None = None) -> torch.Tensor:
     """y[b] = concat_i(W_i x[b] + bias_i) of 1..32 rows in the chunks of :func:`rows16`; modes and results as in :func:`gemv`, activations in 16 bits."""
     dev, total = weights[0].units.device, sum(w.n for w in weights)
     if out is None:
         out = torch.empty(nb, total // 2 if mode == MODE_GLU else total, device=dev, dtype=torch.float32)
-    a, ws, off = SgArgs(), workspace(dev), 0
+    a, ws, off = SgArgs(), ws or workspace(dev), 0
     for i, w in enumerate(weights):
         s = a.seg[i]
         s.w, s.bias, s.type, s.n, s.out_off = w.units.data_ptr(), K.ptr(w.bias), w.wtype, w.n, off

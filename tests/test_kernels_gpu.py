@@ -694,6 +694,35 @@ def test_engine_prefill_gemm_modes(tmp_path, mode, keep):
     assert K_status_ok()
 
 
+@pytest.mark.parametrize("name,ft,kv", [("tiny-qwen3", "Q4_K_M", "f16"), ("tiny-qwen3", "Q4_K_M", "q8_0"), ("tiny-qwen2", "BF16", "f16")])
+@pytest.mark.parametrize("rows", [1, 33, 64, 65])
+def test_engine_prompt_pass_row_counts(tmp_path, name, ft, kv, rows):
+    """Prompt passes launched from native code, on both sides of the row count up to which they read the unit-ordered matrices: every row's logits, a second chunk, and chunks of two
+    sequences in one pass, against the fp32 graph (the bound of the other whole-model tests: 5 % of the largest logit)."""
+    from ollama_b200.engine.b200 import B200Backend
+    from ollama_b200.engine.backend import TorchBackend, open_model
+    from ollama_b200.models.synth import write_synthetic_gguf
+    p = str(tmp_path / "m.gguf")
+    write_synthetic_gguf(p, name, ft)
+    g = open_model(p)
+    ref, eng = TorchBackend(g, "cpu"), B200Backend(g, "cuda", keep_bf16=True, kv_type=kv)
+    ref.alloc(2, 256)
+    eng.alloc(2, 256)
+    assert eng._pass is not None and eng._pass.wide and eng._pass.units == (ft == "Q4_K_M")
+    prompt = torch.randint(259, 4096, (2 * rows,), generator=torch.Generator().manual_seed(rows)).tolist()
+
+    def close(a, b):
+        assert (a.cpu() - b).abs().max().item() < 0.05 * b.abs().max().item()
+
+    close(eng.verify(0, prompt[:rows], 0), ref.verify(0, prompt[:rows], 0))
+    close(eng.prefill(0, prompt[rows:], rows), ref.prefill(0, prompt[rows:], rows))
+    segs = [(0, prompt[:rows], 0), (1, prompt[rows:rows + (rows + 1) // 2], 0)]
+    for a, b in zip(eng.prefill_many(segs, [True, True]), ref.prefill_many(segs, [True, True])):
+        close(a, b)
+    assert K_status_ok()
+    eng.close()
+
+
 @pytest.mark.parametrize("stream_q", ["1", "0"])
 def test_engine_moe_prefill_on_mxfp4_experts(tmp_path, monkeypatch, stream_q):
     """gpt-oss prefill without a resident 16-bit copy of the experts: the grouped kernel that streams the MXFP4 blocks (and, with
