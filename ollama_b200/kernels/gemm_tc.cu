@@ -444,7 +444,7 @@ double tile_cycles(const GemmParams& p, int bn, bool pair) {
 
 template <bool TAIL = false, bool XIELU = false>
 int dispatch(const void* a, const void* b, const GemmParams& p, cudaStream_t st, int b_rows = 0) {
-    if (!TAIL && !XIELU && p.m > BM && p.n >= 64 && p.splits <= 1 && !p.tile_expert && p.cm.n_dst == 0 && !b_rows) {
+    if (!TAIL && !XIELU && p.m > 32 && p.n >= 64 && p.splits <= 1 && !p.tile_expert && p.cm.n_dst == 0 && !b_rows) {
         // the form and width with the fewest cycles, at equal ones the wider tile
         double best = 0;
         int width = 0;
@@ -513,11 +513,12 @@ int split_count(int m, int n, int k) {
     return (int)(s > 16 ? 16 : s);
 }
 
-// Parts of the row length, and their tile width, for a product of more than 128 rows that one round of whole tiles leaves long: where the rounds of parts, their sums through
+// Parts of the row length, and their tile width, for a product that one round of whole tiles leaves long: where the rounds of parts, their sums through
 // memory (about 3400 bytes a cycle) and the launch that adds them take a tenth less than the product in one piece.
-// 331 x 2048 x 5504: 31.6 -> 18.4 us; 512 x 4096 x 14336: 75 -> 61.5 us.
+// 331 x 2048 x 5504: 31.6 -> 18.4 us; 512 x 4096 x 14336: 75 -> 61.5 us; 100 x 4096 x 14336: 72 -> 36 us;
+// 16 x 2880 x 4096: 22.5 -> 12.1 us.
 int long_splits(int m, int n, int k, int& width) {
-    if (m <= BM || n < 128) return 1;
+    if (n < 128) return 1;
     GemmParams p = {};
     p.m = m;
     p.n = n;

@@ -803,11 +803,11 @@ def test_moe_fp4_products(E, d, ff, T, k, chunk, bf16):
     assert torch.equal(by_pair[(lids < 0).cuda()], torch.zeros_like(by_pair[(lids < 0).cuda()]))
 
 
-@pytest.mark.parametrize("m,n,k", [(129, 64, 64), (257, 304, 520), (300, 192, 72), (1153, 5584, 1032), (769, 5408, 2056), (300, 1032, 5512), (512, 4096, 9000)])
+@pytest.mark.parametrize("m,n,k", [(129, 64, 64), (257, 304, 520), (300, 192, 72), (1153, 5584, 1032), (769, 5408, 2056), (300, 1032, 5512), (512, 4096, 9000), (16, 5120, 2888), (100, 1032, 4104)])
 @pytest.mark.parametrize("pdl", [0, 2])
 def test_gemm_bf16_shapes(m, n, k, pdl):
-    """Products of more than 128 rows in the form and width that the estimate picks (1153, 769: CTA pairs, 256 and 192 columns;
-    the last two: split along k), ragged in every direction, all outputs.
+    """Products in the form and width that the estimate picks (1153, 769: CTA pairs, 256 and 192 columns;
+    the last four: split along k), ragged in every direction, all outputs.
     Exact products of bf16 values, fp32 sums: k 2^-24 of the sum of magnitudes; 16-bit results one rounding more."""
     K = _K()
     gen = torch.Generator().manual_seed(m + n)
