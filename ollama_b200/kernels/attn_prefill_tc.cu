@@ -628,7 +628,11 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
         const int qp = q_lo + (DIFF ? r & 63 : r);
         const int row_lo = first_key(qp, chunk, window), last_lo = first_key(q_hi, chunk, window);      // this row's first key (but for kept ones); the last row's
         const float LOG2E = 1.4426950408889634f;
-        const float mult = a.softcap > 0.f ? 1.f : a.scale * LOG2E;      // scores times this are exponents of two; the running maximum is one of plain scores
+        // Scores times `mult` are exponents of two; the running maximum is one of plain scores, which takes a scale above zero (the largest score is the largest exponent, a masked
+        // score of minus infinity stays one).  Other scales are multiplied in ahead of mask and maximum.
+        const float sl2 = a.scale * LOG2E;
+        const bool ahead = !(a.softcap > 0.f) && !(sl2 > 0.f);
+        const float mult = a.softcap > 0.f || ahead ? 1.f : sl2;
         const uint32_t lane_base = (uint32_t)(32 * q) << 16;
         float o[OH];
 #pragma unroll
@@ -668,6 +672,11 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
                 for (int i = 0; i < 2; i++)
 #pragma unroll
                     for (int j = 0; j < 32; j++) v[i][j] = __float_as_uint(cap2 * tanh_exp(__uint_as_float(v[i][j]) * inv_cap));
+            } else if (ahead) {
+#pragma unroll
+                for (int i = 0; i < 2; i++)
+#pragma unroll
+                    for (int j = 0; j < 32; j++) v[i][j] = __float_as_uint(__uint_as_float(v[i][j]) * sl2);
             }
             if (masked) {
                 const int kp0 = n0 + 64 * c;

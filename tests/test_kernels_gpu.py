@@ -396,6 +396,25 @@ def test_attn_prefill_on_tcgen05(hd, H, Hkv, T, pos0, window, softcap, use_sinks
     assert torch.allclose(out, ref, atol=1e-2, rtol=2e-2), (out - ref).abs().max()
 
 
+@pytest.mark.parametrize("scale", [-0.1, 0.0])
+@pytest.mark.parametrize("hd,T,pos0,window,use_sinks", [(128, 300, 517, 0, False), (64, 129, 0, 48, True), (128, 5, 0, 0, False)])
+def test_attn_prefill_of_any_scale(hd, T, pos0, window, use_sinks, scale):
+    """A scale of zero gives every visible key the same weight and a negative one the smallest score the largest, with masked keys in whole and in parts of tiles.  Bound as in the
+    test above: operands and probabilities are f16."""
+    K = _K()
+    n_slots, n_ctx, slot, H, Hkv = 2, 1024, 1, 4, 2
+    g = torch.Generator().manual_seed(hd + T)
+    kc, vc = ((torch.randn(n_slots, Hkv, n_ctx, hd, generator=g) * 0.7).to(torch.float16).cuda() for _ in range(2))
+    q = torch.randn(T, H, hd, generator=g).cuda()
+    sinks = torch.randn(H, generator=g).cuda() if use_sinks else None
+    p_end = pos0 + T
+    out = K.attn_prefill(q, kc, vc, slot, pos0, p_end, scale, True, window, 0.0, sinks, mode="tc").float().cpu().view(T, H, hd)
+    ref = R.attention(q.to(torch.float16).float().cpu(), kc[slot, :, :p_end].transpose(0, 1).float().cpu(), vc[slot, :, :p_end].transpose(0, 1).float().cpu(),
+                      torch.arange(pos0, p_end), torch.arange(p_end), scale=scale, causal=True, window=window, sinks=sinks.cpu() if use_sinks else None)
+    assert torch.allclose(out, ref, atol=1e-2, rtol=2e-2), (out - ref).abs().max()
+    assert K.attn_prefill_tc_status(clear=True) == 0
+
+
 @pytest.fixture
 def attn_mode():
     """Selects the decode-attention kernel for one test and restores the automatic choice afterwards."""

@@ -210,6 +210,17 @@ def test_paged_decode_attention(shape, splits):
         at = p + 1
 
 
+@pytest.mark.parametrize("scale", [-0.1, 0.0])
+@pytest.mark.parametrize("chunk", [0, 33])
+def test_paged_attention_of_any_scale(chunk, scale):
+    """Scales of zero and below, which a configuration may name, in prompts and in steps; tolerances as above."""
+    a = Attn(4, 2, 64, 64, chunk, 290, n_rot=32, seed=2)
+    a.scale = scale
+    want = a.expected()
+    close(a.rows(0, 290), want, 8e-3)
+    close(a.decode(289, 3)[0], want[289], 3e-3)
+
+
 @pytest.mark.parametrize("kind", ["tc", "f16", "f32"])
 @pytest.mark.parametrize("chunk", [0, 96, 128, 160])
 def test_a_single_key_stands_out_near_edges_and_far_away(chunk, kind):
