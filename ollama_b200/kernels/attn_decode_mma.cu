@@ -493,15 +493,20 @@ int launch_d(const AttnDecodeArgs& a, const AttnRopeArgs& r, int nb, int pdl, cu
 
 }  // namespace
 
+// 1 if the tensor-core kernel takes caches like these, 0 if the scalar one has to (nothing is launched).  A row's int8 scales are fetched at once, hd / 16 bytes of them.
+B2_API int b2_attn_decode_mma_takes(const AttnDecodeArgs* a, int hd) {
+    if (hd != 64 && hd != 128) return 0;
+    if (a->n_kv_heads < 1 || a->n_heads % a->n_kv_heads || a->n_heads / a->n_kv_heads > ROWS) return 0;
+    return !a->k_scale || !(((uintptr_t)a->k_scale | (uintptr_t)a->v_scale) & (hd / 16 - 1));
+}
+
 int attn_decode_mma_rope_launch(const AttnDecodeArgs& a, const AttnRopeArgs& r, int nb, int hd, int pdl, cudaStream_t st) {
-    if (a.n_kv_heads < 1 || a.n_heads % a.n_kv_heads || a.n_heads / a.n_kv_heads > ROWS) return (int)cudaErrorNotSupported;
+    if (!b2_attn_decode_mma_takes(&a, hd)) return (int)cudaErrorNotSupported;
     if (r.qkv && (a.k_scale || a.v_scale || r.n_rot > 256 || r.n_rot > hd || (r.n_rot & 1) || (a.page_table ? r.n_rot && !r.freqs : !r.inv_freq))) return (int)cudaErrorNotSupported;
     if (a.page_table && (r.maps < 1 || r.maps > 2 || a.n_heads / a.n_kv_heads % r.maps || (r.maps > 1 && r.q_norm) || (r.no_append && r.q_norm))) return (int)cudaErrorInvalidValue;
     if (a.page_table && (!r.qkv || !r.neox || r.dim < 1 || r.maps * r.dim > hd || r.vdim < 1 || r.vdim > hd || r.n_rot > r.dim || a.max_pages < 1 || a.window < 0 || a.keep < 0 || r.v_off < 0 ||
                          (!r.no_append && r.v_off + a.n_kv_heads * r.vdim > r.ldq))) return (int)cudaErrorInvalidValue;
-    if (hd == 128) return launch_d<128>(a, r, nb, pdl, st);
-    if (hd == 64) return launch_d<64>(a, r, nb, pdl, st);
-    return (int)cudaErrorNotSupported;
+    return hd == 128 ? launch_d<128>(a, r, nb, pdl, st) : launch_d<64>(a, r, nb, pdl, st);
 }
 
 // Pipeline depth of the tensor-core decode kernel: 0 = chosen per launch (default), 2, 3 or 4 = forced.  Returns the previous setting.

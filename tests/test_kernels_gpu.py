@@ -331,6 +331,30 @@ def test_attn_decode_tensor_core_long_context(hd, H, Hkv, q8, attn_mode):
         assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
 
 
+@pytest.mark.parametrize("hd,off", [(128, 1), (128, 2), (64, 1)])
+def test_attn_decode_with_scales_off_their_alignment(hd, off, attn_mode):
+    """int8 caches whose scale arrays begin ``off`` f16 values off the alignment that the ring's copies need: the scalar kernel takes them, with the bits that it gives for aligned ones."""
+    K = _K()
+    n_slots, n_ctx, H, Hkv = 2, 192, 8, 2
+    g = torch.Generator().manual_seed(hd + off)
+    kc, vc = (torch.randint(-127, 128, (n_slots, Hkv, n_ctx, hd), generator=g, dtype=torch.int8).cuda() for _ in range(2))
+    ks, vs = (torch.rand(n_slots, Hkv, n_ctx, hd // 32, generator=g).to(torch.float16).cuda() * 0.01 for _ in range(2))
+    q = torch.randn(2, H, hd, generator=g).cuda()
+    pos, slots = torch.tensor([150, 33], dtype=torch.int32).cuda(), torch.tensor([1, 0], dtype=torch.int32).cuda()
+
+    def shifted(t):
+        flat = torch.zeros(t.numel() + 8, device="cuda", dtype=t.dtype)
+        flat[off:off + t.numel()] = t.flatten()
+        return flat[off:off + t.numel()].view(t.shape)
+
+    attn_mode(0)
+    ref, _ = K.attn_decode(q, kc, vc, pos, slots, scale=hd ** -0.5, n_splits=3, k_scale=ks, v_scale=vs)
+    attn_mode(1)
+    for a, b in ((shifted(ks), shifted(vs)), (ks, shifted(vs))):
+        got, _ = K.attn_decode(q, kc, vc, pos, slots, scale=hd ** -0.5, n_splits=3, k_scale=a, v_scale=b)
+        assert torch.equal(got, ref)
+
+
 def test_embed_and_argmax():
     K = _K()
     qw, _ = _weight(GGMLType.Q6_K, 300, 512)
