@@ -507,7 +507,7 @@ class B200Backend(StepEngine):
         c, b = self.cfg, self.buf
         k = ws[0].k
         xin = x[:nb, :k]
-        if nb > INT8_ROWS:
+        if nb > INT8_ROWS and (norm_w is None or k <= SK.ROWS16_MAX_NORM):      # longer rows that are normalised first stay int8
             self._rows_sk(ws, xin, out[:nb], norm_w, mode, b.x16)
             self._n += 2
             return

@@ -229,3 +229,24 @@ def test_gemm16_glu_matches_reference():
     ref = torch.nn.functional.silu(y[:, 0::2]) * y[:, 1::2]
     got = sk.gemm16([w], sk.rows16(x), 19, mode=sk.MODE_GLU)
     assert (got.double() - ref).norm() < 2 ** -9 * ref.norm()
+
+
+def test_steps_of_models_wider_than_the_normalising_pass():
+    """Rows longer than ROWS16_MAX_NORM that are normalised on the way stay in the int8 form at any number of sequences (nine: the first that the 16-bit form takes)."""
+    from types import SimpleNamespace
+
+    from ollama_b200.engine.b200 import INT8_ROWS, B200Backend
+    _, sk = _mods()
+    k, nb = sk.ROWS16_MAX_NORM + 256, INT8_ROWS + 1
+    gen = torch.Generator().manual_seed(1)
+    q = _qw(GGMLType.Q4_K, 32, k, 2)
+    x, nw = torch.randn(nb, k, generator=gen), torch.rand(k, generator=gen) + 0.5
+    dev = dict(device="cuda")
+    be = SimpleNamespace(cfg=SimpleNamespace(norm_eps=1e-5, act="silu", swiglu_alpha=1.702, swiglu_limit=7.0), pdl=False, _n=0, buf=SimpleNamespace(
+        x16=torch.zeros(sk.rows16_bytes(nb, k), dtype=torch.uint8, **dev),
+        sk_x=(torch.zeros(nb * k, dtype=torch.int8, **dev), torch.zeros(nb * (k // 256), **dev), torch.zeros(nb * (k // 32), dtype=torch.int16, **dev))))
+    be._rows_sk = lambda *a, **kw: B200Backend._rows_sk(be, *a, **kw)
+    out = torch.zeros(nb, 32, **dev)
+    B200Backend._sk(be, [sk.repack(q, "cuda")], x.cuda(), out, nb, norm_w=nw.cuda())
+    ref = _quant256_ref(R.rmsnorm(x, nw, 1e-5)) @ q.dequant().t()
+    assert _close(out.cpu(), ref), (out.cpu() - ref).abs().max()
