@@ -48,6 +48,9 @@ FP4_MIN_PAIRS = 16
 # Prompts of up to so many rows an expert do too; beyond them the 128-row tiles of gemm_q_grouped.cu are full: 769 us against 1341 at 32 rows, 1227 against 1349 at 64, 1825
 # against 1358 at 96.
 FP4_MAX_ROWS = 64
+# Router logits of a prompt pass, tokens x experts: up to so many from the steps' kernel, whose CTAs share a row's length among all threads, more from the one that gives it to a
+# warp (kernels/moe.cu).  Rows of 2880, 128 experts: 9.4 us against 11.4 at 64 tokens, 14.1 against 11.4 at 128; 32 experts: 9.6 against 11.3 at 256, 16.0 against 11.4 at 512.
+ROUTER_CELLS = 8192
 
 
 def supports(cfg: ModelConfig) -> bool:
@@ -175,10 +178,6 @@ class B200Backend(StepEngine):
                 # experts stay stacked: [E][n][k] planes, the expert index selects a row range inside the kernels
                 L.router = mat(p + "ffn_gate_inp", False)
                 L.router_f32 = get(p + "ffn_gate_inp.weight").dequant().to(dev).contiguous()
-                # the same as three bf16 matrices that add up to it (8 + 8 + 8 bits): prompt rows are bf16, so the products of the three are exact on the tensor core
-                hi = L.router_f32.to(torch.bfloat16)
-                mid = (L.router_f32 - hi.float()).to(torch.bfloat16)
-                L.router_3 = torch.cat([hi, mid, (L.router_f32 - hi.float() - mid.float()).to(torch.bfloat16)])
 
                 def exps(kind):
                     b = vec(p + f"ffn_{kind}_exps.bias")
@@ -454,17 +453,18 @@ class B200Backend(StepEngine):
         """
         c = self.cfg
         T, k = h.shape[0], c.n_experts_used
-        # [T, E] in the precision of fp32, so that near-ties select as the fp32 graph does (as a 32-bit product it took 64 us of a layer at 1024 rows)
-        if c.d_model % 8 == 0 and c.n_experts % 4 == 0:
-            logits = K.gemm_bf16(h, L.router_3, pdl=2 * self.pdl).view(T, 3, -1).sum(1)
+        # [T, E] in fp32 products and sums, so that near-ties select as the fp32 graph does
+        if c.d_model % 4 == 0:
+            logits = torch.empty(T, c.n_experts, device=self.device, dtype=torch.float32)
+            K.router(h if T * c.n_experts > ROUTER_CELLS else h.float(), L.router_f32, L.router.bias, logits, self.pdl)
             self.kernel_launches += 1
         else:
             logits = h.float() @ L.router_f32.t()
-        if L.router.bias is not None:
-            logits += L.router.bias
+            if L.router.bias is not None:
+                logits += L.router.bias
         ids = torch.empty(T * k, device=self.device, dtype=torch.int32)
         lids, wts = torch.empty_like(ids), torch.empty(T * k, device=self.device, dtype=torch.float32)
-        self._route(logits.contiguous(), T, ids, lids, wts, False)
+        self._route(logits, T, ids, lids, wts, False)
         per = T * k / c.n_experts
         if (self.moe_stream_q and getattr(L.gu, "bf16", None) is None and K.moe_fp4_supported(L.gu) and K.moe_fp4_supported(L.down)
                 and (per <= FP4_MAX_ROWS or not (K.gemm_q_grouped_supported(L.gu) and K.gemm_q_grouped_supported(L.down)))):

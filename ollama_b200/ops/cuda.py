@@ -774,9 +774,10 @@ class RouterArgs(C.Structure):
 
 
 def router(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, out: torch.Tensor, pdl: bool = False) -> None:
-    """out[b, e] = w[e] . x[b] + bias[e], all fp32; row length a multiple of 4."""
+    """out[b, e] = w[e] . x[b] + bias[e] in fp32 products and sums; row length a multiple of 4.  ``x``: a step's fp32 rows, or the bf16 rows of a prompt."""
     a = RouterArgs(ptr(x), ptr(w), ptr(bias), ptr(out), x.stride(0), w.shape[0], w.shape[1], x.shape[0], out.stride(0))
-    _check(lib().b2_router(C.byref(a), int(pdl), stream()), "router")
+    f = lib().b2_router_rows if x.dtype == torch.bfloat16 else lib().b2_router
+    _check(f(C.byref(a), int(pdl), stream()), "router")
 
 
 class MoeSortArgs(C.Structure):

@@ -802,6 +802,35 @@ def test_router(nb, n, k):
     assert out[:, n:].abs().max() == 0
 
 
+@pytest.mark.parametrize("T,E,d", [(1, 3, 4), (9, 128, 2880), (65, 33, 516), (600, 32, 2880), (2048, 128, 2880)])
+def test_router_of_a_prompt(T, E, d):
+    """Router logits of a prompt's bf16 rows against 64 bits, as the engine takes them: the choice of experts hangs on them.  Products of 32 bits whose sums are rounded:
+    2^-24 sqrt(d) / 2 of the results' norm, some ten times what the kernels show; sums that are cut off, as the tensor core's are, go beyond it."""
+    from types import SimpleNamespace
+
+    from ollama_b200.engine.b200 import B200Backend
+    gen = torch.Generator(device="cuda").manual_seed(T + d)
+    h, w, bias = (torch.randn(*s, device="cuda", generator=gen) for s in ((T, d), (E, d), (E,)))
+    h, w, got = h.to(torch.bfloat16), w * 0.02, []
+
+    class Enough(Exception):
+        pass
+
+    def route(logits, *_):
+        got.append(logits.clone())
+        raise Enough
+
+    hi = w.to(torch.bfloat16)
+    mid = (w - hi.float()).to(torch.bfloat16)
+    L = SimpleNamespace(router_f32=w, router=SimpleNamespace(bias=bias), router_3=torch.cat([hi, mid, (w - hi.float() - mid.float()).to(torch.bfloat16)]))
+    be = SimpleNamespace(cfg=SimpleNamespace(d_model=d, n_experts=E, n_experts_used=1), device="cuda", pdl=True, kernel_launches=0, _route=route)
+    with pytest.raises(Enough):
+        B200Backend._moe_prefill(be, h, L)
+    ref = h.double() @ w.double().t() + bias.double()
+    err = (got[0].double() - ref).norm() / ref.norm()
+    assert got[0].shape == (T, E) and err < 2 ** -25 * max(d, 64) ** 0.5, err
+
+
 @pytest.mark.parametrize("E,d,ff,T,k,chunk", [(8, 256, 256, 1, 2, 8), (8, 96, 160, 37, 3, 16), (6, 288, 224, 100, 2, 64), (3, 2880, 2880, 70, 2, 32), (40, 64, 32, 9, 4, 8)])
 @pytest.mark.parametrize("bf16", [False, True])
 def test_moe_fp4_products(E, d, ff, T, k, chunk, bf16):
