@@ -67,6 +67,7 @@ class _Layer:
 
 class B200Backend(StepEngine):
     name = "b200"
+    _pass = _ws = None               # native prompt pass, hand-over buffers of the steps: made by alloc
 
     def __init__(self, g: GGUFFile | None, device: str = "cuda", opts=None, cfg: ModelConfig | None = None,
                  tensors: dict[str, QWeight] | None = None, keep_bf16: bool | None = None, prefill_gemm: str = "bf16",
@@ -326,6 +327,7 @@ class B200Backend(StepEngine):
         if any(L.sk is not None for L in self.layers):      # pre-quantised inputs of the streaming GEMV (rows too wide to quantise in place)
             kq = max(kmax, ff)
             b.x16 = torch.zeros(SK.rows16_bytes(MB, kq), device=dev, dtype=torch.uint8) if MB > INT8_ROWS else None
+            self._ws = SK.Workspace(dev)
             b.sk_x = (torch.zeros(MB * kq, device=dev, dtype=i8), torch.zeros(MB * (kq // 256 + 1), device=dev, dtype=f32),
                       torch.zeros(MB * (kq // 32 + 1), device=dev, dtype=torch.int16))
         b.host_in = torch.zeros(3, MB, dtype=i32).pin_memory()
@@ -340,7 +342,12 @@ class B200Backend(StepEngine):
     def close(self) -> None:
         self._graphs.clear()
         self.k_cache = self.v_cache = self.k_scale = self.v_scale = []
-        self.buf = self._pass = None
+        self.buf = self._pass = self._ws = None
+
+    def check_waits(self) -> None:
+        for ws in (self._ws, self._pass.ws if self._pass is not None else None):
+            if ws is not None:
+                ws.check(wait=False)
 
     # -- decode ---------------------------------------------------------------------------------------
     def _norm_quant(self, x, w, nb, k, *, do_norm=True, residual=None, src=None):
@@ -508,7 +515,7 @@ class B200Backend(StepEngine):
         k = ws[0].k
         xin = x[:nb, :k]
         if nb > INT8_ROWS and (norm_w is None or k <= SK.ROWS16_MAX_NORM):      # longer rows that are normalised first stay int8
-            self._rows_sk(ws, xin, out[:nb], norm_w, mode, b.x16)
+            self._rows_sk(ws, xin, out[:nb], norm_w, mode, b.x16, self._ws)
             self._n += 2
             return
         if not SK.fits_fused_input(nb, k):      # wide or many rows: one CTA per row quantises, the GEMV reads int8 from global memory
@@ -517,7 +524,8 @@ class B200Backend(StepEngine):
                               out=(xq[:nb * k].view(nb, k), xd[:nb * (k // 256)].view(nb, k // 256), xbs[:nb * (k // 32)].view(nb, k // 32)))
             norm_w = None
             self._n += 1
-        SK.gemv(ws, xin, norm_w=norm_w, eps=c.norm_eps, out=out, mode=mode, act=c.act, alpha=c.swiglu_alpha, limit=c.swiglu_limit, pdl=self.pdl)
+        SK.gemv(ws, xin, norm_w=norm_w, eps=c.norm_eps, out=out, mode=mode, act=c.act, alpha=c.swiglu_alpha, limit=c.swiglu_limit, pdl=self.pdl,
+                ws=self._ws)
         self._n += 1
 
     def _rows_sk(self, ws, x: torch.Tensor, out: torch.Tensor, norm_w=None, mode: int = SK.MODE_STORE, buf: torch.Tensor | None = None, wsp=None) -> None:
@@ -771,7 +779,7 @@ class B200Backend(StepEngine):
     def _logits(self, x: torch.Tensor) -> torch.Tensor:
         if self._unit_rows(x.shape[0]) and getattr(self, "sk_head", None) is not None:
             out = torch.empty(x.shape[0], self.cfg.vocab_size, device=self.device, dtype=torch.float32)
-            self._rows_sk([self.sk_head], x.contiguous(), out, self.out_norm, wsp=self._pass.ws if self._pass is not None else None)
+            self._rows_sk([self.sk_head], x.contiguous(), out, self.out_norm, wsp=self._pass.ws if self._pass is not None and self._pass.ws is not None else self._ws)
             self.kernel_launches += 2 * ((x.shape[0] + SK.MAX_TOKENS - 1) // SK.MAX_TOKENS)
             return R.softcap(out, self.cfg.final_softcap)
         return R.softcap(self._mm(self._final_norm(x).to(torch.bfloat16), self.head), self.cfg.final_softcap)

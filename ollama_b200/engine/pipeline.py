@@ -168,7 +168,14 @@ class PipelineBackend:
             last.buf.host_out.copy_(last.buf.sampled, non_blocking=True)
             last.d2h_bytes += last.buf.host_out.numel() * 4
             torch.cuda.current_stream().synchronize()
+        self.check_waits()
         return last.buf.host_out_np[:nb].tolist()
+
+    def check_waits(self) -> None:
+        """Raise if a bounded wait ran out in a kernel of a stage whose results the caller has just read on the host."""
+        for s in self.stages:
+            with torch.cuda.device(s.device):
+                s.check_waits()
 
     # -- prefill ----------------------------------------------------------------------------------------
     def _chunk(self, slot: int, tokens: Sequence[int], pos0: int) -> torch.Tensor:

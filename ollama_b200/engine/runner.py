@@ -569,6 +569,7 @@ class Runner:
             hid = self.backend.hidden(s.slot, s.prompt)
             vec = _pool(hid.float(), self.cfg.pooling)
             _sync(hid)
+            self._check_waits()
             s.n_prompt_eval = len(s.prompt)
             s.out.put(CompletionChunk(done=True, done_reason="stop", embedding=vec.tolist(), prompt_eval_count=len(s.prompt),
                                       prompt_eval_duration=time.perf_counter() - t0))
@@ -709,11 +710,19 @@ class Runner:
         """
         try:
             tok, lp = drawn if drawn is not None else s.sampler.sample(logits, s.grammar.allows if s.grammar else None)
+            self._check_waits()
             self._accept(s, tok, lp)
         except Exception as e:
             if _is_device_error(e):
                 raise
             self._fail(s, e)
+
+    def _check_waits(self) -> None:
+        """Results have reached the host: a kernel behind them that gave up waiting is a device error."""
+        for be in (self.backend, self.draft):
+            check = getattr(be, "check_waits", None)
+            if check is not None:
+                check()
 
     def _fail(self, s: _Seq, e: Exception) -> None:
         """End one sequence with an error chunk and free its slot."""
@@ -753,6 +762,7 @@ class Runner:
             proposals.append(tok)
         logits = self.backend.verify(slot, [s.next_token] + proposals, s.n_past)
         target = logits.argmax(-1).tolist()                 # target[i]: the token after position n_past + i
+        self._check_waits()
         n_ok = 0
         while n_ok < k and proposals[n_ok] == target[n_ok]:
             n_ok += 1

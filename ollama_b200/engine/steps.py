@@ -88,7 +88,11 @@ class StepEngine:
         self.buf.host_out.copy_(self.buf.sampled, non_blocking=True)
         self.d2h_bytes += self.buf.host_out.numel() * 4
         torch.cuda.current_stream().synchronize()
+        self.check_waits()
         return self.buf.host_out_np[:nb].tolist()
+
+    def check_waits(self) -> None:
+        """Raise if a bounded wait ran out in a kernel whose results the caller has just read on the host."""
 
     @torch.no_grad()
     def decode(self, slots, tokens, positions) -> torch.Tensor:

@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) gemm_sk_kernel(const __grid_con
             uint32_t turn = 0;
             for (int it = lo; it < hi; it++) {
                 if (turn > 0 && !bar_wait(&empty[s], (turn - 1) & 1)) {
-                    atomicExch(a.status, (int)KS_TIMEOUT);
+                    *(volatile int*)a.status = KS_TIMEOUT;
                     break;
                 }
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&full[s])), "r"(CHUNK) : "memory");
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) gemm_sk_kernel(const __grid_con
             __syncwarp();
             if (!dead && !__all_sync(0xffffffffu, bar_wait(&full[xs], turn & 1))) {
                 dead = true;
-                if (lane == 0) atomicExch(a.status, (int)KS_TIMEOUT);
+                if (lane == 0) *(volatile int*)a.status = KS_TIMEOUT;
             }
             if (mine && !dead) {
                 const uint8_t* sp = ring + slot * a.slot_bytes;
@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) gemm_sk_kernel(const __grid_con
                         const unsigned long long t0 = now_ns();
                         while (!ok && now_ns() - t0 < SG_WAIT_NS) ok = ld_acquire(&a.flags[from]) != 0u;
                     }
-                    if (!ok) atomicExch(a.status, (int)KS_TIMEOUT);
+                    if (!ok) *(volatile int*)a.status = KS_TIMEOUT;
                 }
                 if (!__all_sync(0xffffffffu, ok)) dead = true;
                 const float* w = a.ws + ((size_t)c0 * SG_WARPS + warp) * SG_WS_FLOATS + lane;

@@ -72,7 +72,7 @@ struct SkArgs {
     // split tiles
     float* ws;            // [groups][SK_WS_FLOATS]
     unsigned* flags;      // [groups], zero between launches
-    int* status;          // KStatus, written when a bounded wait gives up
+    int* status;          // KStatus, written when a bounded wait gives up (may be pinned host memory)
     // shared memory offsets and work split (filled in by the launcher)
     int off_red, off_xq, off_xd, off_xbs, off_ring;
     int ring, slot_bytes; // units per warp ring (2..4) and bytes per slot
@@ -578,7 +578,7 @@ __device__ __forceinline__ void grid_barrier(unsigned* bar, unsigned target, int
                 const unsigned long long t0 = global_ns();
                 while (!ok && global_ns() - t0 < SK_WAIT_NS) ok = ld_acquire_gpu_u32(bar) >= target;
             }
-            if (!ok) atomicExch(status, (int)KS_TIMEOUT);
+            if (!ok) *(volatile int*)status = KS_TIMEOUT;
         }
     }
     __syncthreads();
@@ -767,7 +767,7 @@ __global__ void __launch_bounds__(SK_THREADS, NT == 1 ? 2 : 1) gemv_sk_kernel(co
                                     ok = ld_acquire_gpu_u32(&a.flags[c]) != 0u;
                                 }
                             }
-                            if (!ok) atomicExch(a.status, (int)KS_TIMEOUT);
+                            if (!ok) *(volatile int*)a.status = KS_TIMEOUT;
                         }
                         ok = __shfl_sync(0xffffffffu, ok, 0);
                         if (!ok) {

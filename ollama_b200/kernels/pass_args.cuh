@@ -46,7 +46,7 @@ struct SgArgs {
     float alpha, limit;
     float* ws;            // [groups of b2_gemv_sk_max_groups][512]
     unsigned* flags;
-    int* status;
+    int* status;          // KStatus, written when a bounded wait gives up (may be pinned host memory)
     int tiles, ring, slot_bytes, x_slots;      // filled in by the launcher
 };
 

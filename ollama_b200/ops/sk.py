@@ -195,22 +195,27 @@ def unit_weights(w: SkWeight) -> torch.Tensor:
 
 
 class Workspace:
-    """Hand-over buffers of split tiles and the status word, one set per device (launches of one stream share it; prompt passes have their own)."""
+    """Hand-over buffers of split tiles and the status word.  Launches of one stream share a set: an engine has one for its steps and one for its prompt passes, other callers the
+    device's (:func:`workspace`).  The status word lives in host memory that kernels reach, so that reading it costs nothing."""
 
     def __init__(self, device):
         rows = int(K.lib().b2_gemv_sk_max_groups())
         self.ws = torch.zeros(rows * WS_FLOATS, device=device, dtype=torch.float32)
         self.flags = torch.zeros(rows, device=device, dtype=torch.int32)
-        self.status = torch.zeros(1, device=device, dtype=torch.int32)
+        self.status = torch.zeros(1, dtype=torch.int32).pin_memory()
+        self.status_np = self.status.numpy()
         self.bar = torch.zeros(2, device=device, dtype=torch.int32)          # arrival / exit counters of multi-phase launches
 
-    def check(self) -> None:
-        """Raise if a bounded wait inside a launch gave up; the flags are cleared so the next launch starts clean."""
-        if int(self.status.item()) != 0:
-            self.status.zero_()
+    def check(self, wait: bool = True) -> None:
+        """Raise if a bounded wait inside a launch gave up: its sums are wrong, and a flag that was set too late would be taken for the next launch's, so the flags are cleared.
+        ``wait``: for the launches of the current stream first (a caller that has read their results need not)."""
+        if wait:
+            torch.cuda.current_stream(self.ws.device).synchronize()
+        if self.status_np[0] != 0:
+            self.status_np[0] = 0
             self.flags.zero_()
             self.bar.zero_()
-            raise K.CudaKernelError("streaming GEMV: a bounded wait ran out")
+            raise K.CudaKernelError("product of unit-ordered matrices: a bounded wait ran out")
 
 
 _workspaces: dict = {}
@@ -259,7 +264,7 @@ def fill_args(a: SkArgs, weights: list[SkWeight], nb: int, ws: Workspace) -> Non
 
 def gemv(weights: list[SkWeight], x: torch.Tensor | tuple[torch.Tensor, torch.Tensor], *, norm_w: torch.Tensor | None = None, eps: float = 0.0,
          out: torch.Tensor | None = None, mode: int = MODE_STORE, act: str = "silu", alpha: float = 1.702, limit: float = 7.0,
-         max_ctas: int = 0, split: int = 0, ring: int = 0, pdl: bool = False) -> torch.Tensor:
+         max_ctas: int = 0, split: int = 0, ring: int = 0, pdl: bool = False, ws: Workspace | None = None) -> torch.Tensor:
     """y[b] = concat_i(W_i x[b] + bias_i) for 1..32 tokens.
 
     ``x``: fp32 rows [nb, k] (normalised with ``norm_w`` and quantised inside the kernel) or the (int8, scales) pair of
@@ -272,7 +277,7 @@ def gemv(weights: list[SkWeight], x: torch.Tensor | tuple[torch.Tensor, torch.Te
     if out is None:
         out = torch.empty(nb, total // 2 if mode == MODE_GLU else total, device=dev, dtype=torch.float32)
     a = SkArgs()
-    fill_args(a, weights, nb, workspace(dev))
+    fill_args(a, weights, nb, ws or workspace(dev))
     if pre:
         a.xq, a.xd, a.xbs = x[0].data_ptr(), x[1].data_ptr(), x[2].data_ptr()
     else:

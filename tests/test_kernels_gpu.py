@@ -763,6 +763,7 @@ def test_engine_prompt_pass_row_counts(tmp_path, name, ft, kv, rows):
     for a, b in zip(eng.prefill_many(segs, [True, True]), ref.prefill_many(segs, [True, True])):
         close(a, b)
     assert K_status_ok()
+    eng.check_waits()
     eng.close()
 
 

@@ -31,6 +31,25 @@ def test_generate_greedy_f32_and_q8(tiny_llama_path, tiny_llama_q8_path):
     assert "".join(c.content for c in a).startswith(f"<t{ta[0]}>")
 
 
+@pytest.mark.parametrize("embedding", [False, True])
+def test_waits_that_ran_out_end_the_runner(tiny_llama_path, embedding):
+    """A backend whose kernels gave up waiting says so when results have been read: the request gets an error, not the results, and the runner is done for (the scheduler starts another)."""
+    from ollama_b200.ops.cuda import CudaKernelError
+    r = Runner(tiny_llama_path, RunnerOptions(num_ctx=128, device="cpu"))
+
+    def check():
+        raise CudaKernelError("a bounded wait ran out")
+
+    try:
+        r.backend.check_waits = check
+        s = r.submit(CompletionRequest(prompt=_prompt(), sampling=SamplingParams(temperature=0), num_predict=4, embedding=embedding))
+        c = s.out.get(timeout=60)
+        assert c.done and "a bounded wait ran out" in c.error and not c.tokens and not c.embedding
+        assert "a bounded wait ran out" in r.error
+    finally:
+        r.close()
+
+
 def test_prefix_cache_and_parallel_slots(tiny_llama_path):
     r = Runner(tiny_llama_path, RunnerOptions(num_ctx=128, num_parallel=2, device="cpu"))
     try:

@@ -184,8 +184,33 @@ def test_engine_decodes_up_to_32_sequences_in_one_step(tmp_path):
         got = eng.decode(list(range(nb)), toks[:nb], pos[:nb]).cpu()
         assert (got - want[:nb]).abs().max().item() < tol, nb
         assert eng.decode_argmax(list(range(nb)), toks[:nb], pos[:nb]) == got.argmax(-1).tolist()
-    from ollama_b200.ops import sk
-    sk.workspace("cuda").check()
+    eng.check_waits()
+
+
+def test_waits_that_ran_out_are_reported_and_cleared(tmp_path):
+    """What a launch leaves behind that gave up waiting (set from the host: a status word, a flag set too late) ends the next call that reads results, in steps and prompt passes; the
+    calls after it give what they gave before."""
+    from ollama_b200.engine.b200 import B200Backend
+    from ollama_b200.engine.backend import open_model
+    from ollama_b200.models.synth import write_synthetic_gguf
+    K, sk = _mods()
+    p = str(tmp_path / "m.gguf")
+    write_synthetic_gguf(p, "tiny-qwen3", "Q4_K_M")
+    eng = B200Backend(open_model(p), "cuda", keep_bf16=True)
+    eng.alloc(1, 64)
+    assert eng._pass.units and len({id(w) for w in (eng._ws, eng._pass.ws, sk.workspace("cuda"))}) == 3
+    prompt = [300, 301, 302, 303, 304]
+    want = eng.prefill(0, prompt, 0).clone()
+    tok = eng.decode_argmax([0], [5], [5])
+    for ws in (eng._ws, eng._pass.ws):
+        ws.status[0] = 1
+        ws.flags[:] = 1
+        with pytest.raises(K.CudaKernelError):
+            eng.decode_argmax([0], [5], [5])
+        assert int(ws.flags.max()) == 0 and int(ws.status[0]) == 0
+        assert torch.equal(eng.prefill(0, prompt, 0), want) and eng.decode_argmax([0], [5], [5]) == tok
+        eng.check_waits()
+    eng.close()
 
 
 @pytest.mark.parametrize("segs,k", [([(16, GGMLType.Q4_K)], 256), ([(272, GGMLType.Q6_K), (16, GGMLType.Q4_K), (32, GGMLType.Q6_K)], 512), ([(4096, GGMLType.Q4_K)], 2816)])
@@ -242,7 +267,7 @@ def test_steps_of_models_wider_than_the_normalising_pass():
     q = _qw(GGMLType.Q4_K, 32, k, 2)
     x, nw = torch.randn(nb, k, generator=gen), torch.rand(k, generator=gen) + 0.5
     dev = dict(device="cuda")
-    be = SimpleNamespace(cfg=SimpleNamespace(norm_eps=1e-5, act="silu", swiglu_alpha=1.702, swiglu_limit=7.0), pdl=False, _n=0, buf=SimpleNamespace(
+    be = SimpleNamespace(cfg=SimpleNamespace(norm_eps=1e-5, act="silu", swiglu_alpha=1.702, swiglu_limit=7.0), pdl=False, _n=0, _ws=None, buf=SimpleNamespace(
         x16=torch.zeros(sk.rows16_bytes(nb, k), dtype=torch.uint8, **dev),
         sk_x=(torch.zeros(nb * k, dtype=torch.int8, **dev), torch.zeros(nb * (k // 256), **dev), torch.zeros(nb * (k // 32), dtype=torch.int16, **dev))))
     be._rows_sk = lambda *a, **kw: B200Backend._rows_sk(be, *a, **kw)
