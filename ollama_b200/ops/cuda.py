@@ -464,6 +464,13 @@ def attn_decode_rope(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
     return out
 
 
+def _operands(a: torch.Tensor, b: torch.Tensor, pdl: int) -> tuple[torch.Tensor, torch.Tensor, int]:
+    """Both operands without strides.  A copy of ``b`` made here comes from the kernel just before the product, which then must not fetch it early (``pdl`` 2)."""
+    if not b.is_contiguous():
+        b, pdl = b.contiguous(), min(pdl, 1)
+    return a.contiguous(), b, pdl
+
+
 @functools.lru_cache(maxsize=4096)
 def gemm_bf16_scratch(m: int, n: int, k: int) -> int:
     """Floats of scratch with which the tcgen05 product of this size is split along k (0: it is not)."""
@@ -479,7 +486,7 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, bias: torch.Tensor | None = None
     n = b.shape[0]
     if a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16 or b.shape[1] != k:
         raise ValueError("gemm_bf16 needs bf16 operands [m, k] and [n, k]")
-    a, b = a.contiguous(), b.contiguous()
+    a, b, pdl = _operands(a, b, pdl)
     if out is None:
         out = torch.empty(m, n, device=a.device, dtype=torch.float32)
     size = gemm_bf16_scratch(m, n, k)
@@ -495,7 +502,7 @@ def gemm_bf16_out16(a: torch.Tensor, b: torch.Tensor, bias: torch.Tensor | None 
     """Same product as :func:`gemm_bf16` with a bf16 result (n % 8 == 0)."""
     m, k = a.shape
     n = b.shape[0]
-    a, b = a.contiguous(), b.contiguous()
+    a, b, pdl = _operands(a, b, pdl)
     if out is None:
         out = torch.empty(m, n, device=a.device, dtype=torch.bfloat16)
     f = lib().b2_gemm_bf16_out16
@@ -847,7 +854,7 @@ def gemm_bf16_glu(a: torch.Tensor, b: torch.Tensor, act: str, bias: torch.Tensor
     """Gate/up product of a dense FFN with the gated activation in the GEMM epilogue: bf16 [m, n / 2]."""
     m, k = a.shape
     n = b.shape[0]
-    a, b = a.contiguous(), b.contiguous()
+    a, b, pdl = _operands(a, b, pdl)
     out = torch.empty(m, n // 2, device=a.device, dtype=torch.bfloat16)
     f = lib().b2_gemm_bf16_glu
     f.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_float, C.c_float, C.c_int, C.c_void_p]

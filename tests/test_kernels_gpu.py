@@ -900,6 +900,20 @@ def test_gemm_bf16_shapes(m, n, k, pdl):
     assert K_status_ok()
 
 
+@pytest.mark.parametrize("m", [40, 300])
+def test_gemm_bf16_of_a_strided_matrix(m):
+    """A matrix that the wrapper copies first, in a launch that may begin early: the copy's values are the ones that are multiplied (the bits of the contiguous product)."""
+    K = _K()
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    a, wide = (torch.randn(*s, device="cuda", generator=gen).to(torch.bfloat16) for s in ((m, 1024), (4096, 2048)))
+    for b in (wide[:, :1024], wide.view(2048, 4096)[:1024].t()):
+        want = K.gemm_bf16(a, b.contiguous())
+        for _ in range(3):
+            assert torch.equal(K.gemm_bf16(a, b, pdl=2), want)
+        assert torch.equal(K.gemm_bf16_out16(a, b, pdl=2), K.gemm_bf16_out16(a, b.contiguous()))
+        assert torch.equal(K.gemm_bf16_glu(a, b, "silu", pdl=2), K.gemm_bf16_glu(a, b.contiguous(), "silu"))
+
+
 def K_status_ok() -> bool:
     return _K().gemm_status() == 0
 

@@ -21,3 +21,36 @@ def test_int8_caches_whose_scales_are_not_aligned_go_to_the_scalar_decode_kernel
         assert takes(off, 0) == takes(0, off) == takes(off, off) == int(whole), off
     assert takes(0, 0, scales=False) == 1
     assert takes(0, 0, heads=7) == 0 and takes(0, 0, heads=64) == 0
+
+
+class Launches:
+    """Stands for the kernel library: keeps the arguments of each call."""
+
+    def __init__(self):
+        self.calls = []
+
+    def __getattr__(self, name):
+        class Entry:
+            def __call__(_, *args):
+                self.calls.append((name, args))
+                return 0
+        return Entry()
+
+
+@pytest.fixture
+def launches(monkeypatch):
+    got = Launches()
+    monkeypatch.setattr(K, "lib", lambda: got)
+    monkeypatch.setattr(K, "stream", lambda: None)
+    monkeypatch.setattr(K, "gemm_bf16_scratch", lambda *_: 0)
+    return got
+
+
+@pytest.mark.parametrize("call,at", [(K.gemm_bf16, 9), (K.gemm_bf16_out16, 8), (lambda a, b, pdl: K.gemm_bf16_glu(a, b, "silu", pdl=pdl), 11)])
+def test_a_matrix_that_is_copied_for_the_product_is_not_fetched_early(launches, call, at):
+    """pdl 2 says that b does not depend on the kernel just before; where the wrapper copies b, that kernel is the copy."""
+    a, b = torch.zeros(4, 64, dtype=torch.bfloat16), torch.zeros(32, 64, dtype=torch.bfloat16)
+    strided, turned = torch.zeros(32, 128, dtype=torch.bfloat16)[:, :64], torch.zeros(64, 32, dtype=torch.bfloat16).t()
+    for m, pdl, want in ((b, 2, 2), (b, 0, 0), (strided, 2, 1), (turned, 2, 1), (strided, 1, 1), (strided, 0, 0)):
+        call(a, m, pdl=pdl)
+        assert launches.calls[-1][1][at] == want, (want, launches.calls[-1])
