@@ -149,7 +149,7 @@ class Step:
                    pdl=self.pdl, **conv)
         else:
             m = joined or mat
-            O.gemm(h, m.w, out, bias=m.bias, tail=tail)
+            O.gemm(h, m.w, out, bias=m.bias, tail=tail, pdl=self.be.pdl)
         self.launched()
 
     def product(self, h: torch.Tensor, mat: Mat, out: torch.Tensor, **kw) -> None:
@@ -157,7 +157,7 @@ class Step:
         if self.small:
             O.gemv([O.seg(mat.w, mat.w.shape[0], out, rc=mat.bias, **kw)], mat.w.shape[1], h, self.nb, self.be.f32, mul_row=self.m.tokens, pdl=self.pdl)
         else:
-            O.gemm(h, mat.w, out, bias=mat.bias, mul_row=self.m.tokens, **kw)
+            O.gemm(h, mat.w, out, bias=mat.bias, mul_row=self.m.tokens, pdl=self.be.pdl, **kw)
         self.launched()
 
     def add(self, h: torch.Tensor, mat: Mat) -> None:
@@ -279,7 +279,7 @@ class LatentAttention:
         else:
             c = s.buf("latent_cq", n)
             O.norm_rows(proj, m.q_rank, eps, self.q_norm, c, pdl=s.pdl)
-            O.gemm(c, w, q)
+            O.gemm(c, w, q, pdl=s.be.pdl)
             s.launched()
         s.launched()
         return q
@@ -322,7 +322,7 @@ class LatentAttention:
         r = torch.empty(lp.total, max(self.rp, 8), device=dev, dtype=torch.float16)
         A.latent_gather(cache, self.cp, m.rot_dim, lp.seqs, lp.longest, s.be.cache.table, c, r)
         kv = torch.empty(lp.total, self.w_kv.shape[0], device=dev, dtype=torch.float16)
-        O.gemm(c, self.w_kv, kv)
+        O.gemm(c, self.w_kv, kv, pdl=s.be.pdl)
         A.attn_prefill_parts(q, kv, r, lp.tiles, out, heads=H, dp=self.dp, vp=self.vp, rp=self.rp, vdim=m.vdim, scale=m.scale, window=m.window)
         s.launched(4)
 
@@ -435,7 +435,7 @@ class ExpertFFN:
         both = sh is not None and not s.small and s.act == torch.bfloat16
         if both:
             h, fs = s.rows(self.norm), s.buf("shared", up(sh.e.ff), zero=True)
-            O.gemm(h, sh.gu_router.w, fs, act=self.act, limit=sh.e.limit, bias=sh.gu_router.bias, tail=z)
+            O.gemm(h, sh.gu_router.w, fs, act=self.act, limit=sh.e.limit, bias=sh.gu_router.bias, tail=z, pdl=s.be.pdl)
             s.launched()
         else:
             h = s.normed(self.norm, self.router, z, keep=True)

@@ -188,7 +188,7 @@ class StateSpaceHeads:
                 s.product(h, self.w_in, zx)
                 s.product(h, self.w_dt, dt)
             else:
-                O.gemm(h, self.w_all, zx, tail=dt)
+                O.gemm(h, self.w_all, zx, tail=dt, pdl=be.pdl)
                 s.launched()
             O.ssm_conv(xbc, self.ch, *conv, s.m.slots, s.m.positions, s.m.offs, u, shift=s.decode, pdl=s.pdl)
             if not s.decode:

@@ -75,7 +75,7 @@ class SharedNormLayer:
             if s.small:
                 segs = (O.seg(ff.up.w, ff.ffp, f, act=ff.act, nums=ff.nums),)
             else:
-                O.gemm(h, ff.up.w, f, act=ff.act, nums=ff.nums)
+                O.gemm(h, ff.up.w, f, act=ff.act, nums=ff.nums, pdl=s.be.pdl)
                 s.launched()
         mix.mix(s, mix.project(s, h, mem, segs=segs), mem, cat[:, :self.mixp])
         s.add(cat, self.w_last if ff is not None else mix.w_o)

@@ -330,7 +330,7 @@ class StackBackend(StepEngine):
 
     # -- one layer run ----------------------------------------------------------------------------------
     def _mm(self, a, w, out, **kw) -> None:
-        O.gemm(a, w, out, **kw)
+        O.gemm(a, w, out, pdl=self.pdl, **kw)
         self._n += 1
 
     def _layer(self, i: int, x: torch.Tensor, x0: torch.Tensor, B: _Rows, m: _Meta, decode: bool) -> torch.Tensor:

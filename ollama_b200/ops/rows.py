@@ -124,12 +124,13 @@ def gemv(segs: list, k: int, x: torch.Tensor, nb: int, f32: bool, src: int = SRC
 
 def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: str = "", accumulate: bool = False, k: int | None = None, alpha: float = 1.0,
          limit: float = math.inf, nums: tuple[float, float] = NO_NUMS, bias: torch.Tensor | None = None, mul: torch.Tensor | None = None, mul_row: torch.Tensor | None = None,
-         experts: int = 0, tile_expert: torch.Tensor | None = None, copy: torch.Tensor | None = None, tail: torch.Tensor | None = None) -> None:
+         experts: int = 0, tile_expert: torch.Tensor | None = None, copy: torch.Tensor | None = None, tail: torch.Tensor | None = None,
+         pdl: bool = True) -> None:
     """out (+)= alpha * act(a[:, :k] @ w[:, :k]^T + bias) [* mul[mul_row]]; bf16 operands on tcgen05 (result bf16, f16 or fp32), fp32 operands in full
     32 bits.  ``copy``: bf16 rows of out's pitch that receive an fp32 result too.
     ``a``, ``out`` and ``mul`` may be column windows of wider buffers.  Gated activations ("glu:...") halve the columns.  ``experts``: w holds
     that many stacked matrices and a's tiles of 128 rows belong to ``tile_expert``.  ``tail``: fp32 rows that receive the last columns' sums, as they are, instead of
-    ``out`` (bf16 operands)."""
+    ``out`` (bf16 operands).  ``pdl``: the launch may begin while the kernel before it, which may write w too, ends (bf16 operands, no experts)."""
     n = w.shape[0] // max(experts, 1)
     m, k, nt = a.shape[0], w.shape[1] if k is None else k, tail.shape[1] if tail is not None else 0
     cols = (n - nt) // 2 if act.startswith("glu:") else n - nt
@@ -144,7 +145,7 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: str = "", acc
     ws = torch.empty(size, device=a.device) if size else None
     g = GemmRowsArgs(ptr(a), ptr(w), ptr(out), ptr(bias), ptr(mul), ptr(mul_row), ptr(tile_expert), ptr(copy), ptr(ws), size, m, n, k, a.stride(0), w.stride(0), out.stride(0),
                      OUT_TYPE[out.dtype], ACT[act], int(accumulate), experts, mul.stride(0) if mul is not None else 0, alpha, limit, ptr(tail), n - nt,
-                     tail.stride(0) if nt else 0, *nums, 1)      # 1: w may come from the kernel just before
+                     tail.stride(0) if nt else 0, *nums, int(pdl))
     _call("b2_gemm_rows_f32" if f32 else "b2_gemm_rows", g)
 
 

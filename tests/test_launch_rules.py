@@ -54,3 +54,24 @@ def test_a_matrix_that_is_copied_for_the_product_is_not_fetched_early(launches, 
     for m, pdl, want in ((b, 2, 2), (b, 0, 0), (strided, 2, 1), (turned, 2, 1), (strided, 1, 1), (strided, 0, 0)):
         call(a, m, pdl=pdl)
         assert launches.calls[-1][1][at] == want, (want, launches.calls[-1])
+
+
+@pytest.mark.parametrize("pdl", [False, True])
+def test_products_of_stack_models_follow_the_engines_overlap_flag(monkeypatch, pdl):
+    from types import SimpleNamespace as NS
+
+    from ollama_b200.engine.blocks import Step
+    from ollama_b200.engine.stack import StackBackend
+    from ollama_b200.ops import rows as O
+    got = []
+    monkeypatch.setattr(O, "_call", lambda name, g, *_: got.append((name, g.pdl)))
+    monkeypatch.setattr(O, "_split_floats", lambda *_: 0)
+    h, w, out = torch.zeros(40, 64, dtype=torch.bfloat16), torch.zeros(32, 64, dtype=torch.bfloat16), torch.zeros(40, 32)
+    O.gemm(h, w, out)
+    assert got.pop() == ("b2_gemm_rows", 1)
+    O.gemm(h, w, out, pdl=pdl)
+    StackBackend._mm(NS(pdl=pdl, _n=0), h, w, out)
+    step = NS(small=False, be=NS(pdl=pdl), m=NS(tokens=None), launched=lambda: None)
+    Step.product(step, h, NS(w=w, bias=None), out)
+    Step.enter(step, h, NS(w=w, bias=None), out)
+    assert got == [("b2_gemm_rows", int(pdl))] * 4
