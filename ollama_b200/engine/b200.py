@@ -36,11 +36,12 @@ from .steps import StepEngine
 
 MAX_DECODE_BATCH = 8             # sequences per launch of the dp4a kernels (kernels/gemv.cu)
 MAX_STREAM_BATCH = 32            # sequences per step when every matrix runs on the streaming kernel (kernels/gemv_sk.cu)
-# Steps of more sequences than this multiply f16 activations (kernels/gemm_sk.cu) instead of int8 ones: a layer of Llama-8B takes 64 us of products against 70 at eight
-# sequences and 108 against 78 at thirteen.
+# Steps of more sequences than this multiply f16 activations (kernels/gemm_sk.cu) instead of int8 ones.  Products of a layer of Llama-8B (Q4_K_M), int8 against f16: 52 us against
+# 74 at one sequence, 70 against 74 at six, 76 against 74 at eight, 109 against 81 at nine, 121 against 81 at thirteen, 205 against 112 at 32.
 INT8_ROWS = 8
-# Prompt passes of at most this many rows read the units too, 32 rows a launch, instead of the 16-bit copies: a layer of Llama-8B is 124 MB against 436 (70 us of products
-# against 200 up to eight rows, 105 for every 32).
+# Prompt passes of at most this many rows read the units too, 32 rows a launch, instead of the 16-bit copies (a layer of Llama-8B: 124 MB against 436).  Twelve layers and the logits
+# of one row, units against copies: 1350 us against 2240 at 7 rows, 1830 against 2310 at 32, but 2730 against 2310 at 33 and 3230 against 2370 at 64.  From 33 rows on it is the
+# rows' 16 bits that count: the logits are 0.0007 off the graph in 64 bits, 0.0045 on bf16 rows and copies.
 UNIT_ROWS = 64
 # Steps of at least so many (token, expert) pairs, and of one for every eighth expert, read MXFP4 experts once for all rows that chose them (kernels/moe_fp4.cu), smaller ones
 # once per pair: a layer of 128 experts of 13 MB, four a token, takes 72 us against 75 at four tokens and 194 against 280 at sixteen, but 45 against 29 at one.
@@ -214,8 +215,8 @@ class B200Backend(StepEngine):
         # a step takes up to 32 sequences only when no layer falls back to the dp4a kernels (eight per launch)
         if all(L.sk is not None for L in self.layers) and (self.sk_head is not None or not self.last) and type(self) is B200Backend:
             self.max_batch = MAX_STREAM_BATCH
-        # ... and up to 32 when every layer is a mixture of experts (its kernels run one grid row per token-expert pair) whose dense
-        # matrices are 16-bit and multiply on the tensor-core GEMM; the router's GEMV then runs eight rows per launch
+        # ... and up to 32 when every layer is a mixture of experts (their kernels take any number of token-expert pairs) whose dense
+        # matrices are 16-bit and multiply on the tensor-core GEMM
         if (type(self) is B200Backend and 0 < self.tc_decode_min <= MAX_DECODE_BATCH and self.layers and all(L.moe for L in self.layers)
                 and all(self._bf16_of(w) is not None for L in self.layers for w in ((L.wo,) if L.wqkv16 is not None else (L.wq, L.wk, L.wv, L.wo)))
                 and all(w.wtype in (K.WT_BF16, K.WT_F16) for L in self.layers for w in (L.wq, L.wk, L.wv))

@@ -1,4 +1,4 @@
-// Product of 2..32 rows with unit-ordered Q4_K / Q6_K matrices (the layout of gemv_sk.cu) in 16-bit activations, sm_100a.
+// Product of 1..32 rows with unit-ordered Q4_K / Q6_K matrices (the layout of gemv_sk.cu) in 16-bit activations, sm_100a.
 //
 // Decode steps of several sequences and short passes (drafted tokens, ends of prompts) multiply a few rows with matrices that stream from HBM once.
 // The bound is that stream, so nothing else may cost more than it:
@@ -12,7 +12,7 @@
 //     Q6_K code x scale is rounded once to 11 bits.  mma.sync m16n8k16 sums a 256-block in fp32; the block's d and the rows' scales are applied to the sums, and the
 //     Q4_K minima are one more mma per block, whose B fragment holds the rows' sums of 32 in two f16 parts.
 //     So neither operand is rounded to fewer bits than the f16 activation keeps (2^-12 of a block's largest value at worst, against 2^-8 of the int8 form and
-//     2^-9 of products on bf16 copies): relative error of a product against 64 bits 3e-4, int8 form 7e-3.
+//     2^-9 of products on bf16 copies): relative error of a product against 64 bits 2.1e-4 (Q4_K) and 2.6e-4 (Q6_K), int8 form 7e-3.
 //   * Work.  The launch's (group, 256-block) items are dealt out in equal contiguous shares, one CTA per SM; a group that is split between CTAs is finished by the CTA
 //     that holds its first block, which adds the others' sums in a fixed order (workspace + flag per warp, bounded wait), as in gemv_sk.cu.
 #include "pass_args.cuh"

@@ -1,4 +1,5 @@
-// Streaming quantised matrix-vector kernel for decode steps of 1..32 tokens, sm_100a.
+// Streaming quantised matrix-vector kernel for decode steps of 1..32 tokens, sm_100a.  (Engines take it up to eight; more rows go to gemm_sk.cu, but for rows above 16384 values,
+// which the pass that normalises them there does not hold.)
 //
 // In the reference stack this is ggml's mmvq family (one launch per matrix, dp4a dot products).  Here a
 // decode matrix is a linear byte stream of which every SM pulls its share at HBM speed:

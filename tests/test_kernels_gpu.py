@@ -165,7 +165,7 @@ def test_rmsnorm_bf16(k):
 
 
 @pytest.mark.parametrize("neox,qk_norm,hd,n_rot,H,Hkv,q8", [(False, False, 128, 128, 12, 2, False), (True, True, 64, 64, 9, 3, False),
-                                                          (True, False, 64, 32, 4, 2, True), (True, True, 256, 256, 3, 1, False)])
+                                                          (True, True, 128, 128, 12, 2, False), (False, True, 64, 64, 9, 3, False), (True, False, 64, 32, 4, 2, True), (True, True, 256, 256, 3, 1, False)])
 def test_rope_kv_of_a_prefill_chunk(neox, qk_norm, hd, n_rot, H, Hkv, q8):
     """Chunks of 64 tokens and more take the per-token form of the kernel (a warp per head, the sines and cosines once per token):
     rotated queries, and keys / values in the f16 or int8 cache, against the fp32 statement; positions far into a long context."""
