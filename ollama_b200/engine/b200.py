@@ -711,6 +711,9 @@ class B200Backend(StepEngine):
         """One pass over the rows of several chunks, each ``(slot, tokens, first position)`` of a different sequence: the
         projections, the feed-forward block and the cache append see one matrix of all rows, attention runs per sequence
         over its own cache rows.  Returns the hidden states of all rows in the order given."""
+        for sl, toks, p0 in segs:      # the cache append takes positions as they are: refused before anything is launched
+            if not 0 <= sl < self.n_slots or p0 < 0 or p0 + len(toks) > self.n_ctx:
+                raise ValueError(f"positions {p0}..{p0 + len(toks)} of slot {sl}: the cache has {self.n_slots} slots of {self.n_ctx}")
         c, dev = self.cfg, self.device
         flat = [max(int(t), 0) for _, toks, _ in segs for t in toks]      # negative ids stand for rows whose input comes from ``embeds``
         T = len(flat)

@@ -75,3 +75,15 @@ def test_products_of_stack_models_follow_the_engines_overlap_flag(monkeypatch, p
     Step.product(step, h, NS(w=w, bias=None), out)
     Step.enter(step, h, NS(w=w, bias=None), out)
     assert got == [("b2_gemm_rows", int(pdl))] * 4
+
+
+@pytest.mark.parametrize("segs", [[(0, [5] * 9, 56)], [(0, [5], 64)], [(2, [5], 0)], [(-1, [5], 0)], [(0, [5], -1)], [(0, [5] * 4, 0), (1, [5] * 40, 25)]])
+def test_prompt_rows_outside_the_cache_are_refused_before_a_launch(launches, segs):
+    """The cache append writes at slot and position as they come; attention, which looks at the length, follows it."""
+    from types import SimpleNamespace as NS
+
+    from ollama_b200.engine.b200 import B200Backend
+    be = NS(n_slots=2, n_ctx=64, cfg=NS(), device="cpu")
+    with pytest.raises(ValueError):
+        B200Backend._forward_rows(be, segs)
+    assert not launches.calls
