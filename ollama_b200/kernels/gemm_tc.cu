@@ -180,8 +180,8 @@ __device__ __forceinline__ void store4(const GemmParams& p, float4 r, int row, i
 }
 
 // TAIL: some columns are p.tail's.  A form of its own, since a test per stored element made all products 8 % longer.
-// PAIR: a launch of CTA pairs.  One CTA per tile is bound by what the L2 delivers to an SM, 47 to 55 bytes a cycle whatever the tile (880 cycles for the 48 KB of a 128 x 256 x 64 block
-// whose products take 512); the pair asks for 32 KB.
+// PAIR: a launch of CTA pairs.  One CTA per tile takes what the L2 delivers to an SM, 47 to 59 bytes a cycle whatever the tile (880 cycles for the 48 KB of a 128 x 256 x 64 block
+// whose products take 512; tensor pipe 61 % of the cycles); the pair asks for 32 KB (44 bytes a cycle, 68 %).
 template <int BN, bool SPLIT, bool TAIL, bool XIELU, bool PAIR>
 __global__ void __launch_bounds__(192, 1) gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                                                               const __grid_constant__ GemmParams p) {
