@@ -465,10 +465,11 @@ struct Lay2 {
 
 // D: value columns, DK: query / key columns (D unless the form is PARTS).  DIFF: a CTA takes 64 queries of a head of differential attention, rows 0 .. 63 of its tile
 // with the first map, rows 64 .. 127 with the second; the key rows hold both maps' keys, of which a query row has zeros against the other map's.
+// a.scale is above zero, qsign a factor of the queries (positive_scale).
 template <int D, int DK, int FORM, bool DIFF = false>
 __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                                                                        const __grid_constant__ AttnPrefillArgs a, const __grid_constant__ AttnPagedArgs pg,
-                                                                       const __grid_constant__ AttnPartsArgs pt) {
+                                                                       const __grid_constant__ AttnPartsArgs pt, float qsign) {
     using L = Lay2<D, DK>;
     constexpr bool PAGED = FORM != FLAT;       // query tiles come as a list, output rows have a pitch of their own
     constexpr int OH = D / 2, QH = DK / 2;
@@ -530,7 +531,13 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
 #pragma unroll
             for (int j = 0; j < QH / 8; j++) {
                 const int col = QH * c + 8 * j, atom = col >> 6, chunk = (col & 63) >> 3;
-                *(uint4*)(sQ + atom * ATOM_BYTES + r * 128 + ((chunk ^ (r & 7)) << 4)) = live ? *(const uint4*)(qp + 8 * j) : make_uint4(0, 0, 0, 0);
+                uint4 w = live ? *(const uint4*)(qp + 8 * j) : make_uint4(0, 0, 0, 0);
+                if (qsign != 1.f) {
+                    __half2* x = reinterpret_cast<__half2*>(&w);
+#pragma unroll
+                    for (int i = 0; i < 4; i++) x[i] = __hmul2(x[i], __float2half2_rn(qsign));
+                }
+                *(uint4*)(sQ + atom * ATOM_BYTES + r * 128 + ((chunk ^ (r & 7)) << 4)) = w;
             }
         } else {
         const float* qp = a.q + ((size_t)(m0 + qi) * a.H + (DIFF ? 2 * h + (r >> 6) : h)) * D + OH * c;
@@ -544,7 +551,7 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
             const int col = OH * c + 8 * j;
             const int atom = col >> 6, chunk = (col & 63) >> 3;
             *(uint4*)(sQ + atom * ATOM_BYTES + r * 128 + ((chunk ^ (r & 7)) << 4)) =
-                make_uint4(pack_h2(v0.x, v0.y), pack_h2(v0.z, v0.w), pack_h2(v1.x, v1.y), pack_h2(v1.z, v1.w));
+                make_uint4(pack_h2(qsign * v0.x, qsign * v0.y), pack_h2(qsign * v0.z, qsign * v0.w), pack_h2(qsign * v1.x, qsign * v1.y), pack_h2(qsign * v1.z, qsign * v1.w));
         }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -628,11 +635,7 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
         const int qp = q_lo + (DIFF ? r & 63 : r);
         const int row_lo = first_key(qp, chunk, window), last_lo = first_key(q_hi, chunk, window);      // this row's first key (but for kept ones); the last row's
         const float LOG2E = 1.4426950408889634f;
-        // Scores times `mult` are exponents of two; the running maximum is one of plain scores, which takes a scale above zero (the largest score is the largest exponent, a masked
-        // score of minus infinity stays one).  Other scales are multiplied in ahead of mask and maximum.
-        const float sl2 = a.scale * LOG2E;
-        const bool ahead = !(a.softcap > 0.f) && !(sl2 > 0.f);
-        const float mult = a.softcap > 0.f || ahead ? 1.f : sl2;
+        const float mult = a.softcap > 0.f ? 1.f : a.scale * LOG2E;      // scores times this are exponents of two; the running maximum is one of plain scores
         const uint32_t lane_base = (uint32_t)(32 * q) << 16;
         float o[OH];
 #pragma unroll
@@ -672,11 +675,6 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
                 for (int i = 0; i < 2; i++)
 #pragma unroll
                     for (int j = 0; j < 32; j++) v[i][j] = __float_as_uint(cap2 * tanh_exp(__uint_as_float(v[i][j]) * inv_cap));
-            } else if (ahead) {
-#pragma unroll
-                for (int i = 0; i < 2; i++)
-#pragma unroll
-                    for (int j = 0; j < 32; j++) v[i][j] = __float_as_uint(__uint_as_float(v[i][j]) * sl2);
             }
             if (masked) {
                 const int kp0 = n0 + 64 * c;
@@ -867,6 +865,16 @@ int launch(const AttnPrefillArgs& a, int n_slots, cudaStream_t st) {
     return (int)cudaGetLastError();
 }
 
+// The pipelined kernel's running maximum is one of plain scores, which takes a scale above zero: the largest score is the largest exponent, a masked one of minus infinity stays that.
+// So the sign goes to the queries, and with a scale of zero they are zeros and any other scale does.  Returns the factor.  (A branch in the softmax that multiplied such scales in
+// first, or the sign taken apart inside the kernel, cost every scale: 330 us instead of 322 for 2048 rows at 6144.)
+float positive_scale(AttnPrefillArgs& a) {
+    const float s = a.scale;
+    if (s > 0.f) return 1.f;
+    a.scale = s == 0.f ? 1.f : -s;
+    return s == 0.f ? 0.f : -1.f;
+}
+
 template <int D>
 int launch2(const AttnPrefillArgs& a, int n_slots, int pdl, cudaStream_t st) {
     CUtensorMap mk, mv;
@@ -878,7 +886,8 @@ int launch2(const AttnPrefillArgs& a, int n_slots, int pdl, cudaStream_t st) {
     AttnPrefillArgs copy = a;
     AttnPagedArgs pg = {};
     AttnPartsArgs pt = {};
-    void* args[] = {&mk, &mv, &copy, &pg, &pt};
+    float qsign = positive_scale(copy);
+    void* args[] = {&mk, &mv, &copy, &pg, &pt, &qsign};
     return launch_rows((const void*)attn_prefill_tc2_kernel<D, D, FLAT>, grid, dim3(THREADS2), Lay2<D, D>::TOTAL, args, st, pdl);
 }
 
@@ -889,7 +898,9 @@ int launch_paged(const AttnPrefillArgs& a, const AttnPagedArgs& pg, int n_tiles,
     if (!cached_kv_map(&mk, a.k_cache, rows, D, 64) || !cached_kv_map(&mv, a.v_cache, rows, D, 64)) return (int)cudaErrorNotSupported;
     static PerDeviceOnce once;
     if (once.first()) cudaFuncSetAttribute(attn_prefill_tc2_kernel<D, D, PAGED_CACHE, DIFF>, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay2<D, D>::TOTAL);
-    attn_prefill_tc2_kernel<D, D, PAGED_CACHE, DIFF><<<dim3(n_tiles, DIFF ? a.H / 2 : a.H), THREADS2, Lay2<D, D>::TOTAL, st>>>(mk, mv, a, pg, AttnPartsArgs{});
+    AttnPrefillArgs copy = a;
+    const float qsign = positive_scale(copy);
+    attn_prefill_tc2_kernel<D, D, PAGED_CACHE, DIFF><<<dim3(n_tiles, DIFF ? a.H / 2 : a.H), THREADS2, Lay2<D, D>::TOTAL, st>>>(mk, mv, copy, pg, AttnPartsArgs{}, qsign);
     return (int)cudaGetLastError();
 }
 
@@ -906,7 +917,8 @@ int launch_parts(const AttnPartsArgs& p, int n_tiles, cudaStream_t st) {
     a.scale = p.scale;
     a.window = p.window;
     a.out = p.out;
-    attn_prefill_tc2_kernel<D, DK, PARTS><<<dim3(n_tiles, p.H), THREADS2, Lay2<D, DK>::TOTAL, st>>>(mk, ms, a, AttnPagedArgs{}, p);
+    const float qsign = positive_scale(a);
+    attn_prefill_tc2_kernel<D, DK, PARTS><<<dim3(n_tiles, p.H), THREADS2, Lay2<D, DK>::TOTAL, st>>>(mk, ms, a, AttnPagedArgs{}, p, qsign);
     return (int)cudaGetLastError();
 }
 

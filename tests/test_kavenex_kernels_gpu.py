@@ -286,8 +286,9 @@ def test_absorbed_queries_and_cache_rows(ops, rank, cache32):
                 assert (q[..., d:dp] == 0).all() and (q[..., dp + rot:] == 0).all()
 
 
-@pytest.mark.parametrize("heads,dim,rot,vdim", [(2, 20, 8, 28), (3, 128, 64, 128), (1, 64, 64, 100), (4, 100, 40, 64), (2, 64, 0, 64)])
-def test_prompt_tiles_over_keys_in_two_parts(ops, heads, dim, rot, vdim):
+@pytest.mark.parametrize("heads,dim,rot,vdim,scale", [(2, 20, 8, 28, 0.8), (3, 128, 64, 128, 0.8), (1, 64, 64, 100, 0.8), (4, 100, 40, 64, 0.8), (2, 64, 0, 64, 0.8), (2, 20, 8, 28, -0.8),
+                                                      (3, 128, 64, 128, 0.0)])
+def test_prompt_tiles_over_keys_in_two_parts(ops, heads, dim, rot, vdim, scale):
     """Portions of two sequences, one with a past; single standing-out keys first, at tile borders and far away."""
     K, A, R = ops
     dp, rp, vp = up(dim, 64), up(rot, 64), up(vdim, 64)
@@ -315,7 +316,7 @@ def test_prompt_tiles_over_keys_in_two_parts(ops, heads, dim, rot, vdim):
         tiles += [(row0 + t, min(128, n - t), base, past + t) for t in range(0, n, 128)]
         base, row0 = base + past + n, row0 + n
     out = torch.full((rows, heads * vdim + 4), 9.0, dtype=torch.bfloat16, device="cuda")
-    A.attn_prefill_parts(q, kv, sh, torch.tensor(tiles, dtype=torch.int32).cuda(), out, heads=heads, dp=dp, vp=vp, rp=rp, vdim=vdim, scale=0.8)
+    A.attn_prefill_parts(q, kv, sh, torch.tensor(tiles, dtype=torch.int32).cuda(), out, heads=heads, dp=dp, vp=vp, rp=rp, vdim=vdim, scale=scale)
     base = row0 = 0
     for past, n in lens:
         T = past + n
@@ -323,7 +324,7 @@ def test_prompt_tiles_over_keys_in_two_parts(ops, heads, dim, rot, vdim):
             s = q[row0:row0 + n, h, :dp].double() @ k[base:base + T, h].double().t()
             if rot:
                 s += q[row0:row0 + n, h, dp:].double() @ sh[base:base + T, :rp].double().t()
-            s = (s * 0.8).masked_fill(torch.ones(n, T).triu(past + 1).bool().cuda(), -math.inf)
+            s = (s * scale).masked_fill(torch.ones(n, T).triu(past + 1).bool().cuda(), -math.inf)
             close(out[row0:row0 + n, h * vdim:(h + 1) * vdim], torch.softmax(s, -1) @ v[base:base + T, h, :vdim].double(), 1e-2)
         base, row0 = base + T, row0 + n
     assert (out[:, heads * vdim:] == 9.0).all()
