@@ -324,7 +324,8 @@ __global__ void __launch_bounds__(192, 3) moe_fp4_kernel(const __grid_constant__
                 mbar_expect_tx(&full_s, bytes);
                 asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(scales)),
                              "l"(a.s + ((size_t)e * a.n + row0) * blocks), "r"(bytes), "r"(smem_u32(&full_s)) : "memory");
-                for (int st = 0; st < steps && ok; st++) {
+                int st = 0;
+                for (; st < steps; st++) {
                     const int stage = st % STAGES;
                     if (st >= STAGES) ok = mbar_wait(&empty[stage], (st / STAGES - 1) & 1);
                     if (!ok) break;
@@ -332,11 +333,16 @@ __global__ void __launch_bounds__(192, 3) moe_fp4_kernel(const __grid_constant__
                     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(xs + stage * X_STAGE)),
                                  "l"(src + (size_t)st * XB), "r"(XB), "r"(smem_u32(&full_x[stage])) : "memory");
                 }
-                if (!ok) s_failed = 1;
+                if (!ok) {      // copies under way land before the CTA leaves
+                    s_failed = 1;
+                    mbar_wait(&full_s, 0);
+                    for (int i = st - STAGES; i < st; i++) mbar_wait(&full_x[i % STAGES], (i / STAGES) & 1);
+                }
             }
         } else if (lane == 0) {
             bool ok = true;
-            for (int st = 0; st < steps && ok; st++) {
+            int st = 0;
+            for (; st < steps; st++) {
                 const int stage = st % STAGES, phase = (st / STAGES) & 1;
                 ok = mbar_wait(&full_x[stage], phase) && mbar_wait(&full_a[stage], phase);
                 if (!ok) break;
@@ -350,8 +356,13 @@ __global__ void __launch_bounds__(192, 3) moe_fp4_kernel(const __grid_constant__
                 for (int b = 0; b < 4; b++) umma_mx(tmem, adesc + 2 * b, bdesc + 2 * b, mx_idesc(N, b), ta, tb, st != 0 || b != 0);
                 umma_commit(&empty[stage]);
             }
-            if (ok) umma_commit(&done);
-            else s_failed = 1;
+            if (ok) {
+                umma_commit(&done);
+            } else {      // products under way end, and copies that the other warp asked for, before the CTA leaves
+                s_failed = 1;
+                for (int i = max(0, st - STAGES); i < st; i++) mbar_wait(&empty[i % STAGES], (i / STAGES) & 1);
+                for (int i = st; i < min(st + STAGES, steps); i++) mbar_wait(&full_x[i % STAGES], (i / STAGES) & 1);
+            }
         }
     }
     __syncthreads();
