@@ -821,9 +821,7 @@ def test_router_of_a_prompt(T, E, d):
         got.append(logits.clone())
         raise Enough
 
-    hi = w.to(torch.bfloat16)
-    mid = (w - hi.float()).to(torch.bfloat16)
-    L = SimpleNamespace(router_f32=w, router=SimpleNamespace(bias=bias), router_3=torch.cat([hi, mid, (w - hi.float() - mid.float()).to(torch.bfloat16)]))
+    L = SimpleNamespace(router_f32=w, router=SimpleNamespace(bias=bias))
     be = SimpleNamespace(cfg=SimpleNamespace(d_model=d, n_experts=E, n_experts_used=1), device="cuda", pdl=True, kernel_launches=0, _route=route)
     with pytest.raises(Enough):
         B200Backend._moe_prefill(be, h, L)
