@@ -36,13 +36,11 @@ from .steps import StepEngine
 
 MAX_DECODE_BATCH = 8             # sequences per launch of the dp4a kernels (kernels/gemv.cu)
 MAX_STREAM_BATCH = 32            # sequences per step when every matrix runs on the streaming kernel (kernels/gemv_sk.cu)
-# Steps of more sequences than this multiply f16 activations (kernels/gemm_sk.cu) instead of int8 ones.  Products of a layer of Llama-8B (Q4_K_M), int8 against f16: 52 us against
-# 74 at one sequence, 70 against 74 at six, 76 against 74 at eight, 109 against 81 at nine, 121 against 81 at thirteen, 205 against 112 at 32.
-INT8_ROWS = 8
-# Prompt passes of at most this many rows read the units too, 32 rows a launch, instead of the 16-bit copies (a layer of Llama-8B: 124 MB against 436).  Twelve layers and the logits
-# of one row, units against copies: 1350 us against 2240 at 7 rows, 1830 against 2310 at 32, but 2730 against 2310 at 33 and 3230 against 2370 at 64.  From 33 rows on it is the
-# rows' 16 bits that count: the logits are 0.0007 off the graph in 64 bits, 0.0045 on bf16 rows and copies.
-UNIT_ROWS = 64
+# Steps of more sequences than this multiply f16 activations (kernels/gemm_sk.cu) instead of int8 ones.  Products of a layer of Llama-8B (Q4_K_M), int8 against f16: 53 us against
+# 60 at one sequence, 71 against 60 at two, 74 against 63 at seven, 76 against 63 at eight.
+INT8_ROWS = 1
+# Prompt passes of at most this many rows, which is one launch a product, read the units too instead of the 16-bit copies (a layer of Llama-8B: 124 MB against 436).
+UNIT_ROWS = SK.ROWS16_MAX
 # Steps of at least so many (token, expert) pairs, and of one for every eighth expert, read MXFP4 experts once for all rows that chose them (kernels/moe_fp4.cu), smaller ones
 # once per pair: a layer of 128 experts of 13 MB, four a token, takes 72 us against 75 at four tokens and 194 against 280 at sixteen, but 45 against 29 at one.
 FP4_MIN_PAIRS = 16
@@ -530,10 +528,10 @@ class B200Backend(StepEngine):
         self._n += 1
 
     def _rows_sk(self, ws, x: torch.Tensor, out: torch.Tensor, norm_w=None, mode: int = SK.MODE_STORE, buf: torch.Tensor | None = None, wsp=None) -> None:
-        """Rows times unit-ordered matrices in f16 activations, 32 rows a launch: ``out`` stored / added to / gated."""
+        """Rows times unit-ordered matrices in f16 activations, 64 rows a launch: ``out`` stored / added to / gated."""
         c = self.cfg
-        for r in range(0, x.shape[0], SK.MAX_TOKENS):
-            xs = x[r:r + SK.MAX_TOKENS]
+        for r in range(0, x.shape[0], SK.ROWS16_MAX):
+            xs = x[r:r + SK.ROWS16_MAX]
             x16 = SK.rows16(xs, norm_w, c.norm_eps, out=buf, pdl=self.pdl)
             SK.gemm16(ws, x16, xs.shape[0], out=out[r:], mode=mode, act=c.act, alpha=c.swiglu_alpha, limit=c.swiglu_limit, pdl=self.pdl, ws=wsp)
 

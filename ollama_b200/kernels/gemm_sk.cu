@@ -1,30 +1,44 @@
-// Product of 1..32 rows with unit-ordered Q4_K / Q6_K matrices (the layout of gemv_sk.cu) in 16-bit activations, sm_100a.
+// Product of 1..64 rows with unit-ordered Q4_K / Q6_K matrices (the layout of gemv_sk.cu) in 16-bit activations, sm_100a.
 //
 // Decode steps of several sequences and short passes (drafted tokens, ends of prompts) multiply a few rows with matrices that stream from HBM once.
 // The bound is that stream, so nothing else may cost more than it:
-//   * Activations.  b2_rows16 turns fp32 or bf16 rows (optionally RMS-normalised) into f16 values with one power-of-two scale per row and 256-block, stored in the
-//     order in which the lanes of a warp load tensor-core B fragments: [256-block][8 rows][...].  One 256-block of all rows is one contiguous chunk of 4384 bytes per
-//     eight rows that a producer warp copies into shared memory once per CTA (cp.async.bulk, a ring of chunks); all 16 warps of the CTA read it with
-//     conflict-free 16-byte loads.  (The int8 form that this replaces gathered its operand as 4-byte words through L1: per unit of 2.4 KB a warp fetched 8 KB in
-//     sectors of 16 used bytes at 32 rows, and a launch took 69 us where its weights stream in 10.)
-//   * Weights.  Each warp owns one 16-row tile per group of 16 tiles and streams its units through a cp.async ring of its own, requested before the grid-dependency wait.
-//     Codes become f16 A fragments in registers: a 4-bit code under the exponent of 1024 and one fused multiply-add give code x 6-bit scale exactly (at most 945); of
-//     Q6_K code x scale is rounded once to 11 bits.  mma.sync m16n8k16 sums a 256-block in fp32; the block's d and the rows' scales are applied to the sums, and the
-//     Q4_K minima are one more mma per block, whose B fragment holds the rows' sums of 32 in two f16 parts.
+//   * Matrix instructions.  tcgen05.mma kind::f16, M = 128 matrix rows, N = the activation rows (16, 32, 48 or 64), K = a 256-block: its cost hardly depends on the rows (25 cycles
+//     for 16 columns of K at 16 and 32 rows, 35 at 64), so the expansion of the codes is what an item costs beside its bytes.
+//   * Weights.  An item is 128 matrix rows x 256 columns: eight units, which bulk copies bring into a ring that is filled before the grid-dependency wait.  16 warps expand them, one
+//     unit of every second item each.  Codes become f16 in registers: a 4-bit code under the exponent of 1024 or 64 and one fused multiply-add give code x 6-bit scale exactly
+//     (at most 945); of Q6_K code x scale is rounded once to 11 bits.  They go to tensor memory as the A operand (tcgen05.st.16x128b: lane (g, t) writes rows g and g + 8, words
+//     t of every four, which is how the units are dealt to lanes), not to shared memory: 64 KB an item written there and read again would take longer than the item's 19 KB
+//     from HBM.  K is permuted inside a 64-column group by that; the activations are stored in the same order.
+//   * Activations.  b2_rows16 turns fp32 or bf16 rows (optionally RMS-normalised) into f16 values with one power-of-two scale per row and 256-block, in the 128-byte-swizzled
+//     order of the B operand, so that a 256-block of all rows is one bulk copy.
+//   * Sums.  The accumulators of a 256-block are read back by four warps (a thread a matrix row), which apply the block's d and the rows' scales in fp32 and add up; the Q4_K
+//     minima are one more product per block (A: the minima twice, B: the rows' sums of 32 in two f16 parts) into columns of its own.
 //     So neither operand is rounded to fewer bits than the f16 activation keeps (2^-12 of a block's largest value at worst, against 2^-8 of the int8 form and
 //     2^-9 of products on bf16 copies): relative error of a product against 64 bits 2.1e-4 (Q4_K) and 2.6e-4 (Q6_K), int8 form 7e-3.
-//   * Work.  The launch's (group, 256-block) items are dealt out in equal contiguous shares, one CTA per SM; a group that is split between CTAs is finished by the CTA
-//     that holds its first block, which adds the others' sums in a fixed order (workspace + flag per warp, bounded wait), as in gemv_sk.cu.
+//   * Measured (Llama-8B layer, q/k/v + output + gate/up + down with the four b2_rows16 before them, Q4_K_M): 60 us at 2 rows, 65 at 16, 76 at 32, 104 at 64, where mma.sync fragments
+//     expanded in registers took 74, 81, 113 and 226 (two launches), and 124 MB stream in 19.  What is left: 1100 cycles an item of 128 x 256 (expansion issues for 70 % of them), 2000
+//     to 4000 cycles a launch until the first sums, and as many to exchange those of split groups.
+//   * Work.  The launch's items are dealt out in equal contiguous shares, one CTA per SM; a group of 128 rows that is split between CTAs is finished by the CTA
+//     that holds its first block, which adds the others' sums in a fixed order (workspace + flag, bounded wait), as in gemv_sk.cu.
 #include "pass_args.cuh"
+#include "tc_common.cuh"
 
 namespace {
 
-constexpr int SG_WARPS = 16;                        // consumer warps = row tiles of a group
-constexpr int SG_THREADS = (SG_WARPS + 1) * 32;     // and the producer warp
+using namespace tc;
+constexpr int SG_TILES = 8;                                    // 16-row tiles of a group
+// Warps: 16 that expand, in two teams of eight (a team takes every second item, a warp of it one group of 16 rows), 4 that add up, one each for the products of even and of
+// odd items, the activations, the units of even and of odd items, and 3 that finish the rows of a group while the next one is under way.  72 registers a thread at the launch; the
+// last eight warps leave 32 of theirs to those that add up.
+constexpr int SG_EXPAND = 16, SG_SUM = 4, SG_FINISH = 3, SG_THREADS = (SG_EXPAND + SG_SUM + 5 + SG_FINISH) * 32;
+enum { SG_MMA = SG_EXPAND + SG_SUM, SG_LOAD_X = SG_MMA + 2, SG_LOAD_W = SG_LOAD_X + 1, SG_LAST = SG_LOAD_W + 2 };
 constexpr int SG_UNIT_Q4K = 2368, SG_UNIT_Q6K = 3360;
-constexpr int SG_FRAG = 4096, SG_SUMS = 256, SG_CHUNK = SG_FRAG + SG_SUMS + 32;      // bytes per 256-block and eight rows: values, sums of 32, scales
-constexpr int SG_WS_FLOATS = 16 * 32;
-constexpr int SG_MAX_SMEM = 225 * 1024;
+constexpr int SG_ROW = 544, SG_CHUNK = 16 * (SG_ROW + 4);      // bytes of a row's 256-block: values and sums of 32; with the scales of 16 rows
+constexpr int SG_MAX_ROWS = 64, SG_MAX_NT = SG_MAX_ROWS / 16;
+constexpr int SG_WS_FLOATS = 128 * SG_MAX_ROWS;                // a CTA's share of the workspace
+constexpr int SG_MAX_SMEM = 224 * 1024;
+constexpr int SG_SCALE_SLOTS = 8, SG_D_SLOTS = 8, SG_W_SLOTS = 10, SG_X_SLOTS = 4;
+constexpr int SG_A_COLS = 136;                                 // TMEM columns of an item's expanded weights: 256 / 2 of codes x scales, 16 / 2 of minima
 constexpr unsigned long long SG_WAIT_NS = 1000000000ull;
 
 __device__ __forceinline__ unsigned long long now_ns() {
@@ -32,27 +46,30 @@ __device__ __forceinline__ unsigned long long now_ns() {
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     return t;
 }
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void bar_init(uint64_t* bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory"); }
-__device__ __forceinline__ void bar_arrive(uint64_t* bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory"); }
-__device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity) {      // bounded: about a second
+// Bounded wait of about a second, as mbar_wait: a rolled loop, because the code of all roles has to stay in the instruction caches (unrolled waits, activations and halves of a
+// block made it 136 KB).
+__device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity) {
+    if (mbar_try_wait(bar, parity)) return true;
+#pragma unroll 1
     for (int i = 0; i < (1 << 22); i++) {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok) : "r"(smem_addr(bar)), "r"(parity) : "memory");
-        if (ok) return true;
+        if (mbar_try_wait(bar, parity)) return true;
         if (i > 128) __nanosleep(100);
     }
     return false;
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory"); }
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
     unsigned v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void st_release(unsigned* p, unsigned v) { asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
-__device__ __forceinline__ void cp16(uint32_t dst, const void* src, uint64_t policy) {
-    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "l"(policy) : "memory");
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar, uint64_t policy) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(policy) : "memory");
 }
 __device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
     uint32_t d;
@@ -69,141 +86,135 @@ __device__ __forceinline__ uint32_t h2_add(uint32_t a, uint32_t b) {
     asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
 }
-__device__ __forceinline__ void mma16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+// two fp32 values as one operand of the packed instructions
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pack2(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ f2 pack2u(uint32_t a, uint32_t b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    f2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
 }
 
-// f16x2 constants: 1024 under a code, and what takes it (times a scale) away again
-constexpr uint32_t H_1024 = 0x64006400u, H_M1024 = 0xE400E400u, H_M64 = 0xD400D400u, H_16TH = 0x2C002C00u, H_M1152 = 0xE480E480u, H_QUARTER = 0x34003400u,
-                   H_M288 = 0xDC80DC80u;
+// f16 operands, both K-major
+__host__ __device__ constexpr uint32_t sg_idesc(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24); }
 
-// byte b of w (0..255) twice as f16x2, 1024 added
-__device__ __forceinline__ uint32_t byte_h2(uint32_t w, int b) { return __byte_perm(w, H_1024, 0x5050 | b | (b << 8)); }
-
-}  // namespace
-
-namespace {
-
-// Sums of one unit (16 rows x 256 columns) with all rows of the chunk.  `xc`: the chunk in shared memory.
-template <int NT>
-__device__ __forceinline__ void unit16_q4k(const uint8_t* sp, const uint8_t* xc, int lane, float (&facc)[NT][4]) {
-    const int g = lane >> 2, t = lane & 3;
-    const uint4 sg = reinterpret_cast<const uint4*>(sp + 2048)[g], sh = reinterpret_cast<const uint4*>(sp + 2048)[g + 8];
-    const float2 dg = __half22float2(reinterpret_cast<const __half2*>(sp + 2304)[g]);
-    const float2 dh = __half22float2(reinterpret_cast<const __half2*>(sp + 2304)[g + 8]);
-    const uint4* xf = reinterpret_cast<const uint4*>(xc) + lane;
-    float acc[NT == 1 ? 2 : NT][4];      // one group of rows: two chains of dependent products
-#pragma unroll
-    for (int n = 0; n < (NT == 1 ? 2 : NT); n++)
-#pragma unroll
-        for (int i = 0; i < 4; i++) acc[n][i] = 0.f;
-#pragma unroll
-    for (int p = 0; p < 4; p++) {
-        const uint4 w = reinterpret_cast<const uint4*>(sp)[p * 32 + lane];
-        const uint4 v = make_uint4(w.x >> 8, w.y >> 8, w.z >> 8, w.w >> 8);
-        const uint32_t scg = p < 2 ? sg.x : sg.y, sch = p < 2 ? sh.x : sh.y;
-#pragma unroll
-        for (int half = 0; half < 2; half++) {      // low nibbles: sub-block 2p, high nibbles: 2p + 1
-            const int b = ((2 * p) & 3) + half;
-            const uint32_t mask = half ? 0x00f000f0u : 0x000f000fu;
-            const uint32_t s0 = h2_add(byte_h2(scg, b), H_M1024), s1 = h2_add(byte_h2(sch, b), H_M1024);
-            const uint32_t mg = half ? h2_mul(s0, H_16TH) : s0, mh = half ? h2_mul(s1, H_16TH) : s1;
-            const uint32_t cg = h2_mul(s0, half ? H_M64 : H_M1024), ch = h2_mul(s1, half ? H_M64 : H_M1024);
-            const uint32_t a0 = h2_fma((w.x & mask) | H_1024, mg, cg), a1 = h2_fma((w.y & mask) | H_1024, mh, ch);
-            const uint32_t a2 = h2_fma((v.x & mask) | H_1024, mg, cg), a3 = h2_fma((v.y & mask) | H_1024, mh, ch);
-            const uint32_t e0 = h2_fma((w.z & mask) | H_1024, mg, cg), e1 = h2_fma((w.w & mask) | H_1024, mh, ch);
-            const uint32_t e2 = h2_fma((v.z & mask) | H_1024, mg, cg), e3 = h2_fma((v.w & mask) | H_1024, mh, ch);
-#pragma unroll
-            for (int n = 0; n < NT; n++) {
-                const uint4 bv = xf[n * (SG_FRAG / 16) + (2 * p + half) * 32];
-                mma16(acc[n], a0, a1, a2, a3, bv.x, bv.y);
-                mma16(acc[NT == 1 ? 1 : n], e0, e1, e2, e3, bv.z, bv.w);
-            }
-        }
-    }
-    // minima 2t, 2t + 1 of both rows; k slots 0..7 meet the upper, 8..15 the lower parts of the sums of 32
-    const uint32_t wg = (t < 2 ? sg.z : sg.w) >> (16 * (t & 1)), wh = (t < 2 ? sh.z : sh.w) >> (16 * (t & 1));
-    const uint32_t m0 = h2_add(__byte_perm(wg, H_1024, 0x5150), H_M1024), m1 = h2_add(__byte_perm(wh, H_1024, 0x5150), H_M1024);
-    const uint2* xs = reinterpret_cast<const uint2*>(xc + NT * SG_FRAG) + lane;
-    const float2* xd = reinterpret_cast<const float2*>(xc + NT * (SG_FRAG + SG_SUMS)) + t;
-#pragma unroll
-    for (int n = 0; n < NT; n++) {
-        const uint2 bv = xs[n * 32];
-        float am[4] = {0.f, 0.f, 0.f, 0.f};
-        mma16(am, m0, m1, m0, m1, bv.x, bv.y);
-        const float2 d = xd[n * 4];
-        if (NT == 1) {
-#pragma unroll
-            for (int i = 0; i < 4; i++) acc[0][i] += acc[1][i];
-        }
-        facc[n][0] += d.x * (dg.x * acc[n][0] - dg.y * am[0]);
-        facc[n][1] += d.y * (dg.x * acc[n][1] - dg.y * am[1]);
-        facc[n][2] += d.x * (dh.x * acc[n][2] - dh.y * am[2]);
-        facc[n][3] += d.y * (dh.x * acc[n][3] - dh.y * am[3]);
-    }
+// K-major operand without swizzle: cells of eight rows x 16 bytes are contiguous, `lbo` bytes apart along K and 128 along the rows.
+__device__ __forceinline__ uint64_t desc_cells(uint32_t addr, uint32_t lbo) {
+    return (uint64_t)((addr & 0x3FFFF) >> 4) | (uint64_t)(lbo >> 4) << 16 | (uint64_t)(128 >> 4) << 32 | (uint64_t)1 << 46;
+}
+__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {      // A in tensor memory
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                 ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ bool elect() {      // the same lane of a warp every time
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e != 0;
+}
+// 16 rows x 32 words: register 2 j of lane (g, t) is word 4 j + t of row g, register 2 j + 1 of row g + 8
+__device__ __forceinline__ void tmem_st_16x128_x8(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]),
+                 "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+}
+__device__ __forceinline__ void tmem_st_16x128_x2(uint32_t taddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x2.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
+                   "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]) : "r"(taddr));
 }
 
-template <int NT>
-__device__ __forceinline__ void unit16_q6k(const uint8_t* sp, const uint8_t* xc, int lane, float (&facc)[NT][4]) {
-    const int g = lane >> 2, t = lane & 3;
-    const uint4 sg4 = reinterpret_cast<const uint4*>(sp + 3072)[g], sh4 = reinterpret_cast<const uint4*>(sp + 3072)[g + 8];
-    const uint32_t sg[4] = {sg4.x ^ 0x80808080u, sg4.y ^ 0x80808080u, sg4.z ^ 0x80808080u, sg4.w ^ 0x80808080u};
-    const uint32_t sh[4] = {sh4.x ^ 0x80808080u, sh4.y ^ 0x80808080u, sh4.z ^ 0x80808080u, sh4.w ^ 0x80808080u};
-    const float dg = __half2float(reinterpret_cast<const __half*>(sp + 3328)[g]), dh = __half2float(reinterpret_cast<const __half*>(sp + 3328)[g + 8]);
-    const uint4* xf = reinterpret_cast<const uint4*>(xc) + lane;
-    float acc[NT == 1 ? 2 : NT][4];
-#pragma unroll
-    for (int n = 0; n < (NT == 1 ? 2 : NT); n++)
-#pragma unroll
-        for (int i = 0; i < 4; i++) acc[n][i] = 0.f;
+// f16x2 constants: 1024 or 64 under a code, and what takes it (times a scale) away again
+constexpr uint32_t H_1024 = 0x64006400u, H_M1024 = 0xE400E400u, H_64 = 0x54005400u, H_M1024_M64 = 0xD400E400u, H_M1152 = 0xE480E480u, H_QUARTER = 0x34003400u, H_M288 = 0xDC80DC80u;
+
+__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {      // (a & b) | c; written as such it became two instructions
+    uint32_t d;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+// one half twice: an operand form of the packed instructions
+__device__ __forceinline__ uint32_t lower2(uint32_t v) {
+    uint32_t d;
+    asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tmov.b32 %0, {l, l};\n\t}" : "=r"(d) : "r"(v));
+    return d;
+}
+__device__ __forceinline__ uint32_t upper2(uint32_t v) {
+    uint32_t d;
+    asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tmov.b32 %0, {h, h};\n\t}" : "=r"(d) : "r"(v));
+    return d;
+}
+
+// 64 columns of a Q4_K unit (sub-blocks 2p from the low, 2p + 1 from the high nibbles) as 16 words: [j][row g, row g + 8]; `B`: byte of the first sub-block's scale in scg / sch.
+// A low nibble stands under the exponent of 1024 (code + 1024), a high one under that of 64 (code + 64): both times the scale, less 1024 or 64 scales.
+template <int B>
+__device__ __forceinline__ void expand_q4k(const uint4 w, uint32_t scg, uint32_t sch, uint32_t (&r)[16]) {
+    const uint4 v = make_uint4(w.x >> 8, w.y >> 8, w.z >> 8, w.w >> 8);
+    const uint32_t sg = h2_add(__byte_perm(scg, H_1024, 0x5050 | B | ((B + 1) << 8)), H_M1024), sh = h2_add(__byte_perm(sch, H_1024, 0x5050 | B | ((B + 1) << 8)), H_M1024);
+    const uint32_t kg = h2_mul(sg, H_M1024_M64), kh = h2_mul(sh, H_M1024_M64);
 #pragma unroll
     for (int half = 0; half < 2; half++) {
-        uint32_t W[12];
+        const uint32_t mask = half ? 0x00f000f0u : 0x000f000fu, under = half ? H_64 : H_1024;
+        const uint32_t mg = half ? upper2(sg) : lower2(sg), mh = half ? upper2(sh) : lower2(sh), cg = half ? upper2(kg) : lower2(kg), ch = half ? upper2(kh) : lower2(kh);
+        uint32_t* o = r + 8 * half;
+        o[0] = h2_fma(and_or(w.x, mask, under), mg, cg);
+        o[1] = h2_fma(and_or(w.y, mask, under), mh, ch);
+        o[2] = h2_fma(and_or(v.x, mask, under), mg, cg);
+        o[3] = h2_fma(and_or(v.y, mask, under), mh, ch);
+        o[4] = h2_fma(and_or(w.z, mask, under), mg, cg);
+        o[5] = h2_fma(and_or(w.w, mask, under), mh, ch);
+        o[6] = h2_fma(and_or(v.z, mask, under), mg, cg);
+        o[7] = h2_fma(and_or(v.w, mask, under), mh, ch);
+    }
+}
+// The same of a Q6_K unit, from six code words; `sg`, `sh`: the words that hold the scales of its four 16-wide sub-blocks of rows g and g + 8, 128 added to every byte.
+__device__ __forceinline__ void expand_q6k(const uint32_t* W, uint32_t sg, uint32_t sh, uint32_t (&r)[16]) {
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-            const uint4 v = reinterpret_cast<const uint4*>(sp)[(3 * half + c) * 32 + lane];
-            W[4 * c] = v.x; W[4 * c + 1] = v.y; W[4 * c + 2] = v.z; W[4 * c + 3] = v.w;
-        }
+    for (int G = 0; G < 2; G++) {
+        const uint32_t w0 = W[3 * G], w1 = W[3 * G + 1], w2 = W[3 * G + 2];
+        const uint32_t w3 = ((w0 << 6) & 0xc0c0c0c0u) | ((w1 << 4) & 0x30303030u) | ((w2 << 2) & 0x0c0c0c0cu);
+        // bytes 4 (q - 32) + 128 under 1024: times scale / 4, less 288 scales
+        const uint32_t r0 = (w0 & 0xfcfcfcfcu) ^ 0x80808080u, r1 = (w1 & 0xfcfcfcfcu) ^ 0x80808080u, r2 = (w2 & 0xfcfcfcfcu) ^ 0x80808080u, r3 = w3 ^ 0x80808080u;
+        const uint32_t s0 = h2_add(__byte_perm(sg, H_1024, G ? 0x5352 : 0x5150), H_M1152), s1 = h2_add(__byte_perm(sh, H_1024, G ? 0x5352 : 0x5150), H_M1152);
+        const uint32_t m0 = h2_mul(s0, H_QUARTER), m1 = h2_mul(s1, H_QUARTER), c0 = h2_mul(s0, H_M288), c1 = h2_mul(s1, H_M288);
 #pragma unroll
-        for (int G2 = 0; G2 < 4; G2++) {
-            const uint32_t w0 = W[3 * G2], w1 = W[3 * G2 + 1], w2 = W[3 * G2 + 2];
-            const uint32_t w3 = ((w0 << 6) & 0xc0c0c0c0u) | ((w1 << 4) & 0x30303030u) | ((w2 << 2) & 0x0c0c0c0cu);
-            // bytes 4 (q - 32) + 128 under 1024: times scale / 4, less 288 scales
-            const uint32_t r0 = (w0 & 0xfcfcfcfcu) ^ 0x80808080u, r1 = (w1 & 0xfcfcfcfcu) ^ 0x80808080u, r2 = (w2 & 0xfcfcfcfcu) ^ 0x80808080u, r3 = w3 ^ 0x80808080u;
-            uint32_t a[2][4];
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int j = 8 * half + 2 * G2 + h;
-                const uint32_t s0 = h2_add(byte_h2(sg[j >> 2], j & 3), H_M1152), s1 = h2_add(byte_h2(sh[j >> 2], j & 3), H_M1152);
-                const uint32_t m0 = h2_mul(s0, H_QUARTER), m1 = h2_mul(s1, H_QUARTER), c0 = h2_mul(s0, H_M288), c1 = h2_mul(s1, H_M288);
-                const uint32_t x0 = h ? r2 : r0, x1 = h ? r3 : r1;
-                a[h][0] = h2_fma(__byte_perm(x0, H_1024, 0x5250), m0, c0);
-                a[h][1] = h2_fma(__byte_perm(x1, H_1024, 0x5250), m1, c1);
-                a[h][2] = h2_fma(__byte_perm(x0, H_1024, 0x5351), m0, c0);
-                a[h][3] = h2_fma(__byte_perm(x1, H_1024, 0x5351), m1, c1);
-            }
-#pragma unroll
-            for (int n = 0; n < NT; n++) {
-                const uint4 bv = xf[n * (SG_FRAG / 16) + (4 * half + G2) * 32];
-                mma16(acc[n], a[0][0], a[0][1], a[0][2], a[0][3], bv.x, bv.y);
-                mma16(acc[NT == 1 ? 1 : n], a[1][0], a[1][1], a[1][2], a[1][3], bv.z, bv.w);
-            }
+        for (int h = 0; h < 2; h++) {
+            const uint32_t x0 = h ? r2 : r0, x1 = h ? r3 : r1;
+            const uint32_t mg = h ? upper2(m0) : lower2(m0), mh = h ? upper2(m1) : lower2(m1), cg = h ? upper2(c0) : lower2(c0), ch = h ? upper2(c1) : lower2(c1);
+            uint32_t* o = r + 8 * G + 4 * h;
+            o[0] = h2_fma(__byte_perm(x0, H_1024, 0x5250), mg, cg);
+            o[1] = h2_fma(__byte_perm(x1, H_1024, 0x5250), mh, ch);
+            o[2] = h2_fma(__byte_perm(x0, H_1024, 0x5351), mg, cg);
+            o[3] = h2_fma(__byte_perm(x1, H_1024, 0x5351), mh, ch);
         }
     }
-    const float2* xd = reinterpret_cast<const float2*>(xc + NT * (SG_FRAG + SG_SUMS)) + t;
-#pragma unroll
-    for (int n = 0; n < NT; n++) {
-        const float2 d = xd[n * 4];
-        if (NT == 1) {
-#pragma unroll
-            for (int i = 0; i < 4; i++) acc[0][i] += acc[1][i];
-        }
-        facc[n][0] += d.x * dg * acc[n][0];
-        facc[n][1] += d.y * dg * acc[n][1];
-        facc[n][2] += d.x * dh * acc[n][2];
-        facc[n][3] += d.y * dh * acc[n][3];
-    }
+}
+// Columns 64 P .. of a Q6_K unit, `g`, `h`: the words that hold their sub-blocks' scales.
+template <int P>
+__device__ __forceinline__ void part_q6k(const uint8_t* sp, int lane, uint32_t g, uint32_t h, uint32_t (&r)[16]) {
+    const uint4 u = reinterpret_cast<const uint4*>(sp)[(P * 3 / 2) * 32 + lane], v = reinterpret_cast<const uint4*>(sp)[(P * 3 / 2 + 1) * 32 + lane];
+    const uint32_t lo[6] = {u.x, u.y, u.z, u.w, v.x, v.y}, hi[6] = {u.z, u.w, v.x, v.y, v.z, v.w};
+    expand_q6k(P & 1 ? hi : lo, g ^ 0x80808080u, h ^ 0x80808080u, r);
 }
 
 // Which matrix a 16-row tile of the launch belongs to, and its first unit.
@@ -233,220 +244,455 @@ __device__ __forceinline__ TileAt tile_at(const SgArgs& a, int tile, int kts) {
 // First item of CTA c of n; total * n fits 32 bits (checked by the launcher).
 __device__ __forceinline__ int share(int c, int total, int n) { return (int)((unsigned)c * (unsigned)total / (unsigned)n); }
 
-template <int NT>
-__global__ void __launch_bounds__(SG_THREADS, 1) gemm_sk_kernel(const __grid_constant__ SgArgs a) {
-    extern __shared__ __align__(128) uint8_t smem[];
-    __shared__ __align__(8) uint64_t full[4], empty[4];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int kts = a.k >> 8, total = (a.tiles + SG_WARPS - 1) / SG_WARPS * kts;
-    const int lo = share(blockIdx.x, total, gridDim.x), hi = share(blockIdx.x + 1, total, gridDim.x);
-    constexpr int CHUNK = NT * SG_CHUNK;
-    const int XS = a.x_slots;
-    uint8_t* xring = smem;
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < 4; s++) {
-            bar_init(&full[s], 1);
-            bar_init(&empty[s], SG_WARPS);
-        }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    pdl_launch();
-    if (warp == SG_WARPS) {
-        pdl_wait();
-        if (lane == 0) {
-            int s = 0, kb = lo % kts;
-            uint32_t turn = 0;
-            for (int it = lo; it < hi; it++) {
-                if (turn > 0 && !bar_wait(&empty[s], (turn - 1) & 1)) {
-                    *(volatile int*)a.status = KS_TIMEOUT;
-                    break;
-                }
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&full[s])), "r"(CHUNK) : "memory");
-                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                             ::"r"(smem_addr(xring + s * CHUNK)), "l"(a.x + (size_t)kb * CHUNK), "r"(CHUNK), "r"(smem_addr(&full[s])) : "memory");
-                if (++kb == kts) kb = 0;
-                if (++s == XS) {
-                    s = 0;
-                    turn++;
-                }
-            }
-        }
-        return;
-    }
-    // this warp's units, requested R - 1 items ahead
-    const int R = a.ring;
-    uint8_t* ring = smem + XS * CHUNK + (size_t)warp * R * a.slot_bytes;
-    uint64_t policy;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
-    int in_it = lo, in_slot = 0, in_kb = lo % kts, in_tile = lo / kts * SG_WARPS + warp;
-    const uint8_t* in_p = nullptr;
-    bool in_new = true, in_q6 = false;
-    const uint32_t ring_lane = smem_addr(ring) + lane * 16;
-    auto request = [&]() {
-        if (in_it < hi) {
-            if (in_new) {
-                in_p = nullptr;
-                if (in_tile < a.tiles) {
-                    const TileAt ta = tile_at(a, in_tile, kts);
-                    in_q6 = ta.ub == SG_UNIT_Q6K;
-                    in_p = ta.p + (size_t)in_kb * ta.ub + lane * 16;
-                }
-                in_new = false;
-            }
-            if (in_p) {
-                const uint32_t dst = ring_lane + in_slot * a.slot_bytes;
-#pragma unroll
-                for (int i = 0; i < 4; i++) cp16(dst + i * 512, in_p + i * 512, policy);
-                if (in_q6) {
-#pragma unroll
-                    for (int i = 4; i < 6; i++) cp16(dst + i * 512, in_p + i * 512, policy);
-                    if (lane < (SG_UNIT_Q6K - 3072) / 16) cp16(dst + 3072, in_p + 3072, policy);
-                    in_p += SG_UNIT_Q6K;
-                } else {
-                    if (lane < (SG_UNIT_Q4K - 2048) / 16) cp16(dst + 2048, in_p + 2048, policy);
-                    in_p += SG_UNIT_Q4K;
-                }
-            }
-            if (++in_kb == kts) {
-                in_kb = 0;
-                in_new = true;
-                in_tile += SG_WARPS;
-            }
-            in_it++;
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        in_slot = in_slot + 1 == R ? 0 : in_slot + 1;
-    };
-    for (int i = 0; i < R - 1; i++) request();
-    pdl_wait();
+struct SgBars {
+    uint64_t w_full[SG_W_SLOTS], w_free[SG_W_SLOTS];                              // an item's units
+    uint64_t x_full[SG_X_SLOTS], x_free[SG_X_SLOTS], scale[SG_SCALE_SLOTS];       // its activations, their rows' scales
+    uint64_t a_full[2];                                                           // the expanded weights of a team's item; their place is free when the sums are there
+    uint64_t sum_full[2], sum_free[2];                                            // accumulators of even and odd items
+    uint64_t out_full, out_free, last_full;                                       // sums of a group, of the CTA's last one
+    uint64_t done[2];
+    uint32_t tmem;
+    int seen;
+};
 
-    const int g = lane >> 2, t = lane & 3;
-    bool dead = false;
-    int slot = 0, it = lo, xs = 0;
-    uint32_t turn = 0;
-    while (it < hi) {
-        const int group = it / kts, kb0 = it - group * kts, seg_end = min(hi, (group + 1) * kts);
-        const int tile = group * SG_WARPS + warp;
-        const bool mine = tile < a.tiles;
-        const TileAt ta = tile_at(a, mine ? tile : 0, kts);
-        const bool q6 = ta.ub == SG_UNIT_Q6K;
-        float facc[NT][4];
-#pragma unroll
-        for (int n = 0; n < NT; n++)
-#pragma unroll
-            for (int i = 0; i < 4; i++) facc[n][i] = 0.f;
-        const int n_seg = seg_end - it;
-        for (; it < seg_end; it++) {
-            request();
-            if (R == 4) asm volatile("cp.async.wait_group 3;" ::: "memory");
-            else if (R == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
-            else asm volatile("cp.async.wait_group 1;" ::: "memory");
-            __syncwarp();
-            if (!dead && !__all_sync(0xffffffffu, bar_wait(&full[xs], turn & 1))) {
-                dead = true;
-                if (lane == 0) *(volatile int*)a.status = KS_TIMEOUT;
-            }
-            if (mine && !dead) {
-                const uint8_t* sp = ring + slot * a.slot_bytes;
-                const uint8_t* xc = xring + xs * CHUNK;
-                if (q6) unit16_q6k<NT>(sp, xc, lane, facc);
-                else unit16_q4k<NT>(sp, xc, lane, facc);
-            }
-            slot = slot + 1 == R ? 0 : slot + 1;
-            __syncwarp();      // every lane is done with the unit and the chunk
-            if (lane == 0) bar_arrive(&empty[xs]);
-            if (++xs == XS) {
-                xs = 0;
-                turn++;
-            }
-        }
-        if (!mine) continue;
-        const int me = blockIdx.x * SG_WARPS + warp;
-        if (kb0 != 0) {      // the group began in an earlier CTA: hand over the sums
-            float* w = a.ws + (size_t)me * SG_WS_FLOATS;
-#pragma unroll
-            for (int n = 0; n < NT; n++)
-#pragma unroll
-                for (int i = 0; i < 4; i++) w[(n * 4 + i) * 32 + lane] = facc[n][i];
+// The rows of group `group`, whose sums over the CTA's own blocks (from kb0 on) are in `out` [row of x][128], by `threads` threads: handed over to the CTA that holds the group's
+// first block, or completed with what the others hand over, biases and what they are added to, and stored.  The warps do not wait for each other: every one that hands over counts
+// the flag up, every one that collects watches all flags, and the last of them (`seen`, in shared memory) clears them.  Returns whether no wait ran out.
+__device__ __forceinline__ bool finish_group(const SgArgs& a, const float* out, int group, int kb0, int n_seg, int rows, int kts, int total, int tid, int threads, int* seen) {
+    const int lane = tid & 31;
+    if (kb0 != 0) {
+        float* w = a.ws + (size_t)blockIdx.x * SG_WS_FLOATS;
+        for (int e = tid * 4; e < rows * 128; e += threads * 4) *reinterpret_cast<float4*>(w + e) = *reinterpret_cast<const float4*>(out + e);
+        __syncwarp();
+        if (lane == 0) {
             __threadfence();
-            __syncwarp();
-            if (lane == 0) st_release(&a.flags[me], 1u);
-            continue;
+            atomicAdd(&a.flags[blockIdx.x], 1u);
         }
-        // lane (g, t) holds rows g (i < 2) and g + 8 of x rows 8 n + 2 t + (i & 1).  What the results are added to is fetched ahead of the waits below, all of it at
-        // once: loads that take turns with the stores cost 8 us of 24 at 32 rows.
+        return true;
+    }
+    // A lane has one row (or pair of rows) of the matrix and every step-th row of x, four of them under way at once.  Loads are not predicated (rows past the last are read for
+    // nothing) so that all of a round are in flight together.
+    const int glu = a.mode == 2;      // the up value of a gate is the next row
+    const int quads = glu ? 2 : 4, n_warps = threads / 32, warp = tid >> 5;
+    const bool split = n_warps >= quads;
+    const int step = split ? n_warps / quads : n_warps, x_first = split ? warp / quads : warp;
+    bool alive = true;
+    int n_parts = n_seg < kts ? -1 : 0;
+    for (int quad = split ? warp % quads : 0; quad < quads; quad += split ? quads : 1) {
+        const int row = (quad * 32 + lane) << glu, tile = group * SG_TILES + (row >> 4);
+        const bool mine = tile < a.tiles;
+        const TileAt ta = tile_at(a, mine ? tile : a.tiles - 1, kts);
         const float* bias = a.seg[0].bias;
         int out_off = a.seg[0].out_off;
 #pragma unroll
-        for (int i = 1; i < 4; i++)
-            if (i == ta.s) {
-                bias = a.seg[i].bias;
-                out_off = a.seg[i].out_off;
+        for (int s = 1; s < 4; s++)
+            if (s == ta.s) {
+                bias = a.seg[s].bias;
+                out_off = a.seg[s].out_off;
             }
-        const int row0 = ta.local * 16 + g;
-        const float bias0 = bias ? bias[row0] : 0.f, bias1 = bias ? bias[row0 + 8] : 0.f;
-        float* o = a.out + (a.mode == 2 ? (out_off + row0) >> 1 : out_off + row0);
-        float old[NT][4];
+        const int wrow = ta.local * 16 + (row & 15);
+        float* o = a.out + ((out_off + wrow) >> glu);
+        const float b0 = bias ? bias[wrow] : 0.f, b1 = bias && glu ? bias[wrow + 1] : 0.f;
+#pragma unroll 1
+        for (int x0 = x_first; x0 < a.nb; x0 += 4 * step) {
+            float y[4], u[4];
 #pragma unroll
-        for (int n = 0; n < NT; n++)
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int b = 8 * n + 2 * t + (i & 1);
-                old[n][i] = a.mode == 1 && b < a.nb ? __ldcg(o + (size_t)b * a.ldo + 8 * (i >> 1)) : 0.f;
+            for (int j = 0; j < 4; j++) {
+                y[j] = a.mode == 1 ? __ldcg(o + (size_t)min(x0 + j * step, a.nb - 1) * a.ldo) : 0.f;
+                u[j] = 0.f;
             }
-        if (n_seg < kts) {
-            // the CTAs behind this one that hold the rest of the group: lane i watches the flag of the i-th (all at once: one after the other they cost a trip
-            // to L2 each, 12 us of 16 for a product with nine parts a group)
-            const int group_end = (group + 1) * kts;
-            for (int c0 = blockIdx.x + 1; c0 < gridDim.x; c0 += 32) {
-                const bool part = c0 + lane < gridDim.x && share(c0 + lane, total, gridDim.x) < group_end;
-                const int n_parts = __popc(__ballot_sync(0xffffffffu, part));
-                if (n_parts == 0) break;
-                const int from = (c0 + lane) * SG_WARPS + warp;
-                bool ok = true;
-                if (part && !dead) {
-                    ok = ld_acquire(&a.flags[from]) != 0u;
-                    if (!ok) {
-                        const unsigned long long t0 = now_ns();
-                        while (!ok && now_ns() - t0 < SG_WAIT_NS) ok = ld_acquire(&a.flags[from]) != 0u;
+            if (n_parts < 0) {      // the first time, with the loads above under way
+                // the CTAs behind this one that hold the rest of the group: lane i watches the flag of the i-th (all at once: one after the other they cost a trip to L2 each)
+                const int group_end = (group + 1) * kts;
+                n_parts = 0;
+                for (int c0 = blockIdx.x + 1;; c0 += 32) {
+                    const int c = c0 + lane;
+                    const bool part = c < gridDim.x && share(c, total, gridDim.x) < group_end;
+                    const int n = __popc(__ballot_sync(0xffffffffu, part));
+                    n_parts += n;
+                    if (part) {
+                        // a group that ends the CTA's share is handed over by the warps that expand
+                        const unsigned warps = share(c + 1, total, gridDim.x) <= group_end ? SG_EXPAND : SG_FINISH;
+                        bool ok = ld_acquire(&a.flags[c]) == warps;
+                        if (!ok) {
+                            const unsigned long long t0 = now_ns();
+                            while (!ok && now_ns() - t0 < SG_WAIT_NS) ok = ld_acquire(&a.flags[c]) == warps;
+                        }
+                        if (!ok) alive = false;
                     }
-                    if (!ok) *(volatile int*)a.status = KS_TIMEOUT;
+                    if (n < 32) break;
                 }
-                if (!__all_sync(0xffffffffu, ok)) dead = true;
-                const float* w = a.ws + ((size_t)c0 * SG_WARPS + warp) * SG_WS_FLOATS + lane;
-#pragma unroll 4
-                for (int c = 0; c < n_parts; c++)
-#pragma unroll
-                    for (int n = 0; n < NT; n++)
-#pragma unroll
-                        for (int i = 0; i < 4; i++) facc[n][i] += __ldcg(w + (size_t)c * SG_WARPS * SG_WS_FLOATS + (n * 4 + i) * 32);
                 __syncwarp();
-                if (part) a.flags[from] = 0u;
+            }
+#pragma unroll 1
+            for (int c = 0; c < n_parts; c += 2) {
+                const float* w0 = a.ws + (size_t)(blockIdx.x + 1 + c) * SG_WS_FLOATS + row;
+                const float* w1 = c + 1 < n_parts ? w0 + SG_WS_FLOATS : w0;
+                float v0[4], v1[4], t0[4], t1[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const int x = min(x0 + j * step, rows - 1) * 128;
+                    v0[j] = __ldcg(w0 + x);
+                    v1[j] = __ldcg(w1 + x);
+                    if (glu) {
+                        t0[j] = __ldcg(w0 + x + 1);
+                        t1[j] = __ldcg(w1 + x + 1);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    y[j] += v0[j];
+                    if (c + 1 < n_parts) y[j] += v1[j];
+                    if (glu) {
+                        u[j] += t0[j];
+                        if (c + 1 < n_parts) u[j] += t1[j];
+                    }
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int x = x0 + j * step;
+                if (x < a.nb && mine) {
+                    y[j] += out[x * 128 + row] + b0;
+                    if (glu) y[j] = glu_act(y[j], u[j] + out[x * 128 + row + 1] + b1, a.act, a.alpha, a.limit);
+                    o[(size_t)x * a.ldo] = y[j];
+                }
             }
         }
+    }
+    if (n_seg < kts) {      // a warp without rows of x has not looked at the flags, and is done with them too
+        int before = 0;
+        __syncwarp();
+        if (lane == 0) before = atomicAdd(seen, 1);
+        if (__shfl_sync(0xffffffffu, before, 0) == n_warps - 1) {
+            const int group_end = (group + 1) * kts;
+            for (int c = blockIdx.x + 1 + lane; c < gridDim.x && share(c, total, gridDim.x) < group_end; c += 32) a.flags[c] = 0u;
+            if (lane == 0) *seen = 0;
+        }
+    }
+    return alive;
+}
+
+template <int NT>
+__global__ void __launch_bounds__(SG_THREADS, 1) gemm_sk_kernel(const __grid_constant__ SgArgs a) {
+    constexpr int N = 16 * NT, X_BYTES = N * SG_ROW, X_SLOT = (X_BYTES + 1023) & ~1023, CHUNK = NT * SG_CHUNK;
+    constexpr bool ONE_MINS = NT == 4;             // sums of the minima: one place instead of two, where tensor memory is full
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) SgBars bars;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int kts = a.k >> 8, total = (a.tiles + SG_TILES - 1) / SG_TILES * kts;
+    const int lo = share(blockIdx.x, total, gridDim.x), n_items = share(blockIdx.x + 1, total, gridDim.x) - lo;
+    const int group0 = lo / kts, kb_lo = lo - group0 * kts;
+    const int XS = a.x_slots, R = a.ring;
+    uint8_t* x_ring = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
+    float2* dbuf = reinterpret_cast<float2*>(x_ring + XS * X_SLOT);            // [slot][128]
+    float* scales = reinterpret_cast<float*>(dbuf + SG_D_SLOTS * 128);         // [slot][N]
+    float* out = scales + SG_SCALE_SLOTS * N;                                  // [row of x][128]
+    uint8_t* w_ring = reinterpret_cast<uint8_t*>(out + N * 128);               // [slot][tile]
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < R; i++) {
+            mbar_init(&bars.w_full[i], SG_TILES);
+            mbar_init(&bars.w_free[i], SG_TILES);
+        }
+        for (int i = 0; i < XS; i++) {
+            mbar_init(&bars.x_full[i], 1);
+            mbar_init(&bars.x_free[i], 1);
+        }
+        for (int i = 0; i < SG_SCALE_SLOTS; i++) mbar_init(&bars.scale[i], 1);
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&bars.a_full[i], SG_TILES);
+            mbar_init(&bars.sum_full[i], 1);
+            mbar_init(&bars.sum_free[i], SG_SUM);
+            mbar_init(&bars.done[i], 1);
+        }
+        mbar_init(&bars.out_full, SG_SUM);
+        mbar_init(&bars.out_free, SG_FINISH);
+        mbar_init(&bars.last_full, SG_SUM);
+        bars.seen = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    pdl_launch();
+    bool alive = true;      // false: a wait ran out
+    auto wait = [&](uint64_t* bar, uint32_t parity) { return alive = __all_sync(0xffffffffu, bar_wait(bar, parity)) != 0; };
+
+    if (warp < SG_EXPAND) {
+        const int quad = warp & 3, team = warp >> 3, tig = 2 * quad + ((warp >> 2) & 1);      // warp & 3 gives the TMEM lanes it reaches
+        __syncthreads();      // barriers and tensor memory
+        tc_fence_after();
+        const uint32_t a_cols = bars.tmem + ((uint32_t)(quad * 32 + 16 * ((warp >> 2) & 1)) << 16) + team * SG_A_COLS;
+        const int g = lane >> 2, t = lane & 3, row = tig * 16 + g;
+        int slot = team, kb = kb_lo + team, tile = group0 * SG_TILES + tig;
+        uint32_t turn = 0;
+        bool fresh = true, mine = false, q6 = false;
+        for (int i = team; i < n_items; i += 2) {
+            if (kb >= kts) {
+                do {
+                    kb -= kts;
+                    tile += SG_TILES;
+                } while (kb >= kts);
+                fresh = true;
+            }
+            if (fresh) {
+                mine = tile < a.tiles;
+                q6 = mine && tile_at(a, tile, kts).ub == SG_UNIT_Q6K;
+                fresh = false;
+            }
+            if (!wait(&bars.w_full[slot], turn)) break;
+            const uint8_t* sp = w_ring + (size_t)(slot * SG_TILES + tig) * a.slot_bytes;
+            uint4 sg, sh;
+            float2 dg, dh;
+            uint32_t r[16];
+            if (q6) {
+                sg = reinterpret_cast<const uint4*>(sp + 3072)[g];
+                sh = reinterpret_cast<const uint4*>(sp + 3072)[g + 8];
+                dg = make_float2(__half2float(reinterpret_cast<const __half*>(sp + 3328)[g]), 0.f);
+                dh = make_float2(__half2float(reinterpret_cast<const __half*>(sp + 3328)[g + 8]), 0.f);
+                part_q6k<0>(sp, lane, sg.x, sh.x, r);
+            } else {
+                sg = reinterpret_cast<const uint4*>(sp + 2048)[g];
+                sh = reinterpret_cast<const uint4*>(sp + 2048)[g + 8];
+                dg = __half22float2(reinterpret_cast<const __half2*>(sp + 2304)[g]);
+                dh = __half22float2(reinterpret_cast<const __half2*>(sp + 2304)[g + 8]);
+                expand_q4k<0>(reinterpret_cast<const uint4*>(sp)[lane], sg.x, sh.x, r);
+            }
+            if (i > 1) {
+                if (!wait(&bars.sum_full[team], ((i >> 1) - 1) & 1)) break;
+                tc_fence_after();
+            }
+            tmem_st_16x128_x8(a_cols, r);
+            uint32_t m0 = 0, m1 = 0;      // minima 2 t, 2 t + 1 of both rows
+            if (q6) {
+                part_q6k<1>(sp, lane, sg.y, sh.y, r);
+                tmem_st_16x128_x8(a_cols + 32, r);
+                part_q6k<2>(sp, lane, sg.z, sh.z, r);
+                tmem_st_16x128_x8(a_cols + 64, r);
+                part_q6k<3>(sp, lane, sg.w, sh.w, r);
+            } else {
+                expand_q4k<2>(reinterpret_cast<const uint4*>(sp)[32 + lane], sg.x, sh.x, r);
+                tmem_st_16x128_x8(a_cols + 32, r);
+                expand_q4k<0>(reinterpret_cast<const uint4*>(sp)[64 + lane], sg.y, sh.y, r);
+                tmem_st_16x128_x8(a_cols + 64, r);
+                expand_q4k<2>(reinterpret_cast<const uint4*>(sp)[96 + lane], sg.y, sh.y, r);
+                const uint32_t wg = (t < 2 ? sg.z : sg.w) >> (16 * (t & 1)), wh = (t < 2 ? sh.z : sh.w) >> (16 * (t & 1));
+                m0 = h2_add(__byte_perm(wg, H_1024, 0x5150), H_M1024);
+                m1 = h2_add(__byte_perm(wh, H_1024, 0x5150), H_M1024);
+            }
+            __syncwarp();      // every lane has its part of the unit
+            if (lane == 0) mbar_arrive(&bars.w_free[slot]);
+            tmem_st_16x128_x8(a_cols + 96, r);
+            tmem_st_16x128_x2(a_cols + 128, m0, m1, m0, m1);      // for the upper and again for the lower parts of the sums of 32
+            if (t == 0) {
+                // the sums of the item that had the slot before are taken: the products of the one two items ago, which have ended, waited for those of two more before
+                float2* my_d = dbuf + (i & (SG_D_SLOTS - 1)) * 128 + row;
+                my_d[0] = dg;
+                my_d[8] = dh;
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars.a_full[team]);
+            slot += 2;
+            if (slot >= R) {
+                slot -= R;
+                turn ^= 1;
+            }
+            kb += 2;
+        }
+        // nothing more to expand: all sixteen warps finish the last group
+        pdl_wait();
+        const int last = (lo + n_items - 1) / kts, kb0 = last == group0 ? kb_lo : 0;
+        if (alive && wait(&bars.last_full, 0)) alive = __all_sync(0xffffffffu, finish_group(a, out, last, kb0, lo + n_items - last * kts - kb0, N, kts, total, threadIdx.x, SG_EXPAND * 32, &bars.seen));
+    } else if (warp < SG_MMA) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 136;");
+        __syncthreads();
+        tc_fence_after();
+        const int quad = warp & 3, row = quad * 32 + lane;
+        const uint32_t cols = bars.tmem + ((uint32_t)(quad * 32) << 16) + 2 * SG_A_COLS;
+        int group = group0, kb0 = kb_lo;
+        for (int i = 0; i < n_items; group++, kb0 = 0) {
+            const int n_seg = min(n_items - i, kts - kb0);
+            f2 sum[N / 2];
 #pragma unroll
-        for (int n = 0; n < NT; n++)
+            for (int c = 0; c < N / 2; c++) sum[c] = 0ull;
+            for (const int end = i + n_seg; i < end; i++) {
+                const int buf = i & 1;
+                if (!wait(&bars.scale[i & (SG_SCALE_SLOTS - 1)], (i / SG_SCALE_SLOTS) & 1) || !wait(&bars.sum_full[buf], (i >> 1) & 1)) break;
+                tc_fence_after();
+                const float2 d = dbuf[(i & (SG_D_SLOTS - 1)) * 128 + row];
+                const f2 d2 = pack2(d.x, d.x), m2 = pack2(-d.y, -d.y);
+                const ulonglong2* sx = reinterpret_cast<const ulonglong2*>(scales + (i & (SG_SCALE_SLOTS - 1)) * N);
+                const uint32_t at = cols + buf * N, at_m = cols + 2 * N + (ONE_MINS ? 0 : buf * N);
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int b = 8 * n + 2 * t + (i & 1);
-                const float v = facc[n][i] + (i < 2 ? bias0 : bias1);
-                float* at = o + (size_t)b * a.ldo;
-                if (a.mode == 2) {      // the up value of a gate is one row further: lane + 4
-                    const float up = __shfl_down_sync(0xffffffffu, v, 4);
-                    if (!(g & 1) && b < a.nb) at[4 * (i >> 1)] = glu_act(v, up, a.act, a.alpha, a.limit);
-                } else if (b < a.nb) {
-                    at[8 * (i >> 1)] = v + old[n][i];
+                for (int c = 0; c < NT; c++) {
+                    uint32_t v[16], m[16];
+                    tmem_ld16(at + 16 * c, v);
+                    tmem_ld16(at_m + 16 * c, m);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (c == NT - 1) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&bars.sum_free[buf]);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 8; j += 2) {
+                        const ulonglong2 s = sx[4 * c + (j >> 1)];
+                        sum[8 * c + j] = fma2(s.x, fma2(m2, pack2u(m[2 * j], m[2 * j + 1]), mul2(d2, pack2u(v[2 * j], v[2 * j + 1]))), sum[8 * c + j]);
+                        sum[8 * c + j + 1] = fma2(s.y, fma2(m2, pack2u(m[2 * j + 2], m[2 * j + 3]), mul2(d2, pack2u(v[2 * j + 2], v[2 * j + 3]))), sum[8 * c + j + 1]);
+                    }
                 }
             }
+            if (!alive) break;
+            // the rows are finished by other warps: here the stores and their fence took 6000 cycles, in which nothing moved
+            const bool last = i == n_items;
+            if (group > group0 && !wait(&bars.out_free, (group - group0 - 1) & 1)) break;
+#pragma unroll
+            for (int c = 0; c < N / 2; c++) {
+                const float2 v = unpack2(sum[c]);
+                out[(2 * c) * 128 + row] = v.x;
+                out[(2 * c + 1) * 128 + row] = v.y;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(last ? &bars.last_full : &bars.out_full);
+        }
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        if (warp == SG_MMA) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&bars.tmem)) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+            tc_fence_before();
+        }
+        __syncthreads();
+        tc_fence_after();
+        if (warp < SG_LOAD_X) {
+            // products of every second item: with one warp for all, its waits and the issue of 17 instructions (1250 cycles an item) were the slowest part
+            const int par = warp - SG_MMA;
+            const uint32_t tmem = __shfl_sync(0xffffffffu, bars.tmem, 0);
+            const uint32_t d = tmem + 2 * SG_A_COLS + par * N, dm = tmem + 2 * SG_A_COLS + 2 * N + (ONE_MINS ? 0 : par * N), at = tmem + par * SG_A_COLS;
+            const uint64_t x_desc = umma_desc(x_ring), s_desc = desc_cells(smem_u32(x_ring) + N * 512, N * 16);
+            int s = par;
+            uint32_t turn = 0, lap = 0;
+            for (int i = par; i < n_items; i += 2, lap ^= 1) {
+                if (!wait(&bars.x_full[s], turn) || (i > 1 && !wait(&bars.sum_free[par], lap ^ 1)) || !wait(&bars.a_full[par], lap)) break;
+                tc_fence_after();
+                const uint64_t x0 = (uint64_t)((s * X_SLOT) >> 4), xd = x_desc + x0;
+                if (elect()) {
+#pragma unroll
+                    for (int c = 0; c < 16; c++) mma_ts(d, at + c * 8, xd + (uint64_t)(((c >> 2) * N * 128 + (c & 3) * 32) >> 4), sg_idesc(N), c > 0);
+                }
+                __syncwarp();
+                if (ONE_MINS && i > 0) {
+                    if (!wait(&bars.sum_free[par ^ 1], ((i - 1) >> 1) & 1)) break;
+                    tc_fence_after();
+                }
+                if (elect()) {
+                    mma_ts(dm, at + 128, s_desc + x0, sg_idesc(N), 0);
+                    umma_commit(&bars.sum_full[par]);
+                    umma_commit(&bars.x_free[s]);
+                }
+                __syncwarp();
+                s += 2;
+                if (s >= XS) {
+                    s -= XS;
+                    turn ^= 1;
+                }
+            }
+            if (!alive) {      // what is under way ends before the CTA leaves
+                if (elect()) umma_commit(&bars.done[par]);
+                bar_wait(&bars.done[par], 0);
+            }
+        } else if (warp == SG_LOAD_X) {
+            pdl_wait();
+            int kb = kb_lo, s = 0, i = 0;
+            uint32_t turn = 0;
+            for (; i < n_items; i++) {
+                if (i >= XS && !wait(&bars.x_free[s], turn ^ 1)) break;
+                const int q = i & (SG_SCALE_SLOTS - 1);      // free: the accumulators of two items before the one that had the slot of x were
+                if (lane == 0) {
+                    const uint8_t* src = a.x + (size_t)kb * CHUNK;
+                    mbar_expect_tx(&bars.x_full[s], X_BYTES);
+                    bulk_copy(smem_u32(x_ring + s * X_SLOT), src, X_BYTES, &bars.x_full[s]);
+                    mbar_expect_tx(&bars.scale[q], N * 4);
+                    bulk_copy(smem_u32(scales + q * N), src + X_BYTES, N * 4, &bars.scale[q]);
+                }
+                __syncwarp();
+                if (++kb == kts) kb = 0;
+                if (++s == XS) {
+                    s = 0;
+                    turn ^= 1;
+                }
+            }
+            if (!alive)      // what is under way ends before the CTA leaves
+                for (int j = i - XS; j < i; j++) {
+                    bar_wait(&bars.x_full[j % XS], (j / XS) & 1);
+                    bar_wait(&bars.scale[j & (SG_SCALE_SLOTS - 1)], (j / SG_SCALE_SLOTS) & 1);
+                }
+        } else if (warp < SG_LAST) {
+            // units of every second item: lane i copies the one of the group's i-th tile (eight copies take a warp 1000 cycles)
+            uint64_t policy;
+            asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+            const int par = warp - SG_LOAD_W;
+            int kb = kb_lo + par, tile = group0 * SG_TILES + lane, slot = par, i = par;
+            uint32_t turn = 0, bytes = 0;
+            const uint8_t* p = nullptr;
+            bool fresh = true;
+            for (; i < n_items; i += 2) {
+                if (kb >= kts) {
+                    do {
+                        kb -= kts;
+                        tile += SG_TILES;
+                    } while (kb >= kts);
+                    fresh = true;
+                }
+                if (fresh) {
+                    bytes = 0;
+                    if (lane < SG_TILES && tile < a.tiles) {
+                        const TileAt ta = tile_at(a, tile, kts);
+                        bytes = ta.ub;
+                        p = ta.p + (size_t)kb * bytes;
+                    }
+                    fresh = false;
+                }
+                if (i >= R && !wait(&bars.w_free[slot], turn ^ 1)) break;
+                if (bytes) {
+                    mbar_expect_tx(&bars.w_full[slot], bytes);
+                    bulk_copy(smem_u32(w_ring + (size_t)(slot * SG_TILES + lane) * a.slot_bytes), p, bytes, &bars.w_full[slot], policy);
+                    p += 2 * bytes;
+                } else if (lane < SG_TILES) {
+                    mbar_arrive(&bars.w_full[slot]);
+                }
+                __syncwarp();
+                slot += 2;
+                if (slot >= R) {
+                    slot -= R;
+                    turn ^= 1;
+                }
+                kb += 2;
+            }
+            if (!alive)      // what is under way ends before the CTA leaves
+                for (int j = max(par, i - (R & ~1)); j < i; j += 2) bar_wait(&bars.w_full[j % R], (j / R) & 1);
+        } else {
+            pdl_wait();
+            int kb0 = kb_lo;
+            const int last = (lo + n_items - 1) / kts, tid = threadIdx.x - SG_LAST * 32;
+            for (int g = group0; g < last; g++, kb0 = 0) {
+                if (!wait(&bars.out_full, (g - group0) & 1)) break;
+                alive = __all_sync(0xffffffffu, finish_group(a, out, g, kb0, kts - kb0, N, kts, total, tid, SG_FINISH * 32, &bars.seen));
+                if (lane == 0) mbar_arrive(&bars.out_free);
+                if (!alive) break;
+            }
+        }
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    if (dead)      // the producer may have chunks in flight: they land before the CTA leaves
-        for (int i = max(0, hi - lo - XS); i < hi - lo; i++) bar_wait(&full[i % XS], (i / XS) & 1);
+    if (!alive && lane == 0) *(volatile int*)a.status = KS_TIMEOUT;
+    tc_fence_before();
+    __syncthreads();
+    if (warp == SG_MMA) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(bars.tmem));
+    }
 }
 
 // One warp per (row, 256-block): eight columns per lane.  A row that is normalised belongs to one CTA (its sum of squares is needed first).
-// Rows nb .. 8 ceil(nb / 8) - 1 of the last group are written as zeros.
+// Rows nb .. 16 ceil(nb / 16) - 1 are written as zeros.
 template <bool BF16>
 __device__ __forceinline__ void load8(const void* x, size_t at, float (&v)[8]) {
     if (BF16) {
@@ -466,7 +712,9 @@ __device__ __forceinline__ void load8(const void* x, size_t at, float (&v)[8]) {
 
 constexpr int R16_WARPS = 8, R16_KEEP = 8;      // blocks that a warp keeps in registers between the sum of squares and the stores
 
-__device__ __forceinline__ void store_block(const Rows16Args& a, int nt, int ntile, int gg, int blk, int lane, const float (&v)[8]) {
+// A 256-block of `n` rows: [64 columns][n rows][128 bytes, 16-byte pieces xor row & 7] values, [two parts][n rows][16 bytes] sums of 32 (upper f16 parts of the eight, then
+// lower parts), [n] scales.  Place 8 j + 2 t + e of 64 columns holds column 32 (j / 4) + 16 (j / 2 & 1) + 4 t + (j & 1) + 2 e.
+__device__ __forceinline__ void store_block(const Rows16Args& a, int n, int row, int blk, int lane, const float (&v)[8]) {
     float m = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; i++) m = fmaxf(m, fabsf(v[i]));
@@ -482,22 +730,22 @@ __device__ __forceinline__ void store_block(const Rows16Args& a, int nt, int nti
     }
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
     sum += __shfl_xor_sync(0xffffffffu, sum, 2);                                    // the 32 columns of four lanes
-    uint8_t* c = a.out + (size_t)blk * nt * SG_CHUNK;
-    // lane: columns 8 lane .. + 7 of the block = t values 2 (lane & 1) and + 1 of 16-column group lane / 2, fragment pair lane / 4
-    __half2* f = reinterpret_cast<__half2*>(c + ntile * SG_FRAG + ((size_t)(lane >> 2) * 32 + gg * 4 + 2 * (lane & 1)) * 16 + ((lane >> 1) & 1) * 8);
-    f[0] = __halves2half2(h[0], h[2]);
-    f[1] = __halves2half2(h[1], h[3]);
-    f[4] = __halves2half2(h[4], h[6]);
-    f[5] = __halves2half2(h[5], h[7]);
-    // sums of sub-blocks 2t, 2t + 1: lanes 8 t and 8 t + 4 hold them
+    uint8_t* c = a.out + (size_t)blk * n * (SG_ROW + 4);
+    // lane: columns 8 lane .. + 7 = t values 2 (lane & 1) and + 1 of 16-column group lane / 2
+    const int j = 2 * ((lane >> 1) & 3);
+    uint8_t* f = c + (size_t)((lane >> 3) * n + row) * 128 + 8 * (lane & 1);
+    const __half2 p[4] = {__halves2half2(h[0], h[2]), __halves2half2(h[4], h[6]), __halves2half2(h[1], h[3]), __halves2half2(h[5], h[7])};
+    *reinterpret_cast<uint2*>(f + ((j ^ (row & 7)) << 4)) = *reinterpret_cast<const uint2*>(p);
+    *reinterpret_cast<uint2*>(f + (((j + 1) ^ (row & 7)) << 4)) = *reinterpret_cast<const uint2*>(p + 2);
+    // sums of two neighbouring sub-blocks: lanes 8 i and 8 i + 4 hold them
     const float next = __shfl_down_sync(0xffffffffu, sum, 4);
     if ((lane & 7) == 0) {
         const __half h0 = __float2half_rn(sum), h1 = __float2half_rn(next);
-        __half2* s = reinterpret_cast<__half2*>(c + nt * SG_FRAG + ntile * SG_SUMS + (gg * 4 + (lane >> 3)) * 8);
+        __half2* s = reinterpret_cast<__half2*>(c + (size_t)n * 512 + row * 16 + (lane >> 3) * 4);
         s[0] = __halves2half2(h0, h1);
-        s[1] = __halves2half2(__float2half_rn(sum - __half2float(h0)), __float2half_rn(next - __half2float(h1)));
+        s[n * 4] = __halves2half2(__float2half_rn(sum - __half2float(h0)), __float2half_rn(next - __half2float(h1)));
     }
-    if (lane == 0) *reinterpret_cast<float*>(c + nt * (SG_FRAG + SG_SUMS) + (ntile * 8 + gg) * 4) = scale;
+    if (lane == 0) *reinterpret_cast<float*>(c + (size_t)n * SG_ROW + row * 4) = scale;
 }
 
 template <bool BF16>
@@ -505,15 +753,14 @@ __global__ void __launch_bounds__(R16_WARPS * 32) rows16_kernel(const __grid_con
     __shared__ float ssq[R16_WARPS];
     pdl_launch();
     pdl_wait();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = blockIdx.x, nkb = a.k >> 8, nt = gridDim.x >> 3;
-    const int ntile = row >> 3, gg = row & 7;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = blockIdx.x, nkb = a.k >> 8, n = gridDim.x;
     const int b0 = blockIdx.y * R16_WARPS + warp, step = gridDim.y * R16_WARPS;
     const bool pad = row >= nb;
     if (!a.norm_w) {
         for (int blk = b0; blk < nkb; blk += step) {
             float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             if (!pad) load8<BF16>(a.x, (size_t)row * a.ldx + blk * 256 + lane * 8, v);
-            store_block(a, nt, ntile, gg, blk, lane, v);
+            store_block(a, n, row, blk, lane, v);
         }
         return;
     }
@@ -547,7 +794,7 @@ __global__ void __launch_bounds__(R16_WARPS * 32) rows16_kernel(const __grid_con
         const float w[8] = {n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, n1.z, n1.w};
 #pragma unroll
         for (int j = 0; j < 8; j++) v[i][j] *= rstd * w[j];
-        store_block(a, nt, ntile, gg, blk, lane, v[i]);
+        store_block(a, n, row, blk, lane, v[i]);
     }
 }
 
@@ -577,25 +824,26 @@ int go(const void* fn, dim3 grid, dim3 block, size_t smem, void** args, cudaStre
 }  // namespace
 
 // Bytes of the activation chunks of nb rows of length k.
-B2_API long long b2_rows16_bytes(int nb, int k) { return (long long)(k >> 8) * ((nb + 7) >> 3) * SG_CHUNK; }
+B2_API long long b2_rows16_bytes(int nb, int k) { return (long long)(k >> 8) * ((nb + 15) >> 4) * SG_CHUNK; }
 
 // Rows in the order that b2_gemm_sk reads.  k a multiple of 256 (at most 16384 with a norm), x and out 16-byte aligned, ldx a multiple of 8 (fp32: of 4).
 B2_API int b2_rows16(const Rows16Args* in, int nb, int pdl, cudaStream_t st) {
     Rows16Args a = *in;
-    if (nb < 1 || nb > 32 || a.k < 256 || (a.k & 255) || !a.x || !a.out || (((uintptr_t)a.x | (uintptr_t)a.out | (uintptr_t)a.norm_w) & 15) || (a.ldx & (a.bf16 ? 7 : 3)))
+    if (nb < 1 || nb > SG_MAX_ROWS || a.k < 256 || (a.k & 255) || !a.x || !a.out || (((uintptr_t)a.x | (uintptr_t)a.out | (uintptr_t)a.norm_w) & 15) ||
+        (a.ldx & (a.bf16 ? 7 : 3)))
         return (int)cudaErrorInvalidValue;
     if (a.norm_w && (a.k >> 8) > R16_WARPS * R16_KEEP) return (int)cudaErrorNotSupported;
-    const int nkb = a.k >> 8, rows = (nb + 7) & ~7;
+    const int nkb = a.k >> 8, rows = (nb + 15) & ~15;
     void* args[] = {&a, &nb};
     const dim3 grid(rows, a.norm_w ? 1 : (nkb + R16_WARPS - 1) / R16_WARPS);
     return go(a.bf16 ? (const void*)rows16_kernel<true> : (const void*)rows16_kernel<false>, grid, dim3(R16_WARPS * 32), 0, args, st, pdl);
 }
 
-// y = W x for 1..32 rows in the chunks of b2_rows16, up to four matrices of one row length.  Returns a cudaError_t value.
+// y = W x for 1..64 rows in the chunks of b2_rows16, up to four matrices of one row length.  Returns a cudaError_t value.
 B2_API int b2_gemm_sk(const SgArgs* in, int max_ctas, int pdl, cudaStream_t st) {
     SgArgs a = *in;
-    if (a.nseg < 1 || a.nseg > 4 || a.nb < 1 || a.nb > 32 || a.k < 256 || (a.k & 255) || !a.x || ((uintptr_t)a.x & 15) || !a.out || !a.ws || !a.flags || !a.status || a.mode < 0 ||
-        a.mode > 2)
+    if (a.nseg < 1 || a.nseg > 4 || a.nb < 1 || a.nb > SG_MAX_ROWS || a.k < 256 || (a.k & 255) || !a.x || ((uintptr_t)a.x & 15) || !a.out || !a.ws || !a.flags || !a.status ||
+        a.mode < 0 || a.mode > 2)
         return (int)cudaErrorInvalidValue;
     int slot = 0, tiles = 0;
     for (int s = 0; s < a.nseg; s++) {
@@ -605,26 +853,31 @@ B2_API int b2_gemm_sk(const SgArgs* in, int max_ctas, int pdl, cudaStream_t st) 
         tiles += g.n >> 4;
         slot = slot > (g.type == WT_Q6_K ? SG_UNIT_Q6K : SG_UNIT_Q4K) ? slot : (g.type == WT_Q6_K ? SG_UNIT_Q6K : SG_UNIT_Q4K);
     }
-    const int nt = a.nb <= 8 ? 1 : a.nb <= 16 ? 2 : a.nb <= 24 ? 3 : 4;
+    const int nt = (a.nb + 15) >> 4, rows = 16 * nt;
     a.tiles = tiles;
     a.slot_bytes = slot;
-    const size_t chunk = (size_t)nt * SG_CHUNK;
-    // weights in flight first: four slots a warp where they fit beside three chunks
-    a.ring = SG_WARPS * 4 * slot + 3 * chunk <= SG_MAX_SMEM ? 4 : 3;
-    a.x_slots = (SG_MAX_SMEM - (size_t)SG_WARPS * a.ring * slot) / chunk >= 4 ? 4 : 3;
-    const size_t smem = SG_WARPS * a.ring * slot + a.x_slots * chunk;
-    if (smem > SG_MAX_SMEM) return (int)cudaErrorInvalidValue;
+    const size_t chunk = (size_t)((rows * SG_ROW + 1023) & ~1023);
+    const size_t fixed = 1024 + SG_D_SLOTS * 128 * 8 + SG_SCALE_SLOTS * rows * 4 + rows * 512, item = (size_t)SG_TILES * slot;
+    // Four chunks of activations where at least four items fit beside them, else two (32 rows and fewer: six or eight items beside four chunks; 64: four or six beside two).  Both
+    // rings are even, so that a slot always belongs to even or to odd items: the warps that fill or use it wait for every phase of its barriers, as the parity of a phase demands.
+    a.x_slots = fixed + 4 * chunk + 4 * item <= SG_MAX_SMEM ? 4 : 2;
+    const size_t slots = (SG_MAX_SMEM - fixed - a.x_slots * chunk) / item;
+    a.ring = (slots < SG_W_SLOTS ? (int)slots : SG_W_SLOTS) & ~1;
+    const size_t smem = fixed + a.x_slots * chunk + a.ring * item;
     const void* fn = nt == 1 ? (const void*)gemm_sk_kernel<1> : nt == 2 ? (const void*)gemm_sk_kernel<2> : nt == 3 ? (const void*)gemm_sk_kernel<3> : (const void*)gemm_sk_kernel<4>;
-    static PerDeviceOnce once[4];
+    static PerDeviceOnce once[SG_MAX_NT];
     if (once[nt - 1].first()) {
         const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SG_MAX_SMEM);
         if (e != cudaSuccess) return (int)e;
     }
-    const int total = (tiles + SG_WARPS - 1) / SG_WARPS * (a.k >> 8);
+    const int total = (tiles + SG_TILES - 1) / SG_TILES * (a.k >> 8);
     if (total >= 1 << 23) return (int)cudaErrorNotSupported;
-    int grid = total < sms() ? total : sms();      // one CTA per SM: all are resident, so waits on other CTAs end
-    if (grid > 4096 / SG_WARPS) grid = 4096 / SG_WARPS;
+    // one CTA per SM: all are resident, so waits on other CTAs end.  No more of them than give every CTA as many items as the fullest has.
+    int grid = total < sms() ? total : sms();
+    if (grid > 256) grid = 256;                    // CTAs that the workspace holds
     if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
+    const int most = (total + grid - 1) / grid;
+    grid = (total + most - 1) / most;
     void* args[] = {&a};
     return go(fn, dim3((unsigned)grid), dim3(SG_THREADS), smem, args, st, pdl);
 }

@@ -44,7 +44,7 @@ struct SgArgs {
     float* out;
     int ldo, act;
     float alpha, limit;
-    float* ws;            // [groups of b2_gemv_sk_max_groups][512]
+    float* ws;            // b2_gemv_sk_max_groups() x 512 floats, and as many flags
     unsigned* flags;
     int* status;          // KStatus, written when a bounded wait gives up (may be pinned host memory)
     int tiles, ring, slot_bytes, x_slots;      // filled in by the launcher
@@ -57,7 +57,7 @@ struct Rows16Args {
     const float* norm_w;  // RMSNorm weight or null
     float eps;
     int k;
-    uint8_t* out;         // [k / 256][ceil(nb / 8)][SG_CHUNK] regrouped: per 256-block all values, then all sums, then all scales
+    uint8_t* out;         // [k / 256][ceil(nb / 16)][SG_CHUNK] regrouped: per 256-block all values, then all sums, then all scales
 };
 
 struct AttnPrefillArgs {

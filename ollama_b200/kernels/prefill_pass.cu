@@ -39,7 +39,7 @@ struct PassArgs {
     float *x, *qkv, *q;                           // residual stream [rows][d]; [rows][(H + 2 Hkv) hd]; [rows][H hd]
     void *o, *h;                                  // bf16 [rows][H hd], [rows][d]
     void* f;                                      // bf16 [rows][ff], units: fp32
-    uint8_t* x16;                                 // units: b2_rows16_bytes(32, widest row)
+    uint8_t* x16;                                 // units: b2_rows16_bytes(min(rows, 64), widest row)
     float* ws;                                    // units: workspace of b2_gemm_sk, otherwise scratch of b2_gemm_bf16
     long long ws_floats;
     unsigned* flags;
@@ -50,7 +50,7 @@ struct PassArgs {
 
 namespace {
 
-constexpr int UNIT_ROWS = 32;
+constexpr int UNIT_ROWS = 64;
 
 // Rows of `x` (fp32, or bf16 when ldx counts those), normalised with `w` where given, times unit-ordered matrices.
 int unit_product(const PassArgs& a, const SgSeg* w, int n, const void* x, int bf16, int k, const float* norm, float* out, int ldo, int mode, int& count, cudaStream_t st) {

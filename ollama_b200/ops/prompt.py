@@ -62,7 +62,7 @@ class PromptPass:
         qkv, q, o = rows((c.n_heads + 2 * c.n_kv_heads) * c.head_dim), rows(c.q_dim), rows(c.q_dim, torch.bfloat16)
         h = None if units else rows(c.d_model, torch.bfloat16)
         f = rows(c.d_ff, torch.float32 if units else torch.bfloat16)
-        x16 = torch.empty(SK.rows16_bytes(min(n, SK.MAX_TOKENS), max(c.d_model, c.q_dim, c.d_ff)), device=dev, dtype=torch.uint8) if units else None
+        x16 = torch.empty(SK.rows16_bytes(min(n, SK.ROWS16_MAX), max(c.d_model, c.q_dim, c.d_ff)), device=dev, dtype=torch.uint8) if units else None
         ws = self.ws if units else None
         size = 0 if units else max(K.gemm_bf16_scratch(n, *nk) for nk in (((c.n_heads + 2 * c.n_kv_heads) * c.head_dim, c.d_model), (c.d_model, c.q_dim), (c.d_model, c.d_ff)))
         parts = torch.empty(size, device=dev, dtype=torch.float32) if size else None

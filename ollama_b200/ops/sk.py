@@ -288,12 +288,13 @@ def gemv(weights: list[SkWeight], x: torch.Tensor | tuple[torch.Tensor, torch.Te
     return out
 
 
-ROWS16_CHUNK = 4384              # bytes of the activation chunk of one 256-block and eight rows (kernels/gemm_sk.cu)
+ROWS16_CHUNK = 8768              # bytes of the activation chunk of one 256-block and sixteen rows (kernels/gemm_sk.cu)
+ROWS16_MAX = 64                  # rows of one product
 ROWS16_MAX_NORM = 16384          # longest row that is normalised on the way
 
 
 def rows16_bytes(nb: int, k: int) -> int:
-    return (k // 256) * ((nb + 7) // 8) * ROWS16_CHUNK
+    return (k // 256) * ((nb + 15) // 16) * ROWS16_CHUNK
 
 
 def rows16(x: torch.Tensor, norm_w: torch.Tensor | None = None, eps: float = 0.0, out: torch.Tensor | None = None, pdl: bool = False) -> torch.Tensor:
@@ -313,7 +314,7 @@ def rows16(x: torch.Tensor, norm_w: torch.Tensor | None = None, eps: float = 0.0
 
 def gemm16(weights: list[SkWeight], x: torch.Tensor, nb: int, *, out: torch.Tensor | None = None, mode: int = MODE_STORE, act: str = "silu", alpha: float = 1.702,
            limit: float = 7.0, max_ctas: int = 0, pdl: bool = False, ws: Workspace | None = None) -> torch.Tensor:
-    """y[b] = concat_i(W_i x[b] + bias_i) of 1..32 rows in the chunks of :func:`rows16`; modes and results as in :func:`gemv`, activations in 16 bits."""
+    """y[b] = concat_i(W_i x[b] + bias_i) of 1..64 rows in the chunks of :func:`rows16`; modes and results as in :func:`gemv`, activations in 16 bits."""
     dev, total = weights[0].units.device, sum(w.n for w in weights)
     if out is None:
         out = torch.empty(nb, total // 2 if mode == MODE_GLU else total, device=dev, dtype=torch.float32)

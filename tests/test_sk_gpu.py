@@ -245,6 +245,32 @@ def test_gemm16_matches_reference(segs, k, nb):
     sk.workspace("cuda").check()
 
 
+@pytest.mark.parametrize("segs,k", [([(16, GGMLType.Q6_K)], 256), ([(2064, GGMLType.Q4_K)], 256), ([(400, GGMLType.Q6_K), (2000, GGMLType.Q4_K)], 1280),
+                                    ([(272, GGMLType.Q4_K)], 14336), ([(4096, GGMLType.Q6_K)], 1024), ([(20480, GGMLType.Q4_K)], 768)])
+@pytest.mark.parametrize("nb", [2, 16, 17, 33, 48, 49, 64])
+def test_gemm16_items_and_rows(segs, k, nb):
+    """Every number of 16-row groups of x, with a block a group of matrix rows, groups that end inside a share (finished while the next is under way), shares that end inside a group
+    (handed over by either set of warps), one group over all CTAs, and partly filled groups; bound as above."""
+    _, sk = _mods()
+    gen = torch.Generator().manual_seed(nb + k)
+    ws = [sk.repack(QWeight.from_float("w", torch.randn(n, k, generator=gen) * 0.05, t), "cuda") for n, t in segs]
+    W = torch.cat([sk.unit_weights(w) for w in ws]).double().cuda()
+    x = torch.randn(nb, k, generator=gen).cuda()
+    ref = x.double() @ W.t()
+    tol = 2 ** -9 * ref.std(1, keepdim=True) + 1e-6
+    chunks = sk.rows16(x)
+    out = torch.ones(nb, W.shape[0], device="cuda")
+    for ctas in (0, 7):                                 # as many CTAs as SMs, and a few with long shares
+        assert ((sk.gemm16(ws, chunks, nb, max_ctas=ctas).double() - ref).abs() <= tol).all()
+        assert torch.equal(sk.gemm16(ws, chunks, nb, max_ctas=ctas), sk.gemm16(ws, chunks, nb, max_ctas=ctas))
+    sk.gemm16(ws, chunks, nb, out=out, mode=sk.MODE_ACCUM)
+    assert ((out.double() - 1 - ref).abs() <= tol + 2e-6).all()
+    if all(n % 2 == 0 for n, _ in segs):
+        glu = torch.nn.functional.silu(ref[:, 0::2]) * ref[:, 1::2]
+        assert (sk.gemm16(ws, chunks, nb, mode=sk.MODE_GLU).double() - glu).norm() < 2 ** -9 * glu.norm()
+    sk.workspace("cuda").check()
+
+
 def test_gemm16_glu_matches_reference():
     _, sk = _mods()
     gen = torch.Generator().manual_seed(3)
