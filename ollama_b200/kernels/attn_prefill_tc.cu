@@ -452,6 +452,36 @@ bool cached_kv_map(CUtensorMap* out, const void* base, size_t rows, int d, int b
 constexpr int THREADS2 = (SOFTMAX_WARPS + 3) * 32;
 constexpr int TMEM_COLS2 = 512;
 
+__device__ __forceinline__ uint32_t cluster_size() {
+    uint32_t v;
+    asm volatile("mov.u32 %0, %cluster_nctaid.x;" : "=r"(v));
+    return v;
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t v;
+    asm volatile("mov.u32 %0, %cluster_ctaid.x;" : "=r"(v));
+    return v;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Shared memory of CTA `rank` of the cluster, at this CTA's address `at`.
+__device__ __forceinline__ uint32_t peer_at(uint32_t at, int rank) {
+    uint32_t p;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(p) : "r"(at), "r"(rank));
+    return p;
+}
+__device__ __forceinline__ float2 ld_cluster2(uint32_t at, int rank) {
+    float2 v;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(peer_at(at, rank)));
+    return v;
+}
+__device__ __forceinline__ float4 ld_cluster4(uint32_t at, int rank) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(peer_at(at, rank)));
+    return v;
+}
+
 enum CacheForm : int { FLAT = 0, PAGED_CACHE = 1, PARTS = 2 };
 
 template <int D, int DK>
@@ -466,7 +496,9 @@ struct Lay2 {
 // D: value columns, DK: query / key columns (D unless the form is PARTS).  DIFF: a CTA takes 64 queries of a head of differential attention, rows 0 .. 63 of its tile
 // with the first map, rows 64 .. 127 with the second; the key rows hold both maps' keys, of which a query row has zeros against the other map's.
 // a.scale is above zero, qsign a factor of the queries (positive_scale).
-template <int D, int DK, int FORM, bool DIFF = false>
+// SPLIT (flat caches): the CTAs of a cluster share the keys of a query tile, equal runs of tiles each, and merge their sums through distributed shared memory.  A few query rows
+// behind a long context are one tile a head, which left 116 of 148 SMs idle.
+template <int D, int DK, int FORM, bool DIFF = false, bool SPLIT = false>
 __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                                                                        const __grid_constant__ AttnPrefillArgs a, const __grid_constant__ AttnPagedArgs pg,
                                                                        const __grid_constant__ AttnPartsArgs pt, float qsign) {
@@ -491,7 +523,8 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
     float* x_sum = x_max + 256;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int mt = gridDim.x - 1 - blockIdx.x;
+    const int parts = SPLIT ? (int)cluster_size() : 1, part = SPLIT ? (int)cluster_rank() : 0;
+    const int mt = gridDim.x / parts - 1 - blockIdx.x / parts;
     const int4 tile = FORM == PARTS ? pt.tiles[mt] : PAGED ? pg.tiles[mt] : make_int4(mt * BQ, min(BQ, a.T - mt * BQ), a.slot, a.pos0 + mt * BQ);
     const int m0 = tile.x, rows = tile.y, h = blockIdx.y, hkv = FORM == PARTS ? h : h / (a.H / (DIFF ? 2 : 1) / a.Hkv);
     const int q_lo = tile.w, q_hi = q_lo + rows - 1;
@@ -501,8 +534,9 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
     const int window = FORM == PAGED_CACHE ? pg.window : a.window, keep = FORM == PAGED_CACHE && window > 0 ? pg.keep : 0;
     const int k_begin = first_key(q_lo, chunk, window) & ~(BKV - 1);
     const int front = kept_tiles(keep, k_begin, BKV);      // tiles at the sequence's start, for its kept keys
-    const int n_tiles = front + (k_end > k_begin ? (k_end - k_begin + BKV - 1) / BKV : 0);
-    auto first_of = [&](int t) { return t < front ? t * BKV : k_begin + (t - front) * BKV; };
+    const int all_tiles = front + (k_end > k_begin ? (k_end - k_begin + BKV - 1) / BKV : 0);
+    const int t_lo = SPLIT ? all_tiles * part / parts : 0, n_tiles = SPLIT ? all_tiles * (part + 1) / parts - t_lo : all_tiles;
+    auto first_of = [&](int t) { return t < front ? t * BKV : k_begin + (t + t_lo - front) * BKV; };
 
     if (threadIdx.x == 0) {
         *failed = 0;
@@ -561,7 +595,7 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     pdl_launch();      // not before the tensor memory is there: CTAs of the next kernel that came first would keep it until this one ends
-    const int row0 = FORM == PARTS ? tile.z + k_begin : PAGED ? 0 : (a.slot * a.Hkv + hkv) * a.n_ctx + k_begin;
+    const int row0 = FORM == PARTS ? tile.z + k_begin : PAGED ? 0 : (a.slot * a.Hkv + hkv) * a.n_ctx + k_begin + t_lo * BKV;
     const int* table = FORM == PAGED_CACHE ? pg.page_table + (size_t)tile.z * pg.max_pages : nullptr;
 
     if (warp == 8 || warp == 10) {
@@ -729,7 +763,14 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
             ok = false;
             atomicExch(failed, 1);
         }
-        if constexpr (DIFF) {      // the second map's rows meet the first's in the key buffers, which no product reads any more; every softmax thread passes the barriers
+        if constexpr (SPLIT) {      // unnormalised rows and their maximum and sum to the key buffers, which no product reads any more
+            float* mine = reinterpret_cast<float*>(sm + L::OFF_K) + r * (D + 4) + OH * c;
+            if (r < rows) {
+#pragma unroll
+                for (int j = 0; j < OH; j += 4) *(float4*)(mine + j) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
+            }
+            if (c == 0) reinterpret_cast<float2*>(x_max)[r] = make_float2(m_run * mult, l_run + x_sum[128 + r]);
+        } else if constexpr (DIFF) {      // the second map's rows meet the first's in the key buffers, which no product reads any more; every softmax thread passes the barriers
             constexpr int LDX = D + 4;
             float* other = reinterpret_cast<float*>(sm + L::OFF_K);      // [64][LDX]
             const float l = l_run + x_sum[(c ^ 1) * 128 + r], inv = l > 0.f ? 1.f / l : 0.f;
@@ -841,6 +882,34 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
             }
         }
     }
+    if constexpr (SPLIT) {
+        __syncwarp();
+        cluster_sync();      // all threads of all CTAs get here: every wait before it is bounded
+        if (warp < SOFTMAX_WARPS) {
+            const uint32_t o_at = smem_u32(sm + L::OFF_K), ml_at = smem_u32(x_max);
+            const float sink = a.sinks ? a.sinks[h] * 1.4426950408889634f : -INFINITY;
+            for (int e = part * SOFTMAX_WARPS * 32 + threadIdx.x; e < rows * (D / 4); e += parts * SOFTMAX_WARPS * 32) {
+                const int r = e / (D / 4), col = 4 * (e % (D / 4));
+                float m = sink;
+                for (int s = 0; s < parts; s++) m = fmaxf(m, ld_cluster2(ml_at + r * 8, s).x);
+                float l = sink == -INFINITY ? 0.f : ex2(sink - m);
+                float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int s = 0; s < parts; s++) {
+                    const float2 ml = ld_cluster2(ml_at + r * 8, s);
+                    const float4 v = ld_cluster4(o_at + (r * (D + 4) + col) * 4, s);
+                    const float w = ml.x == -INFINITY ? 0.f : ex2(ml.x - m);
+                    l += ml.y * w;
+                    y.x += v.x * w; y.y += v.y * w; y.z += v.z * w; y.w += v.w * w;
+                }
+                const float inv = l > 0.f ? 1.f / l : 0.f;
+                const __nv_bfloat162 lo = __floats2bfloat162_rn(y.x * inv, y.y * inv), hi = __floats2bfloat162_rn(y.z * inv, y.w * inv);
+                *(uint2*)(a.out + (size_t)(m0 + r) * a.H * D + (size_t)h * D + col) =
+                    make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+            }
+        }
+        __syncwarp();
+        cluster_sync();      // no CTA leaves while others read its memory
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == 9) {
@@ -875,6 +944,21 @@ float positive_scale(AttnPrefillArgs& a) {
     return s == 0.f ? 0.f : -1.f;
 }
 
+// CTAs that share the keys of a query tile (a cluster): as many of 8, 4 or 2 as there are SMs for and as leave each of them two tiles of 128 keys.  The cluster and its merge cost
+// about 3 us, a tile 1.3, so eight tiles are the least: 32 heads of 128, 7 rows behind 901: 15.7 -> 10.5 us, 64 behind 4000: 46.6 -> 19.8, 128 behind 6000: 68.6 -> 27.8, but 100
+// behind 300 12.7 -> 14.3.
+int key_parts(const AttnPrefillArgs& a, int tiles) {
+    static int sms[64] = {};
+    int d = 0;
+    cudaGetDevice(&d);
+    d &= 63;
+    if (!sms[d]) cudaDeviceGetAttribute(&sms[d], cudaDevAttrMultiProcessorCount, d);
+    const int keys = a.window > 0 && a.causal ? (a.kv_len < a.window + BQ ? a.kv_len : a.window + BQ) : a.kv_len;
+    for (int p = 8; p > 1; p >>= 1)
+        if (tiles * p <= sms[d] && keys > (p > 4 ? 2 * p - 1 : 7) * BKV) return p;
+    return 1;
+}
+
 template <int D>
 int launch2(const AttnPrefillArgs& a, int n_slots, int pdl, cudaStream_t st) {
     CUtensorMap mk, mv;
@@ -888,6 +972,26 @@ int launch2(const AttnPrefillArgs& a, int n_slots, int pdl, cudaStream_t st) {
     AttnPartsArgs pt = {};
     float qsign = positive_scale(copy);
     void* args[] = {&mk, &mv, &copy, &pg, &pt, &qsign};
+    const int parts = key_parts(a, (int)(grid.x * grid.y));
+    if (parts > 1) {
+        const void* fn = (const void*)attn_prefill_tc2_kernel<D, D, FLAT, false, true>;
+        static PerDeviceOnce split_once;
+        if (split_once.first()) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay2<D, D>::TOTAL);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(grid.x * parts, grid.y);
+        cfg.blockDim = dim3(THREADS2);
+        cfg.dynamicSmemBytes = Lay2<D, D>::TOTAL;
+        cfg.stream = st;
+        cudaLaunchAttribute at[2];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = parts;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[1].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
+        cfg.attrs = at;
+        cfg.numAttrs = 2;
+        return (int)cudaLaunchKernelExC(&cfg, fn, args);
+    }
     return launch_rows((const void*)attn_prefill_tc2_kernel<D, D, FLAT>, grid, dim3(THREADS2), Lay2<D, D>::TOTAL, args, st, pdl);
 }
 

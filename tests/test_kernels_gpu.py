@@ -420,6 +420,25 @@ def test_attn_prefill_on_tcgen05(hd, H, Hkv, T, pos0, window, softcap, use_sinks
     assert torch.allclose(out, ref, atol=1e-2, rtol=2e-2), (out - ref).abs().max()
 
 
+@pytest.mark.parametrize("hd,H,Hkv", [(128, 8, 2), (64, 16, 4)])
+@pytest.mark.parametrize("T,pos0,window,softcap,use_sinks", [(1, 896, 0, 0.0, False), (7, 1020, 0, 0.0, True), (128, 1920, 0, 0.0, False), (130, 2100, 0, 30.0, True),
+                                                              (200, 2500, 1000, 0.0, False), (66, 2700, 1, 0.0, False), (257, 2000, 2200, 0.0, True)])
+def test_attn_prefill_shares_keys(hd, H, Hkv, T, pos0, window, softcap, use_sinks):
+    """Few query tiles behind a long context: clusters of two to eight CTAs share a tile's keys, with windows that leave some of them none.  Bound as above."""
+    K = _K()
+    n_slots, n_ctx, slot = 2, 3072, 1
+    g = torch.Generator().manual_seed(hd + T)
+    kc, vc = ((torch.randn(n_slots, Hkv, n_ctx, hd, generator=g) * 0.7).to(torch.float16).cuda() for _ in range(2))
+    q = torch.randn(T, H, hd, generator=g).cuda()
+    sinks = torch.randn(H, generator=g).cuda() if use_sinks else None
+    scale, p_end = 1 / math.sqrt(hd), pos0 + T
+    out = K.attn_prefill(q, kc, vc, slot, pos0, p_end, scale, True, window, softcap, sinks, mode="tc").float().cpu().view(T, H, hd)
+    assert K.attn_prefill_tc_status(clear=True) == 0
+    ref = R.attention(q.to(torch.float16).float().cpu(), kc[slot, :, :p_end].transpose(0, 1).float().cpu(), vc[slot, :, :p_end].transpose(0, 1).float().cpu(),
+                      torch.arange(pos0, p_end), torch.arange(p_end), scale=scale, causal=True, window=window, softcap=softcap, sinks=sinks.cpu() if use_sinks else None)
+    assert torch.allclose(out, ref, atol=1e-2, rtol=2e-2), (out - ref).abs().max()
+
+
 @pytest.mark.parametrize("scale", [-0.1, 0.0])
 @pytest.mark.parametrize("hd,T,pos0,window,use_sinks", [(128, 300, 517, 0, False), (64, 129, 0, 48, True), (128, 5, 0, 0, False)])
 def test_attn_prefill_of_any_scale(hd, T, pos0, window, use_sinks, scale):
