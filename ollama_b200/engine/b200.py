@@ -782,7 +782,7 @@ class B200Backend(StepEngine):
         if self._unit_rows(x.shape[0]) and getattr(self, "sk_head", None) is not None:
             out = torch.empty(x.shape[0], self.cfg.vocab_size, device=self.device, dtype=torch.float32)
             self._rows_sk([self.sk_head], x.contiguous(), out, self.out_norm, wsp=self._pass.ws if self._pass is not None and self._pass.ws is not None else self._ws)
-            self.kernel_launches += 2 * ((x.shape[0] + SK.MAX_TOKENS - 1) // SK.MAX_TOKENS)
+            self.kernel_launches += 2
             return R.softcap(out, self.cfg.final_softcap)
         return R.softcap(self._mm(self._final_norm(x).to(torch.bfloat16), self.head), self.cfg.final_softcap)
 

@@ -920,6 +920,31 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
 }
 
 
+// Rows [lo, hi) of an int8 cache of one slot as f16, [K, V][Hkv][pitch][D]; rows from kv_len on are zeros (a masked key's value still meets a probability of zero).  A thread has
+// 16 dims, half of a scale's block.
+__global__ void __launch_bounds__(256) expand_q8_kernel(const __grid_constant__ AttnPrefillArgs a, int D, int lo, int hi, int pitch, __half* out) {
+    pdl_launch();
+    pdl_wait();
+    const int per = D / 16, n = (hi - lo) * per, i = blockIdx.x * 256 + threadIdx.x, hkv = blockIdx.y >> 1, is_v = blockIdx.y & 1;
+    if (i >= n) return;
+    const int pos = lo + i / per, col = 16 * (i % per);
+    uint32_t w[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+    if (pos < a.kv_len) {
+        const size_t row = ((size_t)a.slot * a.Hkv + hkv) * a.n_ctx + pos;
+        const uint4 q = *reinterpret_cast<const uint4*>(reinterpret_cast<const int8_t*>(is_v ? a.v_cache : a.k_cache) + row * D + col);
+        const float d = __half2float((is_v ? a.v_scale : a.k_scale)[row * (D / 32) + (col >> 5)]);
+        const uint32_t u[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const uint32_t b = u[j >> 1] >> (16 * (j & 1));
+            w[j] = pack_h2(d * (float)(int8_t)(b & 0xff), d * (float)(int8_t)((b >> 8) & 0xff));
+        }
+    }
+    uint4* o = reinterpret_cast<uint4*>(out + (((size_t)is_v * a.Hkv + hkv) * pitch + pos) * D + col);
+    o[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    o[1] = make_uint4(w[4], w[5], w[6], w[7]);
+}
+
 int g_variant = 2;      // 0: probabilities through shared memory, 1: probabilities in TMEM, 2: the pipelined kernel (default)
 
 template <int D, bool PT>
@@ -1100,4 +1125,36 @@ B2_API int b2_attn_prefill_tc_status() {
 B2_API void b2_attn_prefill_tc_clear_status() {
     const int v = 0;
     cudaMemcpyToSymbol(g_attn_tc_status, &v, sizeof(int));
+}
+
+// Halves of scratch that b2_attn_prefill_q8 takes for kv_len keys.
+B2_API long long b2_attn_prefill_q8_scratch(int kv_len, int n_kv_heads, int head_dim) { return 2ll * n_kv_heads * ((kv_len + BKV - 1) / BKV * BKV) * head_dim; }
+
+// The same on an int8 cache with scales: its rows that queries may see are expanded into `scratch` (16-byte aligned, b2_attn_prefill_q8_scratch halves) once, where the kernel that
+// expands them on the way (attn_prefill.cu) does so for every 64 queries of a head and multiplies with mma.sync.  32 heads of 128: 7 rows behind 901 57 -> 14 us, 64 behind 4000
+// 236 -> 25, 2048 behind 4000 1401 -> 253; 2 rows behind 50 6.6 -> 8.4, so up to 64 keys stay there.  Head size 64 or 128 (anything else, and other alignments:
+// cudaErrorNotSupported, nothing launched).
+B2_API int b2_attn_prefill_q8(const AttnPrefillArgs* in, int head_dim, int n_slots, void* scratch, int pdl, cudaStream_t st) {
+    if (!in || !in->k_scale || !in->v_scale || !scratch || in->T < 1 || in->H < 1 || in->Hkv < 1 || in->Hkv > 32767 || in->H % in->Hkv || in->kv_len < 1 || in->kv_len > in->n_ctx ||
+        n_slots < 1 || in->slot < 0 || in->slot >= n_slots || in->pos0 < 0)
+        return (int)cudaErrorInvalidValue;
+    AttnPrefillArgs a = *in;
+    if ((head_dim != 64 && head_dim != 128) || g_variant != 2 || a.kv_len <= 64 ||
+        (((uintptr_t)a.k_cache | (uintptr_t)a.v_cache | (uintptr_t)a.q | (uintptr_t)a.out | (uintptr_t)scratch) & 15))
+        return (int)cudaErrorNotSupported;
+    const int pitch = (a.kv_len + BKV - 1) / BKV * BKV;
+    if ((size_t)a.Hkv * pitch >= ((size_t)1 << 31)) return (int)cudaErrorNotSupported;
+    int lo = a.window > 0 && a.pos0 >= a.window ? (a.pos0 - a.window + 1) / BKV * BKV : 0, hi = pitch;
+    if (lo >= hi) lo = hi - BKV;
+    __half* out = (__half*)scratch;
+    void* args[] = {&a, &head_dim, &lo, &hi, (void*)&pitch, &out};
+    const int rc = launch_rows((const void*)expand_q8_kernel, dim3(((hi - lo) * (head_dim / 16) + 255) / 256, 2 * a.Hkv), dim3(256), 0, args, st, pdl);
+    if (rc) return rc;
+    AttnPrefillArgs c = a;
+    c.k_cache = out;
+    c.v_cache = out + (size_t)a.Hkv * pitch * head_dim;
+    c.k_scale = c.v_scale = nullptr;
+    c.slot = 0;
+    c.n_ctx = pitch;
+    return head_dim == 128 ? launch2<128>(c, 1, pdl, st) : launch2<64>(c, 1, pdl, st);
 }

@@ -9,6 +9,7 @@ extern "C" {
 int b2_rmsnorm_bf16(const NormCastArgs* a, int rows, int pdl, cudaStream_t st);
 int b2_rope_kv(const RopeKvArgs* a, int nt, int pdl, cudaStream_t st);
 int b2_attn_prefill_tc(const AttnPrefillArgs* a, int head_dim, int n_slots, int pdl, cudaStream_t st);
+int b2_attn_prefill_q8(const AttnPrefillArgs* in, int head_dim, int n_slots, void* scratch, int pdl, cudaStream_t st);
 int b2_attn_prefill(const AttnPrefillArgs* a, int head_dim, cudaStream_t st);
 int b2_gemm_bf16(const void* a, const void* b, int m, int n, int k, float* out, int ldo, const float* bias, int accumulate, int pdl, float* ws,
                  long long ws_floats, cudaStream_t st);
@@ -45,6 +46,7 @@ struct PassArgs {
     unsigned* flags;
     int* status;
     int units, tc, pdl;                           // tc: attention on tcgen05 where it applies
+    void* kv16;                                   // int8 caches: b2_attn_prefill_q8_scratch halves for the longest sequence, or null
     int launches;                                 // out
 };
 
@@ -110,7 +112,12 @@ B2_API int b2_prefill_pass(const PassLayer* layers, int n, PassArgs* io, const P
             const PassSeg& g = segs[s];
             const AttnPrefillArgs at{a.q + (size_t)g.row0 * qd, L.k_cache, L.v_cache, (__nv_bfloat16*)a.o + (size_t)g.row0 * qd, L.sinks, g.rows, a.n_heads, a.n_kv_heads, a.n_ctx,
                                      g.slot, g.pos0, g.pos0 + g.rows, a.causal, L.window, a.scale, a.softcap, L.k_scale, L.v_scale};
-            rc = a.tc && (a.hd == 64 || a.hd == 128) && !L.k_scale ? b2_attn_prefill_tc(&at, a.hd, a.n_slots, a.pdl, st) : (int)cudaErrorNotSupported;
+            rc = (int)cudaErrorNotSupported;
+            if (a.tc && (a.hd == 64 || a.hd == 128))
+                rc = !L.k_scale ? b2_attn_prefill_tc(&at, a.hd, a.n_slots, a.pdl, st)
+                     : a.kv16   ? b2_attn_prefill_q8(&at, a.hd, a.n_slots, a.kv16, a.pdl, st)
+                                : (int)cudaErrorNotSupported;
+            if (!rc && L.k_scale) count++;
             if (rc == (int)cudaErrorNotSupported) rc = b2_attn_prefill(&at, a.hd, st);      // nothing was launched
         }
         if (rc) break;

@@ -612,12 +612,19 @@ ATTN_PREFILL_HEAD_DIMS = (32, 64, 128, 256)
 ATTN_PREFILL_DEFAULT = "auto"       # the kernel prefill attention runs on unless told otherwise (see attn_prefill)
 
 
+def attn_prefill_q8_scratch(kv_len: int, n_kv_heads: int, head_dim: int, device) -> torch.Tensor:
+    """Room for the visible rows of a slot's int8 cache as f16 (kernels/attn_prefill_tc.cu)."""
+    f = lib().b2_attn_prefill_q8_scratch
+    f.restype = C.c_longlong
+    return torch.empty(f(kv_len, n_kv_heads, head_dim), device=device, dtype=torch.float16)
+
+
 def attn_prefill(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, slot: int, pos0: int, kv_len: int, scale: float,
                  causal: bool = True, window: int = 0, softcap: float = 0.0, sinks: torch.Tensor | None = None,
                  k_scale: torch.Tensor | None = None, v_scale: torch.Tensor | None = None, mode: str | None = None, pdl: bool = False) -> torch.Tensor:
     """Flash attention of a prefill chunk: q [T, H, D] fp32 -> bf16 [T, H * D].  ``mode``: "tc" = the tcgen05 kernel
     (kernels/attn_prefill_tc.cu: f16 caches, head size 64 / 128), "mma" = the mma.sync kernel (kernels/attn_prefill.cu), "auto" =
-    tcgen05 where it applies.  Default: B200_ATTN_PREFILL, else ATTN_PREFILL_DEFAULT."""
+    tcgen05 where it applies, int8 caches as expanded rows.  Default: B200_ATTN_PREFILL, else ATTN_PREFILL_DEFAULT."""
     T, H, D = q.shape
     n_slots, Hkv, n_ctx, _ = k_cache.shape
     out = torch.empty(T, H * D, device=q.device, dtype=torch.bfloat16)
@@ -632,6 +639,13 @@ def attn_prefill(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
             _check(rc, "attn_prefill_tc")
     elif mode == "tc":
         raise RuntimeError("attn_prefill: the tcgen05 kernel takes f16 caches and head size 64 or 128")
+    elif mode == "auto" and D in (64, 128) and k_scale is not None and q.dtype == torch.float32:
+        scratch = attn_prefill_q8_scratch(kv_len, Hkv, D, q.device)
+        rc = lib().b2_attn_prefill_q8(C.byref(a), D, n_slots, C.c_void_p(ptr(scratch)), int(pdl), stream())
+        if rc == 0:
+            return out
+        if rc != 801:
+            _check(rc, "attn_prefill_q8")
     _check(lib().b2_attn_prefill(C.byref(a), D, stream()), "attn_prefill")
     return out
 

@@ -439,6 +439,32 @@ def test_attn_prefill_shares_keys(hd, H, Hkv, T, pos0, window, softcap, use_sink
     assert torch.allclose(out, ref, atol=1e-2, rtol=2e-2), (out - ref).abs().max()
 
 
+@pytest.mark.parametrize("hd,H,Hkv", [(128, 8, 2), (64, 6, 3)])
+@pytest.mark.parametrize("T,pos0,window,causal", [(65, 0, 0, True), (7, 120, 0, True), (130, 700, 0, True), (100, 900, 300, True), (3, 1020, 1, True), (150, 0, 0, False)])
+def test_attn_prefill_of_int8_caches_expanded(hd, H, Hkv, T, pos0, window, causal):
+    """Visible rows of an int8 cache, expanded once, against the same cache expanded on the host (f16, as both kernels round) and against the kernel that expands on the way; what lies
+    behind the last key in the scratch must not matter.  Bound as above."""
+    K = _K()
+    n_slots, n_ctx, slot, p_end = 2, 1100, 1, pos0 + T
+    g = torch.Generator().manual_seed(hd + T)
+    kc, vc = (torch.randint(-127, 128, (n_slots, Hkv, n_ctx, hd), generator=g, dtype=torch.int8) for _ in range(2))
+    ks, vs = ((torch.rand(n_slots, Hkv, n_ctx, hd // 32, generator=g) * 0.02).to(torch.float16) for _ in range(2))
+    q = torch.randn(T, H, hd, generator=g)
+    poison = torch.full((8 << 20,), float("nan"), device="cuda", dtype=torch.float16)
+    del poison                                         # what the scratch is likely to get
+    args = (slot, pos0, p_end, 1 / math.sqrt(hd), causal, window)
+    dev = [t.cuda() for t in (q, kc, vc, ks, vs)]
+    out = K.attn_prefill(*dev[:3], *args, k_scale=dev[3], v_scale=dev[4])
+    old = K.attn_prefill(*dev[:3], *args, k_scale=dev[3], v_scale=dev[4], mode="mma")
+    assert K.attn_prefill_tc_status(clear=True) == 0
+    k, v = ((c.float().view(n_slots, Hkv, n_ctx, -1, 32) * s.float()[..., None]).to(torch.float16).float().view(n_slots, Hkv, n_ctx, hd)[slot, :, :p_end].transpose(0, 1)
+            for c, s in ((kc, ks), (vc, vs)))
+    ref = R.attention(q.to(torch.float16).float(), k, v, torch.arange(pos0, p_end), torch.arange(p_end), scale=1 / math.sqrt(hd), causal=causal, window=window)
+    for o in (out, old):
+        got = o.float().cpu().view(T, H, hd)
+        assert torch.allclose(got, ref, atol=1e-2, rtol=2e-2), (got - ref).abs().max()
+
+
 @pytest.mark.parametrize("scale", [-0.1, 0.0])
 @pytest.mark.parametrize("hd,T,pos0,window,use_sinks", [(128, 300, 517, 0, False), (64, 129, 0, 48, True), (128, 5, 0, 0, False)])
 def test_attn_prefill_of_any_scale(hd, T, pos0, window, use_sinks, scale):
