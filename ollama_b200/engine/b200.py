@@ -474,14 +474,14 @@ class B200Backend(StepEngine):
         per = T * k / c.n_experts
         if (self.moe_stream_q and getattr(L.gu, "bf16", None) is None and K.moe_fp4_supported(L.gu) and K.moe_fp4_supported(L.down)
                 and (per <= FP4_MAX_ROWS or not (K.gemm_q_grouped_supported(L.gu) and K.gemm_q_grouped_supported(L.down)))):
-            # experts without a resident 16-bit copy: their 4-bit blocks are multiplied as they are, once for up to 64 rows.  Chunks of about twice
-            # the mean, so that few experts need a second one: at 32 rows 769 us a layer in chunks of 64, 830 of 32; at 8 rows 512 of 16, 541 of 32
-            m = K.MoeFp4(T * k, self.e_cnt, c.d_model, c.d_ff_expert, self.device, 8 if per <= 4 else 16 if per <= 8 else 32 if per <= 20 else 64)
-            m.sort(lids, T * k)
-            m.take(h, k, T * k)
-            m.product(L.gu, T * k, c.act, c.swiglu_alpha, c.swiglu_limit)
+            # experts without a resident 16-bit copy: their 4-bit blocks are multiplied as they are, once for a chunk of rows.  Chunks that few experts
+            # need a second one of (1024 tokens of 128 experts, 32 rows a mean: 765 us a layer in chunks of 48, 787 of 40, 942 of 32, 794 of 64)
+            m = K.MoeFp4(T * k, self.e_cnt, c.d_model, c.d_ff_expert, self.device, K.moe_fp4_chunk(per))
+            m.sort(lids, T * k, self.pdl)
+            m.take(h, k, T * k, self.pdl)
+            m.product(L.gu, T * k, c.act, c.swiglu_alpha, c.swiglu_limit, pdl=self.pdl)
             ys = torch.empty(m.rows, c.d_model, device=self.device, dtype=torch.float32)
-            m.product(L.down, T * k, out=ys)
+            m.product(L.down, T * k, out=ys, pdl=self.pdl)
             self.kernel_launches += 6
             return K.moe_scatter_combine(ys, m.row_of_pair, wts, T, k, out=x, accumulate=x is not None)
         row, tile_expert, rows = K.moe_plan(lids, self.e_cnt)

@@ -12,9 +12,11 @@
 //     (to 2^-18 of the block's largest value).  They are two rows of N; the epilogue adds their columns.
 //   * The codes of a 32-column block are stored as bytes of columns c and 16 + c; the rows are written in that order of columns too (moe_rows_kernel), tile by tile in the layout
 //     and swizzle that shared memory has, so that a step's rows are one bulk copy; the scales of a tile's matrix rows are one more.
-//   * What bounds it now is the path through L1 and shared memory: 690 cycles a step of 128 x 128 codes, in which the loads and stores of the codes keep it busy for 440 and the
-//     tensor core's reads for 170.  Three CTAs an SM with two stages each are best (two with three stages 10 % slower; four leave the L1 too small for the loads under way, 70 %
-//     slower).  128 bytes of a matrix row per request instead of 64 cost 10 % (the stores fall apart), 16-byte stores with the padding 10 %.
+//   * What bounds it now is the path through L1 and shared memory: 660 cycles a step of 128 x 128 codes at eight rows, in which a product of 32 columns takes 70 cycles to fetch its
+//     128 matrix rows however few rows it has (280 a step) and the loads and stores of the codes 256.  Three CTAs an SM with two stages each are best up to 24 rows (two with three
+//     stages 10 % slower; four leave the L1 too small for the loads under way, 70 % slower), two from 32 rows on.  128 bytes of a matrix row per request instead of 64 cost 10 %
+//     (the stores fall apart), 16-byte stores with the padding 10 %; codes through a cp.async ring in shared memory instead of registers, and two teams of warps that bring
+//     alternate steps, 20 % at eight rows (two CTAs fit) and nothing at 48.
 #include <cuda_fp8.h>
 
 #include "tc_common.cuh"
@@ -393,7 +395,8 @@ int launch(const MoeFp4Args& a, int max_chunks, int pdl, cudaStream_t st) {
     if (once.first()) cudaFuncSetAttribute(moe_fp4_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM);
     // No more shared memory than the CTAs need (1 KB each of static and of reserved memory): the rest is the L1 that the loads under way live in.  Left to itself the SM keeps the
     // split of a kernel before it: 16 tokens behind a GEMM of 200 KB took 173 us instead of 109.
-    const int fit = 228 * 1024 / (smem + 2048), ctas = fit < 3 ? fit : 3;
+    // At least 36 KB of it: with three CTAs of 32 to 48 rows an SM kept 3 to 27 KB, and 2048 pairs of 128 experts took 864 us at 32 rows, 677 with two CTAs.
+    const int fit = 192 * 1024 / (smem + 2048), ctas = fit < 1 ? 1 : fit < 3 ? fit : 3;
     cudaFuncSetAttribute(moe_fp4_kernel<R>, cudaFuncAttributePreferredSharedMemoryCarveout, (ctas * (smem + 2048) * 100 + 228 * 1024 - 1) / (228 * 1024));
     MoeFp4Args copy = a;
     void* args[] = {&copy};
@@ -422,7 +425,7 @@ B2_API int b2_moe_rows(const void* x, int bf16, int ldx, int cols, int per_token
     return go(bf16 ? (const void*)moe_rows_kernel<true> : (const void*)moe_rows_kernel<false>, dim3(pairs), dim3(256), args, st, pdl);
 }
 
-// chunk_rows: 8, 16, 32 or 64, what moe_sort and moe_rows were given.  Returns a cudaError_t value (cudaErrorNotSupported: other shapes; nothing launched).
+// chunk_rows: 8, 16, 24, 32, 40, 48 or 64, what moe_sort and moe_rows were given.  Returns a cudaError_t value (cudaErrorNotSupported: other shapes; nothing launched).
 B2_API int b2_moe_fp4(const MoeFp4Args* in, int chunk_rows, int max_chunks, int pdl, cudaStream_t st) {
     const MoeFp4Args a = *in;
     if (!a.q || !a.s || !a.x || !a.chunks || !a.out || max_chunks < 1 || max_chunks > 65535 || a.glu < 0 || a.glu > 3 || (((uintptr_t)a.q | (uintptr_t)a.s | (uintptr_t)a.x) & 15))
@@ -431,7 +434,10 @@ B2_API int b2_moe_fp4(const MoeFp4Args* in, int chunk_rows, int max_chunks, int 
     switch (chunk_rows) {
         case 8: return launch<8>(a, max_chunks, pdl, st);
         case 16: return launch<16>(a, max_chunks, pdl, st);
+        case 24: return launch<24>(a, max_chunks, pdl, st);
         case 32: return launch<32>(a, max_chunks, pdl, st);
+        case 40: return launch<40>(a, max_chunks, pdl, st);
+        case 48: return launch<48>(a, max_chunks, pdl, st);
         case 64: return launch<64>(a, max_chunks, pdl, st);
     }
     return (int)cudaErrorInvalidValue;

@@ -816,11 +816,17 @@ def moe_fp4_supported(w: DevWeight) -> bool:
     return w.wtype == WT_MXFP4 and w.n % 16 == 0 and w.k % 32 == 0 and w.k <= 16384
 
 
+def moe_fp4_chunk(rows: float) -> int:
+    """Rows of a chunk for so many rows an expert on average.  A layer of 128 experts of 13 MB by mean and chunk, us: 4: 439 (8), 496 (16); 8: 534 (16), 556 (24), 631 (8); 12: 581 (24),
+    606 (16), 652 (32); 16: 616 (24), 677 (32), 736 (16); 20: 690 (24), 703 (32); 24: 729 (48), 736 (40), 760 (32), 810 (24); 32: 765 (48), 794 (64); 40: 863 (64), 870 (48)."""
+    return 8 if rows <= 5 else 16 if rows <= 9 else 24 if rows <= 20 else 48 if rows <= 36 else 64
+
+
 class MoeFp4:
     """The (token, expert) pairs of a step or a prompt times MXFP4 experts, each expert read once for all rows that chose it (kernels/moe_fp4.cu).
 
     Holds the sorted places of the pairs and the row buffers, so that a decode step can keep one for its CUDA graph; sizes that depend on the choice of
-    experts never visit the host.  ``chunk``: rows of an expert that a block multiplies at once, 8 / 16 / 32 / 64."""
+    experts never visit the host.  ``chunk``: rows of an expert that a block multiplies at once, 8 / 16 / 24 / 32 / 40 / 48 / 64."""
 
     def __init__(self, pairs: int, n_experts: int, d: int, ff: int, device, chunk: int):
         self.n_experts, self.d, self.ff, self.chunk = n_experts, d, ff, chunk

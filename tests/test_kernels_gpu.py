@@ -919,6 +919,12 @@ def test_moe_fp4_products(E, d, ff, T, k, chunk, bf16):
     assert torch.equal(by_pair[(lids < 0).cuda()], torch.zeros_like(by_pair[(lids < 0).cuda()]))
 
 
+@pytest.mark.parametrize("E,d,ff,T,k,chunk", [(5, 288, 160, 75, 2, 24), (5, 288, 160, 75, 2, 40), (4, 160, 288, 100, 2, 48), (1, 96, 64, 49, 1, 48)])
+def test_moe_fp4_chunks_between(E, d, ff, T, k, chunk):
+    """Chunks of 24, 40 and 48 rows, whose scales and accumulators end between powers of two; full chunks and a row more."""
+    test_moe_fp4_products(E, d, ff, T, k, chunk, True)
+
+
 @pytest.mark.parametrize("m,n,k", [(129, 64, 64), (257, 304, 520), (300, 192, 72), (1153, 5584, 1032), (769, 5408, 2056), (300, 1032, 5512), (512, 4096, 9000), (16, 5120, 2888), (100, 1032, 4104)])
 @pytest.mark.parametrize("pdl", [0, 2])
 def test_gemm_bf16_shapes(m, n, k, pdl):
