@@ -169,17 +169,35 @@ __global__ void attn_combine_kernel(const __grid_constant__ AttnCombineArgs a) {
     const int h = blockIdx.x, b = blockIdx.y, d = threadIdx.x;
     pdl_launch();
     pdl_wait();
+    // A split that holds no keys says so with a sum of zero and leaves its accumulators as they are.  Lane i looks at split i, so that the loads of what there is go out together.
     const size_t p0 = ((size_t)b * a.n_heads + h) * a.n_splits;
-    float mn = -1e30f;
-    for (int s = 0; s < a.n_splits; s++) mn = fmaxf(mn, a.part_ml[p0 + s].x);
-    if (a.sinks) mn = fmaxf(mn, a.sinks[h]);
+    const int lane = d & 31;
+    float mn = a.sinks ? a.sinks[h] : -1e30f;
+    const float2 first = lane < a.n_splits ? a.part_ml[p0 + lane] : make_float2(-1e30f, 0.f);
+    mn = fmaxf(mn, first.x);
+    for (int s0 = 32; s0 < a.n_splits; s0 += 32) mn = fmaxf(mn, s0 + lane < a.n_splits ? a.part_ml[p0 + s0 + lane].x : -1e30f);
+    mn = warp_max(mn);
     float o = 0.f, l = 0.f;
-    for (int s = 0; s < a.n_splits; s++) {
-        const float2 ml = a.part_ml[p0 + s];
-        const float c = __expf(ml.x - mn);
-        o += a.part_acc[(p0 + s) * a.hd + d] * c;
-        l += ml.y * c;
+    for (int s0 = 0; s0 < a.n_splits; s0 += 32) {
+        const float2 ml = s0 == 0 ? first : s0 + lane < a.n_splits ? a.part_ml[p0 + s0 + lane] : make_float2(-1e30f, 0.f);
+        const float w = ml.y > 0.f ? __expf(ml.x - mn) : 0.f;
+        const float* acc = a.part_acc + (p0 + s0) * a.hd + d;
+        unsigned used = __ballot_sync(0xffffffffu, ml.y > 0.f);
+        l += ml.y * w;
+        while (used) {      // eight at a time
+            float v[8], c[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const int i = __ffs(used) - 1;
+                c[j] = __shfl_sync(0xffffffffu, w, i < 0 ? 0 : i);
+                v[j] = i < 0 ? 0.f : acc[(size_t)i * a.hd];
+                used &= used - 1;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; j++) o += v[j] * c[j];
+        }
     }
+    l = warp_sum(l);
     if (a.sinks) l += __expf(a.sinks[h] - mn);
     const float v = l > 0.f ? o / l : 0.f;
     const size_t oi = ((size_t)b * a.n_heads + h) * a.hd + d;
@@ -310,10 +328,15 @@ B2_API int b2_attn_decode(const AttnDecodeArgs* a, const AttnCombineArgs* c, int
     AttnDecodeArgs ca = *a;
     void* args[] = {&ca};
     cudaError_t e = cudaErrorNotSupported;
-    if (use_mma(*a, hd)) e = (cudaError_t)attn_decode_mma_launch(*a, nb, hd, pdl, st);
+    AttnCombineArgs cc = *c;
+    if (use_mma(*a, hd)) {
+        AttnDecodeArgs m = *a;
+        m.n_splits = attn_decode_mma_splits(m, nb);
+        e = (cudaError_t)attn_decode_mma_launch(m, nb, hd, pdl, st);
+        if (e == cudaSuccess) cc.n_splits = m.n_splits;
+    }
     if (e == cudaErrorNotSupported) e = launch1(fn, grid, dim3(128), args, st, pdl);
     if (e != cudaSuccess) return (int)e;
-    AttnCombineArgs cc = *c;
     void* args2[] = {&cc};
     return (int)launch1((const void*)attn_combine_kernel, dim3(a->n_heads, nb), dim3(hd), args2, st, pdl);
 }
@@ -324,9 +347,12 @@ B2_API int b2_attn_decode(const AttnDecodeArgs* a, const AttnCombineArgs* c, int
 // b2_rope_kv + b2_attn_decode.
 B2_API int b2_attn_decode_rope(const AttnDecodeArgs* a, const AttnRopeArgs* r, const AttnCombineArgs* c, int nb, int hd, int pdl, cudaStream_t st) {
     if (!r || !r->qkv) return (int)cudaErrorInvalidValue;
-    const cudaError_t e = (cudaError_t)attn_decode_mma_rope_launch(*a, *r, nb, hd, pdl, st);
+    AttnDecodeArgs m = *a;
+    m.n_splits = attn_decode_mma_splits(m, nb);
+    const cudaError_t e = (cudaError_t)attn_decode_mma_rope_launch(m, *r, nb, hd, pdl, st);
     if (e != cudaSuccess) return (int)e;
     AttnCombineArgs cc = *c;
+    cc.n_splits = m.n_splits;
     void* args2[] = {&cc};
     return (int)launch1((const void*)attn_combine_kernel, dim3(a->n_heads, nb), dim3(hd), args2, st, pdl);
 }

@@ -331,6 +331,33 @@ def test_attn_decode_tensor_core_long_context(hd, H, Hkv, q8, attn_mode):
         assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
 
 
+@pytest.mark.parametrize("hd,H,Hkv,nb,n_splits,window", [(128, 32, 8, 24, 16, 0), (64, 64, 8, 17, 8, 0), (128, 16, 16, 32, 5, 0), (64, 16, 8, 32, 16, 130), (128, 32, 8, 9, 32, 0)])
+@pytest.mark.parametrize("q8", [False, True])
+def test_attn_decode_deals_positions_out(hd, H, Hkv, nb, n_splits, window, q8, attn_mode):
+    """More CTAs than fit at once: sequences of 1 to 2000 positions in equal shares, splits without keys whose accumulators hold NaN, against the scalar kernel (f16 products of
+    values of about one: 2^-9 of them)."""
+    K = _K()
+    n_ctx = 2048
+    g = torch.Generator().manual_seed(nb)
+    pos = torch.randint(0, 2000, (nb,), generator=g, dtype=torch.int32)
+    pos[0], pos[-1] = 0, 1999
+    if q8:
+        kc, vc = (torch.randint(-127, 128, (nb, Hkv, n_ctx, hd), generator=g, dtype=torch.int8).cuda() for _ in range(2))
+        ks, vs = ((torch.rand(nb, Hkv, n_ctx, hd // 32, generator=g) * 0.01).to(torch.float16).cuda() for _ in range(2))
+    else:
+        kc, vc = ((torch.randn(nb, Hkv, n_ctx, hd, generator=g) * 0.7).to(torch.float16).cuda() for _ in range(2))
+        ks = vs = None
+    q, slots = torch.randn(nb, H, hd, generator=g).cuda(), torch.randperm(nb, generator=g).to(torch.int32).cuda()
+
+    def run(mode):
+        attn_mode(mode)
+        scratch = tuple(torch.full((n,), float("nan"), device="cuda") for n in (nb * H * n_splits * hd, nb * H * n_splits * 2))
+        return K.attn_decode(q, kc, vc, pos.cuda(), slots, scale=hd ** -0.5, n_splits=n_splits, window=window, scratch=scratch, k_scale=ks, v_scale=vs, quant_out=False)[0]
+
+    ref, got = run(0), run(1)
+    assert (got - ref).abs().max() <= 2 ** -9 * max(1.0, float(ref.abs().max()))
+
+
 @pytest.mark.parametrize("hd,off", [(128, 1), (128, 2), (64, 1)])
 def test_attn_decode_with_scales_off_their_alignment(hd, off, attn_mode):
     """int8 caches whose scale arrays begin ``off`` f16 values off the alignment that the ring's copies need: the scalar kernel takes them, with the bits that it gives for aligned ones."""
