@@ -33,6 +33,9 @@
 //   * The activations are quantised by the CTA itself while its first units are in flight: the kernel
 //     reads the fp32 rows (optionally RMS-normalising them first), so a decode layer needs no separate
 //     norm / quantise launch.  Inputs too large for shared memory come pre-quantised from b2_quant256.
+//   * What bounds one token now: gate/up of Llama-8B streams 66 MB in 10 to 11.5 us once its inputs are there; the four products of a layer spend 1 us each from a CTA's start to
+//     its first request, 1.3 to 2.3 us on the inputs (a trip to L2, a barrier, two reductions) and 1 to 2 us on the slowest CTA.  Arguments of one phase instead of four, shares and
+//     rows by multiplication, norm weights fetched before the wait and one barrier instead of two took the four from 52.3 to 41.9 us a layer.
 #include "comm.cuh"
 
 constexpr int SK_WARPS = 8;
@@ -78,7 +81,9 @@ struct SkArgs {
     int off_red, off_xq, off_xd, off_xbs, off_ring;
     int ring, slot_bytes; // units per warp ring (2..4) and bytes per slot
     int wpt_log2;         // warps of a CTA that share one range of units: 1 << wpt_log2
-    int n_groups;         // ranges the launch's units are divided into
+    int n_groups;         // ranges the launch's units are divided into: group i begins at i share_q + min(i, share_r)
+    int share_q, share_r;
+    unsigned kt_magic;    // u / (k / 256) = the upper half of u times this, for units u of a launch; 0: divide
     CommSend cm;          // cm.n_dst > 0: the result goes to every rank of the group as (value, epoch) pairs (pitch ldo)
 };
 
@@ -89,13 +94,15 @@ constexpr int SK_MAX_DYN_SMEM = 224 * 1024;     // 227 KB per CTA less the kerne
 // Q/K/V, say).  All CTAs of the launch are resident at once; between two phases they meet at a barrier in global memory,
 // and every warp's ring keeps requesting weights across that barrier, so the memory stream does not stop while the
 // CTAs exchange the few kilobytes of activations.
-struct SkChain {
-    SkArgs ph[SK_MAX_PHASES];
+template <int PHASES>
+struct SkLaunch {
+    SkArgs ph[PHASES];
     int n;
     unsigned* bar;        // two counters (arrivals, exits), zero between launches; unused when n == 1
     int tune;             // experiments: bits 0-1 = units per warp requested before the inputs are read (0: ring - 1), bit 2 = no requests across a phase end
     unsigned long long* trace;   // optional: [grid][16] nanosecond time stamps of thread 0 (launch, inputs ready, per phase: quantised, done)
 };
+using SkChain = SkLaunch<SK_MAX_PHASES>;
 
 struct Quant256Args {
     const float* x;       // [nb][ldx]
@@ -495,24 +502,93 @@ __device__ __forceinline__ void quantise_rows(const float* x, int ldx, const flo
     else quantise_pairs<false, PR>(x, ldx, norm_w, eps, k, nb, xq, ldq, xd, xbs, ssq, perm);
 }
 
+// The same of one row of up to 16 blocks, in the one-token word order: every warp has two blocks and their norm weights `nw` in registers, so that a trip to L2 and one barrier are all
+// it waits for.
+__device__ __forceinline__ void quantise_short(const SkArgs& a, const float4 (&nw)[2][2], int8_t* xq, float* xd, int16_t* xbs, float* ssq) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nkb = a.k >> 8;
+    float v[2][8];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int blk = warp + i * SK_WARPS;
+        float4 u0 = make_float4(0.f, 0.f, 0.f, 0.f), u1 = u0;
+        if (blk < nkb) {
+            const float4* p = reinterpret_cast<const float4*>(a.x + blk * 256 + lane * 8);
+            u0 = __ldcg(p);
+            u1 = __ldcg(p + 1);
+        }
+        v[i][0] = u0.x; v[i][1] = u0.y; v[i][2] = u0.z; v[i][3] = u0.w;
+        v[i][4] = u1.x; v[i][5] = u1.y; v[i][6] = u1.z; v[i][7] = u1.w;
+    }
+    if (a.norm_w) {
+        float ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int j = 0; j < 8; j++) ss += v[i][j] * v[i][j];
+        ss = warp_sum(ss);
+        if (lane == 0) ssq[warp] = ss;
+        __syncthreads();
+        const float4 s0 = reinterpret_cast<const float4*>(ssq)[0], s1 = reinterpret_cast<const float4*>(ssq)[1];
+        const float rstd = rsqrtf((((s0.x + s0.y) + (s0.z + s0.w)) + ((s1.x + s1.y) + (s1.z + s1.w))) / (float)a.k + a.eps);
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const float w[8] = {nw[i][0].x, nw[i][0].y, nw[i][0].z, nw[i][0].w, nw[i][1].x, nw[i][1].y, nw[i][1].z, nw[i][1].w};
+#pragma unroll
+            for (int j = 0; j < 8; j++) v[i][j] *= rstd * w[j];
+        }
+    }
+    float amax[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        amax[i] = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; j++) amax[i] = fmaxf(amax[i], fabsf(v[i][j]));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        amax[0] = fmaxf(amax[0], __shfl_xor_sync(0xffffffffu, amax[0], o));
+        amax[1] = fmaxf(amax[1], __shfl_xor_sync(0xffffffffu, amax[1], o));
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int blk = warp + i * SK_WARPS;
+        if (blk >= nkb) break;
+        const float id = amax[i] > 0.f ? 127.f / amax[i] : 0.f;
+        int q[8], sum = 0;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            q[j] = __float2int_rn(v[i][j] * id);
+            sum += q[j];
+        }
+        uint32_t* w = reinterpret_cast<uint32_t*>(xq + blk * 256);
+        w[(2 * (lane & 1)) * 16 + (lane >> 1)] = (uint32_t)(q[0] & 0xff) | ((uint32_t)(q[1] & 0xff) << 8) | ((uint32_t)(q[2] & 0xff) << 16) | ((uint32_t)(q[3] & 0xff) << 24);
+        w[(2 * (lane & 1) + 1) * 16 + (lane >> 1)] = (uint32_t)(q[4] & 0xff) | ((uint32_t)(q[5] & 0xff) << 8) | ((uint32_t)(q[6] & 0xff) << 16) | ((uint32_t)(q[7] & 0xff) << 24);
+        if (lane == 0) xd[blk] = amax[i] / 127.f;
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        if ((lane & 3) == 0) xbs[blk * 8 + (lane >> 2)] = (int16_t)sum;
+    }
+}
+
 __device__ __forceinline__ void decode_unit(const SkArgs& a, int kts, int u, int& s, int& tile, int& kt) {
     s = 0;
 #pragma unroll
     for (int i = 1; i < 4; i++)
         if (i < a.nseg && u >= a.seg[i].unit0) s = i;
     const int l = u - a.seg[s].unit0;
-    tile = l / kts;
+    tile = a.kt_magic ? (int)__umulhi((unsigned)l, a.kt_magic) : l / kts;
     kt = l - tile * kts;
 }
 
-// Units [lo, hi) of group `gg` of `n_groups`: an equal share of the launch's units.
-__device__ __forceinline__ void group_range(int gg, int total, int n_groups, int& lo, int& hi) {
-    lo = (int)((long long)gg * total / n_groups);
-    hi = (int)((long long)(gg + 1) * total / n_groups);
+// Units [lo, hi) of group `gg`: an equal share of the launch's units.  (Quotients of 64 bits, and of 32 by the row length, were a third of the 1.5 us until the first request.)
+__device__ __forceinline__ void group_range(const SkArgs& a, int gg, int& lo, int& hi) {
+    lo = gg * a.share_q + min(gg, a.share_r);
+    hi = lo + a.share_q + (gg < a.share_r);
 }
 
 // Points the walker at phase w.ph: this warp's place in that phase's split; returns where its group's range starts.
-__device__ __forceinline__ int walker_enter(Walker& w, const SkChain& c, int warp) {
+template <int PHASES>
+__device__ __forceinline__ int walker_enter(Walker& w, const SkLaunch<PHASES>& c, int warp) {
     const SkArgs& a = c.ph[w.ph];
     w.l2 = a.wpt_log2;
     w.kts = a.k >> 8;
@@ -520,14 +596,15 @@ __device__ __forceinline__ int walker_enter(Walker& w, const SkChain& c, int war
     const int gg = blockIdx.x * (SK_WARPS >> w.l2) + (warp >> w.l2);
     int glo = 0;
     w.ghi = 0;
-    if (gg < a.n_groups) group_range(gg, a.total_units, a.n_groups, glo, w.ghi);
+    if (gg < a.n_groups) group_range(a, gg, glo, w.ghi);
     return glo;
 }
 
 // Moves `w` to this warp's first unit at or after segment start `from` of phase w.ph, or of the next phase that has one.
 // Inside a segment (the part of one 16-row tile that lies in the group's range) the 2^l2 warps of the group take equal
 // contiguous runs of units.
-__device__ __forceinline__ void walker_find(Walker& w, const SkChain& c, int warp, int from) {
+template <int PHASES>
+__device__ __forceinline__ void walker_find(Walker& w, const SkLaunch<PHASES>& c, int warp, int from) {
     w.valid = false;
     for (;;) {
         const SkArgs& a = c.ph[w.ph];
@@ -548,11 +625,12 @@ __device__ __forceinline__ void walker_find(Walker& w, const SkChain& c, int war
             }
             sl = sh;
         }
-        if (++w.ph >= c.n) return;
+        if (PHASES == 1 || ++w.ph >= c.n) return;
         from = walker_enter(w, c, warp);
     }
 }
-__device__ __forceinline__ void walker_next(Walker& w, const SkChain& c, int warp) {
+template <int PHASES>
+__device__ __forceinline__ void walker_next(Walker& w, const SkLaunch<PHASES>& c, int warp) {
     if (++w.u < w.ub) w.p += unit_bytes(w.type);
     else walker_find(w, c, warp, w.seg_end);
 }
@@ -585,18 +663,19 @@ __device__ __forceinline__ void grid_barrier(unsigned* bar, unsigned target, int
     __syncthreads();
 }
 
-template <int NT, bool ONE, bool XSMEM>
-__global__ void __launch_bounds__(SK_THREADS, NT == 1 ? 2 : 1) gemv_sk_kernel(const __grid_constant__ SkChain c_param) {
+// PHASES 1: the launch of one product, whose arguments are a quarter of a chain's.
+template <int NT, bool ONE, bool XSMEM, int PHASES>
+__global__ void __launch_bounds__(SK_THREADS, NT == 1 ? 2 : 1) gemv_sk_kernel(const __grid_constant__ SkLaunch<PHASES> c_param) {
     constexpr int FRAG = NT * 4 * 32;           // floats of one warp's accumulator fragment
     extern __shared__ __align__(128) uint8_t smem[];
     // The argument block is more than a kilobyte and is indexed at run time (phase, matrix): read from the constant bank
     // field by field, every first touch of a line is a miss of about a microsecond, one after the other.  All threads copy
     // it to shared memory in one sweep instead.
-    __shared__ __align__(16) SkChain c;
+    __shared__ __align__(16) SkLaunch<PHASES> c;
     {
         const uint32_t* src = reinterpret_cast<const uint32_t*>(&c_param);
         uint32_t* dst = reinterpret_cast<uint32_t*>(&c);
-        for (int i = threadIdx.x; i < (int)(sizeof(SkChain) / 4); i += SK_THREADS) dst[i] = src[i];
+        for (int i = threadIdx.x; i < (int)(sizeof(c) / 4); i += SK_THREADS) dst[i] = src[i];
     }
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -640,12 +719,23 @@ __global__ void __launch_bounds__(SK_THREADS, NT == 1 ? 2 : 1) gemv_sk_kernel(co
         else held++;
     }
     if (tr) tr[tr_n++] = global_ns();
+    // one row of up to 16 blocks: the norm's weights of the lane's two eights do not depend on the kernel before
+    const bool short_row = ONE && XSMEM && PHASES == 1 && c.ph[0].k <= 2 * SK_WARPS * 256;
+    float4 nw[2][2];
+    if (ONE && XSMEM && PHASES == 1 && short_row && c.ph[0].norm_w) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const float4* p = reinterpret_cast<const float4*>(c.ph[0].norm_w + min(warp + i * SK_WARPS, (c.ph[0].k >> 8) - 1) * 256 + lane * 8);
+            nw[i][0] = __ldg(p);
+            nw[i][1] = __ldg(p + 1);
+        }
+    }
     pdl_wait();
     if (tr) tr[tr_n++] = global_ns();
     bool dead = false;                      // a bounded wait gave up: stop waiting, the status word is set
-    for (int ph = 0; ph < c.n; ph++) {
+    for (int ph = 0; ph < (PHASES == 1 ? 1 : c.n); ph++) {
         const SkArgs& a = c.ph[ph];
-        if (ph > 0) grid_barrier(c.bar, gridDim.x * (unsigned)ph, a.status, dead);
+        if (PHASES > 1 && ph > 0) grid_barrier(c.bar, gridDim.x * (unsigned)ph, a.status, dead);
         if (tr) tr[tr_n++] = global_ns();
         const int kts = a.k >> 8;
         // a group of 2^l2 warps of this CTA works through one contiguous range of units, tile segment by tile segment
@@ -653,7 +743,7 @@ __global__ void __launch_bounds__(SK_THREADS, NT == 1 ? 2 : 1) gemv_sk_kernel(co
         const int gi = warp >> l2, wi = warp & (wpt - 1);
         const int n_groups = a.n_groups, gg = blockIdx.x * (SK_WARPS >> l2) + gi;
         int glo = 0, ghi = 0;
-        if (gg < n_groups) group_range(gg, a.total_units, n_groups, glo, ghi);
+        if (gg < n_groups) group_range(a, gg, glo, ghi);
         unsigned ep = 0;
         if (a.cm.n_dst > 0) ep = comm_next_epoch(a.cm);
         XOp x;
@@ -666,7 +756,8 @@ __global__ void __launch_bounds__(SK_THREADS, NT == 1 ? 2 : 1) gemv_sk_kernel(co
             float* xd_s = reinterpret_cast<float*>(smem + a.off_xd);
             int16_t* xbs_s = reinterpret_cast<int16_t*>(smem + a.off_xbs);
             // token rows are 16 bytes apart from a multiple of 128, so the eight tokens of a B fragment hit different banks
-            quantise_rows<2>(a.x, a.ldx, a.norm_w, a.eps, a.k, a.nb, xq_s, a.k + 16, xd_s, ONE ? xbs_s : nullptr, ssq, ONE);
+            if (ONE && PHASES == 1 && short_row) quantise_short(a, nw, xq_s, xd_s, xbs_s, ssq);
+            else quantise_rows<2>(a.x, a.ldx, a.norm_w, a.eps, a.k, a.nb, xq_s, a.k + 16, xd_s, ONE ? xbs_s : nullptr, ssq, ONE);
             top_up(SK_MAX_PHASES);
             __syncthreads();
             x.kw = (a.k + 16) >> 2;
@@ -755,7 +846,7 @@ __global__ void __launch_bounds__(SK_THREADS, NT == 1 ? 2 : 1) gemv_sk_kernel(co
                     const int tile_end = u_seg + kts;
                     for (int c = gg + 1; c < n_groups; c++) {
                         int clo, chi;
-                        group_range(c, a.total_units, n_groups, clo, chi);
+                        group_range(a, c, clo, chi);
                         if (clo >= tile_end) break;
                         if (clo == chi) continue;
                         bool ok = true;
@@ -832,7 +923,7 @@ __global__ void __launch_bounds__(SK_THREADS, NT == 1 ? 2 : 1) gemv_sk_kernel(co
 
         if (tr) tr[tr_n++] = global_ns();
     }
-    if (c.n > 1) {
+    if (PHASES > 1 && c.n > 1) {
         // the last CTA to leave puts the counters back to zero for the next launch
         __syncthreads();
         if (threadIdx.x == 0 && atomicAdd(c.bar + 1, 1u) == gridDim.x - 1) {
@@ -875,8 +966,9 @@ int sm_count() {
 }
 
 template <int NT, bool ONE>
-const void* pick_x(bool xsmem) {
-    return xsmem ? (const void*)gemv_sk_kernel<NT, ONE, true> : (const void*)gemv_sk_kernel<NT, ONE, false>;
+const void* pick_x(bool xsmem, bool chain) {
+    if (chain) return xsmem ? (const void*)gemv_sk_kernel<NT, ONE, true, SK_MAX_PHASES> : (const void*)gemv_sk_kernel<NT, ONE, false, SK_MAX_PHASES>;
+    return xsmem ? (const void*)gemv_sk_kernel<NT, ONE, true, 1> : (const void*)gemv_sk_kernel<NT, ONE, false, 1>;
 }
 
 cudaError_t launch(const void* fn, dim3 grid, dim3 block, size_t smem, void** args, cudaStream_t st, int pdl) {
@@ -893,7 +985,7 @@ cudaError_t launch(const void* fn, dim3 grid, dim3 block, size_t smem, void** ar
     return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
-PerDeviceOnce g_attr[8];
+PerDeviceOnce g_attr[16];
 
 }  // namespace
 
@@ -940,8 +1032,9 @@ B2_API int b2_gemv_sk_chain(const SkChain* in, int max_ctas, int split, int ring
     const int off_x = off;
     off += (xbytes + 127) & ~127;
     const int off_ring = off;
-    const void* fn = one ? pick_x<1, true>(xsmem) : nt == 1 ? pick_x<1, false>(xsmem) : nt == 2 ? pick_x<2, false>(xsmem) : pick_x<4, false>(xsmem);
-    const int which = (one ? 0 : nt == 1 ? 1 : nt == 2 ? 2 : 3) * 2 + (xsmem ? 1 : 0);
+    const bool chain = c.n > 1;
+    const void* fn = one ? pick_x<1, true>(xsmem, chain) : nt == 1 ? pick_x<1, false>(xsmem, chain) : nt == 2 ? pick_x<2, false>(xsmem, chain) : pick_x<4, false>(xsmem, chain);
+    const int which = (one ? 0 : nt == 1 ? 1 : nt == 2 ? 2 : 3) * 4 + (xsmem ? 2 : 0) + (chain ? 1 : 0);
     if (g_attr[which].first()) {
         const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_MAX_DYN_SMEM);
         if (e != cudaSuccess) return (int)e;
@@ -987,6 +1080,9 @@ B2_API int b2_gemv_sk_chain(const SkChain* in, int max_ctas, int split, int ring
         }
         a.wpt_log2 = l2;
         a.n_groups = groups;
+        a.share_q = units / groups;
+        a.share_r = units % groups;
+        a.kt_magic = kts > 1 && (long long)units * kts < 1ll << 32 ? 0xffffffffu / (unsigned)kts + 1u : 0u;      // beyond, the quotient's error would show
         const int per_cta = SK_WARPS >> l2;
         grid = max(grid, (groups + per_cta - 1) / per_cta);
         a.off_red = off_red;
@@ -997,7 +1093,8 @@ B2_API int b2_gemv_sk_chain(const SkChain* in, int max_ctas, int split, int ring
         a.ring = ring;
         a.slot_bytes = slot;
     }
-    void* args[] = {&c};
+    SkLaunch<1> single{{c.ph[0]}, 1, c.bar, c.tune, c.trace};
+    void* args[] = {chain ? (void*)&c : (void*)&single};
     return (int)launch(fn, dim3((unsigned)grid), dim3(SK_THREADS), smem, args, st, pdl);
 }
 

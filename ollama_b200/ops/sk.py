@@ -36,7 +36,7 @@ class SkArgs(C.Structure):
                 ("mode", C.c_int), ("out", C.c_void_p), ("ldo", C.c_int), ("act", C.c_int), ("alpha", C.c_float), ("limit", C.c_float),
                 ("ws", C.c_void_p), ("flags", C.c_void_p), ("status", C.c_void_p),
                 ("off_red", C.c_int), ("off_xq", C.c_int), ("off_xd", C.c_int), ("off_xbs", C.c_int), ("off_ring", C.c_int), ("ring", C.c_int),
-                ("slot_bytes", C.c_int), ("wpt_log2", C.c_int), ("n_groups", C.c_int),
+                ("slot_bytes", C.c_int), ("wpt_log2", C.c_int), ("n_groups", C.c_int), ("share_q", C.c_int), ("share_r", C.c_int), ("kt_magic", C.c_uint),
                 ("cm", K.CommSend)]
 
 

@@ -245,6 +245,24 @@ def test_gemm16_matches_reference(segs, k, nb):
     sk.workspace("cuda").check()
 
 
+@pytest.mark.parametrize("k", [256, 2048, 2304, 4096, 4352])
+@pytest.mark.parametrize("t", [GGMLType.Q4_K, GGMLType.Q6_K])
+def test_one_row_quantised_inside(k, t):
+    """One row that the launch quantises itself, up to 16 blocks (a warp's two in registers) and beyond: the same bits as the row quantised before; normalised, against the statement
+    in fp32, from which the few values that lie between two codes may differ by one (1 / 127 of a block's largest, in a row of thousands less than 2e-3 of the result's norm)."""
+    _, sk = _mods()
+    gen = torch.Generator().manual_seed(k)
+    ws = [sk.repack(_qw(t, n, k, n), "cuda") for n in (48, 4096)]
+    x, nw = torch.randn(1, k, generator=gen).cuda(), (torch.rand(k, generator=gen) + 0.5).cuda()
+    x[0, :min(k - 1, 300)] = 0                         # a block of zeros
+    assert torch.equal(sk.gemv(ws, x), sk.gemv(ws, sk.quant256(x)))
+    W = torch.cat([sk.unit_weights(w) for w in ws])
+    ref = _quant256_ref(R.rmsnorm(x.cpu(), nw.cpu(), 1e-5)).cuda() @ W.t()
+    got = sk.gemv(ws, x, norm_w=nw, eps=1e-5)
+    assert (got - ref).norm() <= 2e-3 * ref.norm()
+    sk.workspace("cuda").check()
+
+
 @pytest.mark.parametrize("segs,k", [([(16, GGMLType.Q6_K)], 256), ([(2064, GGMLType.Q4_K)], 256), ([(400, GGMLType.Q6_K), (2000, GGMLType.Q4_K)], 1280),
                                     ([(272, GGMLType.Q4_K)], 14336), ([(4096, GGMLType.Q6_K)], 1024), ([(20480, GGMLType.Q4_K)], 768)])
 @pytest.mark.parametrize("nb", [2, 16, 17, 33, 48, 49, 64])
