@@ -15,11 +15,12 @@
 //     minima are one more product per block (A: the minima twice, B: the rows' sums of 32 in two f16 parts) into columns of its own.
 //     So neither operand is rounded to fewer bits than the f16 activation keeps (2^-12 of a block's largest value at worst, against 2^-8 of the int8 form and
 //     2^-9 of products on bf16 copies): relative error of a product against 64 bits 2.1e-4 (Q4_K) and 2.6e-4 (Q6_K), int8 form 7e-3.
-//   * Measured (Llama-8B layer, q/k/v + output + gate/up + down with the four b2_rows16 before them, Q4_K_M): 60 us at 2 rows, 65 at 16, 76 at 32, 104 at 64, where mma.sync fragments
+//   * Measured (Llama-8B layer, q/k/v + output + gate/up + down with the four b2_rows16 before them, Q4_K_M): 56 us at 2 rows, 57 at 16, 65 at 32, 87 at 64, where mma.sync fragments
 //     expanded in registers took 74, 81, 113 and 226 (two launches), and 124 MB stream in 19.  What is left: 1100 cycles an item of 128 x 256 (expansion issues for 70 % of them), 2000
-//     to 4000 cycles a launch until the first sums, and as many to exchange those of split groups.
-//   * Work.  The launch's items are dealt out in equal contiguous shares, one CTA per SM; a group of 128 rows that is split between CTAs is finished by the CTA
-//     that holds its first block, which adds the others' sums in a fixed order (workspace + flag, bounded wait), as in gemv_sk.cu.
+//     to 4000 cycles a launch until the first sums, and 3000 to exchange those of split groups.
+//   * Work.  The launch's items are dealt out in equal contiguous shares, one CTA per SM.  The CTAs of a split group each finish a share of its values, adding the others' parts in a
+//     fixed order.  Parts are handed over through a workspace without flags or fences (see handed(); bounded wait).  With the first CTA collecting everything behind flags, and all
+//     warps watching flags that shared a line, a layer took 61, 64, 76 and 104 us.
 #include "pass_args.cuh"
 #include "tc_common.cuh"
 
@@ -36,6 +37,8 @@ constexpr int SG_UNIT_Q4K = 2368, SG_UNIT_Q6K = 3360;
 constexpr int SG_ROW = 544, SG_CHUNK = 16 * (SG_ROW + 4);      // bytes of a row's 256-block: values and sums of 32; with the scales of 16 rows
 constexpr int SG_MAX_ROWS = 64, SG_MAX_NT = SG_MAX_ROWS / 16;
 constexpr int SG_WS_FLOATS = 128 * SG_MAX_ROWS;                // a CTA's share of the workspace
+constexpr int SG_CTAS = 148;
+constexpr uint32_t SG_EMPTY = 0xffffffffu;                     // a place of the workspace that holds no value
 constexpr int SG_MAX_SMEM = 224 * 1024;
 constexpr int SG_SCALE_SLOTS = 8, SG_D_SLOTS = 8, SG_W_SLOTS = 10, SG_X_SLOTS = 4;
 constexpr int SG_A_COLS = 136;                                 // TMEM columns of an item's expanded weights: 256 / 2 of codes x scales, 16 / 2 of minima
@@ -58,11 +61,6 @@ __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity) {
     return false;
 }
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory"); }
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
 __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
@@ -252,125 +250,142 @@ struct SgBars {
     uint64_t out_full, out_free, last_full;                                       // sums of a group, of the CTA's last one
     uint64_t done[2];
     uint32_t tmem;
-    int seen;
 };
 
-// The rows of group `group`, whose sums over the CTA's own blocks (from kb0 on) are in `out` [row of x][128], by `threads` threads: handed over to the CTA that holds the group's
-// first block, or completed with what the others hand over, biases and what they are added to, and stored.  The warps do not wait for each other: every one that hands over counts
-// the flag up, every one that collects watches all flags, and the last of them (`seen`, in shared memory) clears them.  Returns whether no wait ran out.
-__device__ __forceinline__ bool finish_group(const SgArgs& a, const float* out, int group, int kb0, int n_seg, int rows, int kts, int total, int tid, int threads, int* seen) {
-    const int lane = tid & 31;
-    if (kb0 != 0) {
-        float* w = a.ws + (size_t)blockIdx.x * SG_WS_FLOATS;
-        for (int e = tid * 4; e < rows * 128; e += threads * 4) *reinterpret_cast<float4*>(w + e) = *reinterpret_cast<const float4*>(out + e);
-        __syncwarp();
-        if (lane == 0) {
-            __threadfence();
-            atomicAdd(&a.flags[blockIdx.x], 1u);
-        }
-        return true;
-    }
-    // A lane has one row (or pair of rows) of the matrix and every step-th row of x, four of them under way at once.  Loads are not predicated (rows past the last are read for
-    // nothing) so that all of a round are in flight together.
-    const int glu = a.mode == 2;      // the up value of a gate is the next row
-    const int quads = glu ? 2 : 4, n_warps = threads / 32, warp = tid >> 5;
-    const bool split = n_warps >= quads;
-    const int step = split ? n_warps / quads : n_warps, x_first = split ? warp / quads : warp;
-    bool alive = true;
-    int n_parts = n_seg < kts ? -1 : 0;
-    for (int quad = split ? warp % quads : 0; quad < quads; quad += split ? quads : 1) {
-        const int row = (quad * 32 + lane) << glu, tile = group * SG_TILES + (row >> 4);
-        const bool mine = tile < a.tiles;
-        const TileAt ta = tile_at(a, mine ? tile : a.tiles - 1, kts);
-        const float* bias = a.seg[0].bias;
-        int out_off = a.seg[0].out_off;
+// The CTAs that hold blocks of a group: `n` from `first` on.  Of the first `ends` of them it is the last group, and the first `finish` of these finish it together, a share of its values
+// each; the others (one that goes on with the next group, and those of a group in very many parts) only hand their sums over.  Finishers wait for CTAs before and behind them: there are
+// eight at most, so that CTAs which wait for others that are not resident yet cannot fill the GPU, however many streams launch at once.
+struct Parts {
+    int first, n, ends, finish;
+};
+__device__ __forceinline__ Parts parts_of(int group, int kts, int total) {
+    const unsigned n = gridDim.x, end = (unsigned)(group + 1) * kts;
+    Parts p;
+    p.first = (int)(((unsigned)group * kts * n + n - 1) / (unsigned)total);      // the largest c whose share does not begin behind the group's first item
+    const int last = (int)((end * n - 1) / (unsigned)total);
+    p.n = last - p.first + 1;
+    p.ends = share(last + 1, total, n) == (int)end ? p.n : p.n - 1;
+    p.finish = min(p.ends, 8);
+    return p;
+}
+// A CTA's sums of its last group and of the one that its share begins in, as the others read them: values are handed over without flags.  A place holds SG_EMPTY until its value is
+// written; its one reader asks for it until it is there and empties it again.  (With a flag behind a fence, the value took two more trips to L2: 1 us a launch.)
+__device__ __forceinline__ uint32_t* handed(const SgArgs& a, int cta, bool last) { return reinterpret_cast<uint32_t*>(a.ws) + (size_t)(2 * cta + last) * SG_WS_FLOATS; }
+__device__ __forceinline__ uint32_t no_empty(float v) { return __float_as_uint(v) == SG_EMPTY ? 0x7fffffffu : __float_as_uint(v); }      // SG_EMPTY would be a NaN
+__device__ __forceinline__ uint4 ld_relaxed(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_relaxed(uint4* p, uint4 v) {
+    asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+
+// Quads of neighbouring rows [e0, e1) of group `group`, 32 to a row of x: the sums of this CTA (`out`, [row of x][128], complete when `ready` is), of the others of `p`, biases and what
+// they are added to, stored by `threads` threads.  ITEMS quads of a thread and PARTS parts of each are under way at once; loads are not predicated (the last quad or part is read again)
+// so that all of a round are.  Returns whether no wait ran out.
+template <int ITEMS, int PARTS>
+__device__ __forceinline__ bool finish_rows(const SgArgs& a, const float* out, int group, int kts, const Parts& p, int e0, int e1, int tid, int threads, uint64_t* ready) {
+    const int lane = tid & 31, others = p.n - 1;
+    const int row = ((e0 + lane) & 31) * 4, tile = group * SG_TILES + (row >> 4);      // the same in all rounds
+    const bool glu = a.mode == 2;      // the up value of a gate is the next row
+    const TileAt ta = tile_at(a, min(tile, a.tiles - 1), kts);
+    const float* bias = a.seg[0].bias;
+    int out_off = a.seg[0].out_off;
 #pragma unroll
-        for (int s = 1; s < 4; s++)
-            if (s == ta.s) {
-                bias = a.seg[s].bias;
-                out_off = a.seg[s].out_off;
-            }
-        const int wrow = ta.local * 16 + (row & 15);
-        float* o = a.out + ((out_off + wrow) >> glu);
-        const float b0 = bias ? bias[wrow] : 0.f, b1 = bias && glu ? bias[wrow + 1] : 0.f;
+    for (int s = 1; s < 4; s++)
+        if (s == ta.s) {
+            bias = a.seg[s].bias;
+            out_off = a.seg[s].out_off;
+        }
+    const int wrow = ta.local * 16 + (row & 15);
+    float* o = a.out + ((out_off + wrow) >> glu);
+    const bool wide = !(((uintptr_t)o | ((uintptr_t)a.ldo * 4)) & 15);
+    float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (bias) b = make_float4(bias[wrow], bias[wrow + 1], bias[wrow + 2], bias[wrow + 3]);
 #pragma unroll 1
-        for (int x0 = x_first; x0 < a.nb; x0 += 4 * step) {
-            float y[4], u[4];
+    for (int base = e0 + tid - lane; base < e1; base += ITEMS * threads) {
+        float4 y[ITEMS];
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                y[j] = a.mode == 1 ? __ldcg(o + (size_t)min(x0 + j * step, a.nb - 1) * a.ldo) : 0.f;
-                u[j] = 0.f;
+        for (int i = 0; i < ITEMS; i++) {
+            const int e = base + i * threads + lane;
+            const float* r = o + (size_t)(e >> 5) * a.ldo;
+            y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (a.mode == 1 && e < e1 && tile < a.tiles) {
+                if (wide)
+                    y[i] = __ldcg(reinterpret_cast<const float4*>(r));
+                else
+                    y[i] = make_float4(__ldcg(r), __ldcg(r + 1), __ldcg(r + 2), __ldcg(r + 3));
             }
-            if (n_parts < 0) {      // the first time, with the loads above under way
-                // the CTAs behind this one that hold the rest of the group: lane i watches the flag of the i-th (all at once: one after the other they cost a trip to L2 each)
-                const int group_end = (group + 1) * kts;
-                n_parts = 0;
-                for (int c0 = blockIdx.x + 1;; c0 += 32) {
-                    const int c = c0 + lane;
-                    const bool part = c < gridDim.x && share(c, total, gridDim.x) < group_end;
-                    const int n = __popc(__ballot_sync(0xffffffffu, part));
-                    n_parts += n;
-                    if (part) {
-                        // a group that ends the CTA's share is handed over by the warps that expand
-                        const unsigned warps = share(c + 1, total, gridDim.x) <= group_end ? SG_EXPAND : SG_FINISH;
-                        bool ok = ld_acquire(&a.flags[c]) == warps;
-                        if (!ok) {
-                            const unsigned long long t0 = now_ns();
-                            while (!ok && now_ns() - t0 < SG_WAIT_NS) ok = ld_acquire(&a.flags[c]) == warps;
-                        }
-                        if (!ok) alive = false;
-                    }
-                    if (n < 32) break;
-                }
-                __syncwarp();
-            }
+        }
+        // the others' last sums come when this CTA's do: asking for them before only gets in the way of what they write (at 64 rows 2 us of a launch)
+        if (p.finish > 1 && ready) {
+            if (!__all_sync(0xffffffffu, bar_wait(ready, 0))) return false;
+            ready = nullptr;
+        }
 #pragma unroll 1
-            for (int c = 0; c < n_parts; c += 2) {
-                const float* w0 = a.ws + (size_t)(blockIdx.x + 1 + c) * SG_WS_FLOATS + row;
-                const float* w1 = c + 1 < n_parts ? w0 + SG_WS_FLOATS : w0;
-                float v0[4], v1[4], t0[4], t1[4];
+        for (int c0 = 0; c0 < others; c0 += PARTS) {
+            uint4 v[ITEMS][PARTS];
+            unsigned long long t0 = 0;
+            for (;;) {
+                bool there = true;
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const int x = min(x0 + j * step, rows - 1) * 128;
-                    v0[j] = __ldcg(w0 + x);
-                    v1[j] = __ldcg(w1 + x);
-                    if (glu) {
-                        t0[j] = __ldcg(w0 + x + 1);
-                        t1[j] = __ldcg(w1 + x + 1);
-                    }
+                for (int c = 0; c < PARTS; c++) {
+                    const int part = p.first + min(c0 + c, others - 1), cta = part + (part >= (int)blockIdx.x);
+                    const uint4* w = reinterpret_cast<const uint4*>(handed(a, cta, cta < p.first + p.ends));
+#pragma unroll
+                    for (int i = 0; i < ITEMS; i++) v[i][c] = ld_relaxed(w + min(base + i * threads + lane, e1 - 1));
                 }
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    y[j] += v0[j];
-                    if (c + 1 < n_parts) y[j] += v1[j];
-                    if (glu) {
-                        u[j] += t0[j];
-                        if (c + 1 < n_parts) u[j] += t1[j];
-                    }
-                }
+                for (int c = 0; c < PARTS; c++)
+#pragma unroll
+                    for (int i = 0; i < ITEMS; i++)
+                        there &= base + i * threads + lane >= e1 || c0 + c >= others ||
+                                 (v[i][c].x != SG_EMPTY && v[i][c].y != SG_EMPTY && v[i][c].z != SG_EMPTY && v[i][c].w != SG_EMPTY);
+                if (__all_sync(0xffffffffu, there)) break;
+                const unsigned long long t = __shfl_sync(0xffffffffu, now_ns(), 0);
+                if (t0 == 0) t0 = t;
+                if (t - t0 > SG_WAIT_NS) return false;
             }
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int x = x0 + j * step;
-                if (x < a.nb && mine) {
-                    y[j] += out[x * 128 + row] + b0;
-                    if (glu) y[j] = glu_act(y[j], u[j] + out[x * 128 + row + 1] + b1, a.act, a.alpha, a.limit);
-                    o[(size_t)x * a.ldo] = y[j];
+            for (int c = 0; c < PARTS; c++)
+                if (c0 + c < others) {
+                    const int part = p.first + c0 + c, cta = part + (part >= (int)blockIdx.x);
+                    uint4* w = reinterpret_cast<uint4*>(handed(a, cta, cta < p.first + p.ends));
+#pragma unroll
+                    for (int i = 0; i < ITEMS; i++) {
+                        const int e = base + i * threads + lane;
+                        if (e < e1) st_relaxed(w + e, make_uint4(SG_EMPTY, SG_EMPTY, SG_EMPTY, SG_EMPTY));
+                        y[i] = add4(y[i], make_float4(__uint_as_float(v[i][c].x), __uint_as_float(v[i][c].y), __uint_as_float(v[i][c].z), __uint_as_float(v[i][c].w)));
+                    }
+                }
+        }
+        if (ready) {
+            if (!__all_sync(0xffffffffu, bar_wait(ready, 0))) return false;
+            ready = nullptr;
+        }
+#pragma unroll
+        for (int i = 0; i < ITEMS; i++) {
+            const int e = base + i * threads + lane;
+            if (e < e1 && tile < a.tiles) {
+                const float4 v = add4(add4(y[i], *reinterpret_cast<const float4*>(out + 4 * e)), b);
+                float* r = o + (size_t)(e >> 5) * a.ldo;
+                if (glu) {
+                    r[0] = glu_act(v.x, v.y, a.act, a.alpha, a.limit);
+                    r[1] = glu_act(v.z, v.w, a.act, a.alpha, a.limit);
+                } else if (wide) {
+                    *reinterpret_cast<float4*>(r) = v;
+                } else {
+                    r[0] = v.x;
+                    r[1] = v.y;
+                    r[2] = v.z;
+                    r[3] = v.w;
                 }
             }
         }
     }
-    if (n_seg < kts) {      // a warp without rows of x has not looked at the flags, and is done with them too
-        int before = 0;
-        __syncwarp();
-        if (lane == 0) before = atomicAdd(seen, 1);
-        if (__shfl_sync(0xffffffffu, before, 0) == n_warps - 1) {
-            const int group_end = (group + 1) * kts;
-            for (int c = blockIdx.x + 1 + lane; c < gridDim.x && share(c, total, gridDim.x) < group_end; c += 32) a.flags[c] = 0u;
-            if (lane == 0) *seen = 0;
-        }
-    }
-    return alive;
+    return true;
 }
 
 template <int NT>
@@ -379,6 +394,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) gemm_sk_kernel(const __grid_con
     constexpr bool ONE_MINS = NT == 4;             // sums of the minima: one place instead of two, where tensor memory is full
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) SgBars bars;
+    __shared__ Parts last_parts;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int kts = a.k >> 8, total = (a.tiles + SG_TILES - 1) / SG_TILES * kts;
     const int lo = share(blockIdx.x, total, gridDim.x), n_items = share(blockIdx.x + 1, total, gridDim.x) - lo;
@@ -408,7 +424,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) gemm_sk_kernel(const __grid_con
         mbar_init(&bars.out_full, SG_SUM);
         mbar_init(&bars.out_free, SG_FINISH);
         mbar_init(&bars.last_full, SG_SUM);
-        bars.seen = 0;
+        last_parts = parts_of((lo + n_items - 1) / kts, kts, total);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     pdl_launch();
@@ -500,8 +516,16 @@ __global__ void __launch_bounds__(SG_THREADS, 1) gemm_sk_kernel(const __grid_con
         }
         // nothing more to expand: all sixteen warps finish the last group
         pdl_wait();
-        const int last = (lo + n_items - 1) / kts, kb0 = last == group0 ? kb_lo : 0;
-        if (alive && wait(&bars.last_full, 0)) alive = __all_sync(0xffffffffu, finish_group(a, out, last, kb0, lo + n_items - last * kts - kb0, N, kts, total, threadIdx.x, SG_EXPAND * 32, &bars.seen));
+        const int last = (lo + n_items - 1) / kts, quads = a.nb * 32;
+        const Parts p = last_parts;
+        if (!alive) {
+        } else if (p.finish > 1) {
+            const int j = blockIdx.x - p.first;
+            if (j < p.finish)
+                alive = finish_rows<1, 4>(a, out, last, kts, p, share(j, quads, p.finish), share(j + 1, quads, p.finish), threadIdx.x, SG_EXPAND * 32, &bars.last_full);
+        } else {
+            alive = finish_rows<4, 1>(a, out, last, kts, p, 0, quads, threadIdx.x, SG_EXPAND * 32, &bars.last_full);
+        }
     } else if (warp < SG_MMA) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 136;");
         __syncthreads();
@@ -545,6 +569,20 @@ __global__ void __launch_bounds__(SG_THREADS, 1) gemm_sk_kernel(const __grid_con
             // the rows are finished by other warps: here the stores and their fence took 6000 cycles, in which nothing moved
             const bool last = i == n_items;
             if (group > group0 && !wait(&bars.out_free, (group - group0 - 1) & 1)) break;
+            const auto hand_over = [&] {      // all but what this CTA finishes itself
+                const Parts p = last_parts;
+                if (!last || p.ends < 2) return;
+                uint32_t* w = handed(a, blockIdx.x, true) + row;
+                const int j = blockIdx.x - p.first, quad = row >> 2;
+                const int e0 = j < p.finish ? share(j, a.nb * 32, p.finish) : 0, e1 = j < p.finish ? share(j + 1, a.nb * 32, p.finish) : 0;
+#pragma unroll
+                for (int c = 0; c < N; c++) {
+                    const float2 v = unpack2(sum[c >> 1]);
+                    if (c < a.nb && (c * 32 + quad < e0 || c * 32 + quad >= e1)) __stcg(w + c * 128, no_empty(c & 1 ? v.y : v.x));
+                }
+            };
+            // the others wait for it, so it goes first; but 64 stores in a row hold up the sums for this CTA's own threads (a layer at 64 rows: 93 us, 87 after them; 65 and 66 at 32)
+            if (NT < 4) hand_over();
 #pragma unroll
             for (int c = 0; c < N / 2; c++) {
                 const float2 v = unpack2(sum[c]);
@@ -553,6 +591,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) gemm_sk_kernel(const __grid_con
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(last ? &bars.last_full : &bars.out_full);
+            if (NT == 4) hand_over();
         }
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
@@ -676,9 +715,17 @@ __global__ void __launch_bounds__(SG_THREADS, 1) gemm_sk_kernel(const __grid_con
             const int last = (lo + n_items - 1) / kts, tid = threadIdx.x - SG_LAST * 32;
             for (int g = group0; g < last; g++, kb0 = 0) {
                 if (!wait(&bars.out_full, (g - group0) & 1)) break;
-                alive = __all_sync(0xffffffffu, finish_group(a, out, g, kb0, kts - kb0, N, kts, total, tid, SG_FINISH * 32, &bars.seen));
+                if (kb0) {
+                    uint4* w = reinterpret_cast<uint4*>(handed(a, blockIdx.x, false));
+                    for (int e = tid; e < a.nb * 32; e += SG_FINISH * 32) {
+                        const float4 v = *reinterpret_cast<const float4*>(out + 4 * e);
+                        st_relaxed(w + e, make_uint4(no_empty(v.x), no_empty(v.y), no_empty(v.z), no_empty(v.w)));
+                    }
+                } else {
+                    finish_rows<1, 1>(a, out, g, kts, Parts{(int)blockIdx.x, 1, 1, 1}, 0, a.nb * 32, tid, SG_FINISH * 32, nullptr);
+                }
+                __syncwarp();
                 if (lane == 0) mbar_arrive(&bars.out_free);
-                if (!alive) break;
             }
         }
     }
@@ -839,10 +886,13 @@ B2_API int b2_rows16(const Rows16Args* in, int nb, int pdl, cudaStream_t st) {
     return go(a.bf16 ? (const void*)rows16_kernel<true> : (const void*)rows16_kernel<false>, grid, dim3(R16_WARPS * 32), 0, args, st, pdl);
 }
 
+// Floats of the workspace of b2_gemm_sk, every byte of which is 255 before the first launch and whenever a launch has ended (unless a wait ran out).
+B2_API long long b2_gemm_sk_ws() { return 2ll * SG_CTAS * SG_WS_FLOATS; }
+
 // y = W x for 1..64 rows in the chunks of b2_rows16, up to four matrices of one row length.  Returns a cudaError_t value.
 B2_API int b2_gemm_sk(const SgArgs* in, int max_ctas, int pdl, cudaStream_t st) {
     SgArgs a = *in;
-    if (a.nseg < 1 || a.nseg > 4 || a.nb < 1 || a.nb > SG_MAX_ROWS || a.k < 256 || (a.k & 255) || !a.x || ((uintptr_t)a.x & 15) || !a.out || !a.ws || !a.flags || !a.status ||
+    if (a.nseg < 1 || a.nseg > 4 || a.nb < 1 || a.nb > SG_MAX_ROWS || a.k < 256 || (a.k & 255) || !a.x || ((uintptr_t)a.x & 15) || !a.out || !a.ws || ((uintptr_t)a.ws & 15) || !a.status ||
         a.mode < 0 || a.mode > 2)
         return (int)cudaErrorInvalidValue;
     int slot = 0, tiles = 0;
@@ -874,7 +924,7 @@ B2_API int b2_gemm_sk(const SgArgs* in, int max_ctas, int pdl, cudaStream_t st) 
     if (total >= 1 << 23) return (int)cudaErrorNotSupported;
     // one CTA per SM: all are resident, so waits on other CTAs end.  No more of them than give every CTA as many items as the fullest has.
     int grid = total < sms() ? total : sms();
-    if (grid > 256) grid = 256;                    // CTAs that the workspace holds
+    if (grid > SG_CTAS) grid = SG_CTAS;            // CTAs that the workspace holds two parts of
     if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
     const int most = (total + grid - 1) / grid;
     grid = (total + most - 1) / most;

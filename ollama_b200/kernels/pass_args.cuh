@@ -44,8 +44,7 @@ struct SgArgs {
     float* out;
     int ldo, act;
     float alpha, limit;
-    float* ws;            // b2_gemv_sk_max_groups() x 512 floats, and as many flags
-    unsigned* flags;
+    float* ws;            // b2_gemm_sk_ws() floats, all bytes 255
     int* status;          // KStatus, written when a bounded wait gives up (may be pinned host memory)
     int tiles, ring, slot_bytes, x_slots;      // filled in by the launcher
 };

@@ -43,7 +43,6 @@ struct PassArgs {
     uint8_t* x16;                                 // units: b2_rows16_bytes(min(rows, 64), widest row)
     float* ws;                                    // units: workspace of b2_gemm_sk, otherwise scratch of b2_gemm_bf16
     long long ws_floats;
-    unsigned* flags;
     int* status;
     int units, tc, pdl;                           // tc: attention on tcgen05 where it applies
     void* kv16;                                   // int8 caches: b2_attn_prefill_q8_scratch halves for the longest sequence, or null
@@ -79,7 +78,6 @@ int unit_product(const PassArgs& a, const SgSeg* w, int n, const void* x, int bf
         s.alpha = a.alpha;
         s.limit = a.limit;
         s.ws = a.ws;
-        s.flags = a.flags;
         s.status = a.status;
         rc = b2_gemm_sk(&s, 0, a.pdl, st);
         if (rc) return rc;

@@ -23,7 +23,7 @@ class PassSeg(C.Structure):
 class PassArgs(C.Structure):
     _fields_ = [("rows", I), ("d", I), ("n_heads", I), ("n_kv_heads", I), ("hd", I), ("n_rot", I), ("neox", I), ("n_ctx", I), ("n_slots", I), ("ff", I), ("causal", I), ("act", I),
                 ("eps", F), ("scale", F), ("softcap", F), ("alpha", F), ("limit", F), ("positions", P), ("slots", P), ("x", P), ("qkv", P), ("q", P), ("o", P), ("h", P), ("f", P),
-                ("x16", P), ("ws", P), ("ws_floats", C.c_longlong), ("flags", P), ("status", P), ("units", I), ("tc", I), ("pdl", I), ("kv16", P), ("launches", I)]
+                ("x16", P), ("ws", P), ("ws_floats", C.c_longlong), ("status", P), ("units", I), ("tc", I), ("pdl", I), ("kv16", P), ("launches", I)]
 
 
 class PromptPass:
@@ -70,7 +70,7 @@ class PromptPass:
         kv16 = K.attn_prefill_q8_scratch(max(p0 + r for _, r, _, p0 in segs), c.n_kv_heads, c.head_dim, dev) if q8 else None
         a = PassArgs(n, c.d_model, c.n_heads, c.n_kv_heads, c.head_dim, c.rope_dim, int(c.rope_style == "neox"), be.n_ctx, be.n_slots, c.d_ff, int(c.causal), K._ACT[c.act],
                      c.norm_eps, be.attn_scale, c.attn_softcap, c.swiglu_alpha, c.swiglu_limit, K.ptr(positions), K.ptr(slots), K.ptr(x), K.ptr(qkv), K.ptr(q), K.ptr(o), K.ptr(h),
-                     K.ptr(f), K.ptr(x16), *((K.ptr(ws.ws), 0, K.ptr(ws.flags), K.ptr(ws.status)) if units else (K.ptr(parts), size, None, None)), int(units), int(tc),
+                     K.ptr(f), K.ptr(x16), *((K.ptr(ws.parts), 0, K.ptr(ws.status)) if units else (K.ptr(parts), size, None)), int(units), int(tc),
                      int(be.pdl), K.ptr(kv16), 0)
         sg = (PassSeg * len(segs))(*[PassSeg(*s) for s in segs])
         fn = K.lib().b2_prefill_pass

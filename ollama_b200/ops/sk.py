@@ -59,7 +59,7 @@ class SgSeg(C.Structure):
 
 class SgArgs(C.Structure):
     _fields_ = [("seg", SgSeg * 4), ("nseg", C.c_int), ("k", C.c_int), ("nb", C.c_int), ("x", C.c_void_p), ("mode", C.c_int), ("out", C.c_void_p), ("ldo", C.c_int),
-                ("act", C.c_int), ("alpha", C.c_float), ("limit", C.c_float), ("ws", C.c_void_p), ("flags", C.c_void_p), ("status", C.c_void_p), ("tiles", C.c_int),
+                ("act", C.c_int), ("alpha", C.c_float), ("limit", C.c_float), ("ws", C.c_void_p), ("status", C.c_void_p), ("tiles", C.c_int),
                 ("ring", C.c_int), ("slot_bytes", C.c_int), ("x_slots", C.c_int)]
 
 
@@ -202,18 +202,20 @@ class Workspace:
         rows = int(K.lib().b2_gemv_sk_max_groups())
         self.ws = torch.zeros(rows * WS_FLOATS, device=device, dtype=torch.float32)
         self.flags = torch.zeros(rows, device=device, dtype=torch.int32)
+        self.parts = torch.full((int(K.lib().b2_gemm_sk_ws()),), -1, device=device, dtype=torch.int32)      # of gemm16; -1: no value
         self.status = torch.zeros(1, dtype=torch.int32).pin_memory()
         self.status_np = self.status.numpy()
         self.bar = torch.zeros(2, device=device, dtype=torch.int32)          # arrival / exit counters of multi-phase launches
 
     def check(self, wait: bool = True) -> None:
-        """Raise if a bounded wait inside a launch gave up: its sums are wrong, and a flag that was set too late would be taken for the next launch's, so the flags are cleared.
+        """Raise if a bounded wait inside a launch gave up: its sums are wrong, and a flag or part that came too late would be taken for the next launch's, so all are cleared.
         ``wait``: for the launches of the current stream first (a caller that has read their results need not)."""
         if wait:
             torch.cuda.current_stream(self.ws.device).synchronize()
         if self.status_np[0] != 0:
             self.status_np[0] = 0
             self.flags.zero_()
+            self.parts.fill_(-1)
             self.bar.zero_()
             raise K.CudaKernelError("product of unit-ordered matrices: a bounded wait ran out")
 
@@ -325,7 +327,7 @@ def gemm16(weights: list[SkWeight], x: torch.Tensor, nb: int, *, out: torch.Tens
         off += w.n
     a.nseg, a.k, a.nb, a.x = len(weights), weights[0].k, nb, K.ptr(x)
     a.mode, a.out, a.ldo, a.act, a.alpha, a.limit = mode, out.data_ptr(), out.stride(0), K._ACT[act], alpha, limit
-    a.ws, a.flags, a.status = ws.ws.data_ptr(), ws.flags.data_ptr(), ws.status.data_ptr()
+    a.ws, a.status = ws.parts.data_ptr(), ws.status.data_ptr()
     K._check(K.lib().b2_gemm_sk(C.byref(a), max_ctas, int(pdl), K.stream()), "gemm_sk")
     return out
 

@@ -289,6 +289,31 @@ def test_gemm16_items_and_rows(segs, k, nb):
     sk.workspace("cuda").check()
 
 
+@pytest.mark.parametrize("n,k,nb", [(272, 14336, 3), (1040, 2048, 5), (4096, 4096, 64), (20480, 1024, 17)])
+def test_gemm16_parts_are_handed_over_once(n, k, nb):
+    """Groups in more parts than finish them, in a few, and with parts of CTAs that go on; outputs of any alignment and stride; a row that is not a number arrives like any other.
+    Whatever a launch handed over is taken: the workspace is empty again."""
+    _, sk = _mods()
+    gen = torch.Generator().manual_seed(n)
+    w = sk.repack(QWeight.from_float("w", torch.randn(n, k, generator=gen) * 0.05, GGMLType.Q4_K), "cuda")
+    w.bias = torch.randn(n + 1, generator=gen).cuda()[1:]
+    x, ws = torch.randn(nb, k, generator=gen).cuda(), sk.workspace("cuda")
+    want = sk.gemm16([w], sk.rows16(x), nb)
+    ref = x.double() @ sk.unit_weights(w).double().cuda().t() + w.bias.double()
+    assert ((want.double() - ref).abs() <= 2 ** -9 * ref.std(1, keepdim=True) + 1e-6).all()
+    odd = torch.zeros(nb, n + 3, device="cuda")
+    assert torch.equal(sk.gemm16([w], sk.rows16(x), nb, out=odd[:, 1:n + 1]), want) and (odd[:, 0] == 0).all() and (odd[:, n + 1:] == 0).all()
+    odd = odd[:, 1:n + 1]
+    sk.gemm16([w], sk.rows16(x), nb, out=odd, mode=sk.MODE_ACCUM)
+    assert (odd - 2 * want).abs().max() <= 2 ** -20 * want.abs().max()      # two orders of the same sums
+    x[nb // 2] = float("nan")
+    got = sk.gemm16([w], sk.rows16(x), nb)
+    rest = [b for b in range(nb) if b != nb // 2]
+    assert torch.equal(got[rest], want[rest]) and got[nb // 2].isnan().all()
+    ws.check()
+    assert (ws.parts == -1).all()
+
+
 def test_gemm16_glu_matches_reference():
     _, sk = _mods()
     gen = torch.Generator().manual_seed(3)
