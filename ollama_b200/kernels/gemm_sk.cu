@@ -19,8 +19,9 @@
 //     expanded in registers took 74, 81, 113 and 226 (two launches), and 124 MB stream in 19.  What is left: 1100 cycles an item of 128 x 256 (expansion issues for 70 % of them), 2000
 //     to 4000 cycles a launch until the first sums, and 3000 to exchange those of split groups.
 //   * Work.  The launch's items are dealt out in equal contiguous shares, one CTA per SM.  The CTAs of a split group each finish a share of its values, adding the others' parts in a
-//     fixed order.  Parts are handed over through a workspace without flags or fences (see handed(); bounded wait).  With the first CTA collecting everything behind flags, and all
+//     fixed order.  Parts are handed over through a workspace without flags or fences (handed.cuh; bounded wait).  With the first CTA collecting everything behind flags, and all
 //     warps watching flags that shared a line, a layer took 61, 64, 76 and 104 us.
+#include "handed.cuh"
 #include "pass_args.cuh"
 #include "tc_common.cuh"
 
@@ -38,7 +39,6 @@ constexpr int SG_ROW = 544, SG_CHUNK = 16 * (SG_ROW + 4);      // bytes of a row
 constexpr int SG_MAX_ROWS = 64, SG_MAX_NT = SG_MAX_ROWS / 16;
 constexpr int SG_WS_FLOATS = 128 * SG_MAX_ROWS;                // a CTA's share of the workspace
 constexpr int SG_CTAS = 148;
-constexpr uint32_t SG_EMPTY = 0xffffffffu;                     // a place of the workspace that holds no value
 constexpr int SG_MAX_SMEM = 224 * 1024;
 constexpr int SG_SCALE_SLOTS = 8, SG_D_SLOTS = 8, SG_W_SLOTS = 10, SG_X_SLOTS = 4;
 constexpr int SG_A_COLS = 136;                                 // TMEM columns of an item's expanded weights: 256 / 2 of codes x scales, 16 / 2 of minima
@@ -268,18 +268,8 @@ __device__ __forceinline__ Parts parts_of(int group, int kts, int total) {
     p.finish = min(p.ends, 8);
     return p;
 }
-// A CTA's sums of its last group and of the one that its share begins in, as the others read them: values are handed over without flags.  A place holds SG_EMPTY until its value is
-// written; its one reader asks for it until it is there and empties it again.  (With a flag behind a fence, the value took two more trips to L2: 1 us a launch.)
+// A CTA's sums of its last group and of the one that its share begins in, as the others read them.  (With flags behind fences a launch took 1 us longer.)
 __device__ __forceinline__ uint32_t* handed(const SgArgs& a, int cta, bool last) { return reinterpret_cast<uint32_t*>(a.ws) + (size_t)(2 * cta + last) * SG_WS_FLOATS; }
-__device__ __forceinline__ uint32_t no_empty(float v) { return __float_as_uint(v) == SG_EMPTY ? 0x7fffffffu : __float_as_uint(v); }      // SG_EMPTY would be a NaN
-__device__ __forceinline__ uint4 ld_relaxed(const uint4* p) {
-    uint4 v;
-    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_relaxed(uint4* p, uint4 v) {
-    asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
-}
 __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 
 // Quads of neighbouring rows [e0, e1) of group `group`, 32 to a row of x: the sums of this CTA (`out`, [row of x][128], complete when `ready` is), of the others of `p`, biases and what
@@ -342,7 +332,7 @@ __device__ __forceinline__ bool finish_rows(const SgArgs& a, const float* out, i
 #pragma unroll
                     for (int i = 0; i < ITEMS; i++)
                         there &= base + i * threads + lane >= e1 || c0 + c >= others ||
-                                 (v[i][c].x != SG_EMPTY && v[i][c].y != SG_EMPTY && v[i][c].z != SG_EMPTY && v[i][c].w != SG_EMPTY);
+                                 (v[i][c].x != HANDED_EMPTY && v[i][c].y != HANDED_EMPTY && v[i][c].z != HANDED_EMPTY && v[i][c].w != HANDED_EMPTY);
                 if (__all_sync(0xffffffffu, there)) break;
                 const unsigned long long t = __shfl_sync(0xffffffffu, now_ns(), 0);
                 if (t0 == 0) t0 = t;
@@ -356,7 +346,7 @@ __device__ __forceinline__ bool finish_rows(const SgArgs& a, const float* out, i
 #pragma unroll
                     for (int i = 0; i < ITEMS; i++) {
                         const int e = base + i * threads + lane;
-                        if (e < e1) st_relaxed(w + e, make_uint4(SG_EMPTY, SG_EMPTY, SG_EMPTY, SG_EMPTY));
+                        if (e < e1) st_relaxed(w + e, make_uint4(HANDED_EMPTY, HANDED_EMPTY, HANDED_EMPTY, HANDED_EMPTY));
                         y[i] = add4(y[i], make_float4(__uint_as_float(v[i][c].x), __uint_as_float(v[i][c].y), __uint_as_float(v[i][c].z), __uint_as_float(v[i][c].w)));
                     }
                 }
@@ -578,7 +568,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) gemm_sk_kernel(const __grid_con
 #pragma unroll
                 for (int c = 0; c < N; c++) {
                     const float2 v = unpack2(sum[c >> 1]);
-                    if (c < a.nb && (c * 32 + quad < e0 || c * 32 + quad >= e1)) __stcg(w + c * 128, no_empty(c & 1 ? v.y : v.x));
+                    if (c < a.nb && (c * 32 + quad < e0 || c * 32 + quad >= e1)) st_relaxed(w + c * 128, handed_bits(c & 1 ? v.y : v.x));
                 }
             };
             // the others wait for it, so it goes first; but 64 stores in a row hold up the sums for this CTA's own threads (a layer at 64 rows: 93 us, 87 after them; 65 and 66 at 32)
@@ -719,7 +709,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) gemm_sk_kernel(const __grid_con
                     uint4* w = reinterpret_cast<uint4*>(handed(a, blockIdx.x, false));
                     for (int e = tid; e < a.nb * 32; e += SG_FINISH * 32) {
                         const float4 v = *reinterpret_cast<const float4*>(out + 4 * e);
-                        st_relaxed(w + e, make_uint4(no_empty(v.x), no_empty(v.y), no_empty(v.z), no_empty(v.w)));
+                        st_relaxed(w + e, make_uint4(handed_bits(v.x), handed_bits(v.y), handed_bits(v.z), handed_bits(v.w)));
                     }
                 } else {
                     finish_rows<1, 1>(a, out, g, kts, Parts{(int)blockIdx.x, 1, 1, 1}, 0, a.nb * 32, tid, SG_FINISH * 32, nullptr);

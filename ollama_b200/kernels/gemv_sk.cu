@@ -1,4 +1,4 @@
-// Streaming quantised matrix-vector kernel for decode steps of 1..32 tokens, sm_100a.  (Engines take it up to eight; more rows go to gemm_sk.cu, but for rows above 16384 values,
+// Streaming quantised matrix-vector kernel for decode steps of 1..32 tokens, sm_100a.  (Engines take it for one; more rows go to gemm_sk.cu, but for rows above 16384 values,
 // which the pass that normalises them there does not hold.)
 //
 // In the reference stack this is ggml's mmvq family (one launch per matrix, dp4a dot products).  Here a
@@ -27,7 +27,7 @@
 //   * A warp that has all 16 units of a 16-row tile finishes the rows from its registers: store, add to the residual
 //     stream, gated activation of interleaved gate/up rows, or (value, epoch) stores to the peers of a
 //     tensor-parallel group.  A tile that is split between warps is finished by the warp that holds its first unit;
-//     the others hand their partial sums over through a small workspace and a flag (bounded wait, fixed
+//     the others hand their partial sums over through a small workspace (handed.cuh; bounded wait, fixed
 //     summation order).  A warp meets a split tile first (it computes it at the start of its range), so the warp
 //     that finishes a tile at the end of its own range finds the partial sums waiting.
 //   * The activations are quantised by the CTA itself while its first units are in flight: the kernel
@@ -35,8 +35,10 @@
 //     norm / quantise launch.  Inputs too large for shared memory come pre-quantised from b2_quant256.
 //   * What bounds one token now: gate/up of Llama-8B streams 66 MB in 10 to 11.5 us once its inputs are there; the four products of a layer spend 1 us each from a CTA's start to
 //     its first request, 1.3 to 2.3 us on the inputs (a trip to L2, a barrier, two reductions) and 1 to 2 us on the slowest CTA.  Arguments of one phase instead of four, shares and
-//     rows by multiplication, norm weights fetched before the wait and one barrier instead of two took the four from 52.3 to 41.9 us a layer.
+//     rows by multiplication, norm weights fetched before the wait and one barrier instead of two took the four from 52.3 to 41.9 us a layer; parts of split tiles
+//     handed over without flags, whose fences held up the warps that stream, to 39.0.
 #include "comm.cuh"
+#include "handed.cuh"
 
 constexpr int SK_WARPS = 8;
 constexpr int SK_THREADS = SK_WARPS * 32;
@@ -74,8 +76,7 @@ struct SkArgs {
     int act;
     float alpha, limit;
     // split tiles
-    float* ws;            // [groups][SK_WS_FLOATS]
-    unsigned* flags;      // [groups], zero between launches
+    uint32_t* ws;         // [groups][SK_WS_FLOATS], see handed.cuh
     int* status;          // KStatus, written when a bounded wait gives up (may be pinned host memory)
     // shared memory offsets and work split (filled in by the launcher)
     int off_red, off_xq, off_xd, off_xbs, off_ring;
@@ -832,15 +833,12 @@ __global__ void __launch_bounds__(SK_THREADS, NT == 1 ? 2 : 1) gemv_sk_kernel(co
             const bool starts = kt0 == 0, ends = kt0 + n_seg == kts;
             if (wi == 0 && !starts) {
                 // the tile began in an earlier group: hand the partial sums to the group that owns its first unit
-                float* wsp = a.ws + (size_t)gg * SK_WS_FLOATS;
+                uint32_t* wsp = a.ws + (size_t)gg * SK_WS_FLOATS;
     #pragma unroll
                 for (int n = 0; n < NT; n++)
     #pragma unroll
                     for (int i = 0; i < 4; i++)
-                        if (!ONE || !(i & 1)) wsp[(n * 4 + i) * 32 + lane] = facc[n][i];
-                __threadfence();
-                __syncwarp();
-                if (lane == 0) st_release_gpu_u32(&a.flags[gg], 1u);
+                        if (!ONE || !(i & 1)) st_relaxed(wsp + (n * 4 + i) * 32 + lane, handed_bits(facc[n][i]));
             } else if (wi == 0) {
                 if (!ends) {
                     const int tile_end = u_seg + kts;
@@ -849,31 +847,36 @@ __global__ void __launch_bounds__(SK_THREADS, NT == 1 ? 2 : 1) gemv_sk_kernel(co
                         group_range(a, c, clo, chi);
                         if (clo >= tile_end) break;
                         if (clo == chi) continue;
-                        bool ok = true;
-                        if (lane == 0 && !dead) {
-                            ok = ld_acquire_gpu_u32(&a.flags[c]) != 0u;
-                            if (!ok) {
-                                const unsigned long long t0 = global_ns();
-                                while (!ok && global_ns() - t0 < SK_WAIT_NS) {
-                                    __nanosleep(32);
-                                    ok = ld_acquire_gpu_u32(&a.flags[c]) != 0u;
-                                }
+                        uint32_t* wsp = a.ws + (size_t)c * SK_WS_FLOATS + lane;
+                        uint32_t part[NT][4];
+                        unsigned long long t0 = 0;
+                        while (!dead) {
+                            bool there = true;
+    #pragma unroll
+                            for (int n = 0; n < NT; n++)
+    #pragma unroll
+                                for (int i = 0; i < 4; i++)
+                                    if (!ONE || !(i & 1)) {
+                                        part[n][i] = ld_relaxed(wsp + (n * 4 + i) * 32);
+                                        there &= part[n][i] != HANDED_EMPTY;
+                                    }
+                            if (__all_sync(0xffffffffu, there)) break;
+                            const unsigned long long now = __shfl_sync(0xffffffffu, global_ns(), 0);
+                            if (t0 == 0) t0 = now;
+                            if (now - t0 > SK_WAIT_NS) {
+                                dead = true;
+                                if (lane == 0) *(volatile int*)a.status = KS_TIMEOUT;
                             }
-                            if (!ok) *(volatile int*)a.status = KS_TIMEOUT;
                         }
-                        ok = __shfl_sync(0xffffffffu, ok, 0);
-                        if (!ok) {
-                            dead = true;
-                            continue;
-                        }
-                        const float* wsp = a.ws + (size_t)c * SK_WS_FLOATS;
+                        if (dead) continue;
     #pragma unroll
                         for (int n = 0; n < NT; n++)
     #pragma unroll
                             for (int i = 0; i < 4; i++)
-                                if (!ONE || !(i & 1)) facc[n][i] += __ldcg(wsp + (n * 4 + i) * 32 + lane);
-                        __syncwarp();
-                        if (lane == 0) a.flags[c] = 0u;
+                                if (!ONE || !(i & 1)) {
+                                    facc[n][i] += __uint_as_float(part[n][i]);
+                                    st_relaxed(wsp + (n * 4 + i) * 32, HANDED_EMPTY);
+                                }
                     }
                 }
                 // finish the 16 rows: lane (g, t) holds rows g (i < 2) and g + 8 of tokens 8 n + 2 t + (i & 1); one token: every t
@@ -989,7 +992,7 @@ PerDeviceOnce g_attr[16];
 
 }  // namespace
 
-// Rows of the workspace / flag arrays a caller must provide (one per group of the largest launch).
+// Rows of 512 values of the workspace a caller must provide (one per group of the largest launch).
 B2_API int b2_gemv_sk_max_groups() { return 4096; }
 
 // Runs the phases of `in` (y = W x for 1..32 tokens on unit-ordered Q4_K / Q6_K matrices, the same token count in every phase)
@@ -1009,7 +1012,7 @@ B2_API int b2_gemv_sk_chain(const SkChain* in, int max_ctas, int split, int ring
     for (int p = 0; p < c.n; p++) {
         SkArgs& a = c.ph[p];
         if (a.nb != nb || (a.x != nullptr) != xsmem || a.nseg < 1 || a.nseg > 4 || (a.k & 255) || a.k <= 0) return (int)cudaErrorInvalidValue;
-        if (!a.ws || !a.flags || !a.status || (!a.x && (!a.xq || !a.xd || (nb == 1 && !a.xbs)))) return (int)cudaErrorInvalidValue;
+        if (!a.ws || !a.status || (!a.x && (!a.xq || !a.xd || (nb == 1 && !a.xbs)))) return (int)cudaErrorInvalidValue;
         if (a.cm.n_dst < 0 || a.cm.n_dst > COMM_MAX_RANKS || (a.cm.n_dst > 0 && (!a.cm.ll || a.mode != 0))) return (int)cudaErrorInvalidValue;
         if (xsmem && (((uintptr_t)a.x & 15) || (a.ldx & 3) || (a.norm_w && ((uintptr_t)a.norm_w & 15)))) return (int)cudaErrorInvalidValue;
         const int kts = a.k >> 8;

@@ -34,7 +34,7 @@ class SkArgs(C.Structure):
     _fields_ = [("seg", SkSeg * 4), ("nseg", C.c_int), ("k", C.c_int), ("nb", C.c_int), ("total_units", C.c_int),
                 ("x", C.c_void_p), ("ldx", C.c_int), ("norm_w", C.c_void_p), ("eps", C.c_float), ("xq", C.c_void_p), ("xd", C.c_void_p), ("xbs", C.c_void_p),
                 ("mode", C.c_int), ("out", C.c_void_p), ("ldo", C.c_int), ("act", C.c_int), ("alpha", C.c_float), ("limit", C.c_float),
-                ("ws", C.c_void_p), ("flags", C.c_void_p), ("status", C.c_void_p),
+                ("ws", C.c_void_p), ("status", C.c_void_p),
                 ("off_red", C.c_int), ("off_xq", C.c_int), ("off_xd", C.c_int), ("off_xbs", C.c_int), ("off_ring", C.c_int), ("ring", C.c_int),
                 ("slot_bytes", C.c_int), ("wpt_log2", C.c_int), ("n_groups", C.c_int), ("share_q", C.c_int), ("share_r", C.c_int), ("kt_magic", C.c_uint),
                 ("cm", K.CommSend)]
@@ -199,24 +199,22 @@ class Workspace:
     device's (:func:`workspace`).  The status word lives in host memory that kernels reach, so that reading it costs nothing."""
 
     def __init__(self, device):
-        rows = int(K.lib().b2_gemv_sk_max_groups())
-        self.ws = torch.zeros(rows * WS_FLOATS, device=device, dtype=torch.float32)
-        self.flags = torch.zeros(rows, device=device, dtype=torch.int32)
-        self.parts = torch.full((int(K.lib().b2_gemm_sk_ws()),), -1, device=device, dtype=torch.int32)      # of gemm16; -1: no value
+        sizes = int(K.lib().b2_gemv_sk_max_groups()) * WS_FLOATS, int(K.lib().b2_gemm_sk_ws())
+        self.ws, self.parts = (torch.full((n,), -1, device=device, dtype=torch.int32) for n in sizes)       # of gemv, of gemm16; -1: no value
         self.status = torch.zeros(1, dtype=torch.int32).pin_memory()
         self.status_np = self.status.numpy()
-        self.bar = torch.zeros(2, device=device, dtype=torch.int32)          # arrival / exit counters of multi-phase launches
+        self.flags = torch.zeros(2, device=device, dtype=torch.int32)        # arrival / exit counters of multi-phase launches
 
     def check(self, wait: bool = True) -> None:
-        """Raise if a bounded wait inside a launch gave up: its sums are wrong, and a flag or part that came too late would be taken for the next launch's, so all are cleared.
+        """Raise if a bounded wait inside a launch gave up: its sums are wrong, and a part that came too late would be taken for the next launch's, so all are cleared.
         ``wait``: for the launches of the current stream first (a caller that has read their results need not)."""
         if wait:
             torch.cuda.current_stream(self.ws.device).synchronize()
         if self.status_np[0] != 0:
             self.status_np[0] = 0
             self.flags.zero_()
+            self.ws.fill_(-1)
             self.parts.fill_(-1)
-            self.bar.zero_()
             raise K.CudaKernelError("product of unit-ordered matrices: a bounded wait ran out")
 
 
@@ -261,7 +259,7 @@ def fill_args(a: SkArgs, weights: list[SkWeight], nb: int, ws: Workspace) -> Non
         a.seg[i] = w.seg(out_off=off)
         off += w.n
     a.nseg, a.k, a.nb = len(weights), weights[0].k, nb
-    a.ws, a.flags, a.status = ws.ws.data_ptr(), ws.flags.data_ptr(), ws.status.data_ptr()
+    a.ws, a.status = ws.ws.data_ptr(), ws.status.data_ptr()
 
 
 def gemv(weights: list[SkWeight], x: torch.Tensor | tuple[torch.Tensor, torch.Tensor], *, norm_w: torch.Tensor | None = None, eps: float = 0.0,
@@ -351,7 +349,7 @@ def gemv_chain(phases: list[SkArgs], device, max_ctas: int = 0, split: int = 0, 
     c = SkChain()
     for i, a in enumerate(phases):
         c.ph[i] = a
-    c.n, c.bar = len(phases), workspace(device).bar.data_ptr()
+    c.n, c.bar = len(phases), workspace(device).flags.data_ptr()
     c.tune = TUNE
     c.trace = trace.data_ptr() if trace is not None else None      # int64 [grid, 16]: time stamps of thread 0 of every CTA
     K._check(K.lib().b2_gemv_sk_chain(C.byref(c), max_ctas, split, ring, int(pdl), K.stream()), "gemv_sk_chain")

@@ -314,6 +314,23 @@ def test_gemm16_parts_are_handed_over_once(n, k, nb):
     assert (ws.parts == -1).all()
 
 
+@pytest.mark.parametrize("n,k,split", [(16, 16384, 1), (6144, 4096, 0), (4000, 1792, 2), (28672, 512, 0)])
+@pytest.mark.parametrize("nb", [1, 7])
+def test_gemv_parts_are_handed_over_once(n, k, split, nb):
+    """A tile in as many parts as it has blocks, and parts of warps that go on: launches one behind the other give the same and leave the workspace empty."""
+    _, sk = _mods()
+    gen = torch.Generator().manual_seed(n + nb)
+    w = sk.repack(QWeight.from_float("w", torch.randn(n, k, generator=gen) * 0.05, GGMLType.Q4_K), "cuda")
+    x, ws = torch.randn(nb, k, generator=gen).cuda(), sk.workspace("cuda")
+    xin = x if sk.fits_fused_input(nb, k) else sk.quant256(x)
+    want = sk.gemv([w], xin, split=split)
+    ref = _quant256_ref(x.cpu()).cuda() @ sk.unit_weights(w).cuda().t()
+    assert (want - ref).norm() <= 2e-3 * ref.norm()      # values at a rounding tie may be quantised to the code beside
+    assert all(torch.equal(sk.gemv([w], xin, split=split), want) for _ in range(3))
+    ws.check()
+    assert (ws.ws == -1).all()
+
+
 def test_gemm16_glu_matches_reference():
     _, sk = _mods()
     gen = torch.Generator().manual_seed(3)
