@@ -544,6 +544,8 @@ class B200Backend(StepEngine):
         inv_freq, mscale = (self.inv_freq_local, 1.0) if local else (self.inv_freq, self.mscale)
         ca = K.AttnCombineArgs(K.ptr(b.part_acc), K.ptr(b.part_ml), K.ptr(L.sinks), c.n_heads, self.n_splits, c.head_dim,
                                K.ptr(b.ao), None, None)
+        # the merge of the splits writes the rows as the output product reads them
+        x16 = b.x16 if INT8_ROWS < nb <= SK.ROWS16_MAX and c.q_dim % 256 == 0 and 256 % c.head_dim == 0 else None
         fused = self.fuse_rope and (L.q_norm is None) == (L.k_norm is None) and self.k_scale[i] is None
         aa = K.AttnDecodeArgs(None if fused else K.ptr(b.q), K.ptr(self.k_cache[i]), K.ptr(self.v_cache[i]), K.ptr(b.positions), K.ptr(b.slots),
                               c.n_heads, c.n_kv_heads, self.n_ctx, self.n_splits, self.attn_scale, c.attn_softcap,
@@ -552,8 +554,7 @@ class B200Backend(StepEngine):
         if fused:
             # rotary embedding of the queries, rotation + cache append of the new key / value and the attention in one launch
             rr = K.AttnRopeArgs(K.ptr(b.qkv), K.ptr(inv_freq), mscale, c.rope_dim, int(c.rope_style == "neox"), K.ptr(L.q_norm), K.ptr(L.k_norm), c.norm_eps)
-            lib.b2_attn_decode_rope.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p]
-            rc = lib.b2_attn_decode_rope(C.byref(aa), C.byref(rr), C.byref(ca), nb, c.head_dim, int(self.pdl), st())
+            rc = K.attn_decode_into(aa, rr, ca, nb, c.head_dim, self.pdl, x16)
             if rc == 801:               # cudaErrorNotSupported: nothing was launched; this model keeps the separate kernel
                 self.fuse_rope = fused = False
                 aa.q = K.ptr(b.q)
@@ -566,9 +567,13 @@ class B200Backend(StepEngine):
                               c.head_dim, c.rope_dim, int(c.rope_style == "neox"), self.n_ctx, K.ptr(b.q), K.ptr(self.k_cache[i]),
                               K.ptr(self.v_cache[i]), K.ptr(self.k_scale[i]), K.ptr(self.v_scale[i]))
             K._check(lib.b2_rope_kv(C.byref(ra), nb, int(self.pdl), st()), "rope_kv")
-            K._check(lib.b2_attn_decode(C.byref(aa), C.byref(ca), nb, c.head_dim, int(self.pdl), st()), "attn_decode")
+            K._check(K.attn_decode_into(aa, None, ca, nb, c.head_dim, self.pdl, x16), "attn_decode")
             self._n += 3
-        self._sk([L.sk.o], b.ao, b.x, nb, mode=SK.MODE_ACCUM)
+        if x16 is None:
+            self._sk([L.sk.o], b.ao, b.x, nb, mode=SK.MODE_ACCUM)
+        else:
+            SK.gemm16([L.sk.o], x16, nb, out=b.x[:nb], mode=SK.MODE_ACCUM, pdl=self.pdl, ws=self._ws)
+            self._n += 1
         self._sk([L.sk.gu], b.x, b.hf, nb, norm_w=L.ffn_norm, mode=SK.MODE_GLU)
         self._sk([L.sk.down], b.hf, b.x, nb, mode=SK.MODE_ACCUM)
 

@@ -23,6 +23,7 @@
 //     warps watching flags that shared a line, a layer took 61, 64, 76 and 104 us.
 #include "handed.cuh"
 #include "pass_args.cuh"
+#include "rows16.cuh"
 #include "tc_common.cuh"
 
 namespace {
@@ -35,8 +36,7 @@ constexpr int SG_TILES = 8;                                    // 16-row tiles o
 constexpr int SG_EXPAND = 16, SG_SUM = 4, SG_FINISH = 3, SG_THREADS = (SG_EXPAND + SG_SUM + 5 + SG_FINISH) * 32;
 enum { SG_MMA = SG_EXPAND + SG_SUM, SG_LOAD_X = SG_MMA + 2, SG_LOAD_W = SG_LOAD_X + 1, SG_LAST = SG_LOAD_W + 2 };
 constexpr int SG_UNIT_Q4K = 2368, SG_UNIT_Q6K = 3360;
-constexpr int SG_ROW = 544, SG_CHUNK = 16 * (SG_ROW + 4);      // bytes of a row's 256-block: values and sums of 32; with the scales of 16 rows
-constexpr int SG_MAX_ROWS = 64, SG_MAX_NT = SG_MAX_ROWS / 16;
+constexpr int SG_MAX_NT = SG_MAX_ROWS / 16;
 constexpr int SG_WS_FLOATS = 128 * SG_MAX_ROWS;                // a CTA's share of the workspace
 constexpr int SG_CTAS = 148;
 constexpr int SG_MAX_SMEM = 224 * 1024;
@@ -749,42 +749,6 @@ __device__ __forceinline__ void load8(const void* x, size_t at, float (&v)[8]) {
 
 constexpr int R16_WARPS = 8, R16_KEEP = 8;      // blocks that a warp keeps in registers between the sum of squares and the stores
 
-// A 256-block of `n` rows: [64 columns][n rows][128 bytes, 16-byte pieces xor row & 7] values, [two parts][n rows][16 bytes] sums of 32 (upper f16 parts of the eight, then
-// lower parts), [n] scales.  Place 8 j + 2 t + e of 64 columns holds column 32 (j / 4) + 16 (j / 2 & 1) + 4 t + (j & 1) + 2 e.
-__device__ __forceinline__ void store_block(const Rows16Args& a, int n, int row, int blk, int lane, const float (&v)[8]) {
-    float m = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; i++) m = fmaxf(m, fabsf(v[i]));
-    m = warp_max(m);
-    const int e = max((int)(__float_as_uint(m) >> 23), 16);                        // scale 2^(e - 135): the largest value lands in 256..512
-    const float inv = __uint_as_float((uint32_t)(262 - e) << 23), scale = __uint_as_float((uint32_t)(e - 8) << 23);
-    __half h[8];
-    float sum = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        h[i] = __float2half_rn(v[i] * inv);
-        sum += __half2float(h[i]);
-    }
-    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 2);                                    // the 32 columns of four lanes
-    uint8_t* c = a.out + (size_t)blk * n * (SG_ROW + 4);
-    // lane: columns 8 lane .. + 7 = t values 2 (lane & 1) and + 1 of 16-column group lane / 2
-    const int j = 2 * ((lane >> 1) & 3);
-    uint8_t* f = c + (size_t)((lane >> 3) * n + row) * 128 + 8 * (lane & 1);
-    const __half2 p[4] = {__halves2half2(h[0], h[2]), __halves2half2(h[4], h[6]), __halves2half2(h[1], h[3]), __halves2half2(h[5], h[7])};
-    *reinterpret_cast<uint2*>(f + ((j ^ (row & 7)) << 4)) = *reinterpret_cast<const uint2*>(p);
-    *reinterpret_cast<uint2*>(f + (((j + 1) ^ (row & 7)) << 4)) = *reinterpret_cast<const uint2*>(p + 2);
-    // sums of two neighbouring sub-blocks: lanes 8 i and 8 i + 4 hold them
-    const float next = __shfl_down_sync(0xffffffffu, sum, 4);
-    if ((lane & 7) == 0) {
-        const __half h0 = __float2half_rn(sum), h1 = __float2half_rn(next);
-        __half2* s = reinterpret_cast<__half2*>(c + (size_t)n * 512 + row * 16 + (lane >> 3) * 4);
-        s[0] = __halves2half2(h0, h1);
-        s[n * 4] = __halves2half2(__float2half_rn(sum - __half2float(h0)), __float2half_rn(next - __half2float(h1)));
-    }
-    if (lane == 0) *reinterpret_cast<float*>(c + (size_t)n * SG_ROW + row * 4) = scale;
-}
-
 template <bool BF16>
 __global__ void __launch_bounds__(R16_WARPS * 32) rows16_kernel(const __grid_constant__ Rows16Args a, int nb) {
     __shared__ float ssq[R16_WARPS];
@@ -797,7 +761,7 @@ __global__ void __launch_bounds__(R16_WARPS * 32) rows16_kernel(const __grid_con
         for (int blk = b0; blk < nkb; blk += step) {
             float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             if (!pad) load8<BF16>(a.x, (size_t)row * a.ldx + blk * 256 + lane * 8, v);
-            store_block(a, n, row, blk, lane, v);
+            store_block16(a.out, n, row, blk, lane, v);
         }
         return;
     }
@@ -831,7 +795,7 @@ __global__ void __launch_bounds__(R16_WARPS * 32) rows16_kernel(const __grid_con
         const float w[8] = {n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, n1.z, n1.w};
 #pragma unroll
         for (int j = 0; j < 8; j++) v[i][j] *= rstd * w[j];
-        store_block(a, n, row, blk, lane, v[i]);
+        store_block16(a.out, n, row, blk, lane, v[i]);
     }
 }
 

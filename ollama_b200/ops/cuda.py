@@ -417,6 +417,21 @@ def attn_decode_stages(n: int) -> int:
     return int(lib().b2_attn_decode_stages(int(n)))
 
 
+def attn_decode_into(a: AttnDecodeArgs, r: AttnRopeArgs | None, c: AttnCombineArgs, nb: int, hd: int, pdl: bool, out16: torch.Tensor | None = None) -> int:
+    """Decode attention (with ``r``: on raw projections), merged into the outputs of ``c`` or, with ``out16``, into the 16-bit chunks that the products of unit-ordered matrices read.
+    Returns the CUDA error; 801 (nothing was launched) where the form with ``r`` is not taken."""
+    rp, cp = C.byref(r) if r is not None else None, C.byref(c)
+    if out16 is not None:
+        f = lib().b2_attn_decode_rows16
+        f.argtypes = [C.c_void_p] * 4 + [C.c_int] * 3 + [C.c_void_p]
+        return f(C.byref(a), rp, cp, ptr(out16), nb, hd, int(pdl), stream())
+    if r is None:
+        return lib().b2_attn_decode(C.byref(a), cp, nb, hd, int(pdl), stream())
+    f = lib().b2_attn_decode_rope
+    f.argtypes = [C.c_void_p] * 3 + [C.c_int] * 3 + [C.c_void_p]
+    return f(C.byref(a), rp, cp, nb, hd, int(pdl), stream())
+
+
 def attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, positions: torch.Tensor, slots: torch.Tensor, *,
                 scale: float, n_splits: int, window: int = 0, softcap: float = 0.0, sinks: torch.Tensor | None = None,
                 scratch: tuple[torch.Tensor, torch.Tensor] | None = None, quant_out: bool = True, pdl: bool = False,

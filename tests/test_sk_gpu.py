@@ -331,6 +331,29 @@ def test_gemv_parts_are_handed_over_once(n, k, split, nb):
     assert (ws.ws == -1).all()
 
 
+@pytest.mark.parametrize("hd,H,Hkv", [(128, 8, 2), (64, 12, 4), (32, 8, 8), (256, 3, 1)])
+@pytest.mark.parametrize("nb", [2, 16, 17, 64])
+def test_attention_merged_into_chunks(hd, H, Hkv, nb):
+    """The merge of the splits that writes the output product's chunks gives the bits of the merge and b2_rows16, rows of zeros included; heads of half, of quarter, of eighth and of
+    whole blocks, with the tensor-core and with the scalar kernel before it."""
+    K, sk = _mods()
+    n_ctx, splits = 256, 4
+    gen = torch.Generator().manual_seed(nb + hd)
+    kc, vc = (torch.randn(nb, Hkv, n_ctx, hd, generator=gen).half().cuda() for _ in range(2))
+    q, sinks = torch.randn(nb, H, hd, generator=gen).cuda(), torch.randn(H, generator=gen).cuda()
+    pos, slots = torch.randint(0, n_ctx, (nb,), generator=gen, dtype=torch.int32).cuda(), torch.arange(nb, dtype=torch.int32).cuda()
+    acc, ml = torch.empty(nb * H * splits * hd, device="cuda"), torch.empty(nb * H * splits * 2, device="cuda")
+    out = torch.empty(nb, H * hd, device="cuda")
+    chunks = torch.full((sk.rows16_bytes(nb, H * hd),), 0xAA, device="cuda", dtype=torch.uint8)
+    a = K.AttnDecodeArgs(K.ptr(q), K.ptr(kc), K.ptr(vc), K.ptr(pos), K.ptr(slots), H, Hkv, n_ctx, splits, hd ** -0.5, 0.0, 0, K.ptr(acc), K.ptr(ml), None, None)
+    c = K.AttnCombineArgs(K.ptr(acc), K.ptr(ml), K.ptr(sinks), H, splits, hd, K.ptr(out), None, None)
+    assert K.attn_decode_into(a, None, c, nb, hd, False) == 0
+    c.out = None
+    assert K.attn_decode_into(a, None, c, nb, hd, True, chunks) == 0
+    assert torch.equal(chunks, sk.rows16(out, out=torch.full_like(chunks, 0x55)))
+    assert K.attn_decode_into(a, None, c, 65, hd, True, chunks) != 0 and K.attn_decode_into(a, None, c, nb, hd, True, chunks[4:]) != 0
+
+
 def test_gemm16_glu_matches_reference():
     _, sk = _mods()
     gen = torch.Generator().manual_seed(3)
