@@ -70,7 +70,7 @@ class PromptPass:
         kv16 = K.attn_prefill_q8_scratch(max(p0 + r for _, r, _, p0 in segs), c.n_kv_heads, c.head_dim, dev) if q8 else None
         a = PassArgs(n, c.d_model, c.n_heads, c.n_kv_heads, c.head_dim, c.rope_dim, int(c.rope_style == "neox"), be.n_ctx, be.n_slots, c.d_ff, int(c.causal), K._ACT[c.act],
                      c.norm_eps, be.attn_scale, c.attn_softcap, c.swiglu_alpha, c.swiglu_limit, K.ptr(positions), K.ptr(slots), K.ptr(x), K.ptr(qkv), K.ptr(q), K.ptr(o), K.ptr(h),
-                     K.ptr(f), K.ptr(x16), *((K.ptr(ws.parts), 0, K.ptr(ws.status)) if units else (K.ptr(parts), size, None)), int(units), int(tc),
+                     K.ptr(f), K.ptr(x16), *((K.ptr(ws.ws), 0, K.ptr(ws.status)) if units else (K.ptr(parts), size, None)), int(units), int(tc),
                      int(be.pdl), K.ptr(kv16), 0)
         sg = (PassSeg * len(segs))(*[PassSeg(*s) for s in segs])
         fn = K.lib().b2_prefill_pass

@@ -199,8 +199,8 @@ class Workspace:
     device's (:func:`workspace`).  The status word lives in host memory that kernels reach, so that reading it costs nothing."""
 
     def __init__(self, device):
-        sizes = int(K.lib().b2_gemv_sk_max_groups()) * WS_FLOATS, int(K.lib().b2_gemm_sk_ws())
-        self.ws, self.parts = (torch.full((n,), -1, device=device, dtype=torch.int32) for n in sizes)       # of gemv, of gemm16; -1: no value
+        # parts of gemv or of gemm16, whichever runs; -1: no value
+        self.ws = torch.full((max(int(K.lib().b2_gemv_sk_max_groups()) * WS_FLOATS, int(K.lib().b2_gemm_sk_ws())),), -1, device=device, dtype=torch.int32)
         self.status = torch.zeros(1, dtype=torch.int32).pin_memory()
         self.status_np = self.status.numpy()
         self.flags = torch.zeros(2, device=device, dtype=torch.int32)        # arrival / exit counters of multi-phase launches
@@ -214,7 +214,6 @@ class Workspace:
             self.status_np[0] = 0
             self.flags.zero_()
             self.ws.fill_(-1)
-            self.parts.fill_(-1)
             raise K.CudaKernelError("product of unit-ordered matrices: a bounded wait ran out")
 
 
@@ -325,7 +324,7 @@ def gemm16(weights: list[SkWeight], x: torch.Tensor, nb: int, *, out: torch.Tens
         off += w.n
     a.nseg, a.k, a.nb, a.x = len(weights), weights[0].k, nb, K.ptr(x)
     a.mode, a.out, a.ldo, a.act, a.alpha, a.limit = mode, out.data_ptr(), out.stride(0), K._ACT[act], alpha, limit
-    a.ws, a.status = ws.parts.data_ptr(), ws.status.data_ptr()
+    a.ws, a.status = ws.ws.data_ptr(), ws.status.data_ptr()
     K._check(K.lib().b2_gemm_sk(C.byref(a), max_ctas, int(pdl), K.stream()), "gemm_sk")
     return out
 

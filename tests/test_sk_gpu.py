@@ -311,7 +311,7 @@ def test_gemm16_parts_are_handed_over_once(n, k, nb):
     rest = [b for b in range(nb) if b != nb // 2]
     assert torch.equal(got[rest], want[rest]) and got[nb // 2].isnan().all()
     ws.check()
-    assert (ws.parts == -1).all()
+    assert (ws.ws == -1).all()
 
 
 @pytest.mark.parametrize("n,k,split", [(16, 16384, 1), (6144, 4096, 0), (4000, 1792, 2), (28672, 512, 0)])
