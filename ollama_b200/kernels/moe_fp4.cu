@@ -425,7 +425,7 @@ B2_API int b2_moe_rows(const void* x, int bf16, int ldx, int cols, int per_token
     return go(bf16 ? (const void*)moe_rows_kernel<true> : (const void*)moe_rows_kernel<false>, dim3(pairs), dim3(256), args, st, pdl);
 }
 
-// chunk_rows: 8, 16, 24, 32, 40, 48 or 64, what moe_sort and moe_rows were given.  Returns a cudaError_t value (cudaErrorNotSupported: other shapes; nothing launched).
+// chunk_rows: 8, 16, 24, 32, 48 or 64, what moe_sort and moe_rows were given.  Returns a cudaError_t value (cudaErrorNotSupported: other shapes; nothing launched).
 B2_API int b2_moe_fp4(const MoeFp4Args* in, int chunk_rows, int max_chunks, int pdl, cudaStream_t st) {
     const MoeFp4Args a = *in;
     if (!a.q || !a.s || !a.x || !a.chunks || !a.out || max_chunks < 1 || max_chunks > 65535 || a.glu < 0 || a.glu > 3 || (((uintptr_t)a.q | (uintptr_t)a.s | (uintptr_t)a.x) & 15))
@@ -436,7 +436,6 @@ B2_API int b2_moe_fp4(const MoeFp4Args* in, int chunk_rows, int max_chunks, int 
         case 16: return launch<16>(a, max_chunks, pdl, st);
         case 24: return launch<24>(a, max_chunks, pdl, st);
         case 32: return launch<32>(a, max_chunks, pdl, st);
-        case 40: return launch<40>(a, max_chunks, pdl, st);
         case 48: return launch<48>(a, max_chunks, pdl, st);
         case 64: return launch<64>(a, max_chunks, pdl, st);
     }

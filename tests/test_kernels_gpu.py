@@ -946,9 +946,9 @@ def test_moe_fp4_products(E, d, ff, T, k, chunk, bf16):
     assert torch.equal(by_pair[(lids < 0).cuda()], torch.zeros_like(by_pair[(lids < 0).cuda()]))
 
 
-@pytest.mark.parametrize("E,d,ff,T,k,chunk", [(5, 288, 160, 75, 2, 24), (5, 288, 160, 75, 2, 40), (4, 160, 288, 100, 2, 48), (1, 96, 64, 49, 1, 48)])
+@pytest.mark.parametrize("E,d,ff,T,k,chunk", [(5, 288, 160, 75, 2, 24), (4, 160, 288, 100, 2, 48), (1, 96, 64, 49, 1, 48)])
 def test_moe_fp4_chunks_between(E, d, ff, T, k, chunk):
-    """Chunks of 24, 40 and 48 rows, whose scales and accumulators end between powers of two; full chunks and a row more."""
+    """Chunks of 24 and 48 rows, whose scales and accumulators end between powers of two; full chunks and a row more."""
     test_moe_fp4_products(E, d, ff, T, k, chunk, True)
 
 
