@@ -36,10 +36,11 @@ from .steps import StepEngine
 
 MAX_DECODE_BATCH = 8             # sequences per launch of the dp4a kernels (kernels/gemv.cu)
 MAX_STREAM_BATCH = 32            # sequences per step when every matrix runs on the streaming kernel (kernels/gemv_sk.cu)
-# Steps of more sequences than this multiply f16 activations (kernels/gemm_sk.cu) instead of int8 ones.  Products of a layer of Llama-8B (Q4_K_M), int8 against f16: 53 us against
-# 60 at one sequence, 71 against 60 at two, 74 against 63 at seven, 76 against 63 at eight.
+# Steps of more sequences than this multiply f16 activations (kernels/gemm_sk.cu) instead of int8 ones.  Products of a layer of Llama-8B (Q4_K_M), int8 against f16: 39 us against
+# 55 at one sequence, 59 against 56 at two and at four, 64 against 56 at six, 70 against 56 at eight.
 INT8_ROWS = 1
 # Prompt passes of at most this many rows, which is one launch a product, read the units too instead of the 16-bit copies (a layer of Llama-8B: 124 MB against 436).
+# Twelve layers at 64 rows: 1526 us against 2324; with two launches, at 65 rows 2255 against 2321, at 96 2362 against 2295.
 UNIT_ROWS = SK.ROWS16_MAX
 # Steps of at least so many (token, expert) pairs, and of one for every eighth expert, read MXFP4 experts once for all rows that chose them (kernels/moe_fp4.cu), smaller ones
 # once per pair: a layer of 128 experts of 13 MB, four a token, takes 72 us against 75 at four tokens and 194 against 280 at sixteen, but 45 against 29 at one.
