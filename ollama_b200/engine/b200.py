@@ -547,7 +547,7 @@ class B200Backend(StepEngine):
                                K.ptr(b.ao), None, None)
         # the merge of the splits writes the rows as the output product reads them
         x16 = b.x16 if INT8_ROWS < nb <= SK.ROWS16_MAX and c.q_dim % 256 == 0 and 256 % c.head_dim == 0 else None
-        fused = self.fuse_rope and (L.q_norm is None) == (L.k_norm is None) and self.k_scale[i] is None
+        fused = self.fuse_rope and (L.q_norm is None) == (L.k_norm is None)
         aa = K.AttnDecodeArgs(None if fused else K.ptr(b.q), K.ptr(self.k_cache[i]), K.ptr(self.v_cache[i]), K.ptr(b.positions), K.ptr(b.slots),
                               c.n_heads, c.n_kv_heads, self.n_ctx, self.n_splits, self.attn_scale, c.attn_softcap,
                               c.sliding_window if L.swa else 0, K.ptr(b.part_acc), K.ptr(b.part_ml), K.ptr(self.k_scale[i]),

@@ -24,7 +24,7 @@ struct AttnDecodeArgs {
 
 // Optional second argument of the tensor-core kernel: with `qkv` set the kernel takes the query rows straight from the
 // projection output and rotates them itself, and the CTA whose split holds the query's own position rotates the new key,
-// appends key and value to the cache (f16 caches only) and uses them from shared memory, so that no rotary-embedding launch
+// appends key and value to the cache and uses them from shared memory, so that no rotary-embedding launch
 // precedes the attention.
 struct AttnRopeArgs {
     const float* qkv;        // [nb][(H + 2 Hkv) * HD] raw projections (q | k | v), or null: q comes rotated from a.q

@@ -352,7 +352,8 @@ __global__ void __launch_bounds__(128) attn_decode_paged_kernel(const __grid_con
 // 35.2 -> 23.2, f16 29.2 -> 26.0 (bytes 15); 32 about 467 22.3 -> 20.6 (bytes 9.3), with sixteen splits allocated 34.6 -> 22.2; 64 heads of 64, 16 about 1024 18.3 -> 15.9.
 // What is left: three CTAs of four warps an SM (registers) whose turn takes about as long as its rows, the launch, the first rows' latency and the merge (6 us).
 // Q8: rows stay int8 in the ring.  A key word (four dims) becomes two B-fragment registers in place, which is why the queries' fragments have a lane's dims in that order;
-// values are expanded into a tile of the warp's own.
+// values are expanded into a tile of the warp's own.  With raw projections the owning split quantises the new rows as b2_rope_kv does, instead of that launch before this one: a step of 8
+// sequences of 12 layers 1096 -> 1073 us.
 template <int D, int NS, bool Q8>
 __global__ void __launch_bounds__(128) attn_decode_flat_kernel(const __grid_constant__ AttnDecodeArgs a, const __grid_constant__ AttnRopeArgs r, int room) {
     constexpr int LD = D + PAD, NW = 16;                          // positions of a warp's turn
@@ -363,6 +364,7 @@ __global__ void __launch_bounds__(128) attn_decode_flat_kernel(const __grid_cons
     __shared__ float s_m[4][ROWS], s_l[4][ROWS];
     __shared__ float s_cs[128], s_sn[128];                        // cos / sin of the query position per rotated pair (fused form)
     __shared__ __half s_newk[D], s_newv[D];                       // the query token's own key and value rows (fused form, owning split)
+    __shared__ int8_t s_new8[2][D];                               // Q8: their codes, whose scales are s_newk[i], s_newv[i] of dims 32 i ..
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
     unsigned char* ring = smem_raw + ROWS * LD * 2 + warp * (NS * STAGE + WIDE);
     __half* wide = reinterpret_cast<__half*>(ring + NS * STAGE);  // Q8: [NW][LD] values
@@ -436,7 +438,7 @@ __global__ void __launch_bounds__(128) attn_decode_flat_kernel(const __grid_cons
 #pragma unroll
     for (int i = 0; i < NS - 1; i++) request(i);
 
-    const bool fresh = !Q8 && r.qkv != nullptr;
+    const bool fresh = r.qkv != nullptr;
     const bool owner = fresh && qpos >= p0 && qpos < p1;          // this split holds the query token's own position
     // element i of a raw head row after the rotary embedding (pairs (2p, 2p+1), or (p, p + n_rot/2) in the neox order)
     auto rotated = [&](const float* row, int i) -> float {
@@ -451,7 +453,7 @@ __global__ void __launch_bounds__(128) attn_decode_flat_kernel(const __grid_cons
     if (fresh) {
         // the raw rows (query heads of this group, the key and the value) are staged from the last warp's last stage on, which no request has reached yet; cos / sin of the
         // position are computed once per CTA meanwhile
-        float* raw = reinterpret_cast<float*>(smem_raw + ROWS * LD * 2 + (4 * NS - 1) * STAGE);       // [group + 2][D]
+        float* raw = reinterpret_cast<float*>(smem_raw + ROWS * LD * 2 + 3 * (NS * STAGE + WIDE) + (NS - 1) * STAGE);       // [group + 2][D]
         const int nrows = group + (owner ? 2 : 0);
         const float* tok = r.qkv + (size_t)b * (a.n_heads + 2 * a.n_kv_heads) * D;
         for (int c = tid; c < nrows * (D / 4); c += 128) {
@@ -488,7 +490,23 @@ __global__ void __launch_bounds__(128) attn_decode_flat_kernel(const __grid_cons
             __half* kc = const_cast<__half*>(a.k_cache) + (row0 + qpos) * D;
             __half* vc = const_cast<__half*>(a.v_cache) + (row0 + qpos) * D;
             for (int i = tid; i < D; i += 128) {
-                const __half kh = __float2half_rn(rotated(krow, i)), vh = __float2half_rn(vrow[i]);
+                const float k = rotated(krow, i), v = vrow[i];
+                if (Q8) {      // a warp has a block of 32 dims
+                    const __half hk = __float2half_rn(warp_max(fabsf(k)) / 127.f), hv = __float2half_rn(warp_max(fabsf(v)) / 127.f);
+                    const float dk = __half2float(hk), dv = __half2float(hv);
+                    const int8_t qk = (int8_t)(dk > 0.f ? max(-127, min(127, __float2int_rn(k / dk))) : 0), qv = (int8_t)(dv > 0.f ? max(-127, min(127, __float2int_rn(v / dv))) : 0);
+                    s_new8[0][i] = qk;
+                    s_new8[1][i] = qv;
+                    const_cast<int8_t*>(reinterpret_cast<const int8_t*>(a.k_cache))[(row0 + qpos) * D + i] = qk;
+                    const_cast<int8_t*>(reinterpret_cast<const int8_t*>(a.v_cache))[(row0 + qpos) * D + i] = qv;
+                    if (lane == 0) {
+                        const size_t at = (row0 + qpos) * (D / 32) + (i >> 5);
+                        const_cast<__half*>(a.k_scale)[at] = s_newk[i >> 5] = hk;
+                        const_cast<__half*>(a.v_scale)[at] = s_newv[i >> 5] = hv;
+                    }
+                    continue;
+                }
+                const __half kh = __float2half_rn(k), vh = __float2half_rn(v);
                 s_newk[i] = kh;
                 s_newv[i] = vh;
                 kc[i] = kh;
@@ -541,10 +559,22 @@ __global__ void __launch_bounds__(128) attn_decode_flat_kernel(const __grid_cons
         __half* tk = reinterpret_cast<__half*>(st);
         const __half* tv = Q8 ? wide : tk + NW * LD;
         if (owner && n0 <= qpos && qpos < n0 + NW) {      // the query's own row did not come from the cache
-            __half* dk = tk + (qpos - n0) * LD;
+            const int rr = qpos - n0;
+            __half* dk = tk + rr * LD;
             for (int d = lane; d < D; d += 32) {
-                dk[d] = s_newk[d];
-                dk[NW * LD + d] = s_newv[d];
+                if (Q8) {
+                    unsigned char* to = st + rr * D + ((D == 128 ? (d >> 4) ^ (4 * (rr & 1)) : d >> 4) << 4) + (d & 15);
+                    to[0] = (unsigned char)s_new8[0][d];
+                    to[NW * D + SCALES] = (unsigned char)s_new8[1][d];
+                } else {
+                    dk[d] = s_newk[d];
+                    dk[NW * LD + d] = s_newv[d];
+                }
+            }
+            if (Q8 && lane < D / 32) {
+                __half* sc = reinterpret_cast<__half*>(st + NW * D) + rr * (D / 32) + lane;
+                sc[0] = s_newk[lane];
+                sc[(NW * D + SCALES) / 2] = s_newv[lane];
             }
             __syncwarp();
         }
@@ -724,7 +754,8 @@ template <int D, int NS, bool Q8 = false>
 int launch_flat(const AttnDecodeArgs& a, const AttnRopeArgs& r, int nb, int pdl, cudaStream_t st) {
     constexpr int WARP = Q8 ? NS * 2 * (16 * D + D) + 16 * (D + PAD) * 2 : NS * 2 * 16 * (D + PAD) * 2;
     constexpr int RINGS = ROWS * (D + PAD) * 2 + 4 * WARP, MERGE = ROWS * (D + PAD) * 2 + 4 * ROWS * D * 4;
-    const int raw = r.qkv ? RINGS - WARP / NS + (a.n_heads / a.n_kv_heads + 2) * D * 4 : 0;      // where the raw rows end (f16 caches)
+    constexpr int LAST = Q8 ? 2 * 17 * D + 16 * (D + PAD) * 2 : WARP / NS;                        // the last warp's last stage and what lies behind it
+    const int raw = r.qkv ? RINGS - LAST + (a.n_heads / a.n_kv_heads + 2) * D * 4 : 0;            // where the raw rows end
     int smem = RINGS > MERGE ? RINGS : MERGE;
     if (raw > smem) smem = raw;
     const void* fn = (const void*)attn_decode_flat_kernel<D, NS, Q8>;
@@ -775,7 +806,7 @@ int attn_decode_mma_splits(const AttnDecodeArgs& a, int nb) {
 
 int attn_decode_mma_rope_launch(const AttnDecodeArgs& a, const AttnRopeArgs& r, int nb, int hd, int pdl, cudaStream_t st) {
     if (!b2_attn_decode_mma_takes(&a, hd)) return (int)cudaErrorNotSupported;
-    if (r.qkv && (a.k_scale || a.v_scale || r.n_rot > 256 || r.n_rot > hd || (r.n_rot & 1) || (a.page_table ? r.n_rot && !r.freqs : !r.inv_freq))) return (int)cudaErrorNotSupported;
+    if (r.qkv && ((a.page_table && (a.k_scale || a.v_scale)) || r.n_rot > 256 || r.n_rot > hd || (r.n_rot & 1) || (a.page_table ? r.n_rot && !r.freqs : !r.inv_freq))) return (int)cudaErrorNotSupported;
     if (a.page_table && (r.maps < 1 || r.maps > 2 || a.n_heads / a.n_kv_heads % r.maps || (r.maps > 1 && r.q_norm) || (r.no_append && r.q_norm))) return (int)cudaErrorInvalidValue;
     if (a.page_table && (!r.qkv || !r.neox || r.dim < 1 || r.maps * r.dim > hd || r.vdim < 1 || r.vdim > hd || r.n_rot > r.dim || a.max_pages < 1 || a.window < 0 || a.keep < 0 || r.v_off < 0 ||
                          (!r.no_append && r.v_off + a.n_kv_heads * r.vdim > r.ldq))) return (int)cudaErrorInvalidValue;

@@ -456,9 +456,9 @@ def attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, p
 def attn_decode_rope(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, positions: torch.Tensor, slots: torch.Tensor,
                      inv_freq: torch.Tensor, *, n_heads: int, n_rot: int, neox: bool, mscale: float, scale: float, n_splits: int,
                      window: int = 0, softcap: float = 0.0, sinks: torch.Tensor | None = None, pdl: bool = False, q_norm: torch.Tensor | None = None,
-                     k_norm: torch.Tensor | None = None, eps: float = 1e-6) -> torch.Tensor | None:
+                     k_norm: torch.Tensor | None = None, eps: float = 1e-6, k_scale: torch.Tensor | None = None, v_scale: torch.Tensor | None = None) -> torch.Tensor | None:
     """Decode attention on raw projections ``qkv`` [nb, (H + 2 Hkv) * hd]: the kernel rotates the queries and the new key,
-    appends key and value to the f16 caches at ``positions`` and attends over positions 0..position.  ``q_norm`` / ``k_norm`` [hd]: each query and key head is
+    appends key and value to the caches (f16, or int8 with scales) at ``positions`` and attends over positions 0..position.  ``q_norm`` / ``k_norm`` [hd]: each query and key head is
     RMS-normalised first.  Returns the output [nb, H * hd], or None when the tensor-core kernel does not take the shape (nothing was launched)."""
     nb = qkv.shape[0]
     Hkv, n_ctx, hd = k_cache.shape[1], k_cache.shape[2], k_cache.shape[3]
@@ -467,7 +467,7 @@ def attn_decode_rope(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
     ml = torch.empty(nb * n_heads * n_splits * 2, device=dev, dtype=torch.float32)
     out = torch.empty(nb, n_heads * hd, device=dev, dtype=torch.float32)
     a = AttnDecodeArgs(None, ptr(k_cache), ptr(v_cache), ptr(positions), ptr(slots), n_heads, Hkv, n_ctx, n_splits, scale, softcap,
-                       window, ptr(acc), ptr(ml), None, None)
+                       window, ptr(acc), ptr(ml), ptr(k_scale), ptr(v_scale))
     r = AttnRopeArgs(ptr(qkv), ptr(inv_freq), mscale, n_rot, int(neox), ptr(q_norm), ptr(k_norm), eps)
     c = AttnCombineArgs(ptr(acc), ptr(ml), ptr(sinks), n_heads, n_splits, hd, ptr(out), None, None)
     f = lib().b2_attn_decode_rope

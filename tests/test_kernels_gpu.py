@@ -266,6 +266,37 @@ def test_attn_decode_with_rotary_embedding_and_cache_append_inside(hd, H, Hkv, n
                               pos[:1], slots[:1] * 0, inv, n_heads=1, n_rot=64, neox=neox, mscale=1.0, scale=1.0, n_splits=1) is None
 
 
+@pytest.mark.parametrize("hd,H,Hkv,n_rot,neox,norm", [(128, 32, 8, 128, False, False), (128, 32, 2, 64, True, True), (64, 12, 4, 64, True, False), (64, 16, 1, 32, False, True)])
+@pytest.mark.parametrize("window,n_splits", [(0, 1), (0, 4), (48, 4)])
+def test_attn_decode_rotates_and_appends_to_int8_caches(hd, H, Hkv, n_rot, neox, norm, window, n_splits, attn_mode):
+    """The same for int8 caches, against rope_kv and the tensor-core attention: the same codes and scales (a key's code may be the one beside where the sum of squares of its norm ends in
+    another bit) and the same output (one code in 127 of a value of a position), whatever the cache row held; up to sixteen heads a group, whose raw rows reach behind the ring."""
+    K = _K()
+    attn_mode(1)
+    n_slots, n_ctx, nb = 4, 320, 4
+    g = torch.Generator().manual_seed(hd + H)
+    kc, vc = (torch.randint(-127, 128, (n_slots, Hkv, n_ctx, hd), generator=g, dtype=torch.int8).cuda() for _ in range(2))
+    ks, vs = ((torch.rand(n_slots, Hkv, n_ctx, hd // 32, generator=g) * 0.01).half().cuda() for _ in range(2))
+    qkv = torch.randn(nb, (H + 2 * Hkv) * hd, generator=g).cuda()
+    pos, slots = torch.tensor([0, 63, 64, 301], dtype=torch.int32).cuda(), torch.tensor([2, 0, 3, 1], dtype=torch.int32).cuda()
+    inv = (1.0 / (10000.0 ** (torch.arange(0, n_rot, 2).float() / n_rot))).cuda()
+    w = dict(q_norm=torch.rand(hd, generator=g).cuda() + 0.5, k_norm=torch.rand(hd, generator=g).cuda() + 0.5, eps=1e-5) if norm else {}
+    kc2, vc2, ks2, vs2 = kc.clone(), vc.clone(), ks.clone(), vs.clone()
+    q = K.rope_kv(qkv, pos, slots, inv, n_heads=H, n_kv_heads=Hkv, hd=hd, n_rot=n_rot, neox=neox, mscale=1.3, k_cache=kc, v_cache=vc, k_scale=ks, v_scale=vs, **w)
+    want, _ = K.attn_decode(q, kc, vc, pos, slots, scale=hd ** -0.5, n_splits=n_splits, window=window, quant_out=False, k_scale=ks, v_scale=vs)
+    for b in range(nb):
+        at = (int(slots[b]), slice(None), int(pos[b]))
+        kc2[at] = vc2[at] = -128
+        ks2[at] = vs2[at] = float("nan")
+    got = K.attn_decode_rope(qkv, kc2, vc2, pos, slots, inv, n_heads=H, n_rot=n_rot, neox=neox, mscale=1.3, scale=hd ** -0.5, n_splits=n_splits, window=window, k_scale=ks2, v_scale=vs2, **w)
+    assert got is not None and torch.equal(vc2, vc) and torch.equal(vs2, vs)
+    if norm:
+        assert (kc2.int() - kc.int()).abs().max() <= 1 and torch.allclose(ks2, ks, rtol=2 ** -10)
+    else:
+        assert torch.equal(kc2, kc) and torch.equal(ks2, ks)
+    assert torch.allclose(got, want, atol=2e-3, rtol=2e-3), (got - want).abs().max()
+
+
 @pytest.mark.parametrize("hd,H,Hkv", [(128, 8, 2), (64, 3, 3)])
 @pytest.mark.parametrize("n_splits", [1, 3, 16])
 def test_attn_decode_head_norm(hd, H, Hkv, n_splits, attn_mode):
