@@ -497,6 +497,22 @@ def test_attn_prefill_shares_keys(hd, H, Hkv, T, pos0, window, softcap, use_sink
     assert torch.allclose(out, ref, atol=1e-2, rtol=2e-2), (out - ref).abs().max()
 
 
+@pytest.mark.parametrize("hd,H,T", [(128, 16, 64), (128, 16, 128), (64, 32, 64)])
+def test_attn_prefill_of_keys_from_memory(hd, H, T):
+    """Caches larger than L2 in turn, so that the warps of a tile wait for keys and are woken at different times: every launch gives the bits of the first one on its cache."""
+    K = _K()
+    n_ctx, pos0, g = 6144, 6000, torch.Generator(device="cuda").manual_seed(hd + T)
+    caches = [[torch.randn(1, H, n_ctx, hd, generator=g, device="cuda").mul_(0.7).half() for _ in range(2)] for _ in range(5)]
+    q = torch.randn(T, H, hd, generator=g, device="cuda")
+    first, bad = {}, torch.zeros((), device="cuda", dtype=torch.int64)
+    for i in range(4000):
+        n = i % len(caches)
+        out = K.attn_prefill(q, *caches[n], 0, pos0, pos0 + T, hd ** -0.5, mode="tc")
+        bad += (out != first.setdefault(n, out)).any()
+    assert K.attn_prefill_tc_status(clear=True) == 0
+    assert int(bad) == 0
+
+
 @pytest.mark.parametrize("hd,H,Hkv", [(128, 8, 2), (64, 6, 3)])
 @pytest.mark.parametrize("T,pos0,window,causal", [(65, 0, 0, True), (7, 120, 0, True), (130, 700, 0, True), (100, 900, 300, True), (3, 1020, 1, True), (150, 0, 0, False)])
 def test_attn_prefill_of_int8_caches_expanded(hd, H, Hkv, T, pos0, window, causal):
