@@ -375,6 +375,8 @@ static int attn_decode(const AttnDecodeArgs* a, const AttnCombineArgs* c, int nb
 
 static int attn_decode_rope(const AttnDecodeArgs* a, const AttnRopeArgs* r, const AttnCombineArgs* c, int nb, int hd, uint8_t* out16, int pdl, cudaStream_t st) {
     if (!r || !r->qkv) return (int)cudaErrorInvalidValue;
+    // int8 caches keep the choice between the kernels: with one query head a KV head the scalar one, whose products and probabilities are fp32
+    if (a->k_scale && !use_mma(*a, hd)) return (int)cudaErrorNotSupported;
     AttnDecodeArgs m = *a;
     m.n_splits = attn_decode_mma_splits(m, nb);
     const cudaError_t e = (cudaError_t)attn_decode_mma_rope_launch(m, *r, nb, hd, pdl, st);
@@ -389,8 +391,8 @@ B2_API int b2_attn_decode(const AttnDecodeArgs* a, const AttnCombineArgs* c, int
 
 // Split-K attention on raw projections: rotary embedding of the queries, rotation + cache append of the new key / value and the
 // attention itself in one launch (tensor-core kernel only), then the merge of the splits.  Returns cudaErrorNotSupported
-// (nothing launched) for shapes, cache encodings or rotary settings that kernel does not take: the caller then runs
-// b2_rope_kv + b2_attn_decode.
+// (nothing launched) for shapes, cache encodings or rotary settings that kernel does not take, and for int8 caches whose steps
+// b2_attn_decode gives to the scalar kernel: the caller then runs b2_rope_kv + b2_attn_decode.
 B2_API int b2_attn_decode_rope(const AttnDecodeArgs* a, const AttnRopeArgs* r, const AttnCombineArgs* c, int nb, int hd, int pdl, cudaStream_t st) {
     return attn_decode_rope(a, r, c, nb, hd, nullptr, pdl, st);
 }

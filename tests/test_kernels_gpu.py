@@ -297,6 +297,25 @@ def test_attn_decode_rotates_and_appends_to_int8_caches(hd, H, Hkv, n_rot, neox,
     assert torch.allclose(got, want, atol=2e-3, rtol=2e-3), (got - want).abs().max()
 
 
+@pytest.mark.parametrize("hd,H,Hkv,mode", [(128, 8, 8, -1), (64, 4, 4, -1), (128, 8, 2, 0)])
+def test_int8_steps_keep_the_choice_of_kernel(hd, H, Hkv, mode, attn_mode):
+    """One query head a KV head, or the scalar kernel asked for: the form that rotates and appends inside is refused before anything is launched, so that such steps stay on the kernel whose
+    products and probabilities are fp32."""
+    K = _K()
+    attn_mode(mode)
+    n_ctx, g = 128, torch.Generator().manual_seed(hd + H)
+    kc, vc = (torch.randint(-127, 128, (1, Hkv, n_ctx, hd), generator=g, dtype=torch.int8).cuda() for _ in range(2))
+    ks, vs = ((torch.rand(1, Hkv, n_ctx, hd // 32, generator=g) * 0.01).half().cuda() for _ in range(2))
+    kept = [t.clone() for t in (kc, vc, ks, vs)]
+    qkv, at = torch.randn(1, (H + 2 * Hkv) * hd, generator=g).cuda(), torch.tensor([77], dtype=torch.int32).cuda()
+    inv = (1.0 / (10000.0 ** (torch.arange(0, hd, 2).float() / hd))).cuda()
+    args = dict(n_heads=H, n_rot=hd, neox=True, mscale=1.0, scale=hd ** -0.5, n_splits=2, k_scale=ks, v_scale=vs)
+    assert K.attn_decode_rope(qkv, kc, vc, at, at * 0, inv, **args) is None
+    assert all(torch.equal(x, y) for x, y in zip((kc, vc, ks, vs), kept))
+    attn_mode(1)
+    assert K.attn_decode_rope(qkv, kc, vc, at, at * 0, inv, **args) is not None
+
+
 @pytest.mark.parametrize("hd,H,Hkv", [(128, 8, 2), (64, 3, 3)])
 @pytest.mark.parametrize("n_splits", [1, 3, 16])
 def test_attn_decode_head_norm(hd, H, Hkv, n_splits, attn_mode):
