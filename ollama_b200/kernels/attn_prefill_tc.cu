@@ -490,7 +490,7 @@ struct Lay2 {
     static constexpr int Q_BYTES = K_ATOMS * ATOM_BYTES;
     static constexpr int K_BYTES = K_ATOMS * ATOM_BYTES, V_BYTES = V_ATOMS * ATOM_BYTES;
     static constexpr int OFF_K = Q_BYTES, OFF_V = OFF_K + 2 * K_BYTES, OFF_BAR = OFF_V + 2 * V_BYTES;
-    static constexpr int TOTAL = OFF_BAR + 256 + 3 * 2 * 128 * 4 + 1024;
+    static constexpr int TOTAL = OFF_BAR + 1024 + 3 * 2 * 128 * 4 + 1024;
 };
 
 // D: value columns, DK: query / key columns (D unless the form is PARTS).  DIFF: a CTA takes 64 queries of a head of differential attention, rows 0 .. 63 of its tile
@@ -519,7 +519,7 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
     uint64_t* pair = bars + 14;          // [4]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
     int* failed = reinterpret_cast<int*>(bars + 19);
-    float* x_max = reinterpret_cast<float*>(sm + L::OFF_BAR + 256);      // [2][2][128] row maxima of the two column halves, of even and of odd tiles
+    float* x_max = reinterpret_cast<float*>(sm + L::OFF_BAR + 1024);      // [2][2][128] row maxima of even and of odd tiles, of the two column halves
     float* x_sum = x_max + 512;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -675,6 +675,7 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
 #pragma unroll
         for (int j = 0; j < OH; j++) o[j] = 0.f;
         float m_run = -INFINITY, l_run = 0.f, corr_prev = 1.f;
+        const uint32_t x_at = smem_u32(x_max + c * 128 + r);      // the partner's place is 512 bytes off
         bool ok = true;
         auto accumulate = [&](int t, float corr) {      // o = o * corr + O_tile(t)
             const int b = t & 1;
@@ -726,13 +727,16 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
 #pragma unroll
                 for (int j = 0; j < 32; j++) mx = fmaxf(mx, __uint_as_float(v[i][j]));
             // The partner may be woken from this wait a whole tile later than this warp, which has written the next tile's maximum by then: hence a place each for even and odd
-            // tiles.  (With one, 7 rows to 128 of 16 heads behind 6000 keys from HBM had a quarter of a tile's rows on two maxima in up to 9 % of the launches.)
-            float* x_now = x_max + 256 * b;
-            x_now[c * 128 + r] = mx;
+            // tiles.  (With one, 64 to 128 rows of 16 heads behind 6000 keys from HBM had a quarter of a tile's rows on two maxima in up to 9 % of the launches.)  Addresses of
+            // 32 bits: 512 rows of 32 heads at 6000 take 71.8 us, with one place and 64-bit addresses 73.8, with two and those 75.0.
+            const uint32_t x_now = x_at + 1024 * b;
+            float theirs;
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(x_now), "f"(mx) : "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&pair[q]);
             if (!mbar_wait(&pair[q], t & 1)) { ok = false; break; }
-            mx = fmaxf(mx, x_now[(c ^ 1) * 128 + r]);
+            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(theirs) : "r"(x_now ^ 512) : "memory");
+            mx = fmaxf(mx, theirs);
             const float m_new = fmaxf(m_run, mx);
             const float corr = m_new == -INFINITY ? 1.f : ex2((m_run - m_new) * mult);
             const float mref = m_new == -INFINITY ? 0.f : m_new * mult;
