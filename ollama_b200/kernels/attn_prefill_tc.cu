@@ -927,12 +927,12 @@ __global__ void __launch_bounds__(THREADS2, 1) attn_prefill_tc2_kernel(const __g
 }
 
 
-// Rows [lo, hi) of an int8 cache of one slot as f16, [K, V][Hkv][pitch][D]; rows from kv_len on are zeros (a masked key's value still meets a probability of zero).  A thread has
-// 16 dims, half of a scale's block.
-__global__ void __launch_bounds__(256) expand_q8_kernel(const __grid_constant__ AttnPrefillArgs a, int D, int lo, int hi, int pitch, __half* out) {
+// `rows` rows from position `lo` on of KV heads h0 .. h0 + heads - 1 of an int8 cache of one slot as f16, [K, V][heads][rows][D]; rows from kv_len on are zeros (a masked key's value still
+// meets a probability of zero).  A thread has 16 dims, half of a scale's block.
+__global__ void __launch_bounds__(256) expand_q8_kernel(const __grid_constant__ AttnPrefillArgs a, int D, int lo, int rows, int h0, int heads, __half* out) {
     pdl_launch();
     pdl_wait();
-    const int per = D / 16, n = (hi - lo) * per, i = blockIdx.x * 256 + threadIdx.x, hkv = blockIdx.y >> 1, is_v = blockIdx.y & 1;
+    const int per = D / 16, n = rows * per, i = blockIdx.x * 256 + threadIdx.x, hkv = h0 + (blockIdx.y >> 1), is_v = blockIdx.y & 1;
     if (i >= n) return;
     const int pos = lo + i / per, col = 16 * (i % per);
     uint32_t w[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
@@ -947,7 +947,7 @@ __global__ void __launch_bounds__(256) expand_q8_kernel(const __grid_constant__ 
             w[j] = pack_h2(d * (float)(int8_t)(b & 0xff), d * (float)(int8_t)((b >> 8) & 0xff));
         }
     }
-    uint4* o = reinterpret_cast<uint4*>(out + (((size_t)is_v * a.Hkv + hkv) * pitch + pos) * D + col);
+    uint4* o = reinterpret_cast<uint4*>(out + (((size_t)is_v * heads + hkv - h0) * rows + pos - lo) * D + col);
     o[0] = make_uint4(w[0], w[1], w[2], w[3]);
     o[1] = make_uint4(w[4], w[5], w[6], w[7]);
 }
@@ -991,14 +991,14 @@ int key_parts(const AttnPrefillArgs& a, int tiles) {
     return 1;
 }
 
+// The first `heads` query heads, on caches of `rows` rows.
 template <int D>
-int launch2(const AttnPrefillArgs& a, int n_slots, int pdl, cudaStream_t st) {
+int launch2(const AttnPrefillArgs& a, int heads, size_t rows, int pdl, cudaStream_t st) {
     CUtensorMap mk, mv;
-    const size_t rows = (size_t)n_slots * a.Hkv * a.n_ctx;
     if (!cached_kv_map(&mk, a.k_cache, rows, D) || !cached_kv_map(&mv, a.v_cache, rows, D)) return (int)cudaErrorNotSupported;
     static PerDeviceOnce once;
     if (once.first()) cudaFuncSetAttribute(attn_prefill_tc2_kernel<D, D, FLAT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay2<D, D>::TOTAL);
-    dim3 grid((a.T + BQ - 1) / BQ, a.H);
+    dim3 grid((a.T + BQ - 1) / BQ, heads);
     AttnPrefillArgs copy = a;
     AttnPagedArgs pg = {};
     AttnPartsArgs pt = {};
@@ -1108,9 +1108,10 @@ B2_API int b2_attn_prefill_tc(const AttnPrefillArgs* a, int head_dim, int n_slot
         return (int)cudaErrorInvalidValue;
     if (a->k_scale || a->v_scale) return (int)cudaErrorNotSupported;
     if (((uintptr_t)a->k_cache & 15) || ((uintptr_t)a->v_cache & 15) || ((uintptr_t)a->q & 15) || ((uintptr_t)a->out & 15)) return (int)cudaErrorNotSupported;
-    if ((size_t)n_slots * a->Hkv * a->n_ctx >= ((size_t)1 << 31)) return (int)cudaErrorNotSupported;
-    if (g_variant == 2 && head_dim == 128) return launch2<128>(*a, n_slots, pdl, st);
-    if (g_variant == 2 && head_dim == 64) return launch2<64>(*a, n_slots, pdl, st);
+    const size_t rows = (size_t)n_slots * a->Hkv * a->n_ctx;
+    if (rows >= ((size_t)1 << 31)) return (int)cudaErrorNotSupported;
+    if (g_variant == 2 && head_dim == 128) return launch2<128>(*a, a->H, rows, pdl, st);
+    if (g_variant == 2 && head_dim == 64) return launch2<64>(*a, a->H, rows, pdl, st);
     if (head_dim == 128) return g_variant ? launch<128, true>(*a, n_slots, st) : launch<128, false>(*a, n_slots, st);
     if (head_dim == 64) return g_variant ? launch<64, true>(*a, n_slots, st) : launch<64, false>(*a, n_slots, st);
     return (int)cudaErrorNotSupported;
@@ -1134,34 +1135,58 @@ B2_API void b2_attn_prefill_tc_clear_status() {
     cudaMemcpyToSymbol(g_attn_tc_status, &v, sizeof(int));
 }
 
-// Halves of scratch that b2_attn_prefill_q8 takes for kv_len keys.
-B2_API long long b2_attn_prefill_q8_scratch(int kv_len, int n_kv_heads, int head_dim) { return 2ll * n_kv_heads * ((kv_len + BKV - 1) / BKV * BKV) * head_dim; }
+// The positions [lo, lo + rows) of an int8 cache that a pass expands, whole tiles: those from the first query's window on.
+static int expanded_rows(int pos0, int kv_len, int window, int& lo) {
+    const int hi = (kv_len + BKV - 1) / BKV * BKV;
+    lo = window > 0 && pos0 >= window ? (pos0 - window + 1) / BKV * BKV : 0;
+    if (lo >= hi) lo = hi - BKV;
+    return hi - lo;
+}
 
-// The same on an int8 cache with scales: its rows that queries may see are expanded into `scratch` (16-byte aligned, b2_attn_prefill_q8_scratch halves) once, where the kernel that
+// Halves of scratch with which b2_attn_prefill_q8 takes `heads` KV heads at a time, for queries from pos0 on over kv_len keys.
+B2_API long long b2_attn_prefill_q8_scratch(int pos0, int kv_len, int window, int heads, int head_dim) {
+    int lo;
+    return 2ll * heads * expanded_rows(pos0, kv_len, window, lo) * head_dim;
+}
+
+// The same on an int8 cache with scales: its rows that queries may see are expanded into `scratch` (16-byte aligned) once, where the kernel that
 // expands them on the way (attn_prefill.cu) does so for every 64 queries of a head and multiplies with mma.sync.  32 heads of 128: 7 rows behind 901 57 -> 14 us, 64 behind 4000
-// 236 -> 25, 2048 behind 4000 1401 -> 253; 2 rows behind 50 6.6 -> 8.4, so up to 64 keys stay there.  Head size 64 or 128 (anything else, and other alignments:
-// cudaErrorNotSupported, nothing launched).
-B2_API int b2_attn_prefill_q8(const AttnPrefillArgs* in, int head_dim, int n_slots, void* scratch, int pdl, cudaStream_t st) {
-    if (!in || !in->k_scale || !in->v_scale || !scratch || in->T < 1 || in->H < 1 || in->Hkv < 1 || in->Hkv > 32767 || in->H % in->Hkv || in->kv_len < 1 || in->kv_len > in->n_ctx ||
-        n_slots < 1 || in->slot < 0 || in->slot >= n_slots || in->pos0 < 0)
+// 236 -> 25, 2048 behind 4000 1401 -> 253; 2 rows behind 50 6.6 -> 8.4, so up to 64 keys stay there.  Head size 64 or 128 (anything else, other alignments and scratch for less than one
+// KV head: cudaErrorNotSupported, nothing launched).
+// With less scratch than for all KV heads, as many as fit take turns (8 heads of 128 are 537 MB at 131072 positions).  7 rows at 126000 take 456 us with all, 839 in two turns: clusters of
+// eight CTAs do not all fit at once; 2048 rows 5494 and 5601.
+B2_API int b2_attn_prefill_q8(const AttnPrefillArgs* in, int head_dim, int n_slots, void* scratch, long long halves, int pdl, cudaStream_t st) {
+    if (!in || !in->k_scale || !in->v_scale || !scratch || in->T < 1 || in->H < 1 || in->Hkv < 1 || in->H % in->Hkv || in->kv_len < 1 || in->kv_len > in->n_ctx || n_slots < 1 ||
+        in->slot < 0 || in->slot >= n_slots)
         return (int)cudaErrorInvalidValue;
     AttnPrefillArgs a = *in;
-    if ((head_dim != 64 && head_dim != 128) || g_variant != 2 || a.kv_len <= 64 ||
+    if ((head_dim != 64 && head_dim != 128) || g_variant != 2 || a.kv_len <= 64 || a.pos0 < 0 || a.Hkv > 32767 ||
         (((uintptr_t)a.k_cache | (uintptr_t)a.v_cache | (uintptr_t)a.q | (uintptr_t)a.out | (uintptr_t)scratch) & 15))
         return (int)cudaErrorNotSupported;
-    const int pitch = (a.kv_len + BKV - 1) / BKV * BKV;
-    if ((size_t)a.Hkv * pitch >= ((size_t)1 << 31)) return (int)cudaErrorNotSupported;
-    int lo = a.window > 0 && a.pos0 >= a.window ? (a.pos0 - a.window + 1) / BKV * BKV : 0, hi = pitch;
-    if (lo >= hi) lo = hi - BKV;
+    int lo;
+    const int rows = expanded_rows(a.pos0, a.kv_len, a.window, lo), group = a.H / a.Hkv;
+    const long long fit = halves / (2ll * rows * head_dim);
+    if (fit < 1 || (size_t)a.Hkv * rows >= ((size_t)1 << 31)) return (int)cudaErrorNotSupported;
+    const int turns = fit >= a.Hkv ? 1 : (int)((a.Hkv + fit - 1) / fit), some = (a.Hkv + turns - 1) / turns;
     __half* out = (__half*)scratch;
-    void* args[] = {&a, &head_dim, &lo, &hi, (void*)&pitch, &out};
-    const int rc = launch_rows((const void*)expand_q8_kernel, dim3(((hi - lo) * (head_dim / 16) + 255) / 256, 2 * a.Hkv), dim3(256), 0, args, st, pdl);
-    if (rc) return rc;
-    AttnPrefillArgs c = a;
-    c.k_cache = out;
-    c.v_cache = out + (size_t)a.Hkv * pitch * head_dim;
-    c.k_scale = c.v_scale = nullptr;
-    c.slot = 0;
-    c.n_ctx = pitch;
-    return head_dim == 128 ? launch2<128>(c, 1, pdl, st) : launch2<64>(c, 1, pdl, st);
+    for (int h0 = 0; h0 < a.Hkv; h0 += some) {      // launches follow each other: the next heads go where these have been read
+        int heads = a.Hkv - h0 < some ? a.Hkv - h0 : some, first = lo, n = rows;
+        void* args[] = {&a, &head_dim, &first, &n, &h0, &heads, &out};
+        int rc = launch_rows((const void*)expand_q8_kernel, dim3((rows * (head_dim / 16) + 255) / 256, 2 * heads), dim3(256), 0, args, st, pdl);
+        if (rc) return rc;
+        AttnPrefillArgs c = a;      // positions count from `lo`, of which only differences matter
+        c.q += (size_t)h0 * group * head_dim;
+        c.out += (size_t)h0 * group * head_dim;
+        if (c.sinks) c.sinks += h0 * group;
+        c.k_cache = out;
+        c.v_cache = out + (size_t)heads * rows * head_dim;
+        c.k_scale = c.v_scale = nullptr;
+        c.slot = 0;
+        c.n_ctx = rows;
+        c.pos0 -= lo;
+        c.kv_len -= lo;
+        rc = head_dim == 128 ? launch2<128>(c, heads * group, (size_t)heads * rows, pdl, st) : launch2<64>(c, heads * group, (size_t)heads * rows, pdl, st);
+        if (rc) return rc;
+    }
+    return 0;
 }

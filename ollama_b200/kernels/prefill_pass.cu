@@ -9,7 +9,7 @@ extern "C" {
 int b2_rmsnorm_bf16(const NormCastArgs* a, int rows, int pdl, cudaStream_t st);
 int b2_rope_kv(const RopeKvArgs* a, int nt, int pdl, cudaStream_t st);
 int b2_attn_prefill_tc(const AttnPrefillArgs* a, int head_dim, int n_slots, int pdl, cudaStream_t st);
-int b2_attn_prefill_q8(const AttnPrefillArgs* in, int head_dim, int n_slots, void* scratch, int pdl, cudaStream_t st);
+int b2_attn_prefill_q8(const AttnPrefillArgs* in, int head_dim, int n_slots, void* scratch, long long halves, int pdl, cudaStream_t st);
 int b2_attn_prefill(const AttnPrefillArgs* a, int head_dim, cudaStream_t st);
 int b2_gemm_bf16(const void* a, const void* b, int m, int n, int k, float* out, int ldo, const float* bias, int accumulate, int pdl, float* ws,
                  long long ws_floats, cudaStream_t st);
@@ -45,7 +45,8 @@ struct PassArgs {
     long long ws_floats;
     int* status;
     int units, tc, pdl;                           // tc: attention on tcgen05 where it applies
-    void* kv16;                                   // int8 caches: b2_attn_prefill_q8_scratch halves for the longest sequence, or null
+    void* kv16;                                   // int8 caches: scratch of b2_attn_prefill_q8, or null
+    long long kv16_halves;
     int launches;                                 // out
 };
 
@@ -113,7 +114,7 @@ B2_API int b2_prefill_pass(const PassLayer* layers, int n, PassArgs* io, const P
             rc = (int)cudaErrorNotSupported;
             if (a.tc && (a.hd == 64 || a.hd == 128))
                 rc = !L.k_scale ? b2_attn_prefill_tc(&at, a.hd, a.n_slots, a.pdl, st)
-                     : a.kv16   ? b2_attn_prefill_q8(&at, a.hd, a.n_slots, a.kv16, a.pdl, st)
+                     : a.kv16   ? b2_attn_prefill_q8(&at, a.hd, a.n_slots, a.kv16, a.kv16_halves, a.pdl, st)
                                 : (int)cudaErrorNotSupported;
             if (!rc && L.k_scale) count++;
             if (rc == (int)cudaErrorNotSupported) rc = b2_attn_prefill(&at, a.hd, st);      // nothing was launched

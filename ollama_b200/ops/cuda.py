@@ -627,11 +627,22 @@ ATTN_PREFILL_HEAD_DIMS = (32, 64, 128, 256)
 ATTN_PREFILL_DEFAULT = "auto"       # the kernel prefill attention runs on unless told otherwise (see attn_prefill)
 
 
-def attn_prefill_q8_scratch(kv_len: int, n_kv_heads: int, head_dim: int, device) -> torch.Tensor:
-    """Room for the visible rows of a slot's int8 cache as f16 (kernels/attn_prefill_tc.cu)."""
+def attn_prefill_q8_head(pos0: int, kv_len: int, window: int, head_dim: int) -> int:
+    """f16 values that the visible rows of one KV head of an int8 cache take (kernels/attn_prefill_tc.cu)."""
     f = lib().b2_attn_prefill_q8_scratch
     f.restype = C.c_longlong
-    return torch.empty(f(kv_len, n_kv_heads, head_dim), device=device, dtype=torch.float16)
+    return f(pos0, kv_len, window, 1, head_dim)
+
+
+def attn_prefill_q8_scratch(head: int, n_kv_heads: int, device) -> torch.Tensor | None:
+    """Room for such rows, ``head`` values a KV head: of all heads, where that much memory cannot be had of half of them and so on, and None where not even of one (the kernel that expands
+    rows on the way needs none)."""
+    while n_kv_heads:
+        try:
+            return torch.empty(head * n_kv_heads, device=device, dtype=torch.float16)
+        except torch.OutOfMemoryError:
+            n_kv_heads //= 2
+    return None
 
 
 def attn_prefill(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, slot: int, pos0: int, kv_len: int, scale: float,
@@ -655,8 +666,10 @@ def attn_prefill(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
     elif mode == "tc":
         raise RuntimeError("attn_prefill: the tcgen05 kernel takes f16 caches and head size 64 or 128")
     elif mode == "auto" and D in (64, 128) and k_scale is not None and q.dtype == torch.float32:
-        scratch = attn_prefill_q8_scratch(kv_len, Hkv, D, q.device)
-        rc = lib().b2_attn_prefill_q8(C.byref(a), D, n_slots, C.c_void_p(ptr(scratch)), int(pdl), stream())
+        scratch = attn_prefill_q8_scratch(attn_prefill_q8_head(pos0, kv_len, window, D), Hkv, q.device)
+        rc = 801
+        if scratch is not None:
+            rc = lib().b2_attn_prefill_q8(C.byref(a), D, n_slots, C.c_void_p(ptr(scratch)), C.c_longlong(scratch.numel()), int(pdl), stream())
         if rc == 0:
             return out
         if rc != 801:

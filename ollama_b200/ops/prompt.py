@@ -23,7 +23,7 @@ class PassSeg(C.Structure):
 class PassArgs(C.Structure):
     _fields_ = [("rows", I), ("d", I), ("n_heads", I), ("n_kv_heads", I), ("hd", I), ("n_rot", I), ("neox", I), ("n_ctx", I), ("n_slots", I), ("ff", I), ("causal", I), ("act", I),
                 ("eps", F), ("scale", F), ("softcap", F), ("alpha", F), ("limit", F), ("positions", P), ("slots", P), ("x", P), ("qkv", P), ("q", P), ("o", P), ("h", P), ("f", P),
-                ("x16", P), ("ws", P), ("ws_floats", C.c_longlong), ("status", P), ("units", I), ("tc", I), ("pdl", I), ("kv16", P), ("launches", I)]
+                ("x16", P), ("ws", P), ("ws_floats", C.c_longlong), ("status", P), ("units", I), ("tc", I), ("pdl", I), ("kv16", P), ("kv16_halves", C.c_longlong), ("launches", I)]
 
 
 class PromptPass:
@@ -50,6 +50,7 @@ class PromptPass:
             a.mscale, a.window = (1.0 if local else be.mscale), (c.sliding_window if L.swa else 0)
             a.k_cache, a.v_cache, a.k_scale, a.v_scale = map(K.ptr, (be.k_cache[i], be.v_cache[i], be.k_scale[i], be.v_scale[i]))
             self.keep += [ts, be.k_cache[i], be.v_cache[i], be.k_scale[i], be.v_scale[i]]
+        self.windows = {a.window for a in self.layers}
         self.ws = SK.Workspace(be.device) if self.units else None
 
     def run(self, be, x: torch.Tensor, positions: torch.Tensor, slots: torch.Tensor, segs: list[tuple[int, int, int, int]], units: bool, tc: bool) -> int:
@@ -67,11 +68,14 @@ class PromptPass:
         size = 0 if units else max(K.gemm_bf16_scratch(n, *nk) for nk in (((c.n_heads + 2 * c.n_kv_heads) * c.head_dim, c.d_model), (c.d_model, c.q_dim), (c.d_model, c.d_ff)))
         parts = torch.empty(size, device=dev, dtype=torch.float32) if size else None
         q8 = tc and c.head_dim in (64, 128) and be.k_scale[0] is not None
-        kv16 = K.attn_prefill_q8_scratch(max(p0 + r for _, r, _, p0 in segs), c.n_kv_heads, c.head_dim, dev) if q8 else None
+        kv16 = None
+        if q8:
+            head = max(K.attn_prefill_q8_head(p0, p0 + r, w, c.head_dim) for _, r, _, p0 in segs for w in self.windows)
+            kv16 = K.attn_prefill_q8_scratch(head, c.n_kv_heads, dev)
         a = PassArgs(n, c.d_model, c.n_heads, c.n_kv_heads, c.head_dim, c.rope_dim, int(c.rope_style == "neox"), be.n_ctx, be.n_slots, c.d_ff, int(c.causal), K._ACT[c.act],
                      c.norm_eps, be.attn_scale, c.attn_softcap, c.swiglu_alpha, c.swiglu_limit, K.ptr(positions), K.ptr(slots), K.ptr(x), K.ptr(qkv), K.ptr(q), K.ptr(o), K.ptr(h),
                      K.ptr(f), K.ptr(x16), *((K.ptr(ws.ws), 0, K.ptr(ws.status)) if units else (K.ptr(parts), size, None)), int(units), int(tc),
-                     int(be.pdl), K.ptr(kv16), 0)
+                     int(be.pdl), K.ptr(kv16), kv16.numel() if kv16 is not None else 0, 0)
         sg = (PassSeg * len(segs))(*[PassSeg(*s) for s in segs])
         fn = K.lib().b2_prefill_pass
         fn.argtypes = [P, I, P, P, I, P]

@@ -133,11 +133,13 @@ def predict_memory(model: Any, num_ctx: int, num_parallel: int, free: int | None
     kvh = _first_int(kv.get(f"{arch}.attention.head_count_kv"), heads) or heads
     d = _first_int(kv.get(f"{arch}.embedding_length"))
     hd = _first_int(kv.get(f"{arch}.attention.key_length"), d // heads if heads else 0)
-    per_elem = 2.0                                   # f16 cache
+    per_elem, expanded = 2.0, 0                      # f16 cache
     if (envconfig.kv_cache_type() or "f16").lower() in ("q8_0", "q4_0") and hd % 32 == 0:
         per_elem = 1.0 + 2.0 / 32                    # int8 + one f16 scale per 32 dims (q4_0 requests are served as q8_0)
+        if hd in (64, 128):
+            expanded = 2 * kvh * hd * num_ctx * 2    # a prompt's attention reads a layer's rows of one sequence as f16
     extra = sum(os.path.getsize(p) for p in list(getattr(model, "draft_paths", None) or []) if os.path.exists(p))
-    total = size + extra + int(2 * layers * kvh * hd * num_ctx * num_parallel * per_elem)
+    total = size + extra + expanded + int(2 * layers * kvh * hd * num_ctx * num_parallel * per_elem)
     if free:
         ff = _first_int(kv.get(f"{arch}.feed_forward_length"))
         vocab = _first_int(kv.get(f"{arch}.vocab_size")) or len(kv.get("tokenizer.ggml.tokens") or ())

@@ -558,6 +558,35 @@ def test_attn_prefill_of_int8_caches_expanded(hd, H, Hkv, T, pos0, window, causa
         assert torch.allclose(got, ref, atol=1e-2, rtol=2e-2), (got - ref).abs().max()
 
 
+@pytest.mark.parametrize("T,pos0,window", [(130, 2000, 0), (7, 3000, 0), (200, 4000, 1500), (128, 5000, 5001)])
+@pytest.mark.parametrize("heads", [8, 7, 3, 1, 0])
+def test_attn_prefill_of_int8_caches_in_little_memory(T, pos0, window, heads, monkeypatch):
+    """Memory for the rows of so many KV heads only, which take turns, or for none; windows that see a part of the rows, sinks: the values of the kernel that expands on the way, its bits
+    without scratch.  Bound as above."""
+    K = _K()
+    hd, H, Hkv, n_ctx = 128, 16, 8, pos0 + T + 60
+    g = torch.Generator(device="cuda").manual_seed(T)
+    kc, vc = (torch.randint(-127, 128, (1, Hkv, n_ctx, hd), generator=g, device="cuda", dtype=torch.int8) for _ in range(2))
+    ks, vs = ((torch.rand(1, Hkv, n_ctx, hd // 32, generator=g, device="cuda") * 0.02).half() for _ in range(2))
+    q, sinks = torch.randn(T, H, hd, generator=g, device="cuda"), torch.randn(H, generator=g, device="cuda")
+    room = K.attn_prefill_q8_head(pos0, pos0 + T, window, hd)
+    seen = min(pos0 + T, window + T) if window else pos0 + T
+    assert seen <= room // (2 * hd) < seen + 3 * 128
+    empty = torch.empty
+
+    def little(*shape, dtype=torch.float32, **kw):      # full at more than `heads` heads, with a part of a head to spare
+        if dtype == torch.float16 and shape[0] > heads * room + room // 2:
+            raise torch.OutOfMemoryError("as a full GPU says it")
+        return empty(*shape, dtype=dtype, **kw)
+
+    args = dict(window=window, sinks=sinks, k_scale=ks, v_scale=vs)
+    old = K.attn_prefill(q, kc, vc, 0, pos0, pos0 + T, hd ** -0.5, mode="mma", **args).float()
+    monkeypatch.setattr(torch, "empty", little)
+    out = K.attn_prefill(q, kc, vc, 0, pos0, pos0 + T, hd ** -0.5, mode="auto", **args).float()
+    assert K.attn_prefill_tc_status(clear=True) == 0
+    assert torch.equal(out, old) if heads == 0 else torch.allclose(out, old, atol=1e-2, rtol=2e-2), (out - old).abs().max()
+
+
 @pytest.mark.parametrize("scale", [-0.1, 0.0])
 @pytest.mark.parametrize("hd,T,pos0,window,use_sinks", [(128, 300, 517, 0, False), (64, 129, 0, 48, True), (128, 5, 0, 0, False)])
 def test_attn_prefill_of_any_scale(hd, T, pos0, window, use_sinks, scale):

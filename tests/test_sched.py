@@ -166,6 +166,12 @@ def test_auto_context_shrinks_when_memory_is_short():
     s.unload_all()
 
 
+def test_predicted_memory_counts_the_rows_that_prompts_expand_from_int8_caches(monkeypatch):
+    monkeypatch.setenv("OLLAMA_KV_CACHE_TYPE", "q8_0")
+    values = 2 * 2 * 64 * 4096                            # keys and values of a layer: 2 KV heads of 64
+    assert predict_memory(FakeModel("a", 1 * GiB), 4096, 3) == 1 * GiB + 2 * 3 * values * 34 // 32 + 2 * values
+
+
 def test_queue_limit_and_single_loader(monkeypatch):
     monkeypatch.setenv("OLLAMA_MAX_QUEUE", "1")
     gate = threading.Event()
