@@ -1151,7 +1151,8 @@ B2_API long long b2_attn_prefill_q8_scratch(int pos0, int kv_len, int window, in
 
 // The same on an int8 cache with scales: its rows that queries may see are expanded into `scratch` (16-byte aligned) once, where the kernel that
 // expands them on the way (attn_prefill.cu) does so for every 64 queries of a head and multiplies with mma.sync.  32 heads of 128: 7 rows behind 901 57 -> 14 us, 64 behind 4000
-// 236 -> 25, 2048 behind 4000 1401 -> 253; 2 rows behind 50 6.6 -> 8.4, so up to 64 keys stay there.  Head size 64 or 128 (anything else, other alignments and scratch for less than one
+// 236 -> 25, 2048 behind 4000 1401 -> 253.  Up to 64 keys, and up to 128 of more than 64 rows, stay there (2 rows
+// behind 50 6.6 -> 8.4; prompts of six layers of 16 heads: 65 rows from position 0 672 -> 702, 128 rows 718 -> 755, but 129 rows 811 -> 799 and 7 rows behind 110 392 -> 382).  Head size 64 or 128 (anything else, other alignments and scratch for less than one
 // KV head: cudaErrorNotSupported, nothing launched).
 // With less scratch than for all KV heads, as many as fit take turns (8 heads of 128 are 537 MB at 131072 positions).  7 rows at 126000 take 456 us with all, 839 in two turns: clusters of
 // eight CTAs do not all fit at once; 2048 rows 5494 and 5601.
@@ -1160,7 +1161,7 @@ B2_API int b2_attn_prefill_q8(const AttnPrefillArgs* in, int head_dim, int n_slo
         in->slot < 0 || in->slot >= n_slots)
         return (int)cudaErrorInvalidValue;
     AttnPrefillArgs a = *in;
-    if ((head_dim != 64 && head_dim != 128) || g_variant != 2 || a.kv_len <= 64 || a.pos0 < 0 || a.Hkv > 32767 ||
+    if ((head_dim != 64 && head_dim != 128) || g_variant != 2 || a.kv_len <= (a.T > 64 ? BKV : 64) || a.pos0 < 0 || a.Hkv > 32767 ||
         (((uintptr_t)a.k_cache | (uintptr_t)a.v_cache | (uintptr_t)a.q | (uintptr_t)a.out | (uintptr_t)scratch) & 15))
         return (int)cudaErrorNotSupported;
     int lo;

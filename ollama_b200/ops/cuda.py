@@ -665,7 +665,7 @@ def attn_prefill(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
             _check(rc, "attn_prefill_tc")
     elif mode == "tc":
         raise RuntimeError("attn_prefill: the tcgen05 kernel takes f16 caches and head size 64 or 128")
-    elif mode == "auto" and D in (64, 128) and k_scale is not None and q.dtype == torch.float32:
+    elif mode == "auto" and D in (64, 128) and k_scale is not None and q.dtype == torch.float32 and kv_len > 64:
         scratch = attn_prefill_q8_scratch(attn_prefill_q8_head(pos0, kv_len, window, D), Hkv, q.device)
         rc = 801
         if scratch is not None:

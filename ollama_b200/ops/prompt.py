@@ -67,7 +67,7 @@ class PromptPass:
         ws = self.ws if units else None
         size = 0 if units else max(K.gemm_bf16_scratch(n, *nk) for nk in (((c.n_heads + 2 * c.n_kv_heads) * c.head_dim, c.d_model), (c.d_model, c.q_dim), (c.d_model, c.d_ff)))
         parts = torch.empty(size, device=dev, dtype=torch.float32) if size else None
-        q8 = tc and c.head_dim in (64, 128) and be.k_scale[0] is not None
+        q8 = tc and c.head_dim in (64, 128) and be.k_scale[0] is not None and max(p0 + r for _, r, _, p0 in segs) > 64
         kv16 = None
         if q8:
             head = max(K.attn_prefill_q8_head(p0, p0 + r, w, c.head_dim) for _, r, _, p0 in segs for w in self.windows)

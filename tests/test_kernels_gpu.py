@@ -558,6 +558,20 @@ def test_attn_prefill_of_int8_caches_expanded(hd, H, Hkv, T, pos0, window, causa
         assert torch.allclose(got, ref, atol=1e-2, rtol=2e-2), (got - ref).abs().max()
 
 
+@pytest.mark.parametrize("T,pos0", [(65, 0), (128, 0), (64, 0), (3, 61), (129, 0), (64, 1), (2, 64)])
+def test_short_prompts_on_int8_caches_stay_on_one_launch(T, pos0):
+    """Up to 64 keys, and up to 128 of more rows than that, the kernel that expands rows on the way, with its bits; from one key more on the rows are expanded first."""
+    K = _K()
+    hd, H, Hkv = 128, 8, 2
+    g = torch.Generator(device="cuda").manual_seed(T)
+    kc, vc = (torch.randint(-127, 128, (1, Hkv, 256, hd), generator=g, device="cuda", dtype=torch.int8) for _ in range(2))
+    ks, vs = ((torch.rand(1, Hkv, 256, hd // 32, generator=g, device="cuda") * 0.02).half() for _ in range(2))
+    q = torch.randn(T, H, hd, generator=g, device="cuda")
+    out, old = (K.attn_prefill(q, kc, vc, 0, pos0, pos0 + T, hd ** -0.5, k_scale=ks, v_scale=vs, mode=m) for m in ("auto", "mma"))
+    assert pos0 + T > (128 if T > 64 else 64) or torch.equal(out, old)
+    assert torch.allclose(out.float(), old.float(), atol=1e-2, rtol=2e-2)
+
+
 @pytest.mark.parametrize("T,pos0,window", [(130, 2000, 0), (7, 3000, 0), (200, 4000, 1500), (128, 5000, 5001)])
 @pytest.mark.parametrize("heads", [8, 7, 3, 1, 0])
 def test_attn_prefill_of_int8_caches_in_little_memory(T, pos0, window, heads, monkeypatch):
