@@ -16,8 +16,8 @@
 // The kernel that runs by default is the pipelined form further down (two score buffers, probabilities kept in TMEM, the
 // accumulation of a tile deferred behind the next tile's softmax); the single-buffered forms above it stay selectable.
 //
-// Attention sinks, logit soft-capping and sliding windows follow attn_prefill.cu, which stays the kernel for int8 caches
-// and head sizes other than 64 / 128.  In the reference stack this is ggml-cuda's fattn family (mma / tile / vec).
+// Attention sinks, logit soft-capping and sliding windows follow attn_prefill.cu, which stays the kernel for short int8 caches
+// and head sizes other than 64 / 128.  Rows of longer int8 caches are expanded first (b2_attn_prefill_q8).  In the reference stack this is ggml-cuda's fattn family (mma / tile / vec).
 #include "tc_common.cuh"
 #include "rows.cuh"
 #include "pass_args.cuh"
@@ -976,18 +976,45 @@ float positive_scale(AttnPrefillArgs& a) {
     return s == 0.f ? 0.f : -1.f;
 }
 
-// CTAs that share the keys of a query tile (a cluster): as many of 8, 4 or 2 as there are SMs for and as leave each of them two tiles of 128 keys.  The cluster and its merge cost
+cudaLaunchConfig_t cluster_config(dim3 grid, int smem, int parts, cudaLaunchAttribute* at) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(THREADS2);
+    cfg.dynamicSmemBytes = smem;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = parts;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// CTAs that share the keys of a query tile (a cluster): as many of 8, 4 or 2 as fit the GPU at once (15 clusters of 8, 33 of 4 and 74 of 2 on 148 SMs) and as leave each of them two
+// tiles of the last query tile's keys (the first tiles of a prompt from position 0 have fewer, some CTAs none).  The cluster and its merge cost
 // about 3 us, a tile 1.3, so eight tiles are the least: 32 heads of 128, 7 rows behind 901: 15.7 -> 10.5 us, 64 behind 4000: 46.6 -> 19.8, 128 behind 6000: 68.6 -> 27.8, but 100
-// behind 300 12.7 -> 14.3.
+// behind 300 12.7 -> 14.3.  Clusters that have to wait for others cost more than they save: 34 heads, 7 rows behind 901: 15.5 us in one part, 18.8 in 4, 11.9 in 2; 16 heads, 64 behind
+// 3000: 36.4, 25.2 in 8, 16.4 in 4.
+template <int D>
 int key_parts(const AttnPrefillArgs& a, int tiles) {
-    static int sms[64] = {};
+    static int fit[64][3] = {};      // clusters of 2, 4 and 8
     int d = 0;
     cudaGetDevice(&d);
-    d &= 63;
-    if (!sms[d]) cudaDeviceGetAttribute(&sms[d], cudaDevAttrMultiProcessorCount, d);
     const int keys = a.window > 0 && a.causal ? (a.kv_len < a.window + BQ ? a.kv_len : a.window + BQ) : a.kv_len;
-    for (int p = 8; p > 1; p >>= 1)
-        if (tiles * p <= sms[d] && keys > (p > 4 ? 2 * p - 1 : 7) * BKV) return p;
+    for (int i = 2; i >= 0; i--) {
+        const int p = 2 << i;
+        if (keys <= (p > 4 ? 2 * p - 1 : 7) * BKV) continue;
+        int& n = fit[d & 63][i];
+        if (!n) {
+            const void* fn = (const void*)attn_prefill_tc2_kernel<D, D, FLAT, false, true>;
+            cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay2<D, D>::TOTAL);
+            cudaLaunchAttribute at;
+            const cudaLaunchConfig_t cfg = cluster_config(dim3(p), Lay2<D, D>::TOTAL, p, &at);
+            int most = 0;
+            if (cudaOccupancyMaxActiveClusters(&most, fn, &cfg) != cudaSuccess) cudaGetLastError();
+            n = most > 0 ? most : -1;
+        }
+        if (tiles <= n) return p;
+    }
     return 1;
 }
 
@@ -1004,25 +1031,15 @@ int launch2(const AttnPrefillArgs& a, int heads, size_t rows, int pdl, cudaStrea
     AttnPartsArgs pt = {};
     float qsign = positive_scale(copy);
     void* args[] = {&mk, &mv, &copy, &pg, &pt, &qsign};
-    const int parts = key_parts(a, (int)(grid.x * grid.y));
+    const int parts = key_parts<D>(a, (int)(grid.x * grid.y));
     if (parts > 1) {
-        const void* fn = (const void*)attn_prefill_tc2_kernel<D, D, FLAT, false, true>;
-        static PerDeviceOnce split_once;
-        if (split_once.first()) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay2<D, D>::TOTAL);
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(grid.x * parts, grid.y);
-        cfg.blockDim = dim3(THREADS2);
-        cfg.dynamicSmemBytes = Lay2<D, D>::TOTAL;
-        cfg.stream = st;
         cudaLaunchAttribute at[2];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = parts;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = cluster_config(dim3(grid.x * parts, grid.y), Lay2<D, D>::TOTAL, parts, at);
+        cfg.stream = st;
         at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[1].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
-        cfg.attrs = at;
         cfg.numAttrs = 2;
-        return (int)cudaLaunchKernelExC(&cfg, fn, args);
+        return (int)cudaLaunchKernelExC(&cfg, (const void*)attn_prefill_tc2_kernel<D, D, FLAT, false, true>, args);
     }
     return launch_rows((const void*)attn_prefill_tc2_kernel<D, D, FLAT>, grid, dim3(THREADS2), Lay2<D, D>::TOTAL, args, st, pdl);
 }
@@ -1115,6 +1132,12 @@ B2_API int b2_attn_prefill_tc(const AttnPrefillArgs* a, int head_dim, int n_slot
     if (head_dim == 128) return g_variant ? launch<128, true>(*a, n_slots, st) : launch<128, false>(*a, n_slots, st);
     if (head_dim == 64) return g_variant ? launch<64, true>(*a, n_slots, st) : launch<64, false>(*a, n_slots, st);
     return (int)cudaErrorNotSupported;
+}
+
+// CTAs that share the keys of a query tile in a launch of b2_attn_prefill_tc: 1, or a cluster of 2, 4 or 8.
+B2_API int b2_attn_prefill_key_parts(const AttnPrefillArgs* a, int head_dim) {
+    const int tiles = (a->T + BQ - 1) / BQ * a->H;
+    return head_dim == 128 ? key_parts<128>(*a, tiles) : key_parts<64>(*a, tiles);
 }
 
 // 0: the probabilities go through shared memory; 1: they stay in TMEM; 2: the pipelined kernel (default).  Returns the previous setting.

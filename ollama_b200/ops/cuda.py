@@ -678,6 +678,13 @@ def attn_prefill(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
     return out
 
 
+def attn_prefill_key_parts(q: torch.Tensor, k_cache: torch.Tensor, pos0: int, window: int = 0) -> int:
+    """CTAs that share the keys of a query tile when :func:`attn_prefill` runs on tcgen05 (1: no clusters)."""
+    T, H, D = q.shape
+    a = AttnPrefillArgs(None, None, None, None, None, T, H, k_cache.shape[1], k_cache.shape[2], 0, pos0, pos0 + T, 1, window, 1.0, 0.0, None, None)
+    return lib().b2_attn_prefill_key_parts(C.byref(a), D)
+
+
 def attn_prefill_tc_variant(v: int) -> int:
     """Where the tcgen05 attention kernel keeps the probabilities between its two products: 0 = a shared-memory tile,
     1 = TMEM (they overwrite the scores and feed the second product from there), 2 = the pipelined kernel (two score buffers and

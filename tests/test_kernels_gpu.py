@@ -501,7 +501,7 @@ def test_attn_prefill_on_tcgen05(hd, H, Hkv, T, pos0, window, softcap, use_sinks
 @pytest.mark.parametrize("T,pos0,window,softcap,use_sinks", [(1, 896, 0, 0.0, False), (7, 1020, 0, 0.0, True), (128, 1920, 0, 0.0, False), (130, 2100, 0, 30.0, True),
                                                               (200, 2500, 1000, 0.0, False), (66, 2700, 1, 0.0, False), (257, 2000, 2200, 0.0, True)])
 def test_attn_prefill_shares_keys(hd, H, Hkv, T, pos0, window, softcap, use_sinks):
-    """Few query tiles behind a long context: clusters of two to eight CTAs share a tile's keys, with windows that leave some of them none.  Bound as above."""
+    """Few query tiles behind a long context: clusters of two to eight CTAs share a tile's keys, with windows (of one key: one CTA).  Bound as above."""
     K = _K()
     n_slots, n_ctx, slot = 2, 3072, 1
     g = torch.Generator().manual_seed(hd + T)
@@ -513,6 +513,26 @@ def test_attn_prefill_shares_keys(hd, H, Hkv, T, pos0, window, softcap, use_sink
     assert K.attn_prefill_tc_status(clear=True) == 0
     ref = R.attention(q.to(torch.float16).float().cpu(), kc[slot, :, :p_end].transpose(0, 1).float().cpu(), vc[slot, :, :p_end].transpose(0, 1).float().cpu(),
                       torch.arange(pos0, p_end), torch.arange(p_end), scale=scale, causal=True, window=window, softcap=softcap, sinks=sinks.cpu() if use_sinks else None)
+    assert torch.allclose(out, ref, atol=1e-2, rtol=2e-2), (out - ref).abs().max()
+
+
+@pytest.mark.parametrize("hd,H,T,pos0,parts", [(64, 4, 1024, 0, 4), (128, 4, 1024, 0, 4), (64, 4, 2048, 0, 2), (64, 2, 1921, 0, 4), (64, 15, 64, 2000, 8), (128, 16, 64, 3000, 4),
+                                               (128, 33, 7, 901, 4), (64, 34, 7, 901, 2), (64, 74, 3, 901, 2), (64, 75, 3, 901, 1), (128, 8, 64, 700, 1)])
+@pytest.mark.parametrize("use_sinks", [False, True])
+def test_attn_prefill_in_so_many_parts(hd, H, T, pos0, parts, use_sinks):
+    """Parts by the clusters that fit 148 SMs at once; prompts from position 0, of whose first query tiles most CTAs of a cluster have no key tile.  Bound as above."""
+    K = _K()
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("counts of another GPU")
+    g = torch.Generator(device="cuda").manual_seed(hd + T)
+    kc, vc = (torch.randn(1, 1, pos0 + T + 70, hd, generator=g, device="cuda").mul_(0.7).half().expand(1, H, -1, -1).contiguous() for _ in range(2))
+    q = torch.randn(T, H, hd, generator=g, device="cuda")
+    sinks = torch.randn(H, generator=g, device="cuda") if use_sinks else None
+    assert K.attn_prefill_key_parts(q, kc, pos0) == parts
+    out = K.attn_prefill(q, kc, vc, 0, pos0, pos0 + T, hd ** -0.5, sinks=sinks, mode="tc").float().view(T, H, hd)
+    assert K.attn_prefill_tc_status(clear=True) == 0
+    ref = R.attention(q.half().float(), kc[0, :, :pos0 + T].transpose(0, 1).float(), vc[0, :, :pos0 + T].transpose(0, 1).float(), torch.arange(pos0, pos0 + T, device="cuda"),
+                      torch.arange(pos0 + T, device="cuda"), scale=hd ** -0.5, causal=True, sinks=sinks)
     assert torch.allclose(out, ref, atol=1e-2, rtol=2e-2), (out - ref).abs().max()
 
 
