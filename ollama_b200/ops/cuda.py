@@ -861,9 +861,14 @@ class MoeFp4:
     """The (token, expert) pairs of a step or a prompt times MXFP4 experts, each expert read once for all rows that chose it (kernels/moe_fp4.cu).
 
     Holds the sorted places of the pairs and the row buffers, so that a decode step can keep one for its CUDA graph; sizes that depend on the choice of
-    experts never visit the host.  ``chunk``: rows of an expert that a block multiplies at once, 8 / 16 / 24 / 32 / 40 / 48 / 64."""
+    experts never visit the host.  ``chunk``: rows of an expert that a block multiplies at once, one of CHUNKS (32 is never the quickest,
+    see :func:`moe_fp4_chunk`)."""
+
+    CHUNKS = (8, 16, 24, 32, 48, 64)
 
     def __init__(self, pairs: int, n_experts: int, d: int, ff: int, device, chunk: int):
+        if chunk not in self.CHUNKS:
+            raise ValueError(f"chunks of {chunk} rows: one of {self.CHUNKS} is wanted")
         self.n_experts, self.d, self.ff, self.chunk = n_experts, d, ff, chunk
         self.max_chunks = min(pairs, n_experts + pairs // chunk)      # full chunks, and one that is not for each expert
         self.rows = self.max_chunks * chunk

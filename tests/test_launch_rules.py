@@ -23,6 +23,13 @@ def test_int8_caches_whose_scales_are_not_aligned_go_to_the_scalar_decode_kernel
     assert takes(0, 0, heads=7) == 0 and takes(0, 0, heads=64) == 0
 
 
+def test_expert_rows_are_not_laid_out_for_chunks_that_no_kernel_takes():
+    for chunk in (0, 4, 12, 40, 56, 128):
+        with pytest.raises(ValueError):
+            K.MoeFp4(8, 4, 64, 64, "cpu", chunk)
+    assert all(K.moe_fp4_chunk(rows / 4) in K.MoeFp4.CHUNKS for rows in range(1, 400))
+
+
 class Launches:
     """Stands for the kernel library: keeps the arguments of each call."""
 
