@@ -37,7 +37,8 @@ from .steps import StepEngine
 MAX_DECODE_BATCH = 8             # sequences per launch of the dp4a kernels (kernels/gemv.cu)
 MAX_STREAM_BATCH = 32            # sequences per step when every matrix runs on the streaming kernel (kernels/gemv_sk.cu)
 # Steps of more sequences than this multiply f16 activations (kernels/gemm_sk.cu) instead of int8 ones.  Products of a layer of Llama-8B (Q4_K_M), int8 against f16: 39 us against
-# 55 at one sequence, 59 against 56 at two and at four, 64 against 56 at six, 70 against 56 at eight.
+# 55 at one sequence, 59 against 56 at two and at four, 64 against 56 at six, 70 against 56 at eight.  Smaller models would be quicker in int8 at two sequences (six layers of 1024 wide
+# 208 us against 233, of 2048 247 against 268) but not at four (247 against 228, 321 against 273), and a product of f16 rows is 30 times as exact (2.1e-4 against 7e-3).
 INT8_ROWS = 1
 # Prompt passes of at most this many rows, which is one launch a product, read the units too instead of the 16-bit copies (a layer of Llama-8B: 124 MB against 436).
 # Twelve layers at 64 rows: 1526 us against 2324; with two launches, at 65 rows 2255 against 2321, at 96 2362 against 2295.
@@ -288,9 +289,8 @@ class B200Backend(StepEngine):
         f32, i8, i32 = torch.float32, torch.int8, torch.int32
         qkv_dim = (c.n_heads + 2 * c.n_kv_heads) * c.head_dim
         kmax = max(c.d_model, c.q_dim)
-        # split-K width of decode attention: one CTA per (sequence, KV head, split).  Measured on Llama-8B (num_ctx 8192,
-        # tensor-core kernel): 16 splits give 442 tok/s at 640 tokens of context and 382 at 6272; 32 splits 428 and 396;
-        # 64 splits 409 and 371
+        # split-K width of decode attention: one CTA per (sequence, KV head, split).  Twelve layers of Llama-8B, num_ctx 8192, one sequence:
+        # 16 splits take 646 us at 640 tokens of context and 716 at 6272; 8 splits 651 and 754; 32 splits 656 and 726; 64 splits 666 and 760
         self.n_splits = max(1, min(envconfig.attn_splits(), n_ctx // envconfig.attn_split_len()))
         b = self.buf = _Layer()
         b.x = torch.zeros(MB, c.d_model, device=dev, dtype=f32)

@@ -92,6 +92,6 @@ struct PagedAttnArgs {
 int attn_decode_mma_launch(const AttnDecodeArgs& a, int nb, int hd, int pdl, cudaStream_t st);
 // The splits that a launch of it uses, at most a.n_splits: to be put into the arguments of the launch and of the merge.
 int attn_decode_mma_splits(const AttnDecodeArgs& a, int nb);
-// The same with the rotary embedding and the cache append inside; cudaErrorNotSupported also for quantised caches and more
-// than 256 rotated dimensions.
+// The same with the rotary embedding and the cache append inside; cudaErrorNotSupported also for quantised caches with pages and
+// more than 256 rotated dimensions.
 int attn_decode_mma_rope_launch(const AttnDecodeArgs& a, const AttnRopeArgs& r, int nb, int hd, int pdl, cudaStream_t st);

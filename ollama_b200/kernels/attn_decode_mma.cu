@@ -767,7 +767,7 @@ int launch_flat(const AttnDecodeArgs& a, const AttnRopeArgs& r, int nb, int pdl,
     return start(fn, smem, a, r, nb, room, pdl, st);
 }
 
-int g_stages = 0;      // 0: by the size of the launch; 2, 3 or 4: forced (tests)
+int g_stages = 0;      // f16 caches, 0: by the size of the launch; 2, 3 or 4: forced (tests).  int8 caches always have three stages (74 KB at 128 columns: three CTAs an SM)
 
 // Four stages take 140 KB of shared memory (one CTA per SM), three 109 KB (two per SM), two 74 KB (three per SM).  A launch that
 // gives every SM at most one CTA runs four stages, one that gives it at most two runs three, larger ones keep two: the bytes in
@@ -813,7 +813,7 @@ int attn_decode_mma_rope_launch(const AttnDecodeArgs& a, const AttnRopeArgs& r, 
     return hd == 128 ? launch_d<128>(a, r, nb, pdl, st) : launch_d<64>(a, r, nb, pdl, st);
 }
 
-// Pipeline depth of the tensor-core decode kernel: 0 = chosen per launch (default), 2, 3 or 4 = forced.  Returns the previous setting.
+// Pipeline depth of the tensor-core decode kernel on f16 caches: 0 = chosen per launch (default), 2, 3 or 4 = forced.  Returns the previous setting.
 B2_API int b2_attn_decode_stages(int n) {
     const int old = g_stages;
     if (n == 0 || (n >= 2 && n <= 4)) g_stages = n;

@@ -254,7 +254,8 @@ struct SgBars {
 
 // The CTAs that hold blocks of a group: `n` from `first` on.  Of the first `ends` of them it is the last group, and the first `finish` of these finish it together, a share of its values
 // each; the others (one that goes on with the next group, and those of a group in very many parts) only hand their sums over.  Finishers wait for CTAs before and behind them: there are
-// eight at most, so that CTAs which wait for others that are not resident yet cannot fill the GPU, however many streams launch at once.
+// eight at most, so that of a launch whose last CTAs are not resident yet up to seven hold an SM meanwhile.  21 launches in as many streams leave an SM free for those that are awaited;
+// with more the waits may run out.
 struct Parts {
     int first, n, ends, finish;
 };
