@@ -368,7 +368,7 @@ def test_attn_decode_tensor_core_long_context(hd, H, Hkv, q8, attn_mode):
         ref, _ = K.attn_decode(q, kc, vc, pos, slots, scale=scale, n_splits=n_splits, k_scale=ks, v_scale=vs)
         attn_mode(1)
         outs = []
-        for stages in (0,) if q8 else (2, 3, 4):      # f16 caches: the pipeline depths of the kernel compute the same sums in the same order
+        for stages in (2, 3, 4):               # the pipeline depths of the kernel compute the same sums in the same order
             K.attn_decode_stages(stages)
             try:
                 a, _ = K.attn_decode(q, kc, vc, pos, slots, scale=scale, n_splits=n_splits, k_scale=ks, v_scale=vs)
@@ -378,7 +378,7 @@ def test_attn_decode_tensor_core_long_context(hd, H, Hkv, q8, attn_mode):
             assert torch.equal(a, b)
             assert torch.allclose(a, ref, atol=3e-3, rtol=2e-2), (a - ref).abs().max()
             outs.append(a)
-        assert all(torch.equal(outs[0], o) for o in outs[1:])
+        assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
 
 
 @pytest.mark.parametrize("hd,H,Hkv,nb,n_splits,window", [(128, 32, 8, 24, 16, 0), (64, 64, 8, 17, 8, 0), (128, 16, 16, 32, 5, 0), (64, 16, 8, 32, 16, 130), (128, 32, 8, 9, 32, 0)])
