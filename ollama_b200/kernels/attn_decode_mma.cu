@@ -767,23 +767,28 @@ int launch_flat(const AttnDecodeArgs& a, const AttnRopeArgs& r, int nb, int pdl,
     return start(fn, smem, a, r, nb, room, pdl, st);
 }
 
-int g_stages = 0;      // f16 caches, 0: by the size of the launch; 2, 3 or 4: forced (tests).  int8 caches always have three stages (74 KB at 128 columns: three CTAs an SM)
+int g_stages = 0;      // 0: by the size of the launch; 2, 3 or 4: forced (tests)
 
 // Four stages take 140 KB of shared memory (one CTA per SM), three 109 KB (two per SM), two 74 KB (three per SM).  A launch that
 // gives every SM at most one CTA runs four stages, one that gives it at most two runs three, larger ones keep two: the bytes in
 // flight per SM stay about the same and no launch needs a second round because of its shared memory.
+// int8 caches take 91 KB in four stages and 74 KB, three CTAs per SM, in three, their least.  Steps of at most one CTA per SM in three and in four stages: Llama-8B, one sequence, 4 layers of
+// Q8_0 433 and 412 us at 400 positions, 455 and 430 at 4000, 12 layers of Q4_K_M 666 and 660, 733 and 715 (at 60 663 and 666); 20 layers of 16 heads on 4, two sequences about 4000 1241
+// and 1171.
 int stages_for(const AttnDecodeArgs& a, int nb) {
-    if (g_stages) return g_stages;
-    const long ctas = (long)a.n_splits * a.n_kv_heads * nb;
-    if (a.n_ctx / a.n_splits < 2 * BN) return 2;
-    return ctas <= sm_count() ? 4 : (ctas <= 2L * sm_count() ? 3 : 2);
+    int ns = g_stages;
+    if (!ns) {
+        const long ctas = (long)a.n_splits * a.n_kv_heads * nb;
+        ns = a.n_ctx / a.n_splits < 2 * BN ? 2 : ctas <= sm_count() ? 4 : ctas <= 2L * sm_count() ? 3 : 2;
+    }
+    return a.k_scale && ns < 3 ? 3 : ns;
 }
 
 template <int D>
 int launch_d(const AttnDecodeArgs& a, const AttnRopeArgs& r, int nb, int pdl, cudaStream_t st) {
     const int ns = stages_for(a, nb);
     if (a.page_table) return ns == 4 ? launch_paged<D, 4>(a, r, nb, pdl, st) : ns == 3 ? launch_paged<D, 3>(a, r, nb, pdl, st) : launch_paged<D, 2>(a, r, nb, pdl, st);
-    if (a.k_scale) return launch_flat<D, 3, true>(a, r, nb, pdl, st);
+    if (a.k_scale) return ns == 4 ? launch_flat<D, 4, true>(a, r, nb, pdl, st) : launch_flat<D, 3, true>(a, r, nb, pdl, st);
     return ns == 4 ? launch_flat<D, 4>(a, r, nb, pdl, st) : ns == 3 ? launch_flat<D, 3>(a, r, nb, pdl, st) : launch_flat<D, 2>(a, r, nb, pdl, st);
 }
 
@@ -813,12 +818,15 @@ int attn_decode_mma_rope_launch(const AttnDecodeArgs& a, const AttnRopeArgs& r, 
     return hd == 128 ? launch_d<128>(a, r, nb, pdl, st) : launch_d<64>(a, r, nb, pdl, st);
 }
 
-// Pipeline depth of the tensor-core decode kernel on f16 caches: 0 = chosen per launch (default), 2, 3 or 4 = forced.  Returns the previous setting.
+// Pipeline depth of the tensor-core decode kernel: 0 = chosen per launch (default), 2, 3 or 4 = forced (int8 caches: three at least).  Returns the previous setting.
 B2_API int b2_attn_decode_stages(int n) {
     const int old = g_stages;
     if (n == 0 || (n >= 2 && n <= 4)) g_stages = n;
     return old;
 }
+
+// The depth of a launch for nb sequences.
+B2_API int b2_attn_decode_depth(const AttnDecodeArgs* a, int nb) { return stages_for(*a, nb); }
 
 int attn_decode_mma_launch(const AttnDecodeArgs& a, int nb, int hd, int pdl, cudaStream_t st) {
     const AttnRopeArgs none = {};

@@ -23,6 +23,23 @@ def test_int8_caches_whose_scales_are_not_aligned_go_to_the_scalar_decode_kernel
     assert takes(0, 0, heads=7) == 0 and takes(0, 0, heads=64) == 0
 
 
+def test_depth_of_decode_attention_by_the_ctas_an_sm_gets():
+    """148 SMs, 8 KV heads, 16 splits: four stages up to one CTA an SM, int8 caches too; three up to two; else as few as there are."""
+    def depth(nb, q8, n_splits=16, n_ctx=8192):
+        at = 1 << 20
+        return K.lib().b2_attn_decode_depth(C.byref(K.AttnDecodeArgs(at, at, at, at, at, 32, 8, n_ctx, n_splits, 1.0, 0.0, 0, at, at, *([at, at] if q8 else [None, None]))), nb)
+
+    assert [depth(nb, False) for nb in (1, 2, 3, 8)] == [4, 3, 2, 2]
+    assert [depth(nb, True) for nb in (1, 2, 3, 8)] == [4, 3, 3, 3]
+    assert depth(1, False, n_splits=4, n_ctx=500) == 2 and depth(1, True, n_splits=4, n_ctx=500) == 3
+    for forced in (2, 3, 4):
+        K.attn_decode_stages(forced)
+        try:
+            assert [depth(nb, False) for nb in (1, 8)] == [forced] * 2 and [depth(nb, True) for nb in (1, 8)] == [max(3, forced)] * 2
+        finally:
+            K.attn_decode_stages(0)
+
+
 def test_expert_rows_are_not_laid_out_for_chunks_that_no_kernel_takes():
     for chunk in (0, 4, 12, 40, 56, 128):
         with pytest.raises(ValueError):
