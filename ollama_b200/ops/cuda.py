@@ -861,8 +861,8 @@ class MoeFp4:
     """The (token, expert) pairs of a step or a prompt times MXFP4 experts, each expert read once for all rows that chose it (kernels/moe_fp4.cu).
 
     Holds the sorted places of the pairs and the row buffers, so that a decode step can keep one for its CUDA graph; sizes that depend on the choice of
-    experts never visit the host.  ``chunk``: rows of an expert that a block multiplies at once, one of CHUNKS (32 is never the quickest,
-    see :func:`moe_fp4_chunk`)."""
+    experts never visit the host.  ``chunk``: rows of an expert that a block multiplies at once, one of CHUNKS (32, which
+    :func:`moe_fp4_chunk` leaves out, is the quickest only for 20 rows of few experts: of 32, 178 us against 186 in chunks of 24 and 183 of 48)."""
 
     CHUNKS = (8, 16, 24, 32, 48, 64)
 
