@@ -9,7 +9,7 @@
 // through shared memory at the end.  The scalar kernel stays the choice for short contexts and for head sizes without an instantiation here.
 // Two kernels: of flat caches every warp streams turns of 16 positions of its own (below); the paged one reads tiles of 64 positions, a page, that the four warps share (16 each), starts at the
 // query's chunk or window (keys that are kept in front of a window come first), and normalises q and k over their whole projections or heads before the rotation.
-// Both take two stages of shared memory, or three / four when the launch has so few CTAs that each SM holds two / one.
+// Both take two stages of shared memory (int8 caches three), or three / four when the launch has so few CTAs that each SM holds two / one.
 #include "attn_args.cuh"
 #include "rows.cuh"
 
